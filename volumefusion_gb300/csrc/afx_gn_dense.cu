@@ -19,8 +19,10 @@
 // order, so x agrees with the reference's to the conditioning of the system, not bit for bit.
 #include <cfloat>
 #include <cstring>
+#include <type_traits>
 
 #include "afx_gn.h"
+#include "afx_host.h"
 #include "afx_internal.h"
 
 namespace afx {
@@ -252,92 +254,439 @@ __global__ void fill_jtr_kernel(float* JTr, const int* coords, const float* elem
 }
 
 // ---- LU with partial pivoting (column-major, lda) ----
+//
+// Blocked right-looking elimination: a panel of NB columns is factorised by one CTA, then every other
+// column gets the panel's row swaps and, right of the panel, the panel's updates.  An element still
+// gets a[i][j] - l[i][k] u[k][j] for k = 0, 1, ... in that order, every product and difference
+// rounded by itself, so the factors, pivots and solution are those of the column-by-column
+// elimination bit for bit; only the passes over the matrix fall from one per column to one per NB.
+// Bound: the chain of n pivots (a search over the column, one CTA barrier, a division and a rank-1
+// update of registers each, about 1350 cycles).  At n = 822, ipiv and x read back: 8.9 ms with one
+// search and one update launch per column, 1.37 ms now (a panel 25 us for up to 512 rows and 38 us for up
+// to 1024, the update of the other columns 10 us, the triangular solves 0.27 ms).
 
+// Best pivot of a warp: the largest key (bits of |a| + 1; 0: no candidate) and, among equal ones, the
+// smallest position.
+AFX_D unsigned redux_max(unsigned v) { return __reduce_max_sync(0xffffffffu, v); }
+AFX_D unsigned redux_min(unsigned v) { return __reduce_min_sync(0xffffffffu, v); }
+
+constexpr int kLuMaxPanelThreads = 512;
+
+// Factorises columns k0 .. k0 + w - 1 (w = min(NB, n - k0)) of rows k0 .. n - 1, at most
+// R * blockDim.x rows.  A thread keeps R rows of the panel in registers for the whole panel; rows
+// are not moved: `pos` is the position a row has after the interchanges so far.  The register row
+// moves down by one per column -- the update writes element j to j - 1, so element 0 is always the
+// current column and the loop body does not depend on it -- and the multipliers go to shared memory.
+// From the middle of the panel on only the lower half of the registers still holds columns.
+// Every warp puts its best row in shared memory beside its key, so a column needs one CTA barrier:
+// after it every thread knows the pivot and reads the pivot row.  NB x R is 64 registers at most
+// (512 threads): 32 columns for up to 1024 rows, 16 up to 2048, 8 up to 4096.
+// Where no pivot is left (all zero or NaN) the column is recorded in *info and, as cuSOLVER's caller
+// treats the factorisation as failed, later columns are searched, swapped and divided but nothing is
+// updated any more.
+template <int NB, int R>
+__global__ void __launch_bounds__(kLuMaxPanelThreads) lu_panel_kernel(float* A, int n, int lda, int k0, int* ipiv,
+                                                                      int* info) {
+    constexpr int kWarps = kLuMaxPanelThreads / 32;
+    __shared__ alignas(16) float cand[2][kWarps][NB];  // each warp's best row, double-buffered over columns
+    __shared__ unsigned ckey[2][kWarps], cpos[2][kWarps];
+    __shared__ float prow[NB][NB + 1];                 // the chosen rows from their diagonal element on
+    extern __shared__ float mult[];                    // [NB][R * blockDim.x] multipliers of each row
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = blockDim.x >> 5;
+    const int m = n - k0, w = min(NB, m);
+    float a[R][NB];
+    unsigned pos[R];
+    bool live[R];  // a row of the matrix that is not a pivot yet
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int s = r * blockDim.x + t;
+        pos[r] = (unsigned)s;
+        live[r] = s < m;
+        const float* col = A + (long)k0 * lda + k0 + s;
+#pragma unroll
+        for (int j = 0; j < NB; ++j) a[r][j] = (live[r] && j < w) ? col[(long)j * lda] : 0.f;
+    }
+    bool failed = *info != 0;
+    const int rows = R * blockDim.x;
+    auto column = [&](int c, auto width) {  // width: registers of a row that still hold columns
+        constexpr int kW = decltype(width)::value;
+        const int par = c & 1;
+        unsigned key = 0, kp = 0xffffffffu;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const float v = fabsf(a[r][0]);
+            const unsigned kr = (live[r] && v == v) ? __float_as_uint(v) + 1u : 0u;
+            if (kr > key || (kr == key && kr != 0u && pos[r] < kp)) {
+                key = kr;
+                kp = pos[r];
+            }
+        }
+        const unsigned wk = redux_max(key);
+        const unsigned wp = redux_min(key == wk ? kp : 0xffffffffu);
+        if (wk != 0u && key == wk && kp == wp) {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (pos[r] == wp) {
+#pragma unroll
+                    for (int j = 0; j < kW; j += 4)
+                        *reinterpret_cast<float4*>(&cand[par][wid][j]) =
+                            make_float4(a[r][j], a[r][j + 1], a[r][j + 2], a[r][j + 3]);
+                }
+        }
+        if (lane == 0) {
+            ckey[par][wid] = wk;
+            cpos[par][wid] = wp;
+        }
+        __syncthreads();
+        const unsigned bk = lane < nw ? ckey[par][lane] : 0u;
+        const unsigned best = redux_max(bk);
+        const unsigned bp = (lane < nw && bk == best) ? cpos[par][lane] : 0xffffffffu;
+        const unsigned p = redux_min(bp);
+        const int win = __ffs(__ballot_sync(0xffffffffu, lane < nw && bk == best && bp == p)) - 1;
+        const float* u = cand[par][win];
+        const float piv = best != 0u ? u[0] : 0.f;
+        if (t == 0) ipiv[k0 + c] = best != 0u ? k0 + (int)p + 1 : n + 1;  // 1-based, as getrf
+        if (piv == 0.f) {                                                 // uniform across the block
+            if (t == 0 && !failed) *info = k0 + c + 1;
+            failed = true;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                mult[c * rows + r * blockDim.x + t] = a[r][0];
+#pragma unroll
+                for (int j = 1; j < kW; ++j) a[r][j - 1] = a[r][j];
+            }
+            return;
+        }
+        if (wid == win && lane < kW) prow[c][lane] = u[lane];
+        float l[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (pos[r] == p) {
+                live[r] = false;
+                pos[r] = (unsigned)c;
+            } else if (pos[r] == (unsigned)c) {
+                pos[r] = p;
+            }
+            l[r] = a[r][0] / piv;  // of a row already chosen: not used
+            if (live[r]) mult[c * rows + r * blockDim.x + t] = l[r];
+        }
+        if (failed) {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int j = 1; j < kW; ++j) a[r][j - 1] = a[r][j];
+        } else {
+#pragma unroll
+            for (int j0 = 0; j0 < kW; j0 += 4) {
+                const float4 v = *reinterpret_cast<const float4*>(u + j0);
+                const float uj[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int j = j0 > 0 ? j0 : 1; j < j0 + 4; ++j)
+#pragma unroll
+                    for (int r = 0; r < R; ++r) a[r][j - 1] = a[r][j] - l[r] * uj[j - j0];
+            }
+        }
+    };
+    const int half = min(w, NB / 2);
+    for (int c = 0; c < half; ++c) column(c, std::integral_constant<int, NB>());
+    for (int c = half; c < w; ++c) column(c, std::integral_constant<int, NB / 2>());
+    __syncthreads();
+    // the multipliers of each row at its position: all of them below the panel, those before its
+    // column for a pivot row, whose other elements are prow's
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int s = r * blockDim.x + t;
+        if (s >= m) continue;
+        const int q = live[r] ? w : (int)pos[r];
+        float* row = A + (long)k0 * lda + k0 + pos[r];
+        for (int j = 0; j < q; ++j) row[(long)j * lda] = mult[j * rows + s];
+        if (!live[r])
+            for (int j = q; j < w; ++j) row[(long)j * lda] = prow[q][j - q];
+    }
+}
+
+// The same panel (8 columns) for more rows than fit in registers: in place in global memory.
+constexpr int kLuBigNB = 8;
 constexpr int kLuThreads = 1024;
 
-// Column k: pivot search over rows k..n-1 (largest |a|, the first on ties), row swap, multipliers.
-__global__ void __launch_bounds__(kLuThreads) lu_pivot_kernel(float* A, int n, int lda, int k, int* ipiv, int* info) {
-    __shared__ float bv[kLuThreads];
-    __shared__ int bi[kLuThreads];
-    const int t = threadIdx.x;
-    float best = -1.f;
-    int arg = n;
-    for (int i = k + t; i < n; i += kLuThreads) {
-        const float v = fabsf(A[i + (long)k * lda]);
-        if (v > best) {
-            best = v;
-            arg = i;
-        }
-    }
-    bv[t] = best;
-    bi[t] = arg;
-    __syncthreads();
-    for (int s = kLuThreads / 2; s > 0; s >>= 1) {
-        if (t < s) {
-            const float v = bv[t + s];
-            const int i = bi[t + s];
-            if (v > bv[t] || (v == bv[t] && i < bi[t])) {
-                bv[t] = v;
-                bi[t] = i;
+__global__ void __launch_bounds__(kLuThreads) lu_panel_big_kernel(float* A, int n, int lda, int k0, int* ipiv,
+                                                                  int* info) {
+    __shared__ unsigned ckey[32], cpos[32];
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    const int w = min(kLuBigNB, n - k0);
+    bool failed = *info != 0;
+    for (int c = 0; c < w; ++c) {
+        float* col = A + (long)(k0 + c) * lda;
+        unsigned key = 0, kp = 0xffffffffu;
+        for (int i = k0 + c + t; i < n; i += kLuThreads) {
+            const float v = fabsf(col[i]);
+            const unsigned kr = v == v ? __float_as_uint(v) + 1u : 0u;
+            if (kr > key) {  // ascending i: the first of equal ones stays
+                key = kr;
+                kp = (unsigned)i;
             }
+        }
+        const unsigned wk = redux_max(key), wp = redux_min(key == wk ? kp : 0xffffffffu);
+        if (lane == 0) {
+            ckey[wid] = wk;
+            cpos[wid] = wp;
+        }
+        __syncthreads();
+        const unsigned best = redux_max(ckey[lane]);
+        const unsigned p = redux_min(ckey[lane] == best ? cpos[lane] : 0xffffffffu);
+        const float piv = best != 0u ? col[p] : 0.f;
+        if (t == 0) ipiv[k0 + c] = best != 0u ? (int)p + 1 : n + 1;
+        __syncthreads();  // every thread has read the pivot and the warps' keys
+        if (piv == 0.f) {
+            if (t == 0 && !failed) *info = k0 + c + 1;
+            failed = true;
+            continue;
+        }
+        if (t < w && (int)p != k0 + c) {
+            float* q = A + (long)(k0 + t) * lda;
+            const float x = q[k0 + c];
+            q[k0 + c] = q[p];
+            q[p] = x;
+        }
+        __syncthreads();
+        for (int i = k0 + c + 1 + t; i < n; i += kLuThreads) {
+            const float l = col[i] / piv;
+            col[i] = l;
+            if (!failed)
+                for (int j = c + 1; j < w; ++j) {
+                    float* q = A + (long)(k0 + j) * lda;
+                    q[i] = q[i] - l * q[k0 + c];
+                }
         }
         __syncthreads();
     }
-    const int p = bi[0];
-    const float piv = p < n ? A[p + (long)k * lda] : 0.f;
-    if (t == 0) ipiv[k] = p + 1;  // 1-based, as getrf
-    if (piv == 0.f) {             // uniform across the block
-        if (t == 0 && *info == 0) *info = k + 1;
-        return;
+}
+
+// Where position d's row stood before the panel's swaps (k0 + i <-> p[i], i = 0 .. w - 1).
+AFX_D int swap_source(int d, const int* p, int k0, int w) {
+#pragma unroll 8
+    for (int i = w - 1; i >= 0; --i) {
+        const int a = k0 + i, b = p[i];
+        d = d == a ? b : (d == b ? a : d);
     }
-    __syncthreads();  // every thread has read the pivot before the rows move
-    if (p != k)
-        for (int j = t; j < n; j += kLuThreads) {
-            const float x = A[k + (long)j * lda];
-            A[k + (long)j * lda] = A[p + (long)j * lda];
-            A[p + (long)j * lda] = x;
-        }
+    return d;
+}
+
+// The columns outside a panel, kLuTC of them per CTA over all rows (so a CTA can move rows in place):
+// the panel's row swaps and, for the columns right of it (the first tiles), U12 = L11^-1 A12 by one
+// warp per column and A22 - L21 U12 with one row per thread and pass.  The last row below the panel is
+// reached in ceil((n - k0 - w) / blockDim.x) passes.  NB: columns per panel.
+constexpr int kLuTC = 8;
+
+template <int NB>
+__global__ void __launch_bounds__(kLuThreads) lu_update_kernel(float* A, int n, int lda, int k0, const int* ipiv,
+                                                               const int* info, int right_tiles) {
+    __shared__ int p[NB], dst[2 * NB], src[2 * NB];
+    __shared__ float tmp[2 * NB][kLuTC];
+    __shared__ float L11[NB][NB];               // [column][row]
+    __shared__ alignas(16) float U[NB][kLuTC];
+    const int t = threadIdx.x, nt = blockDim.x;
+    const int w = min(NB, n - k0);
+    const bool right = (int)blockIdx.x < right_tiles;
+    const int c0 = right ? k0 + w + (int)blockIdx.x * kLuTC : ((int)blockIdx.x - right_tiles) * kLuTC;
+    const int nc = min(kLuTC, (right ? n : k0) - c0);
+    const int bad = *info;  // columns from bad - 1 on have no updates
+    const int nk = bad == 0 ? w : max(0, min(w, bad - 1 - k0));
+    if (t < w) p[t] = ipiv[k0 + t] <= n ? ipiv[k0 + t] - 1 : k0 + t;  // a column without a pivot swaps nothing
     __syncthreads();
-    for (int i = k + 1 + t; i < n; i += kLuThreads) A[i + (long)k * lda] = A[i + (long)k * lda] / piv;
-}
-
-// Trailing update A[i][j] -= l[i] u[j] for i, j > k.
-__global__ void lu_update_kernel(float* A, int n, int lda, int k, const int* info) {
-    if (*info) return;
-    const long m = n - k - 1;
-    AFX_GRID_STRIDE(t, m * m) {
-        const int i = k + 1 + (int)(t % m), j = k + 1 + (int)(t / m);
-        A[i + (long)j * lda] = A[i + (long)j * lda] - A[i + (long)k * lda] * A[k + (long)j * lda];
+    if (t < 2 * w) {
+        const int d = t < w ? k0 + t : p[t - w];
+        dst[t] = d;
+        src[t] = swap_source(d, p, k0, w);
+    }
+    if (right)
+        for (int e = t; e < w * w; e += nt) L11[e / w][e % w] = A[k0 + e % w + (long)(k0 + e / w) * lda];
+    __syncthreads();
+    for (int e = t; e < 2 * w * nc; e += nt) {
+        const int q = e % (2 * w), j = e / (2 * w);
+        tmp[q][j] = A[src[q] + (long)(c0 + j) * lda];
+    }
+    __syncthreads();
+    for (int e = t; e < 2 * w * nc; e += nt) {
+        const int q = e % (2 * w), j = e / (2 * w);
+        if (dst[q] != src[q]) A[dst[q] + (long)(c0 + j) * lda] = tmp[q][j];
+    }
+    if (!right) return;
+    for (int j = t >> 5; j < kLuTC; j += nt >> 5) {
+        const int lane = t & 31;
+        float u = (lane < w && j < nc) ? tmp[lane][j] : 0.f;
+        for (int k = 0; k < nk; ++k) {
+            const float uk = __shfl_sync(0xffffffffu, u, k);
+            if (lane > k && lane < w) u = u - L11[k][lane] * uk;
+        }
+        if (lane < NB) U[lane][j] = u;
+    }
+    __syncthreads();  // U, and the moved rows of this CTA's columns
+    for (int e = t; e < w * nc; e += nt) A[k0 + e % w + (long)(c0 + e / w) * lda] = U[e % w][e / w];
+    for (int i = k0 + w + t; i < n; i += nt) {
+        float acc[kLuTC];
+#pragma unroll
+        for (int j = 0; j < kLuTC; ++j) acc[j] = j < nc ? A[i + (long)(c0 + j) * lda] : 0.f;
+        const float* L = A + i + (long)k0 * lda;
+#pragma unroll 8
+        for (int k = 0; k < nk; ++k) {
+            const float l = L[(long)k * lda];
+            const float4 u0 = *reinterpret_cast<const float4*>(&U[k][0]), u1 = *reinterpret_cast<const float4*>(&U[k][4]);
+            acc[0] = acc[0] - l * u0.x;
+            acc[1] = acc[1] - l * u0.y;
+            acc[2] = acc[2] - l * u0.z;
+            acc[3] = acc[3] - l * u0.w;
+            acc[4] = acc[4] - l * u1.x;
+            acc[5] = acc[5] - l * u1.y;
+            acc[6] = acc[6] - l * u1.z;
+            acc[7] = acc[7] - l * u1.w;
+        }
+#pragma unroll
+        for (int j = 0; j < kLuTC; ++j)
+            if (j < nc) A[i + (long)(c0 + j) * lda] = acc[j];
     }
 }
 
-// getrs (no transpose): row interchanges, L y = P b (unit diagonal), U x = y; one block.
+// getrs (no transpose): row interchanges, L y = P b (unit diagonal), U x = y; one block.  Blocks of 32
+// unknowns: a warp solves the diagonal block by shuffles while the other rows' coefficients, which do
+// not depend on it, are already on their way to registers; then every row subtracts the block's 32
+// terms in the order of the column-by-column substitution.  The unknowns stay in shared memory while
+// they fit (kSolveSmem of them).
+constexpr int kSolveNB = 32;
+constexpr int kSolveSmem = 24576;
+
 __global__ void __launch_bounds__(kLuThreads) lu_solve_kernel(const float* A, int n, int lda, const int* ipiv,
-                                                              float* x, const int* info) {
+                                                              float* xg, const int* info, int in_smem) {
+    __shared__ float D[kSolveNB][kSolveNB];  // [column][row]
+    __shared__ float xb[kSolveNB];
+    __shared__ int p[2][kSolveNB];
+    extern __shared__ float xs[];
     if (*info) return;
-    const int t = threadIdx.x;
-    if (t == 0)
-        for (int k = 0; k < n; ++k) {
-            const int p = ipiv[k] - 1;
-            if (p != k) {
-                const float s = x[k];
-                x[k] = x[p];
-                x[p] = s;
-            }
-        }
+    float* x = in_smem ? xs : xg;
+    const int t = threadIdx.x, lane = t & 31, r = t & 31, c = t >> 5;  // 32 x 32 threads over a block
+    if (in_smem)
+        for (int i = t; i < n; i += kLuThreads) xs[i] = xg[i];
+    if (t < kSolveNB) p[0][t] = t < n ? ipiv[t] - 1 : 0;
     __syncthreads();
-    for (int k = 0; k < n; ++k) {  // forward: x[i] -= l[i][k] x[k], i > k
-        const float xk = x[k];
-        for (int i = k + 1 + t; i < n; i += kLuThreads) x[i] = x[i] - A[i + (long)k * lda] * xk;
+    for (int k0 = 0, b = 0; k0 < n; k0 += kSolveNB, b ^= 1) {
+        const int w = min(kSolveNB, n - k0), next = k0 + kSolveNB + t;
+        int d = 0;
+        float v = 0.f;
+        const int pn = (t < kSolveNB && next < n) ? ipiv[next] - 1 : 0;
+        if (t < 2 * w) {
+            d = t < w ? k0 + t : p[b][t - w];
+            v = x[swap_source(d, p[b], k0, w)];
+        }
+        __syncthreads();
+        if (t < 2 * w) x[d] = v;
+        if (t < kSolveNB) p[b ^ 1][t] = pn;
         __syncthreads();
     }
-    for (int k = n - 1; k >= 0; --k) {  // backward
-        if (t == 0) x[k] = x[k] / A[k + (long)k * lda];
+    // (the element of the next diagonal block that this thread stages is loaded a block ahead)
+    float dn = r < n && c < n ? A[r + (long)c * lda] : 0.f;
+    for (int k0 = 0; k0 < n; k0 += kSolveNB) {  // forward: x[i] -= l[i][k] x[k], i > k
+        const int w = min(kSolveNB, n - k0), k1 = k0 + kSolveNB;
+        const float* P = A + (long)k0 * lda;  // the block's columns
+        D[c][r] = dn;
+        const int i0 = k0 + w + t;
+        float l[kSolveNB];
+#pragma unroll
+        for (int k = 0; k < kSolveNB; ++k) l[k] = (i0 < n && k < w) ? P[i0 + (long)k * lda] : 0.f;
+        dn = (k1 + r < n && k1 + c < n) ? A[k1 + r + (long)(k1 + c) * lda] : 0.f;
         __syncthreads();
-        const float xk = x[k];
-        for (int i = t; i < k; i += kLuThreads) x[i] = x[i] - A[i + (long)k * lda] * xk;
+        if (t < 32) {
+            float v = lane < w ? x[k0 + lane] : 0.f;
+#pragma unroll 8
+            for (int k = 0; k < w; ++k) {
+                const float xk = __shfl_sync(0xffffffffu, v, k), d = D[k][lane];
+                if (lane > k && lane < w) v = v - d * xk;
+            }
+            if (lane < w) x[k0 + lane] = v;
+            xb[lane] = v;
+        }
+        __syncthreads();
+        if (i0 < n) {
+            float v = x[i0];
+#pragma unroll
+            for (int k = 0; k < kSolveNB; ++k)
+                if (k < w) v = v - l[k] * xb[k];
+            x[i0] = v;
+        }
+        for (int i = i0 + kLuThreads; i < n; i += kLuThreads) {
+            float v = x[i];
+#pragma unroll 8
+            for (int k = 0; k < w; ++k) v = v - P[i + (long)k * lda] * xb[k];
+            x[i] = v;
+        }
         __syncthreads();
     }
+    const int last = (n - 1) / kSolveNB * kSolveNB;
+    dn = (last + r < n && last + c < n) ? A[last + r + (long)(last + c) * lda] : 0.f;
+    for (int k0 = last; k0 >= 0; k0 -= kSolveNB) {  // backward
+        const int w = min(kSolveNB, n - k0), k1 = k0 - kSolveNB;
+        const float* P = A + (long)k0 * lda;
+        D[c][r] = dn;
+        float u[kSolveNB];
+#pragma unroll
+        for (int k = 0; k < kSolveNB; ++k) u[k] = (t < k0 && k < w) ? P[t + (long)k * lda] : 0.f;
+        dn = k1 >= 0 ? A[k1 + r + (long)(k1 + c) * lda] : 0.f;
+        __syncthreads();
+        if (t < 32) {
+            float v = lane < w ? x[k0 + lane] : 0.f;
+#pragma unroll 4
+            for (int k = w - 1; k >= 0; --k) {
+                const float d = D[k][lane], xk = __shfl_sync(0xffffffffu, v / d, k);  // lane k: v / u[k][k]
+                if (lane == k) v = xk;
+                if (lane < k) v = v - d * xk;
+            }
+            if (lane < w) x[k0 + lane] = v;
+            xb[lane] = v;
+        }
+        __syncthreads();
+        if (t < k0) {
+            float v = x[t];
+#pragma unroll
+            for (int k = kSolveNB - 1; k >= 0; --k)
+                if (k < w) v = v - u[k] * xb[k];
+            x[t] = v;
+        }
+        for (int i = t + kLuThreads; i < k0; i += kLuThreads) {
+            float v = x[i];
+#pragma unroll 8
+            for (int k = w - 1; k >= 0; --k) v = v - P[i + (long)k * lda] * xb[k];
+            x[i] = v;
+        }
+        __syncthreads();
+    }
+    if (in_smem)
+        for (int i = t; i < n; i += kLuThreads) xg[i] = xs[i];
+}
+
+// One panel of NB columns, R rows per thread, and the update of the other columns.
+template <int NB, int R>
+int lu_step(float* A, int n, int lda, int k0, int* ipiv, int* info, cudaStream_t st) {
+    const int m = n - k0, w = m < NB ? m : NB;
+    if (m > R * kLuMaxPanelThreads) {
+        lu_panel_big_kernel<<<1, kLuThreads, 0, st>>>(A, n, lda, k0, ipiv, info);
+    } else {
+        static ContextOnce once;  // the shared-memory opt-in: NB multipliers for every row
+        const int rc = once_per_context(once, [](int) {
+            return note_cuda_error(cudaFuncSetAttribute(lu_panel_kernel<NB, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                        kLuMaxPanelThreads * R * NB * (int)sizeof(float)));
+        });
+        if (rc) return rc;
+        const int threads = ((m + R - 1) / R + 31) / 32 * 32;
+        lu_panel_kernel<NB, R><<<1, threads, threads * R * NB * sizeof(float), st>>>(A, n, lda, k0, ipiv, info);
+    }
+    AFX_LAUNCH_CHECK();
+    const int right = (m - w + kLuTC - 1) / kLuTC, left = (k0 + kLuTC - 1) / kLuTC;
+    if (right + left > 0) {
+        int threads = (m - w + 31) / 32 * 32;
+        threads = threads < 256 ? 256 : threads > kLuThreads ? kLuThreads : threads;
+        lu_update_kernel<NB><<<right + left, threads, 0, st>>>(A, n, lda, k0, ipiv, info, right);
+        AFX_LAUNCH_CHECK();
+    }
+    return AFX_OK;
 }
 
 }  // namespace
@@ -517,17 +866,25 @@ int afx_lu_solve(float* x, const float* A, int n, int lda, const float* b, int* 
     int* info = reinterpret_cast<int*>(static_cast<char*>(workspace) + (((size_t)lda * n * 4 + 255) / 256) * 256);
     AFX_CUDA(cudaMemcpyAsync(LU, A, (size_t)lda * n * 4, cudaMemcpyDeviceToDevice, st));
     AFX_CUDA(cudaMemsetAsync(info, 0, 4, st));
-    for (int k = 0; k < n; ++k) {
-        lu_pivot_kernel<<<1, kLuThreads, 0, st>>>(LU, n, lda, k, ipiv, info);
-        AFX_LAUNCH_CHECK();
-        if (k + 1 < n) {
-            const long m = n - k - 1;
-            lu_update_kernel<<<grid_for(m * m, 256), 256, 0, st>>>(LU, n, lda, k, info);
-            AFX_LAUNCH_CHECK();
-        }
+    for (int k0 = 0; k0 < n;) {
+        // as many columns per panel as the registers of one CTA hold for the rows that are left
+        const int m = n - k0, T = kLuMaxPanelThreads, nb = m <= 2 * T ? 32 : m <= 4 * T ? 16 : kLuBigNB;
+        const int rc = m <= T       ? lu_step<32, 1>(LU, n, lda, k0, ipiv, info, st)
+                       : m <= 2 * T ? lu_step<32, 2>(LU, n, lda, k0, ipiv, info, st)
+                       : m <= 4 * T ? lu_step<16, 4>(LU, n, lda, k0, ipiv, info, st)
+                                    : lu_step<kLuBigNB, 8>(LU, n, lda, k0, ipiv, info, st);
+        if (rc) return rc;
+        k0 += nb;
     }
     AFX_CUDA(cudaMemcpyAsync(x, b, (size_t)n * 4, cudaMemcpyDeviceToDevice, st));
-    lu_solve_kernel<<<1, kLuThreads, 0, st>>>(LU, n, lda, ipiv, x, info);
+    static ContextOnce once;
+    const int rc = once_per_context(once, [](int) {
+        return note_cuda_error(cudaFuncSetAttribute(lu_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                    kSolveSmem * (int)sizeof(float)));
+    });
+    if (rc) return rc;
+    const bool in_smem = n <= kSolveSmem;
+    lu_solve_kernel<<<1, kLuThreads, in_smem ? n * sizeof(float) : 0, st>>>(LU, n, lda, ipiv, x, info, in_smem);
     AFX_LAUNCH_CHECK();
     int h_info = 0;
     AFX_CUDA(cudaMemcpyAsync(&h_info, info, 4, cudaMemcpyDeviceToHost, st));
