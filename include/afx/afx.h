@@ -486,7 +486,7 @@ int afx_fusion_graph_count(const afx_fusion* f);
 
 /* Marching-cubes tile of the session (no counterpart in the reference): AFX_MC_TILE_TMA16 (default:
  * a CTA's brick of 32x8x16 cubes brought into shared memory by TMA), AFX_MC_TILE_TMA8,
- * AFX_MC_TILE_TMA32 (8 or 32 cubes along z), AFX_MC_TILE_COLUMN (column march from global memory),
+ * AFX_MC_TILE_TMA32 (8 or 32 cubes along z), AFX_MC_TILE_COLUMN (sweep from global memory),
  * AFX_MC_TILE_PIPE8 / AFX_MC_TILE_PIPE16 / AFX_MC_TILE_PIPE4 (a persistent grid whose CTAs keep two
  * bricks of 8, 16 or 4 cubes in flight).  Results are the same with every tile (point and triangle sets; triangle order
  * may differ).  afx_fusion_autotune times each tile on the session's current volume (call it after

@@ -1,7 +1,7 @@
 // afx_mc.cu -- marching cubes (point-cloud and triangle variants, fused into one pass over
 // the volume) with warp-aggregated stream compaction, and the lexicographic sort +
-// unique of the canonical point cloud (a merge sort: bitonic 2048-element tiles in
-// shared memory, then merge-path passes).
+// unique of the canonical point cloud (a merge sort: 2048-element tiles in shared memory,
+// then merge-path passes).
 //
 // Case index, edge interpolation and triangulation follow src/MarchingCubes.cu:294-420
 // (corner bit c set when tsdf > iso, cubes skipped when any corner weight is 0, cubes
@@ -18,31 +18,16 @@
 namespace afx {
 
 __constant__ uint64_t c_tri_table[256];
-__constant__ unsigned short c_edge_table[256];
 
 static const uint64_t kTriTableHost[256] = {
 #include "mc_tables.inc"
 };
 
-// Corner c of cube (x,y,z) is at (x,y,z) + kCorner[c]; edge e joins corners kEdge[e][0] -> kEdge[e][1]
-// (src/MarchingCubes.cu:338-379 and the getVertex calls at :441-507).
-__constant__ int c_corner[8][3] = {{1, 1, 0}, {1, 0, 0}, {0, 0, 0}, {0, 1, 0}, {1, 1, 1}, {1, 0, 1}, {0, 0, 1}, {0, 1, 1}};
-__constant__ int c_edge[12][2] = {{0, 1}, {1, 2}, {2, 3}, {3, 0}, {4, 5}, {5, 6}, {6, 7}, {7, 4}, {0, 4}, {1, 5}, {2, 6}, {3, 7}};
-static const int kEdgeHost[12][2] = {{0, 1}, {1, 2}, {2, 3}, {3, 0}, {4, 5}, {5, 6}, {6, 7}, {7, 4}, {0, 4}, {1, 5}, {2, 6}, {3, 7}};
-
-// The tables are constant: uploaded once per device context (before the first marching-cubes launch,
+// The triangle table is constant: uploaded once per device context (before the first marching-cubes launch,
 // which is never inside a stream capture: a session's first frame runs eagerly).
 static int upload_tables() {
     static ContextOnce once;
     return once_per_context(once, [](int) {
-        unsigned short et[256];
-        for (int c = 0; c < 256; ++c) {
-            int e = 0;
-            for (int i = 0; i < 12; ++i)
-                if (((c >> kEdgeHost[i][0]) & 1) != ((c >> kEdgeHost[i][1]) & 1)) e |= 1 << i;
-            et[c] = (unsigned short)e;
-        }
-        AFX_CUDA(cudaMemcpyToSymbol(c_edge_table, et, sizeof(et)));
         AFX_CUDA(cudaMemcpyToSymbol(c_tri_table, kTriTableHost, sizeof(kTriTableHost)));
         return (int)AFX_OK;
     });
@@ -67,131 +52,194 @@ struct McArgs {
 };
 
 
-// getVertex + interpolate (src/MarchingCubes.cu:294-336)
+// Corners of edge e: corner offsets (x, y, z) of its two ends, one bit each, 6 bits per edge
+// (src/MarchingCubes.cu:338-379; the corner and edge numbers of the tables below), in two registers:
+// lanes look up different edges, which constant memory would serve one after the other.
+constexpr unsigned corner_bits(int c) {  // c0 (1,1,0) c1 (1,0,0) c2 (0,0,0) c3 (0,1,0), c4..c7 one slice up
+    return (unsigned)((c & 3) == 0 || (c & 3) == 1) | (unsigned)((c & 3) == 0 || (c & 3) == 3) << 1 | (unsigned)(c >= 4) << 2;
+}
+constexpr int kEdge[12][2] = {{0, 1}, {1, 2}, {2, 3}, {3, 0}, {4, 5}, {5, 6}, {6, 7}, {7, 4}, {0, 4}, {1, 5}, {2, 6}, {3, 7}};
+constexpr uint64_t edge_ends(int from) {  // of edges from .. from + 5
+    uint64_t v = 0;
+    for (int e = 0; e < 6; ++e)
+        v |= (uint64_t)(corner_bits(kEdge[from + e][0]) | corner_bits(kEdge[from + e][1]) << 3) << (6 * e);
+    return v;
+}
+
+// Edges that a cube of case ci crosses: those whose ends lie on different sides.
+AFX_D unsigned crossed_edges(unsigned ci) {
+    const unsigned lo = ci & 15u, hi = ci >> 4;
+    const unsigned a = lo ^ (((lo >> 1) | (lo << 3)) & 15u), b = hi ^ (((hi >> 1) | (hi << 3)) & 15u);
+    return a | (b << 4) | ((lo ^ hi) << 8);
+}
+
+// (float)((double)a + (double)m * (double)d) for 0 <= m <= 1, from binary32 operations: binary64 issues at
+// about 1/80 of their rate here.  m d is p + e exactly, a + p is s + f exactly (Knuth's TwoSum), and
+// t = f + e has a relative error of at most 2^-24.  So the exact value, and its rounding to binary64,
+// lie between s + t (1 - 2^-20) and s + t (1 + 2^-20); where both round to the same binary32 number,
+// which is all but about one in 2^18 times, that is the result.  Otherwise, and where e could
+// underflow, the binary64 sum is taken.
+AFX_D float blend64(float a, float m, float d) {
+    const float p = m * d, e = fmaf(m, d, -p);
+    const float s = a + p, v = s - a, f = (a - (s - v)) + (p - v);
+    const float t = f + e;
+    const float lo = s + t * (1.0f - 9.5367431640625e-7f), hi = s + t * (1.0f + 9.5367431640625e-7f);
+    if (lo == hi && (fabsf(p) > 1e-25f || p == 0.0f)) return lo;
+    return (float)__dadd_rn((double)a, __dmul_rn((double)m, (double)d));
+}
+
+// getVertex + interpolate (src/MarchingCubes.cu:294-336) of edge e of cube (x, y, z).  The ends differ in one
+// coordinate only; in the others p0 + mu (p1 - p0) is p0 + mu 0 = p0 + 0 for a finite mu.
 template <class TT>
 AFX_D void edge_vertex(const TT* __restrict__ tsdf, const Volume& vol, int x, int y, int z, int e, float iso,
                        float* o) {
-    const int* ca = c_corner[c_edge[e][0]];
-    const int* cb = c_corner[c_edge[e][1]];
+    constexpr uint64_t kLow = edge_ends(0), kHigh = edge_ends(6);
+    const unsigned ends = (unsigned)((e < 6 ? kLow >> (6 * e) : kHigh >> (6 * (e - 6))) & 63u);
     const int X = vol.dims[0], Y = vol.dims[1];
-    int x1 = x + ca[0], y1 = y + ca[1], z1 = z + ca[2];
-    int x2 = x + cb[0], y2 = y + cb[1], z2 = z + cb[2];
-    float t0 = vox_ld_t(tsdf, ((long)z1 * Y + y1) * X + x1);
-    float t1 = vox_ld_t(tsdf, ((long)z2 * Y + y2) * X + x2);
+    const int x1 = x + (ends & 1), y1 = y + ((ends >> 1) & 1), z1 = z + ((ends >> 2) & 1);
+    const int x2 = x + ((ends >> 3) & 1), y2 = y + ((ends >> 4) & 1), z2 = z + (ends >> 5);
+    const float t0 = vox_ld_t(tsdf, ((long)z1 * Y + y1) * X + x1);
+    const float t1 = vox_ld_t(tsdf, ((long)z2 * Y + y2) * X + x2);
     float p0[3], p1[3];
     voxel_to_world(x1, y1, z1, vol.vs, vol.half, p0);
     voxel_to_world(x2, y2, z2, vol.vs, vol.half, p1);
+    o[0] = p0[0];
+    o[1] = p0[1];
+    o[2] = p0[2];
     // (double)v < 1e-7 is v < 1e-7f for every float v: 1e-7f is the smallest float >= 1e-7
-    if (fabsf(iso - t0) < 1e-7f) {
-        o[0] = p0[0]; o[1] = p0[1]; o[2] = p0[2];
-        return;
-    }
+    if (fabsf(iso - t0) < 1e-7f) return;
     if (fabsf(iso - t1) < 1e-7f) {
-        o[0] = p1[0]; o[1] = p1[1]; o[2] = p1[2];
+        o[0] = p1[0];
+        o[1] = p1[1];
+        o[2] = p1[2];
         return;
     }
-    if (fabsf(t0 - t1) < 1e-7f) {
-        o[0] = p0[0]; o[1] = p0[1]; o[2] = p0[2];
-        return;
-    }
-    double mu = (double)((iso - t0) / (t1 - t0));
-    if (mu > 1.0) mu = 1.0;
-    else if (mu < 0) mu = 0.0;
+    if (fabsf(t0 - t1) < 1e-7f) return;
+    float mu = (iso - t0) / (t1 - t0);
+    if (mu > 1.0f) mu = 1.0f;
+    else if (mu < 0.0f) mu = 0.0f;
+    const int axis = (ends ^ (ends >> 3)) & 1 ? 0 : ((ends ^ (ends >> 3)) & 2 ? 1 : 2);
+    const float a = axis == 0 ? p0[0] : axis == 1 ? p0[1] : p0[2], b = axis == 0 ? p1[0] : axis == 1 ? p1[1] : p1[2];
+    const float v = blend64(a, mu, b - a);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) o[c] = (float)__dadd_rn((double)p0[c], __dmul_rn(mu, (double)(p1[c] - p0[c])));
+    for (int c = 0; c < 3; ++c) o[c] = c == axis ? v : (mu == mu ? p0[c] + 0.0f : v);  // not a number: in all three
 }
 
 AFX_D bool vne(const float* a, const float* b) { return a[0] != b[0] || a[1] != b[1] || a[2] != b[2]; }
 
-// Warp-aggregated append: returns this lane's base index for `n` items.
-AFX_D unsigned warp_append(unsigned* counter, unsigned n) {
+// Vertices and triangles of up to 32 cubes, one per lane, by the whole warp: the point-cloud vertices
+// (marchingCubesMeshKernel) and/or the triangles (marchingCubesFullKernel).  The crossed edges of all
+// the cubes are laid out one after the other and interpolated one per lane, so lanes have the same work
+// whatever their cubes' cases are, and points and triangles are written in consecutive words.
+struct McEdges {                    // of one warp
+    int cube[32][3];
+    unsigned short edge[32 * 12];   // cube << 4 | edge
+};
+template <bool kMesh>
+struct McScratch : McEdges {
+    float vert[32 * 12][3];         // vertices in edge order
+    unsigned tri[32 * 5];           // triangles: three indices into vert, 9 bits each
+};
+template <>
+struct McScratch<false> : McEdges {};
+
+template <bool kPoints, bool kMesh, class TT>
+AFX_D void mc_emit(const TT* __restrict__ tsdf, const McArgs& a, int x, int y, int z, int ci, bool active,
+                   McScratch<kMesh>& S) {
     const int lane = threadIdx.x & 31;
-    unsigned x = n;
+    const unsigned et = active ? crossed_edges((unsigned)ci) : 0u;
+    const unsigned ne = __popc(et);
+    unsigned incl = ne;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        unsigned y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
+        const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
     }
-    unsigned total = __shfl_sync(0xffffffffu, x, 31);
+    const unsigned total = __shfl_sync(0xffffffffu, incl, 31), first = incl - ne;
     unsigned base = 0;
-    if (lane == 31 && total) base = atomicAdd(counter, total);
-    base = __shfl_sync(0xffffffffu, base, 31);
-    return base + x - n;
-}
-
-// Vertices and triangles of one cube (all lanes of the warp call this together: the appends are
-// warp-aggregated).  Emits the point-cloud vertices (marchingCubesMeshKernel) and/or the
-// triangles (marchingCubesFullKernel).
-template <bool kPoints, bool kMesh, class TT>
-AFX_D void mc_emit(const TT* __restrict__ tsdf, const McArgs& a, int x, int y, int z, int ci, bool active) {
-    const unsigned et = active ? c_edge_table[ci] : 0u;
-    float ep[12][3];
-    if (active) {
-#pragma unroll
-        for (int e = 0; e < 12; ++e)
-            if (et & (1u << e)) edge_vertex(tsdf, a.vol, x, y, z, e, a.iso, ep[e]);
+    if (kPoints && lane == 0 && total) base = atomicAdd(a.point_count, total);
+    S.cube[lane][0] = x;
+    S.cube[lane][1] = y;
+    S.cube[lane][2] = z;
+    {
+        unsigned k = first;
+        for (unsigned rest = et; rest; rest &= rest - 1) S.edge[k++] = (unsigned short)(lane << 4 | (__ffs(rest) - 1));
     }
-    if (kPoints) {
-        unsigned n = __popc(et);
-        unsigned pos = warp_append(a.point_count, n);
-        if (active)
-            for (int e = 0; e < 12; ++e)
-                if (et & (1u << e)) {
-                    if (pos < a.point_cap) {
-                        float* o = a.points + 3 * (long)pos;
-                        o[0] = ep[e][0]; o[1] = ep[e][1]; o[2] = ep[e][2];
-                    }
-                    ++pos;
-                }
-    }
-    if (kMesh) {
-        uint64_t tri = active ? c_tri_table[ci] : 0xFull;
-        unsigned nt = 0;
-        for (int s = 0; s < 15; s += 3) {
-            int e0 = (int)((tri >> (4 * s)) & 0xF);
-            if (e0 == 0xF) break;
-            int e1 = (int)((tri >> (4 * (s + 1))) & 0xF), e2 = (int)((tri >> (4 * (s + 2))) & 0xF);
-            if (vne(ep[e0], ep[e1]) && vne(ep[e0], ep[e2]) && vne(ep[e1], ep[e2])) ++nt;
+    if (kPoints) base = __shfl_sync(0xffffffffu, base, 0);
+    __syncwarp();
+    for (unsigned i = lane; i < total; i += 32) {
+        const unsigned item = S.edge[i];
+        const int* c = S.cube[item >> 4];
+        float v[3];
+        edge_vertex(tsdf, a.vol, c[0], c[1], c[2], (int)(item & 15u), a.iso, v);
+        if (kPoints && (long)base + i < a.point_cap) {
+            float* o = a.points + 3 * ((long)base + i);
+            o[0] = v[0];
+            o[1] = v[1];
+            o[2] = v[2];
         }
-        unsigned f = warp_append(a.face_count, nt);
-        for (int s = 0; s < 15; s += 3) {
-            int e0 = (int)((tri >> (4 * s)) & 0xF);
-            if (e0 == 0xF) break;
-            int e1 = (int)((tri >> (4 * (s + 1))) & 0xF), e2 = (int)((tri >> (4 * (s + 2))) & 0xF);
-            if (!(vne(ep[e0], ep[e1]) && vne(ep[e0], ep[e2]) && vne(ep[e1], ep[e2]))) continue;
-            if (f < a.face_cap) {
-                float* o = a.verts + 9 * (long)f;
-                const int es[3] = {e0, e1, e2};
+        if constexpr (kMesh) {
+            S.vert[i][0] = v[0];
+            S.vert[i][1] = v[1];
+            S.vert[i][2] = v[2];
+        }
+    }
+    __syncwarp();
+    if constexpr (kMesh) {
+        const uint64_t table = active ? c_tri_table[ci] : 0xFull;
+        unsigned tri[5], nt = 0;  // the cube's triangles without two equal corners
 #pragma unroll
-                for (int t = 0; t < 3; ++t) {
-                    o[3 * t] = ep[es[t]][0];
-                    o[3 * t + 1] = ep[es[t]][1];
-                    o[3 * t + 2] = ep[es[t]][2];
-                }
-                int* fo = a.faces + 3 * (long)f;
-                fo[0] = (int)(3 * f);
-                fo[1] = (int)(3 * f + 1);
-                fo[2] = (int)(3 * f + 2);
+        for (int k = 0; k < 5; ++k) {
+            const unsigned e = (unsigned)(table >> (12 * k)) & 0xFFFu;  // three edges
+            tri[k] = 0xffffffffu;
+            // the table ends a case's list with 0xF; everything after it is not read
+            bool on = true;
+#pragma unroll
+            for (int q = 0; q <= k; ++q) on = on && ((unsigned)(table >> (12 * q)) & 0xFu) != 0xFu;
+            if (!on) continue;
+            unsigned v[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) v[q] = first + __popc(et & ((1u << ((e >> (4 * q)) & 0xFu)) - 1u));
+            if (vne(S.vert[v[0]], S.vert[v[1]]) && vne(S.vert[v[0]], S.vert[v[2]]) && vne(S.vert[v[1]], S.vert[v[2]])) {
+                tri[k] = v[0] | v[1] << 9 | v[2] << 18;
+                ++nt;
             }
-            ++f;
         }
+        incl = nt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        const unsigned tris = __shfl_sync(0xffffffffu, incl, 31);
+        unsigned f = 0;
+        if (lane == 0 && tris) f = atomicAdd(a.face_count, tris);
+        {
+            unsigned k = incl - nt;
+#pragma unroll
+            for (int q = 0; q < 5; ++q)
+                if (tri[q] != 0xffffffffu) S.tri[k++] = tri[q];
+        }
+        f = __shfl_sync(0xffffffffu, f, 0);
+        __syncwarp();
+        const long room = max(0L, min((long)tris, a.face_cap - (long)f));
+        for (unsigned j = lane; j < 9 * (unsigned)room; j += 32) {
+            const unsigned t = j / 9, c = j - 9 * t, q = c / 3;
+            a.verts[9 * (long)f + j] = S.vert[(S.tri[t] >> (9 * q)) & 511u][c - 3 * q];
+        }
+        for (unsigned j = lane; j < 3 * (unsigned)room; j += 32) a.faces[3 * (long)f + j] = (int)(3 * f + j);
+        __syncwarp();
     }
 }
 
-// A CTA covers a 32 x 8 patch of cube columns and a run of kMcZ cubes along z; each thread
-// marches its column, keeping the four corner values of the slice it shares with the next cube
-// (one new tsdf/weight row pair per step instead of eight corners, no index divisions).  Warps
-// are aligned to x rows, so the loads are coalesced and the warp-level append stays converged.
-// Emits the point-cloud vertices (marchingCubesMeshKernel) and/or the triangles
-// (marchingCubesFullKernel) of each cube.
-constexpr int kMcX = 32, kMcY = 8, kMcZ = 16;
+constexpr int kMcX = 32, kMcY = 8;  // cube columns of a TMA tile
 
-// False when no 8^3 brick holding a cube origin of the tile [x0, x0+32) x [y0, y0+8) x [z0, z0+zr)
+// False when no 8^3 brick holding a cube origin of the box [x0, x0+xr) x [y0, y0+yr) x [z0, z0+zr)
 // has a voxel with a weight.  A cube is active only if all eight corners have a weight, its origin
-// corner among them, so such a tile has no active cube.  Every thread evaluates it (same answer).
-AFX_D bool tile_occupied(const McArgs& a, int x0, int y0, int z0, int zr) {
+// corner among them, so such a box has no active cube.  Every thread evaluates it (same answer).
+AFX_D bool box_occupied(const McArgs& a, int x0, int xr, int y0, int yr, int z0, int zr) {
     if (!a.occ) return true;
-    const int bx1 = min((x0 + kMcX - 1) >> 3, a.nbx - 1), by1 = min((y0 + kMcY - 1) >> 3, a.nby - 1);
+    const int bx1 = min((x0 + xr - 1) >> 3, a.nbx - 1), by1 = min((y0 + yr - 1) >> 3, a.nby - 1);
     const int bz1 = min((z0 + zr - 1) >> 3, a.nbz - 1);
     for (int bz = z0 >> 3; bz <= bz1; ++bz)
         for (int by = y0 >> 3; by <= by1; ++by)
@@ -200,61 +248,113 @@ AFX_D bool tile_occupied(const McArgs& a, int x0, int y0, int z0, int zr) {
     return false;
 }
 
-// tsdf/weight of the corners (x, y), (x+1, y), (x, y+1), (x+1, y+1) of slice z
-template <class TT, class WT>
-AFX_D void mc_slice(const TT* __restrict__ tsdf, const WT* __restrict__ w, long row0, long X, float t[4],
-                    float ww[4]) {
-    t[0] = vox_ld_t(tsdf, row0);
-    t[1] = vox_ld_t(tsdf, row0 + 1);
-    t[2] = vox_ld_t(tsdf, row0 + X);
-    t[3] = vox_ld_t(tsdf, row0 + X + 1);
-    ww[0] = vox_ld_w(w, row0);
-    ww[1] = vox_ld_w(w, row0 + 1);
-    ww[2] = vox_ld_w(w, row0 + X);
-    ww[3] = vox_ld_w(w, row0 + X + 1);
+// A TMA tile's box: 32 x 8 cube columns, zr cubes deep.
+AFX_D bool tile_occupied(const McArgs& a, int x0, int y0, int z0, int zr) {
+    return box_occupied(a, x0, kMcX, y0, kMcY, z0, zr);
 }
+
+// Sweep from global memory, for any row length and alignment: a warp marches kSweepZ slices over 32
+// columns and kSweepY + 1 rows of voxels (31 x kSweepY cubes a slice), with no barrier anywhere.  A
+// lane reads one voxel of each row, coalesced, and keeps two bits of it -- weight not zero, value
+// above iso -- so a cube's case comes from its own bits, its right neighbour's by one shuffle and
+// those of the slice before; the weights of the next slice are on their way meanwhile, and values
+// are read only where the warp's rows hold a weight.  Surface cubes wait in a queue of the warp's own
+// until 32 of them are interpolated together.
+// Bound: the latency of a slice and, where there is surface, the shared-memory traffic of the emission.
+// 257 x 230 x 301 voxels (142 MB) with 0.22 m^2 of surface at 2.5 mm: 65 us, 1.6 TB/s of DRAM reads (a
+// thread per column reading eight corners a cube, and interpolating where it stood, took 400 us; runs of
+// 16 slices 111 us, a warp with much surface holding up the rest).
+constexpr int kSweepY = 4, kSweepZ = 8, kSweepWarps = 8;
 
 template <class TT, class WT, bool kPoints, bool kMesh>
-__global__ void __launch_bounds__(kMcX * kMcY) mc_kernel(const TT* __restrict__ tsdf,
-                                                        const WT* __restrict__ weights, McArgs a) {
-    const int nx = a.vol.dims[0] - 2, ny = a.vol.dims[1] - 2, nz = a.vol.dims[2] - 2;
-    const long X = a.vol.dims[0], XY = X * a.vol.dims[1];
-    const int x = blockIdx.x * kMcX + threadIdx.x, y = blockIdx.y * kMcY + threadIdx.y;
-    const int z0 = blockIdx.z * kMcZ, z1 = min(z0 + kMcZ, nz);
-    if (!tile_occupied(a, blockIdx.x * kMcX, blockIdx.y * kMcY, z0, kMcZ)) return;  // uniform over the CTA
-    const bool col = x < nx && y < ny;
-    const long base = (long)y * X + x;
-    float t0[4] = {0.f, 0.f, 0.f, 0.f}, w0[4] = {0.f, 0.f, 0.f, 0.f};
-    if (col) mc_slice(tsdf, weights, (long)z0 * XY + base, X, t0, w0);
-    for (int z = z0; z < z1; ++z) {
-        float t1[4] = {0.f, 0.f, 0.f, 0.f}, w1[4] = {0.f, 0.f, 0.f, 0.f};
-        if (col) mc_slice(tsdf, weights, (long)(z + 1) * XY + base, X, t1, w1);
-        int ci = 0;
-        if (col) {
-            // corners (src/MarchingCubes.cu:338-379): c0 (1,1,0) c1 (1,0,0) c2 (0,0,0) c3 (0,1,0),
-            // c4..c7 the same one slice up; slot s of a slice is (x + (s & 1), y + (s >> 1))
-            const float ct[8] = {t0[3], t0[1], t0[0], t0[2], t1[3], t1[1], t1[0], t1[2]};
-            const float cw[8] = {w0[3], w0[1], w0[0], w0[2], w1[3], w1[1], w1[0], w1[2]};
-            bool any_zero = false;
+__global__ void __launch_bounds__(32 * kSweepWarps) mc_sweep_kernel(const TT* __restrict__ tsdf,
+                                                                    const WT* __restrict__ weights, McArgs a) {
+    __shared__ unsigned queue[kSweepWarps][64];
+    extern __shared__ unsigned char sweep_raw[];
+    McScratch<kMesh>* scratch = reinterpret_cast<McScratch<kMesh>*>(sweep_raw);  // one per warp
+    constexpr int R = kSweepY + 1;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int X = a.vol.dims[0], Y = a.vol.dims[1];
+    const int nx = X - 2, ny = Y - 2, nz = a.vol.dims[2] - 2;
+    const int x0 = blockIdx.x * 31, y0 = (blockIdx.y * kSweepWarps + w) * kSweepY, z0 = blockIdx.z * kSweepZ;
+    const int z1 = min(z0 + kSweepZ, nz);  // the last slice of voxels
+    if (y0 >= ny || !box_occupied(a, x0, 31, y0, kSweepY, z0, kSweepZ)) return;  // uniform over the warp
+    unsigned* q = queue[w];
+    unsigned nq = 0;  // queued cubes (uniform)
+    const int x = x0 + lane;
+    const long XY = (long)X * Y, base = (long)y0 * X + x;
+    const int rows = x < X ? min(R, Y - y0) : 0;
+    const unsigned cubes = (lane < 31 && x < nx) ? (1u << min(kSweepY, ny - y0)) - 1u : 0u;  // rows with a cube here
+    auto emit = [&](unsigned from, unsigned n) {  // n <= 32 cubes of the queue
+        const bool act = (unsigned)lane < n;
+        const unsigned e = act ? q[from + lane] : 0u;
+        mc_emit<kPoints, kMesh>(tsdf, a, x0 + (int)((e >> 8) & 31u), y0 + (int)((e >> 13) & 7u), z0 + (int)(e >> 16),
+                                (int)(e & 255u), act, scratch[w]);
+    };
+    float wn[R];
+    auto load_weights = [&](int z) {
+        const WT* p = weights + z * XY + base;
 #pragma unroll
-            for (int c = 0; c < 8; ++c) any_zero |= (cw[c] == 0.0f);
-            if (!any_zero)
+        for (int r = 0; r < R; ++r) wn[r] = (r < rows && z <= z1) ? vox_ld_w(p, (long)r * X) : 0.f;
+    };
+    load_weights(z0);
+    // of the slice before, per row of cubes: all four corners weighted, any / every one above iso, and
+    // the bits themselves (own column, next column)
+    unsigned full0 = 0, any0 = 0, all0 = 0, f0 = 0, g0 = 0;
+    for (int z = z0; z <= z1; ++z) {
+        unsigned f = 0;  // bit r: weight of row r; bit 8 + r: value above iso
 #pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    if (ct[c] > a.iso) ci |= 1 << c;
+        for (int r = 0; r < R; ++r) f |= (wn[r] == 0.0f ? 0u : 1u) << r;
+        load_weights(z + 1);
+        if (__any_sync(0xffffffffu, f != 0u)) {
+            const TT* p = tsdf + z * XY + base;
+            float t[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) t[r] = (f >> r) & 1u ? vox_ld_t(p, (long)r * X) : 0.f;
+#pragma unroll
+            for (int r = 0; r < R; ++r) f |= ((f >> r) & 1u && t[r] > a.iso ? 1u : 0u) << (8 + r);
         }
+        const unsigned g = __shfl_down_sync(0xffffffffu, f, 1);
+        const unsigned both = f & g, either = f | g;
+        const unsigned full = both & (both >> 1);                                  // low bits: weights
+        const unsigned all = (both & (both >> 1)) >> 8, any = (either | (either >> 1)) >> 8;
+        const unsigned act = full & full0 & (any | any0) & ~(all & all0) & cubes;
+        if (__any_sync(0xffffffffu, act != 0u)) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            t0[q] = t1[q];
-            w0[q] = w1[q];
+            for (int r = 0; r < kSweepY; ++r) {
+                const bool on = (act >> r) & 1u;
+                const unsigned bal = __ballot_sync(0xffffffffu, on);
+                if (bal == 0u) continue;
+                if (on) {
+                    // corners (src/MarchingCubes.cu:338-379): c0 (1,1,0) c1 (1,0,0) c2 (0,0,0) c3 (0,1,0),
+                    // c4..c7 the same one slice up
+                    auto bits = [&](unsigned own, unsigned next) {
+                        const unsigned o = own >> (8 + r), n = next >> (8 + r);
+                        return ((n >> 1) & 1u) | ((n & 1u) << 1) | ((o & 1u) << 2) | (((o >> 1) & 1u) << 3);
+                    };
+                    const unsigned ci = bits(f0, g0) | (bits(f, g) << 4);
+                    q[nq + __popc(bal & ((1u << lane) - 1u))] =
+                        ci | ((unsigned)lane << 8) | ((unsigned)r << 13) | ((unsigned)(z - 1 - z0) << 16);
+                }
+                nq += __popc(bal);
+                __syncwarp();
+                if (nq >= 32) {
+                    emit(nq - 32, 32);
+                    nq -= 32;
+                    __syncwarp();
+                }
+            }
         }
-        const bool active = ci != 0 && ci != 255;
-        if (!__any_sync(0xffffffffu, active)) continue;
-        mc_emit<kPoints, kMesh>(tsdf, a, x, y, z, ci, active);
+        full0 = full;
+        any0 = any;
+        all0 = all;
+        f0 = f;
+        g0 = g;
     }
+    if (nq) emit(0, nq);
 }
 
-// Same cubes as mc_kernel, with the CTA's whole brick of corner values -- 40 x 9 x (ZR + 1)
+// Same cubes again, with the CTA's whole brick of corner values -- 40 x 9 x (ZR + 1)
 // elements of TSDF and of weights, x padded to a 16-byte multiple -- brought into shared memory by
 // two TMA tile loads on one mbarrier, so the march reads no global memory for inactive cubes.
 constexpr int kMcTX = 40;  // box width in elements (>= kMcX + 1; 160 B in FP32, 80 B in FP16)
@@ -262,7 +362,10 @@ constexpr int kMcTX = 40;  // box width in elements (>= kMcX + 1; 160 B in FP32,
 __host__ __device__ constexpr size_t mc_brick_bytes(size_t elem, int zr) {
     return ((size_t)kMcTX * (kMcY + 1) * (zr + 1) * elem + 127) / 128 * 128;
 }
-__host__ __device__ constexpr size_t mc_tma_smem(size_t elem, int zr) { return 2 * mc_brick_bytes(elem, zr) + 128; }
+__host__ __device__ constexpr size_t mc_tma_smem(size_t elem, int zr) {  // the bricks, or the warps' scratch after them
+    const size_t bricks = 2 * mc_brick_bytes(elem, zr), scratch = kMcX * kMcY / 32 * sizeof(McScratch<true>);
+    return (bricks > scratch ? bricks : scratch) + 128;
+}
 
 AFX_D uint32_t mc_smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -373,15 +476,16 @@ __global__ void __launch_bounds__(kMcX * kMcY) mc_tma_kernel(const __grid_consta
         }
     }
     __syncthreads();
-    // edge vertices and triangles of the queued cubes, one per thread: the FP64 interpolation
-    // then runs with full warps instead of one or two surface lanes per warp
+    // edge vertices and triangles of the queued cubes, 32 per warp; the warps' scratch takes the place of
+    // the bricks, which have been read
+    McScratch<kMesh>* scratch = reinterpret_cast<McScratch<kMesh>*>(mc_raw + pad);
     const unsigned nq = q_n;
     for (unsigned r0 = 0; r0 < nq; r0 += kMcX * kMcY) {
         const unsigned qi = r0 + tid;
         const bool act = qi < nq;
         const unsigned e = act ? q[qi] : 0u;
         mc_emit<kPoints, kMesh>(tsdf, a, x0 + (int)((e >> 8) & 31u), y0 + (int)((e >> 13) & 7u),
-                                z0 + (int)((e >> 16) & 63u), (int)(e & 255u), act);
+                                z0 + (int)((e >> 16) & 63u), (int)(e & 255u), act, scratch[tid >> 5]);
     }
 }
 
@@ -427,12 +531,14 @@ __global__ void __launch_bounds__(kMcX * kMcY) mc_pipe_kernel(const __grid_const
     __shared__ alignas(8) unsigned long long mbar[2];
     __shared__ unsigned q[kMcX * kMcY * ZR];
     __shared__ unsigned q_n;
-    const uint32_t pad = (128u - (mc_smem_u32(mc_raw) & 127u)) & 127u;
+    McScratch<kMesh>* scratch = reinterpret_cast<McScratch<kMesh>*>(mc_raw);  // the bricks follow
+    unsigned char* const mc_bricks = mc_raw + kMcX * kMcY / 32 * sizeof(McScratch<kMesh>);
+    const uint32_t pad = (128u - (mc_smem_u32(mc_bricks) & 127u)) & 127u;
     TT* st[2];
     WT* sw[2];
     for (int k = 0; k < 2; ++k) {
-        st[k] = reinterpret_cast<TT*>(mc_raw + pad + (2 * k) * kBrick);
-        sw[k] = reinterpret_cast<WT*>(mc_raw + pad + (2 * k + 1) * kBrick);
+        st[k] = reinterpret_cast<TT*>(mc_bricks + pad + (2 * k) * kBrick);
+        sw[k] = reinterpret_cast<WT*>(mc_bricks + pad + (2 * k + 1) * kBrick);
     }
     const int tid = threadIdx.y * kMcX + threadIdx.x;
     const long nall = (long)tx_n * ty_n * tz_n;
@@ -529,7 +635,7 @@ __global__ void __launch_bounds__(kMcX * kMcY) mc_pipe_kernel(const __grid_const
             const bool act = qi < nq;
             const unsigned e = act ? q[qi] : 0u;
             mc_emit<kPoints, kMesh>(tsdf, a, x0 + (int)((e >> 8) & 31u), y0 + (int)((e >> 13) & 7u),
-                                    z0 + (int)((e >> 16) & 63u), (int)(e & 255u), act);
+                                    z0 + (int)((e >> 16) & 63u), (int)(e & 255u), act, scratch[tid >> 5]);
         }
         __syncthreads();  // the queue is reused by the next tile
     }
@@ -573,7 +679,7 @@ static void mc_launch_tma(const TT* tsdf, const McArgs& a, const CUtensorMap* mt
 template <class TT, class WT, bool kPoints, bool kMesh, int ZR>
 static void mc_launch_pipe(const TT* tsdf, const McArgs& a, const CUtensorMap* mt, const CUtensorMap* mw,
                            cudaStream_t st) {
-    constexpr int smem = (int)(4 * mc_brick_bytes(sizeof(TT), ZR) + 128);
+    constexpr int smem = (int)(4 * mc_brick_bytes(sizeof(TT), ZR) + 128 + kMcX * kMcY / 32 * sizeof(McScratch<kMesh>));
     static ContextOnce once;  // per instantiation: opt-in and resident CTAs per SM, per device
     static int per_sm_dev[kMaxDevices], sms_dev[kMaxDevices];
     once_per_context(once, [](int dev) {
@@ -616,8 +722,8 @@ size_t mc_tile_ws_words(const Volume& vol) {
 // tile: kMcTileTma16 (default), kMcTileTma8, kMcTileTma32 (TMA bricks of that many cubes along z),
 // kMcTilePipe8 / kMcTilePipe16 / kMcTilePipe4 (persistent grid with two stages of bricks 8, 16 or 4
 // cubes deep) or
-// kMcTileColumn (column march from global memory, 16 cubes along z).  mt/mw are the maps encoded for
-// that depth, or null (then the column march runs).
+// kMcTileColumn (sweep from global memory).  mt/mw are the maps encoded for that depth, or null (then the
+// sweep runs).
 template <class TT, class WT, bool kPoints, bool kMesh>
 static void mc_launch(const TT* tsdf, const WT* weights, const McArgs& a, const CUtensorMap* mt, const CUtensorMap* mw,
                       int tile, cudaStream_t st) {
@@ -634,9 +740,16 @@ static void mc_launch(const TT* tsdf, const WT* weights, const McArgs& a, const 
     } else if (mt) {
         mc_launch_tma<TT, WT, kPoints, kMesh, 16>(tsdf, a, mt, mw, st);
     } else {
-        const dim3 grid((unsigned)((a.vol.dims[0] - 2 + kMcX - 1) / kMcX),
-                        (unsigned)((a.vol.dims[1] - 2 + kMcY - 1) / kMcY), (unsigned)((a.vol.dims[2] - 2 + kMcZ - 1) / kMcZ));
-        mc_kernel<TT, WT, kPoints, kMesh><<<grid, dim3(kMcX, kMcY), 0, st>>>(tsdf, weights, a);
+        constexpr int kRows = kSweepY * kSweepWarps;
+        const dim3 grid((unsigned)((a.vol.dims[0] - 2 + 30) / 31), (unsigned)((a.vol.dims[1] - 2 + kRows - 1) / kRows),
+                        (unsigned)((a.vol.dims[2] - 2 + kSweepZ - 1) / kSweepZ));
+        constexpr int smem = kSweepWarps * (int)sizeof(McScratch<kMesh>);
+        static ContextOnce once;
+        once_per_context(once, [](int) {
+            return note_cuda_error(cudaFuncSetAttribute(mc_sweep_kernel<TT, WT, kPoints, kMesh>,
+                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        });
+        mc_sweep_kernel<TT, WT, kPoints, kMesh><<<grid, 32 * kSweepWarps, smem, st>>>(tsdf, weights, a);
     }
 }
 
@@ -713,105 +826,167 @@ AFX_D unsigned f2key(float f) {
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 AFX_D float key2f(unsigned k) { return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k); }
-AFX_D bool key_less(const Key3& a, const Key3& b) {
-    if (a.k[0] != b.k[0]) return a.k[0] < b.k[0];
-    if (a.k[1] != b.k[1]) return a.k[1] < b.k[1];
-    return a.k[2] < b.k[2];
+AFX_D bool key_less(const Key3& a, const Key3& b) {  // without branches: lanes compare different keys
+    const bool l0 = a.k[0] < b.k[0], e0 = a.k[0] == b.k[0], l1 = a.k[1] < b.k[1], e1 = a.k[1] == b.k[1];
+    return l0 | (e0 & (l1 | (e1 & (a.k[2] < b.k[2]))));
+}
+AFX_D Key3 key_pick(bool first, const Key3& a, const Key3& b) {
+    return {{first ? a.k[0] : b.k[0], first ? a.k[1] : b.k[1], first ? a.k[2] : b.k[2]}};
 }
 AFX_D bool key_le(const Key3& a, const Key3& b) { return !key_less(b, a); }
 
+// The points are sorted in tiles of kSortTile (one CTA each), the sorted
+// runs merged pairwise in passes over all SMs, then made unique by float equality of consecutive
+// points and compacted in order back into the cloud.  The number of points is on the device, so as
+// many passes are launched as the capacity can need; those that the live number does not need return
+// at once.  The pass a run length belongs to decides which buffer it reads.
+// Bound: latency of a pass (a search for the split, one load, a merge of kSortPer keys per thread).
+// 450,000 points of a marching-cubes cloud: tiles 20 us, 8 passes of 9 us, unique 15 us; one cluster of
+// 16 CTAs doing all of it took 905 us.
 constexpr int kSortTile = 2048;
-constexpr int kSortThreads = 1024;
-constexpr int kSortCluster = 16;
+constexpr int kSortPer = 8;  // keys per thread
+constexpr int kSortThreads = kSortTile / kSortPer;
+constexpr int kUniqueThreads = 1024;
+constexpr long kSortBlocks = 608;  // four CTAs per SM
 
-AFX_D unsigned sort_rank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-AFX_D unsigned sort_ncta() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-    return r;
-}
-AFX_D void sort_cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+// Passes that merge runs of kSortTile into one of n.
+__host__ __device__ inline int sort_passes(long n) {
+    int p = 0;
+    for (long L = kSortTile; L < n; L <<= 1) ++p;
+    return p;
 }
 
-// Bitonic sort of one tile of up to kSortTile points (padding sorts last) into `out`.
-AFX_D void sort_tile(const float* __restrict__ pts, Key3* out, long base, long n, Key3* s) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < kSortTile; i += blockDim.x) {
-        const long j = base + i;
-        Key3 k;
-        if (j < n) {
-            k.k[0] = f2key(pts[3 * j]);
-            k.k[1] = f2key(pts[3 * j + 1]);
-            k.k[2] = f2key(pts[3 * j + 2]);
-        } else {
-            k.k[0] = k.k[1] = k.k[2] = 0xffffffffu;
-        }
-        s[i] = k;
+AFX_D Key3 sort_key(const float* p) {
+    Key3 k;
+    k.k[0] = f2key(p[0]);
+    k.k[1] = f2key(p[1]);
+    k.k[2] = f2key(p[2]);
+    return k;
+}
+
+// A tile in shared memory, with a key of padding after every kSortPer: a warp's threads then work on
+// kSortPer keys each without meeting in the same banks.
+struct SortTile {
+    Key3 k[kSortTile + kSortTile / kSortPer];
+    AFX_D Key3& operator[](int i) { return k[i + i / kSortPer]; }
+};
+
+// Outputs [q0, q0 + kSortPer) of merging the sorted runs s[at, at + la) and s[at + la, at + la + lb), into
+// registers.
+AFX_D void merge_serial(SortTile& s, int at, int la, int lb, int q0, Key3 (&out)[kSortPer]) {
+    int lo = max(0, q0 - lb), hi = min(q0, la);
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (key_le(s[at + mid], s[at + la + q0 - 1 - mid])) lo = mid + 1;
+        else hi = mid;
     }
-    __syncthreads();
-    for (int size = 2; size <= kSortTile; size <<= 1)
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int p = threadIdx.x; p < kSortTile / 2; p += blockDim.x) {
-                const int i = 2 * stride * (p / stride) + (p % stride), j = i + stride;
-                const bool asc = (i & size) == 0;
-                const Key3 a = s[i], b = s[j];
-                if (key_less(b, a) == asc) {
-                    s[i] = b;
-                    s[j] = a;
-                }
+    int ia = lo, ib = q0 - lo;
+    const int end = at + la + lb - 1;
+    Key3 a = s[min(at + ia, end)], b = s[min(at + la + ib, end)];
+#pragma unroll
+    for (int q = 0; q < kSortPer; ++q) {
+        const bool takeA = (ib >= lb) | ((ia < la) & key_le(a, b));
+        out[q] = key_pick(takeA, a, b);
+        ia += takeA;
+        ib += !takeA;
+        const Key3 next = s[min(takeA ? at + ia : at + la + ib, end)];
+        a = key_pick(takeA, next, a);
+        b = key_pick(takeA, b, next);
+    }
+}
+
+// Each tile of up to kSortTile points (padding sorts last) sorted into `out`: kSortPer keys per thread by a
+// sorting network in registers, then runs merged in shared memory, each thread its kSortPer outputs of
+// a merge through registers (a bitonic sort of the tile in shared memory took 50 us for 112 tiles,
+// bound by shared-memory accesses).
+__global__ void __launch_bounds__(kSortThreads) sort_tiles_kernel(const float* __restrict__ pts, const unsigned* count,
+                                                                 long n_max, Key3* out, unsigned* done) {
+    __shared__ SortTile s;
+    const long n = min((long)*count, n_max);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *done = 0u;
+    for (long base = blockIdx.x * (long)kSortTile; base < n; base += gridDim.x * (long)kSortTile) {
+        Key3 v[kSortPer];
+#pragma unroll
+        for (int k = 0; k < kSortPer; ++k) {
+            const long j = base + k * kSortThreads + threadIdx.x;
+            if (j < n) v[k] = sort_key(pts + 3 * j);
+            else v[k].k[0] = v[k].k[1] = v[k].k[2] = 0xffffffffu;
+        }
+#pragma unroll
+        for (int round = 0; round < kSortPer; ++round)  // odd-even transposition
+#pragma unroll
+            for (int k = round & 1; k + 1 < kSortPer; k += 2) {
+                const bool swap = key_less(v[k + 1], v[k]);
+                const Key3 t = key_pick(swap, v[k], v[k + 1]);
+                v[k] = key_pick(swap, v[k + 1], v[k]);
+                v[k + 1] = t;
             }
+        const int q0 = threadIdx.x * kSortPer;
+#pragma unroll
+        for (int k = 0; k < kSortPer; ++k) s[q0 + k] = v[k];
+        __syncthreads();
+        for (int run = kSortPer; run < kSortTile; run <<= 1) {
+            const int pair = q0 / (2 * run) * (2 * run);
+            merge_serial(s, pair, run, run, q0 - pair, v);
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < kSortPer; ++k) s[q0 + k] = v[k];
             __syncthreads();
         }
-    for (int i = threadIdx.x; i < kSortTile; i += blockDim.x) {
-        const long j = base + i;
-        if (j < n) out[j] = s[i];
+        for (int i = threadIdx.x; i < kSortTile; i += kSortThreads)
+            if (base + i < n) out[base + i] = s[i];
+        __syncthreads();
     }
 }
 
-// Outputs [o0, o0 + kSortTile) of merging the sorted runs of length L around o0 (merge path).
-AFX_D void merge_chunk(const Key3* __restrict__ in, Key3* __restrict__ out, long n, long L, long o0, Key3* s,
-                       long* split) {
-    const long pair = o0 / (2 * L) * (2 * L);
-    const long a0 = pair, na = min(L, n - a0);
-    const long b0 = pair + L, nb = max(0L, min(L, n - b0));
-    const long d0 = o0 - pair, d1 = min(d0 + kSortTile, na + nb);
-    __syncthreads();
-    if (threadIdx.x < 2) {
-        const long d = threadIdx.x == 0 ? d0 : d1;
-        long lo = max(0L, d - nb), hi = min(d, na);
-        while (lo < hi) {
-            const long mid = (lo + hi) >> 1;
-            if (key_le(in[a0 + mid], in[b0 + d - 1 - mid])) lo = mid + 1;
-            else hi = mid;
-        }
-        split[threadIdx.x] = lo;
+// Merge path: how many of the first d merged keys come from A[0, na), the rest from B[0, nb).  One warp:
+// 32 probes per step.
+AFX_D long merge_split(const Key3* __restrict__ A, long na, const Key3* __restrict__ B, long nb, long d) {
+    const int lane = threadIdx.x & 31;
+    long lo = max(0L, d - nb), hi = min(d, na);
+    while (lo < hi) {
+        const long mid = lo + (hi - lo) * lane / 32;  // lane 0: lo; ascending
+        const unsigned yes = __ballot_sync(0xffffffffu, key_le(A[mid], B[d - 1 - mid]));
+        const int t = __popc(yes);  // the first t probes are before the split
+        const long first_no = __shfl_sync(0xffffffffu, mid, t & 31), last_yes = __shfl_sync(0xffffffffu, mid, (t + 31) & 31);
+        if (t < 32) hi = first_no;
+        if (t > 0) lo = last_yes + 1;
     }
-    __syncthreads();
-    const long i0 = split[0], i1 = split[1];
-    const long j0 = d0 - i0, j1 = d1 - i1;
-    const int la = (int)(i1 - i0), lb = (int)(j1 - j0);
-    for (int t = threadIdx.x; t < la + lb; t += blockDim.x) s[t] = t < la ? in[a0 + i0 + t] : in[b0 + j0 + (t - la)];
-    __syncthreads();
-    const int tot = la + lb;
-    const int per = kSortTile / blockDim.x;  // blockDim.x divides kSortTile
-    const int q0 = threadIdx.x * per;
-    if (q0 < tot) {
-        int lo = max(0, q0 - lb), hi = min(q0, la);
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (key_le(s[mid], s[la + q0 - 1 - mid])) lo = mid + 1;
-            else hi = mid;
+    return lo;
+}
+
+// One pass: runs of length L of `in` merged pairwise into `out`, kSortTile outputs per CTA and step.
+__global__ void __launch_bounds__(kSortThreads) merge_pass_kernel(const Key3* __restrict__ in, Key3* __restrict__ out,
+                                                                 const unsigned* count, long n_max, long L) {
+    __shared__ SortTile s;
+    __shared__ long split[2];
+    const long n = min((long)*count, n_max);
+    if (L >= n) return;  // one run already
+    for (long o0 = blockIdx.x * (long)kSortTile; o0 < n; o0 += gridDim.x * (long)kSortTile) {
+        const long pair = o0 / (2 * L) * (2 * L);
+        const Key3 *A = in + pair, *B = in + pair + L;
+        const long na = min(L, n - pair), nb = max(0L, min(L, n - pair - L));
+        const long d0 = o0 - pair, d1 = min(d0 + kSortTile, na + nb);
+        const int w = threadIdx.x >> 5;
+        __syncthreads();  // the step before is done with s and split
+        if (w < 2) {
+            const long i = merge_split(A, na, B, nb, w == 0 ? d0 : d1);
+            if ((threadIdx.x & 31) == 0) split[w] = i;
         }
-        int ia = lo, ib = q0 - lo;
-        for (int q = q0; q < q0 + per && q < tot; ++q) {
-            const bool takeA = ib >= lb || (ia < la && key_le(s[ia], s[la + ib]));
-            out[o0 + q] = takeA ? s[ia++] : s[la + ib++];
-        }
+        __syncthreads();
+        const long i0 = split[0], j0 = d0 - i0;
+        const int la = (int)(split[1] - i0), tot = (int)(d1 - d0), lb = tot - la;
+        for (int t = threadIdx.x; t < tot; t += kSortThreads) s[t] = t < la ? A[i0 + t] : B[j0 + (t - la)];
+        __syncthreads();
+        Key3 v[kSortPer];
+        const int q0 = threadIdx.x * kSortPer;
+        if (q0 < tot) merge_serial(s, 0, la, lb, q0, v);
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kSortPer; ++k)
+            if (q0 + k < tot) s[q0 + k] = v[k];
+        __syncthreads();
+        for (int t = threadIdx.x; t < tot; t += kSortThreads) out[o0 + t] = s[t];
     }
 }
 
@@ -819,78 +994,53 @@ AFX_D bool key_same_point(const Key3& a, const Key3& b) {
     return key2f(a.k[0]) == key2f(b.k[0]) && key2f(a.k[1]) == key2f(b.k[1]) && key2f(a.k[2]) == key2f(b.k[2]);
 }
 
-// Lexicographic sort + unique of the point cloud in one launch of one thread-block cluster:
-// tiles of kSortTile sorted in shared memory, merge-path passes until one run remains (the
-// pass count follows the live count on the device), then unique by float equality of
-// consecutive points and an ordered compaction back into `pts`.  Phases are separated by the
-// hardware cluster barrier.
-__global__ void __launch_bounds__(kSortThreads, 1) sort_unique_kernel(float* pts, unsigned* count, long n_max,
-                                                                     Key3* buf0, Key3* buf1, unsigned* tile_cnt,
-                                                                     const unsigned* only_if) {
-    __shared__ Key3 s[kSortTile];
-    if (only_if && *only_if == 0u) return;  // the column-bucket sort did the work
-    __shared__ long split[2];
-    __shared__ unsigned wsum[kSortThreads / 32];
-    __shared__ unsigned s_base;
-    const long n = min((long)*count, n_max);
-    const unsigned rank = sort_rank(), ncta = sort_ncta();
-    const long tiles = (n + kSortTile - 1) / kSortTile;
-    for (long t = rank; t < tiles; t += ncta) sort_tile(pts, buf0, t * kSortTile, n, s);
-    sort_cluster_barrier();
-    Key3* src = buf0;
-    Key3* dst = buf1;
-    for (long L = kSortTile; L < n; L <<= 1) {
-        for (long t = rank; t < tiles; t += ncta) merge_chunk(src, dst, n, L, t * kSortTile, s, split);
-        sort_cluster_barrier();
-        Key3* tmp = src;
-        src = dst;
-        dst = tmp;
+// Points of each tile that differ from the one before them.
+__global__ void __launch_bounds__(kUniqueThreads) unique_count_kernel(const Key3* buf0, const Key3* buf1,
+                                                                   const unsigned* count, long n_max, unsigned* tile_cnt) {
+    const long n = min((long)*count, n_max), tiles = (n + kSortTile - 1) / kSortTile;
+    const Key3* src = sort_passes(n) & 1 ? buf1 : buf0;
+    for (long t = blockIdx.x; t < tiles; t += gridDim.x) {
+        int c = 0;
+        for (long i0 = t * kSortTile; i0 < min(n, (t + 1) * kSortTile); i0 += kUniqueThreads) {
+            const long i = i0 + threadIdx.x;
+            c += __syncthreads_count(i < n && (i == 0 || !key_same_point(src[i - 1], src[i])));
+        }
+        if (threadIdx.x == 0) tile_cnt[t] = (unsigned)c;
     }
-    // unique flags and per-tile counts
+}
+
+// Ordered compaction: a tile starts after the counts of those before it.  The block that finishes last
+// writes the new number of points (no block reads the old one any more).
+__global__ void __launch_bounds__(kUniqueThreads) unique_compact_kernel(float* pts, const Key3* buf0, const Key3* buf1,
+                                                                     unsigned* count, long n_max,
+                                                                     const unsigned* __restrict__ tile_cnt, unsigned* done) {
+    __shared__ unsigned wsum[kUniqueThreads / 32];
+    const long n = min((long)*count, n_max), tiles = (n + kSortTile - 1) / kSortTile;
+    const Key3* src = sort_passes(n) & 1 ? buf1 : buf0;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (long t = rank; t < tiles; t += ncta) {
+    auto sum_before = [&](long t) {  // of tile_cnt[0, t), in every thread
         unsigned c = 0;
-        for (long i = t * kSortTile + threadIdx.x; i < min(n, (t + 1) * kSortTile); i += blockDim.x)
-            c += (i == 0 || !key_same_point(src[i - 1], src[i])) ? 1u : 0u;
+        for (long k = threadIdx.x; k < t; k += kUniqueThreads) c += tile_cnt[k];
         c = warp_sum(c);
         __syncthreads();
         if (lane == 0) wsum[w] = c;
         __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned tot = 0;
-            for (int k = 0; k < kSortThreads / 32; ++k) tot += wsum[k];
-            tile_cnt[t] = tot;
-        }
-    }
-    sort_cluster_barrier();
-    // ordered compaction: tile base = exclusive prefix of the tile counts
-    for (long t = rank; t < tiles; t += ncta) {
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned b = 0;
-            for (long k = 0; k < t; ++k) b += __ldcg(tile_cnt + k);
-            s_base = b;
-        }
-        __syncthreads();
-        // one element per thread per round, kSortTile / kSortThreads rounds, in index order
-        unsigned run = s_base;
-        for (long r0 = t * kSortTile; r0 < min(n, (t + 1) * kSortTile); r0 += blockDim.x) {
+        return warp_sum(wsum[lane]);
+    };
+    for (long t = blockIdx.x; t < tiles; t += gridDim.x) {
+        unsigned run = sum_before(t);
+        // one element per thread per step, in index order
+        for (long r0 = t * kSortTile; r0 < min(n, (t + 1) * kSortTile); r0 += kUniqueThreads) {
             const long i = r0 + threadIdx.x;
             const bool keep = i < n && (i == 0 || !key_same_point(src[i - 1], src[i]));
             const unsigned bal = __ballot_sync(0xffffffffu, keep);
             __syncthreads();
             if (lane == 0) wsum[w] = __popc(bal);
             __syncthreads();
-            unsigned before = 0, all = 0;
-            for (int k = 0; k < kSortThreads / 32; ++k) {
-                const unsigned v = wsum[k];
-                if (k < w) before += v;
-                all += v;
-            }
+            const unsigned c = wsum[lane], before = warp_sum(lane < w ? c : 0u), all = warp_sum(c);
             if (keep) {
-                const unsigned pos = run + before + __popc(bal & ((1u << lane) - 1));
                 const Key3 k = src[i];
-                float* o = pts + 3 * (long)pos;
+                float* o = pts + 3 * (long)(run + before + __popc(bal & ((1u << lane) - 1)));
                 o[0] = key2f(k.k[0]);
                 o[1] = key2f(k.k[1]);
                 o[2] = key2f(k.k[2]);
@@ -898,12 +1048,13 @@ __global__ void __launch_bounds__(kSortThreads, 1) sort_unique_kernel(float* pts
             run += all;
         }
     }
-    sort_cluster_barrier();
-    if (rank == 0 && threadIdx.x == 0 && n > 0) {
-        unsigned tot = 0;
-        for (long k = 0; k < tiles; ++k) tot += __ldcg(tile_cnt + k);
-        *count = tot;
-    }
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last || n == 0) return;
+    const unsigned total = sum_before(tiles);
+    if (threadIdx.x == 0) *count = total;
 }
 
 static size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -913,69 +1064,30 @@ size_t sort_unique_workspace_size(long n_max) {
     return 2 * al(n_max * sizeof(Key3)) + al(((n_max + kSortTile - 1) / kSortTile) * 4) + 256;
 }
 
-static int sort_cluster_size() {
-    static ContextOnce once;
-    static int cached_dev[kMaxDevices];
-    once_per_context(once, [](int dev) {
-        int cached = 0;
-        cudaFuncSetAttribute(sort_unique_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        const int sizes[2] = {kSortCluster, 8};
-        for (int c : sizes) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(c);
-            cfg.blockDim = dim3(kSortThreads);
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = c;
-            at[0].val.clusterDim.y = 1;
-            at[0].val.clusterDim.z = 1;
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
-            int clusters = 0;
-            if (cudaOccupancyMaxActiveClusters(&clusters, sort_unique_kernel, &cfg) == cudaSuccess && clusters > 0) {
-                cached = c;
-                break;
-            }
-            cudaGetLastError();
-        }
-        cached_dev[dev] = cached ? cached : 8;
-        return (int)AFX_OK;
-    });
-    int dev = 0;
-    cudaGetDevice(&dev);
-    return cached_dev[dev] ? cached_dev[dev] : 8;
-}
-
-static int sort_unique_cluster(float* pts, unsigned* count, long n_max, void* ws, size_t ws_bytes, cudaStream_t st,
-                               const unsigned* only_if);
-
 int sort_unique_impl(float* pts, unsigned* count, long n_max, void* ws, size_t ws_bytes, cudaStream_t st) {
-    return sort_unique_cluster(pts, count, n_max, ws, ws_bytes, st, nullptr);
-}
-
-static int sort_unique_cluster(float* pts, unsigned* count, long n_max, void* ws, size_t ws_bytes, cudaStream_t st,
-                               const unsigned* only_if) {
     if (n_max <= 0) return AFX_OK;
     if (!ws || ws_bytes < sort_unique_workspace_size(n_max)) return AFX_ERR_WORKSPACE;
     char* p = static_cast<char*>(ws);
-    Key3* buf0 = reinterpret_cast<Key3*>(p);
-    p += al(n_max * sizeof(Key3));
-    Key3* buf1 = reinterpret_cast<Key3*>(p);
-    p += al(n_max * sizeof(Key3));
+    Key3* buf[2];
+    for (Key3*& b : buf) {
+        b = reinterpret_cast<Key3*>(p);
+        p += al(n_max * sizeof(Key3));
+    }
     unsigned* tile_cnt = reinterpret_cast<unsigned*>(p);
-    const int c = sort_cluster_size();
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(c);
-    cfg.blockDim = dim3(kSortThreads);
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = c;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    AFX_CUDA(cudaLaunchKernelEx(&cfg, sort_unique_kernel, pts, count, n_max, buf0, buf1, tile_cnt, only_if));
+    p += al(((n_max + kSortTile - 1) / kSortTile) * 4);
+    unsigned* done = reinterpret_cast<unsigned*>(p);
+    const long tiles = (n_max + kSortTile - 1) / kSortTile;
+    const unsigned grid = (unsigned)(tiles < kSortBlocks ? tiles : kSortBlocks);
+    sort_tiles_kernel<<<grid, kSortThreads, 0, st>>>(pts, count, n_max, buf[0], done);
+    AFX_LAUNCH_CHECK();
+    const int passes = sort_passes(n_max);
+    for (int k = 0; k < passes; ++k) {
+        merge_pass_kernel<<<grid, kSortThreads, 0, st>>>(buf[k & 1], buf[(k & 1) ^ 1], count, n_max, (long)kSortTile << k);
+        AFX_LAUNCH_CHECK();
+    }
+    unique_count_kernel<<<grid, kUniqueThreads, 0, st>>>(buf[0], buf[1], count, n_max, tile_cnt);
+    AFX_LAUNCH_CHECK();
+    unique_compact_kernel<<<grid, kUniqueThreads, 0, st>>>(pts, buf[0], buf[1], count, n_max, tile_cnt, done);
     AFX_LAUNCH_CHECK();
     return AFX_OK;
 }
@@ -991,7 +1103,7 @@ static int sort_unique_cluster(float* pts, unsigned* count, long n_max, void* ws
 // compaction back into the cloud.  A bucket larger than kBucketCap (a surface lying along one x
 // column) is sorted by its CTA in runs of kBucketCap in shared memory that are then merged pairwise
 // in global memory (merge path, ties from the left run first) between the key buffer and the second
-// buffer of the workspace, so one crowded column no longer sends the whole cloud to the cluster sort.
+// buffer of the workspace.
 // ------------------------------------------------------------------------------------
 
 constexpr int kBucketCap = 8192;  // keys per bucket sorted in shared memory (96 KB)
@@ -1014,7 +1126,6 @@ struct BucketWs {
     unsigned* cursor;  // [nb]
     unsigned* ucnt;    // [nb]
     unsigned* uoff;    // [nb + 1]
-    unsigned* overflow;
 };
 
 __global__ void bucket_count_kernel(const float* __restrict__ pts, const unsigned* count, long n_max, BucketArgs a,
@@ -1024,20 +1135,14 @@ __global__ void bucket_count_kernel(const float* __restrict__ pts, const unsigne
 }
 
 // Exclusive scan of n values by one CTA of 1024 threads (n up to a few thousand); out[n] = total.
-// With `overflow`, flags it when a value exceeds `cap`; with `total`, also writes the total there
-// unless *skip is set.
+// With `total`, the total is written there too.
 __global__ void __launch_bounds__(1024) small_scan_kernel(const unsigned* in, int n, unsigned* out, unsigned* copy,
-                                                          unsigned cap, unsigned* overflow, unsigned* total,
-                                                          const unsigned* skip) {
+                                                          unsigned* total) {
     __shared__ unsigned part[1024];
     const int per = (n + 1023) / 1024;
     const int lo = threadIdx.x * per, hi = min(n, lo + per);
-    unsigned sum = 0, big = 0;
-    for (int i = lo; i < hi; ++i) {
-        sum += in[i];
-        big |= in[i] > cap;
-    }
-    if (overflow && __syncthreads_or(big) && threadIdx.x == 0) *overflow = 1u;
+    unsigned sum = 0;
+    for (int i = lo; i < hi; ++i) sum += in[i];
     part[threadIdx.x] = sum;
     __syncthreads();
     for (int o = 1; o < 1024; o <<= 1) {
@@ -1054,13 +1159,12 @@ __global__ void __launch_bounds__(1024) small_scan_kernel(const unsigned* in, in
     }
     if (threadIdx.x == 1023) {
         out[n] = part[1023];
-        if (total && !(skip && *skip)) *total = part[1023];
+        if (total) *total = part[1023];
     }
 }
 
 __global__ void bucket_scatter_kernel(const float* __restrict__ pts, const unsigned* count, long n_max, BucketArgs a,
-                                      unsigned* cursor, Key3* keys, const unsigned* overflow, int* error) {
-    if (*overflow) return;
+                                      unsigned* cursor, Key3* keys, int* error) {
     const long n = min((long)*count, n_max);
     AFX_GRID_STRIDE(i, n) {
         Key3 k;
@@ -1126,11 +1230,10 @@ AFX_D void cta_merge(const Key3* A, unsigned la, const Key3* B, unsigned lb, Key
 // One CTA per bucket: sort it in place (in shared memory, or in runs merged through `scratch` when it
 // holds more than kBucketCap points) and count its unique points.
 __global__ void __launch_bounds__(kBucketThreads) bucket_sort_kernel(Key3* keys, Key3* scratch, const unsigned* off,
-                                                                   unsigned* ucnt, const unsigned* overflow, long n_max,
+                                                                   unsigned* ucnt, long n_max,
                                                                    int* error) {
     extern __shared__ Key3 sk[];
     __shared__ unsigned wsum[kBucketThreads / 32];
-    if (*overflow) return;
     const int b = blockIdx.x;
     const unsigned lo = off[b], n = off[b + 1] - lo;
     if (lo > off[b + 1] || (long)off[b + 1] > n_max) {  // never expected: skip, flag
@@ -1180,9 +1283,8 @@ __global__ void __launch_bounds__(kBucketThreads) bucket_sort_kernel(Key3* keys,
 // One CTA per bucket: its unique points, in order, at the bucket's place in the output.
 __global__ void __launch_bounds__(kBucketThreads) bucket_compact_kernel(const Key3* keys, const unsigned* off,
                                                                       const unsigned* uoff, float* pts, long n_max,
-                                                                      const unsigned* overflow, int* error) {
+                                                                      int* error) {
     __shared__ unsigned wsum[kBucketThreads / 32];
-    if (*overflow) return;
     const int b = blockIdx.x;
     if (off[b] > off[b + 1] || (long)off[b + 1] > n_max || (long)uoff[b + 1] > n_max) {
         if (threadIdx.x == 0 && error) atomicOr(error, ERRF_INDEX);
@@ -1227,8 +1329,8 @@ int sort_unique_volume_impl(float* pts, unsigned* count, long n_max, void* ws, s
     if (!ws || ws_bytes < sort_unique_volume_workspace_size(n_max, nb)) return AFX_ERR_WORKSPACE;
     const size_t base = sort_unique_workspace_size(n_max);
     unsigned* u = reinterpret_cast<unsigned*>(static_cast<char*>(ws) + base);
-    BucketWs w{u, u + nb, u + 2 * nb + 1, u + 3 * nb + 1, u + 4 * nb + 1, u + 5 * nb + 2};
-    Key3* keys = reinterpret_cast<Key3*>(ws);  // the cluster sort's first buffer (it rebuilds it from the cloud)
+    BucketWs w{u, u + nb, u + 2 * nb + 1, u + 3 * nb + 1, u + 4 * nb + 1};
+    Key3* keys = reinterpret_cast<Key3*>(ws);
     BucketArgs a{vol.half[0], vol.inv[0], nb};
     static ContextOnce once;
     once_per_context(once, [](int) {
@@ -1236,18 +1338,20 @@ int sort_unique_volume_impl(float* pts, unsigned* count, long n_max, void* ws, s
                                                     (int)(kBucketCap * sizeof(Key3))));
     });
     AFX_CUDA(cudaMemsetAsync(w.cnt, 0, nb * 4, st));
-    AFX_CUDA(cudaMemsetAsync(w.overflow, 0, 4, st));
     bucket_count_kernel<<<grid_for(n_max, 256), 256, 0, st>>>(pts, count, n_max, a, w.cnt);
-    small_scan_kernel<<<1, 1024, 0, st>>>(w.cnt, nb, w.off, w.cursor, 0xffffffffu, nullptr, nullptr, nullptr);
-    bucket_scatter_kernel<<<grid_for(n_max, 256), 256, 0, st>>>(pts, count, n_max, a, w.cursor, keys, w.overflow,
-                                                                 error);
-    Key3* scratch = reinterpret_cast<Key3*>(static_cast<char*>(ws) + al(n_max * sizeof(Key3)));  // the second buffer
-    bucket_sort_kernel<<<nb, kBucketThreads, kBucketCap * sizeof(Key3), st>>>(keys, scratch, w.off, w.ucnt, w.overflow,
-                                                                              n_max, error);
-    small_scan_kernel<<<1, 1024, 0, st>>>(w.ucnt, nb, w.uoff, nullptr, 0xffffffffu, nullptr, count, w.overflow);
-    bucket_compact_kernel<<<nb, kBucketThreads, 0, st>>>(keys, w.off, w.uoff, pts, n_max, w.overflow, error);
     AFX_LAUNCH_CHECK();
-    return sort_unique_cluster(pts, count, n_max, ws, ws_bytes, st, w.overflow);
+    small_scan_kernel<<<1, 1024, 0, st>>>(w.cnt, nb, w.off, w.cursor, nullptr);
+    AFX_LAUNCH_CHECK();
+    bucket_scatter_kernel<<<grid_for(n_max, 256), 256, 0, st>>>(pts, count, n_max, a, w.cursor, keys, error);
+    AFX_LAUNCH_CHECK();
+    Key3* scratch = reinterpret_cast<Key3*>(static_cast<char*>(ws) + al(n_max * sizeof(Key3)));  // the second buffer
+    bucket_sort_kernel<<<nb, kBucketThreads, kBucketCap * sizeof(Key3), st>>>(keys, scratch, w.off, w.ucnt, n_max, error);
+    AFX_LAUNCH_CHECK();
+    small_scan_kernel<<<1, 1024, 0, st>>>(w.ucnt, nb, w.uoff, nullptr, count);
+    AFX_LAUNCH_CHECK();
+    bucket_compact_kernel<<<nb, kBucketThreads, 0, st>>>(keys, w.off, w.uoff, pts, n_max, error);
+    AFX_LAUNCH_CHECK();
+    return AFX_OK;
 }
 
 __global__ void translate_kernel(float* pts, const unsigned* count, long n_max, float tx, float ty, float tz) {
