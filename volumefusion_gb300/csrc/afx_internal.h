@@ -29,6 +29,23 @@ int scan_exclusive_dev(const unsigned* in, unsigned* out, const unsigned* count,
 int frame_prep_impl(const uint16_t* mm, int width, int height, const afx_prep_params* p, float* depth, float* vertices,
                     float* normals, float* centroid, unsigned long long* acc, int* error, cudaStream_t st,
                     const uint32_t* undistort_map = nullptr);
+// The rigid stream's frames: every camera's filtered depth and its points in world space (afx_prep.cu).
+struct StreamCamera {
+    const uint16_t* mm;
+    const uint32_t* umap;  // undistortion map (AFX_UNDISTORT_NEAREST), or null
+    float* depth;
+    float* cloud;
+    Intrinsics K;
+    float fxi, fyi;        // 1 / fx, 1 / fy
+    float T[16];           // camera to world, column-major
+};
+struct StreamPrep {
+    int width, height;
+    float depth_threshold;
+    int bilateral;
+    StreamCamera cam[AFX_MAX_CAMERAS];
+};
+int stream_prep_impl(const StreamPrep& A, int n_cameras, int r, double sigma_i, double sigma_s, float thr, cudaStream_t st);
 // afx_undistort_map / afx_undistort_depth (afx_undistort.cu)
 int undistort_map_impl(uint32_t* map, int width, int height, const float K[9], const afx_camera_distortion* d, int mode,
                        cudaStream_t st);
@@ -40,10 +57,10 @@ int undistort_apply_impl(float* dst, const float* src, int width, int height, co
 int integrate_rigid_impl(void* tsdf, void* weights, int fmt, const float* depth, int W, int H, float delta,
                          const Volume& vol, const float* R, const float* t, const float* K, cudaStream_t st,
                          const float* t_dev = nullptr, unsigned char* occ = nullptr);
-// initialise (-1, 0) + rigid integration in one write-only pass (FP32 volumes, X % 4 == 0, 16-byte
-// aligned arrays; AFX_ERR_UNSUPPORTED otherwise)
+// initialise (-1, 0) + rigid integration in one write-only pass; occ (optional): every byte of it is
+// written, 1 for bricks with a weighted voxel of positive value
 int integrate_fresh_impl(float* tsdf, float* weights, const float* depth, int W, int H, float delta, const Volume& vol,
-                         const float* R, const float* t, const float* K, cudaStream_t st);
+                         const float* R, const float* t, const float* K, cudaStream_t st, unsigned char* occ = nullptr);
 void rotation_inverse(const float* R, float* Rinv);
 
 // ---- marching cubes and sorting (afx_mc.cu) ----
@@ -58,8 +75,10 @@ int mc_fused_impl(const void* tsdf, const void* weights, int fmt, const Volume& 
                   unsigned* face_count, long face_cap, cudaStream_t st, int* error = nullptr, int tile = 0,
                   const unsigned char* occ = nullptr,   // occ: brick occupancy (tiles without an occupied
                                                         // brick hold no active cube and are skipped)
-                  unsigned* tile_ws = nullptr);         // mc_tile_ws_words(vol) words: with occ, the
+                  unsigned* tile_ws = nullptr,          // mc_tile_ws_words(vol) words: with occ, the
                                                         // persistent tiles walk a list of occupied tiles
+                  bool occ_positive = false);           // occ marks bricks with a value above iso (any corner
+                                                        // of a cube) instead of a weight (its origin corner)
 size_t mc_tile_ws_words(const Volume& vol);
 // marching-cubes tiles (the session's autotuner picks one): TMA bricks of 16, 8 or 32 cubes along z,
 // the sweep from global memory, or a persistent grid with two stages of bricks 8 or 16 deep

@@ -46,6 +46,7 @@ struct McArgs {
     int* faces;
     int* error;  // TMA path: set on a tile-load timeout
     const unsigned char* occ;  // brick occupancy (8^3 voxels), or null: process every tile
+    bool occ_positive;         // it marks values above iso, not weights
     int nbx, nby, nbz;
     unsigned* tile_count;      // persistent grid: occupied tiles listed here (with occ), or null
     unsigned* tile_list;
@@ -234,13 +235,15 @@ AFX_D void mc_emit(const TT* __restrict__ tsdf, const McArgs& a, int x, int y, i
 
 constexpr int kMcX = 32, kMcY = 8;  // cube columns of a TMA tile
 
-// False when no 8^3 brick holding a cube origin of the box [x0, x0+xr) x [y0, y0+yr) x [z0, z0+zr)
-// has a voxel with a weight.  A cube is active only if all eight corners have a weight, its origin
-// corner among them, so such a box has no active cube.  Every thread evaluates it (same answer).
+// False when no marked 8^3 brick holds a corner of the cubes [x0, x0+xr) x [y0, y0+yr) x [z0, z0+zr) that
+// an active cube has to have: bricks with a weight hold the origin corners (a cube is active only if
+// all eight corners have a weight), bricks with a value above iso any corner.  Every thread evaluates
+// it (same answer).
 AFX_D bool box_occupied(const McArgs& a, int x0, int xr, int y0, int yr, int z0, int zr) {
     if (!a.occ) return true;
-    const int bx1 = min((x0 + xr - 1) >> 3, a.nbx - 1), by1 = min((y0 + yr - 1) >> 3, a.nby - 1);
-    const int bz1 = min((z0 + zr - 1) >> 3, a.nbz - 1);
+    const int last = a.occ_positive ? 0 : 1;
+    const int bx1 = min((x0 + xr - last) >> 3, a.nbx - 1), by1 = min((y0 + yr - last) >> 3, a.nby - 1);
+    const int bz1 = min((z0 + zr - last) >> 3, a.nbz - 1);
     for (int bz = z0 >> 3; bz <= bz1; ++bz)
         for (int by = y0 >> 3; by <= by1; ++by)
             for (int bx = x0 >> 3; bx <= bx1; ++bx)
@@ -764,7 +767,7 @@ static void mc_launch_any(const TT* tsdf, const WT* weights, const McArgs& a, co
 int mc_fused_impl(const void* tsdf, const void* weights, int fmt, const Volume& vol, float iso, float* points,
                   unsigned* point_count, long point_cap, float* verts, unsigned* vert_count, long vert_cap, int* faces,
                   unsigned* face_count, long face_cap, cudaStream_t st, int* error, int tile,
-                  const unsigned char* occ, unsigned* tile_ws) {
+                  const unsigned char* occ, unsigned* tile_ws, bool occ_positive) {
     int rc = upload_tables();
     if (rc) return rc;
     McArgs a;
@@ -780,6 +783,7 @@ int mc_fused_impl(const void* tsdf, const void* weights, int fmt, const Volume& 
     a.faces = faces;
     a.error = error;
     a.occ = occ;
+    a.occ_positive = occ_positive;
     a.tile_count = tile_ws;
     a.tile_list = tile_ws ? tile_ws + 1 : nullptr;
     a.nbx = (vol.dims[0] + 7) / 8;

@@ -11,6 +11,7 @@
 
 #include "afx_common.cuh"
 #include "afx_host.h"
+#include "afx_internal.h"
 #include "afx_tma.h"
 #include "afx_undistort.cuh"
 
@@ -343,6 +344,48 @@ __global__ void __launch_bounds__(kTW * kTH) prep_kernel(const __grid_constant__
     }
 }
 
+// The rigid stream's frame of every camera in one launch (blockIdx.z: camera): metres and range filter --
+// or, for a distorted camera, the unfiltered metres remapped to the nearest pixel -- into shared memory
+// with a halo, the bilateral filter, back-projection and the camera-to-world transform
+// (CameraData::processNextFrame, src/MeshRecontructionStream.cu:88-112).  The arithmetic is that of the
+// separate kernels below.  Bound: latency and issue of the filter; three cameras of 640 x 576 with
+// a 5 x 5 filter: 16 us, where five launches per camera took 24 us each.
+__global__ void __launch_bounds__(kTW * kTH) stream_prep_kernel(const __grid_constant__ StreamPrep A,
+                                                                const __grid_constant__ BilateralTables tab) {
+    __shared__ float dep[(kTH + 2 * kMaxBilateralR) * (kTW + 2 * kMaxBilateralR)];
+    const StreamCamera& cam = A.cam[blockIdx.z];
+    const int W = A.width, H = A.height, r = tab.r;
+    const int tid = threadIdx.y * kTW + threadIdx.x;
+    const int inW = kTW + 2 * r, inH = kTH + 2 * r;
+    const int gx0 = blockIdx.x * kTW - r, gy0 = blockIdx.y * kTH - r;
+    const uint16_t* __restrict__ mm = cam.mm;
+    for (int i = tid; i < inW * inH; i += kTW * kTH) {
+        const int gx = gx0 + i % inW, gy = gy0 + i / inW;
+        if (gx < 0 || gx >= W || gy < 0 || gy >= H) continue;  // the filter clamps to the image
+        const long p = (long)gy * W + gx;
+        auto metres = [&](int x, int y) { return (float)mm[(long)y * W + x] * 0.001f; };
+        dep[i] = cam.umap ? remap_nearest_at(cam.umap[2 * p], W, H, metres) : filter_value(metres(gx, gy), A.depth_threshold);
+    }
+    __syncthreads();
+    const int x = blockIdx.x * kTW + threadIdx.x, y = blockIdx.y * kTH + threadIdx.y;
+    if (x >= W || y >= H) return;
+    auto at = [&](int xx, int yy) -> float { return dep[(yy - gy0) * inW + (xx - gx0)]; };
+    const float d = A.bilateral ? bilateral_at(x, y, W, H, tab, at) : at(x, y);
+    const long p = (long)y * W + x;
+    cam.depth[p] = d;
+    float v[3] = {0.f, 0.f, 0.f}, o[3];
+    if (!(isinf(d) || d < 1.e-4f)) {
+        const float xr = ((float)x - cam.K.cx) * cam.fxi, yr = ((float)y - cam.K.cy) * cam.fyi;
+        v[0] = xr * d;
+        v[1] = yr * d;
+        v[2] = d;
+    }
+    mat4_point(cam.T, v, o);  // transformKernel (src/VertexManipulation.cu:89-95)
+    cam.cloud[3 * p] = o[0];
+    cam.cloud[3 * p + 1] = o[1];
+    cam.cloud[3 * p + 2] = o[2];
+}
+
 __global__ void centroid_finalize_kernel(unsigned long long* acc, float* centroid) {
     long long cnt = (long long)acc[3];
     for (int c = 0; c < 3; ++c) {
@@ -521,6 +564,16 @@ int frame_prep_impl(const uint16_t* mm, int width, int height, const afx_prep_pa
         centroid_finalize_kernel<<<1, 1, 0, st>>>(acc, centroid);
         AFX_LAUNCH_CHECK();
     }
+    return AFX_OK;
+}
+
+int stream_prep_impl(const StreamPrep& A, int n_cameras, int r, double sigma_i, double sigma_s, float thr, cudaStream_t st) {
+    if (A.bilateral && (r < 0 || r > kMaxBilateralR)) return AFX_ERR_UNSUPPORTED;
+    BilateralTables tab;
+    make_bilateral_tables(A.bilateral ? r : 0, sigma_i, sigma_s, thr, &tab);
+    const dim3 grid((A.width + kTW - 1) / kTW, (A.height + kTH - 1) / kTH, n_cameras), block(kTW, kTH);
+    stream_prep_kernel<<<grid, block, 0, st>>>(A, tab);
+    AFX_LAUNCH_CHECK();
     return AFX_OK;
 }
 

@@ -15,33 +15,6 @@
 
 #include "afx_internal.h"
 
-namespace afx {
-
-struct Mat4 {
-    float m[16];  // column-major
-};
-
-// transformKernel (src/VertexManipulation.cu:89-95): p <- (T * [p; 1]).head(3), in place
-__global__ void transform_points_kernel(float* pts, long n, Mat4 T) {
-    AFX_GRID_STRIDE(i, n) {
-        float p[3] = {pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]}, q[3];
-        mat4_point(T.m, p, q);
-        pts[3 * i] = q[0];
-        pts[3 * i + 1] = q[1];
-        pts[3 * i + 2] = q[2];
-    }
-}
-
-__global__ void stream_init_kernel(float* tsdf, float* weights, long S, unsigned* counts) {
-    if (blockIdx.x == 0 && threadIdx.x < 2) counts[threadIdx.x] = 0;
-    AFX_GRID_STRIDE(i, S) {
-        tsdf[i] = -1.f;
-        weights[i] = 0.f;
-    }
-}
-
-}  // namespace afx
-
 using namespace afx;
 
 struct afx_rigid_stream {
@@ -50,7 +23,6 @@ struct afx_rigid_stream {
     long S = 0, P = 0;
     void* arena = nullptr;
     float* depth;    // [n_cameras * P], the filtered depth of each camera
-    float* scratch;  // [P], bilateral input
     float* cloud;    // [n_cameras * P * 3]
     float* tsdf;
     float* weights;
@@ -58,7 +30,8 @@ struct afx_rigid_stream {
     int* faces;      // [triangle_capacity * 3]
     unsigned* counts;  // faces, vertices
     int* error;
-    float* raw;        // [P], a distorted camera's unfiltered metres
+    unsigned char* occ;   // per 8^3 brick of the volume: 1 where this frame left a positive value
+    unsigned* mc_tiles;   // marching cubes: count + occupied tiles
     uint32_t* umap;    // [n_cameras * P * 2], undistortion maps of the distorted cameras
 };
 
@@ -106,8 +79,9 @@ int afx_rigid_stream_create(const afx_rigid_stream_params* params, afx_rigid_str
     const size_t nc = (size_t)p.n_cameras, P = (size_t)s->P, S = (size_t)s->S, T = (size_t)p.triangle_capacity;
     bool distorted = false;
     for (int c = 0; c < p.n_cameras; ++c) distorted = distorted || p.distortion[c].is_distorted;
-    const size_t sizes[] = {nc * P * 4, P * 4, nc * P * 12, S * 4, S * 4, T * 36, T * 12, 64, 64,
-                            distorted ? P * 4 : 0, distorted ? nc * P * 8 : 0};
+    const size_t bricks = (size_t)((p.dims[0] + 7) / 8) * ((p.dims[1] + 7) / 8) * ((p.dims[2] + 7) / 8);
+    const size_t sizes[] = {nc * P * 4, nc * P * 12, S * 4, S * 4, T * 36, T * 12, 64, 64,
+                            bricks, mc_tile_ws_words(s->vol) * 4, distorted ? nc * P * 8 : 0};
     constexpr int kBuffers = (int)(sizeof(sizes) / sizeof(sizes[0]));
     size_t total = 0;
     for (size_t x : sizes) total += al(x);
@@ -124,15 +98,15 @@ int afx_rigid_stream_create(const afx_rigid_stream_params* params, afx_rigid_str
         q += al(sizes[i]);
     }
     s->depth = (float*)ptr[0];
-    s->scratch = (float*)ptr[1];
-    s->cloud = (float*)ptr[2];
-    s->tsdf = (float*)ptr[3];
-    s->weights = (float*)ptr[4];
-    s->verts = (float*)ptr[5];
-    s->faces = (int*)ptr[6];
-    s->counts = (unsigned*)ptr[7];
-    s->error = (int*)ptr[8];
-    s->raw = distorted ? (float*)ptr[9] : nullptr;
+    s->cloud = (float*)ptr[1];
+    s->tsdf = (float*)ptr[2];
+    s->weights = (float*)ptr[3];
+    s->verts = (float*)ptr[4];
+    s->faces = (int*)ptr[5];
+    s->counts = (unsigned*)ptr[6];
+    s->error = (int*)ptr[7];
+    s->occ = (unsigned char*)ptr[8];
+    s->mc_tiles = (unsigned*)ptr[9];
     s->umap = distorted ? (uint32_t*)ptr[10] : nullptr;
     e = cudaMemset(s->arena, 0, total);
     // each distorted camera's cv::initUndistortRectifyMap(CV_32FC1) map, built once
@@ -172,44 +146,35 @@ int afx_rigid_stream_process(afx_rigid_stream* s, const uint16_t* const* depth_m
         if (!depth_mm[c]) return AFX_ERR_INVALID_ARGUMENT;
     cudaStream_t st = as_stream(stream);
     const long P = s->P;
+    StreamPrep A;
+    A.width = p.width;
+    A.height = p.height;
+    A.depth_threshold = p.depth_threshold;
+    A.bilateral = p.bilateral;
     for (int c = 0; c < p.n_cameras; ++c) {
-        float* d = s->depth + c * P;
-        float* in = p.bilateral ? s->scratch : d;
-        int rc;
-        if (p.distortion[c].is_distorted) {
-            // the filtered device frame is overwritten by the host frame's undistortion: the unfiltered
-            // metres remapped (src/MeshRecontructionStream.cu:91-101)
-            rc = afx_depth_from_mm(s->raw, depth_mm[c], P, st);
-            if (!rc) rc = undistort_apply_impl(in, s->raw, p.width, p.height, s->umap + (size_t)c * P * 2,
-                                               AFX_UNDISTORT_NEAREST, st);
-        } else {
-            rc = afx_depth_from_mm(in, depth_mm[c], P, st);
-            if (!rc) rc = afx_filter_depth(in, P, p.depth_threshold, st);
-        }
-        if (!rc && p.bilateral)
-            rc = afx_bilateral_filter(d, in, p.height, p.width, p.bilateral_r, p.sigma_i, p.sigma_s, p.bilateral_thr, st);
-        float* cloud = s->cloud + 3 * c * P;
-        if (!rc) rc = afx_depth_to_mesh(cloud, d, p.width, p.height, p.K[c], st);
-        if (rc) return rc;
-        Mat4 T;
-        std::memcpy(T.m, p.camera_to_world[c], sizeof(T.m));
-        transform_points_kernel<<<grid_for(P, 256), 256, 0, st>>>(cloud, P, T);
-        AFX_LAUNCH_CHECK();
+        StreamCamera& cam = A.cam[c];
+        cam.mm = depth_mm[c];
+        // a distorted camera's filtered frame is overwritten by the undistortion of the unfiltered metres
+        // (src/MeshRecontructionStream.cu:91-101)
+        cam.umap = p.distortion[c].is_distorted ? s->umap + (size_t)c * P * 2 : nullptr;
+        cam.depth = s->depth + c * P;
+        cam.cloud = s->cloud + 3 * c * P;
+        cam.K = make_intrinsics(p.K[c]);
+        cam.fxi = 1.0f / p.K[c][0];
+        cam.fyi = 1.0f / p.K[c][4];
+        std::memcpy(cam.T, p.camera_to_world[c], sizeof(cam.T));
     }
-    // DeviceTsdf::initDefault + integrate(cameras[0]): one write-only pass where the layout allows
+    int rc = stream_prep_impl(A, p.n_cameras, p.bilateral_r, p.sigma_i, p.sigma_s, p.bilateral_thr, st);
+    if (rc) return rc;
+    // DeviceTsdf::initDefault + integrate(cameras[0]) in one write-only pass, which also says which bricks
+    // marching cubes has to look at
     AFX_CUDA(cudaMemsetAsync(s->counts, 0, 8, st));
-    int rc = integrate_fresh_impl(s->tsdf, s->weights, s->depth, p.width, p.height, p.delta, s->vol, p.rotation,
-                                  p.center, p.K[0], st);
-    if (rc == AFX_ERR_UNSUPPORTED) {
-        stream_init_kernel<<<grid_for(s->S, 256), 256, 0, st>>>(s->tsdf, s->weights, s->S, s->counts);
-        AFX_LAUNCH_CHECK();
-        rc = integrate_rigid_impl(s->tsdf, s->weights, kVoxF32, s->depth, p.width, p.height, p.delta, s->vol,
-                                  p.rotation, p.center, p.K[0], st);
-    }
+    rc = integrate_fresh_impl(s->tsdf, s->weights, s->depth, p.width, p.height, p.delta, s->vol, p.rotation,
+                              p.center, p.K[0], st, s->occ);
     if (rc) return rc;
     const long T = p.triangle_capacity;
     rc = mc_fused_impl(s->tsdf, s->weights, kVoxF32, s->vol, 0.f, nullptr, nullptr, 0, s->verts, s->counts + 1, T * 3,
-                       s->faces, s->counts, T, st, s->error);
+                       s->faces, s->counts, T, st, s->error, kMcTilePipe4, s->occ, s->mc_tiles, true);
     return rc;
 }
 
