@@ -11,8 +11,8 @@
 // Diagonal blocks without any contribution keep the identity (runInitIdentityKernel).
 // J^T J depends only on the canonical geometry, weights and correspondences, so it is
 // assembled once per ICP iteration; J^T r is rebuilt every Gauss-Newton iteration.
-// The solve is a block-Jacobi PCG in one cooperative kernel: FP32 block SpMV, dot products in
-// double-binary32 (shared-memory path) or FP64 (global-memory path), FP64 6x6 block inverses.
+// The solve is a block-Jacobi PCG in one kernel on one cluster: FP32 block SpMV, dot products in
+// triple- (shared-memory path) or double-binary32 (global-memory path), FP64 6x6 block inverses.
 #include <cfloat>
 #include <cstring>
 #include <new>
@@ -528,7 +528,8 @@ __global__ void __launch_bounds__(128) diag_inverse_kernel(GnArgs a) {
 // are stored with st.global.cg and loaded with ld.global.cg, i.e. always from L2.
 // Per iteration:
 //   residuals + energies -> energy test and commit -> J^T r -> PCG (x = 0, block-Jacobi,
-//   FP32 block SpMV, double-float or FP64 dots, two cluster barriers per PCG iteration)
+//   FP32 block SpMV; two exchanges through shared memory per PCG iteration, or three cluster barriers
+//   where the vectors are in global memory)
 //   -> T_pending -= [[x_rot]x, x_t; 0] -> re-warp the canonical vertices with T_pending.
 
 constexpr int kLoopThreads = 512;
@@ -594,6 +595,39 @@ AFX_D DF df_prod(float x, float y) {
     return {p, fmaf(x, y, -p)};
 }
 
+// A sum under way: hi is the running binary32 sum, lo the running sum of its exact rounding errors and c
+// that of lo's.  Adding two of them waits for one addition on hi and two on lo; the error terms follow
+// behind, so a butterfly step costs a shuffle and two additions instead of a double-float addition's
+// thirteen, and the result carries more bits (errors of the PCG's dot products against exact sums, over
+// 12 to 384 terms per CTA and 16 CTAs, relative to the sum of |x y|: about a third of a double-float's; with
+// 66 terms at most 1.8e-15 and 3.2e-16 on average, against 4.7e-15 and 9.5e-16).
+struct TF {
+    float hi, lo, c;
+};
+
+AFX_D TF tf_add(TF a, TF b) {
+    const DF h = two_sum(a.hi, b.hi), l = two_sum(a.lo, b.lo), m = two_sum(l.hi, h.lo);
+    return {h.hi, m.hi, (a.c + b.c) + (l.lo + m.lo)};
+}
+
+AFX_D TF tf_add_prod(TF a, float x, float y) {
+    const float p = x * y;
+    return tf_add(a, {p, fmaf(x, y, -p), 0.f});
+}
+
+// Sum over the lanes that differ in bits kFrom, kFrom / 2, ..., 1 of their number, as a double-float.
+template <int kFrom>
+AFX_D DF tf_butterfly(TF v) {
+#pragma unroll
+    for (int o = kFrom; o > 0; o >>= 1) {
+        const TF u = {__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o),
+                      __shfl_xor_sync(0xffffffffu, v.c, o)};
+        v = tf_add(v, u);
+    }
+    const DF s = fast_two_sum(v.hi, v.lo);
+    return fast_two_sum(s.hi, s.lo + v.c);
+}
+
 AFX_D DF df_shfl_xor(DF v, int o) {
     return {__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
 }
@@ -614,50 +648,7 @@ struct ClusterSums {
     double warp[kLoopWarps * 4];  // per-warp sums
     double total[4];
     int phase;
-    // PCG scalars, written by lane 0 of warp 0 and read by every thread after a __syncthreads
-    DF rz_df, bn_df;  // r.z of the current iterate, b.b (shared-memory path)
-    float alpha, beta;
-    int stop;
 };
-
-// Sums v[0..NV) over every thread of the cluster; all threads of all CTAs get identical totals.
-// Fixed-shape FP64 trees: butterfly within each warp, then over the CTA's warps, then over the
-// CTAs by rank.  Contains one cluster barrier.
-template <int NV>
-AFX_D void cluster_sum(double (&v)[NV], ClusterSums& cs) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-        double s = warp_sum(v[i]);
-        if (lane == 0) cs.warp[w * 4 + i] = s;
-    }
-    __syncthreads();
-    const int ph = cs.phase;
-    if (w == 0) {
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            double s = lane < kLoopWarps ? cs.warp[lane * 4 + i] : 0.0;
-#pragma unroll
-            for (int o = kLoopWarps / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) cs.slot[ph][i] = s;
-        }
-    }
-    cluster_barrier();
-    if (w == 0) {
-        const unsigned ncta = cluster_size();
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            double t = lane < (int)ncta ? dsmem_load(&cs.slot[ph][i], lane) : 0.0;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-            if (lane == 0) cs.total[i] = t;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < NV; ++i) v[i] = cs.total[i];
-    if (threadIdx.x == 0) cs.phase = ph ^ 1;
-}
 
 // Double-floats in this CTA's shared memory and in CTA `rank`'s (8-byte slots, hi first).
 AFX_D void sts_df(double* local, DF v) {
@@ -678,7 +669,7 @@ AFX_D DF dsmem_load_df(const double* p, unsigned rank) {
     return v;
 }
 
-// cluster_sum in double-float arithmetic: the same fixed-shape trees (warp butterfly, the CTA's
+// The like in double-float arithmetic: the same fixed-shape trees (warp butterfly, the CTA's
 // warps, the CTAs by rank) with df_add, so every thread of every CTA gets identical totals.
 // Contains one cluster barrier.
 template <int NV>
@@ -721,6 +712,39 @@ AFX_D void cluster_sum_df(DF (&v)[NV], ClusterSums& cs) {
     if (threadIdx.x == 0) cs.phase = ph ^ 1;
 }
 
+// Sums v[0] and v[1] over every thread of the cluster; all threads of all CTAs get identical totals.
+// Fixed-shape FP64 trees: butterfly within each warp, then over the CTA's warps, then over the
+// CTAs by rank.  FP64 additions issue at one warp in about 20 cycles per SM, so a step of the trees adds
+// both values, one in each half of the warp.  Contains one cluster barrier.
+AFX_D void cluster_sum_pair(double (&v)[2], ClusterSums& cs) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    static_assert(kLoopWarps == 16, "half a warp per value");
+    auto half_sum = [](double s) {  // over the 16 lanes of each half
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        return s;
+    };
+    const int k = lane >> 4, q = lane & 15;  // value and item of this lane
+    const double give = k ? v[0] : v[1], got = __shfl_xor_sync(0xffffffffu, give, 16);
+    const double s = half_sum((k ? v[1] : v[0]) + got);
+    if (q == 0) cs.warp[w * 4 + k] = s;
+    __syncthreads();
+    const int ph = cs.phase;
+    if (w == 0) {
+        const double t = half_sum(cs.warp[q * 4 + k]);
+        if (q == 0) cs.slot[ph][k] = t;
+    }
+    cluster_barrier();
+    if (w == 0) {
+        const double t = half_sum(q < (int)cluster_size() ? dsmem_load(&cs.slot[ph][k], q) : 0.0);
+        if (q == 0) cs.total[k] = t;
+    }
+    __syncthreads();
+    v[0] = cs.total[0];
+    v[1] = cs.total[1];
+    if (threadIdx.x == 0) cs.phase = ph ^ 1;
+}
+
 struct LoopArgs {
     GnArgs g;
     const float* points;  // canonical vertices
@@ -740,14 +764,22 @@ AFX_D void jtr_node(const GnArgs& a, int node, int n, float (&acc)[6]) {
 #pragma unroll
     for (int q = 0; q < 6; ++q) acc[q] = 0.f;
     const unsigned o = a.b.loff[node], e = a.b.loff[node + 1];
-#pragma unroll 4
-    for (unsigned t = o + lane; t < e; t += 32) {
-        const int c = a.b.jc[t];
-        if (c < 0) continue;
-        const float rd = __ldcg(a.b.rdepth + c);
-        const float* J = a.b.jrow + (long)t * 6;
+    constexpr int kAhead = 8;  // entries whose loads are in flight together
+    for (unsigned t0 = o + lane; t0 < e; t0 += 32 * kAhead) {
+        int c[kAhead];
+        float J[kAhead][6], rd[kAhead];
 #pragma unroll
-        for (int q = 0; q < 6; ++q) acc[q] = acc[q] + J[q] * rd;
+        for (int k = 0; k < kAhead; ++k) c[k] = t0 + 32 * k < e ? a.b.jc[t0 + 32 * k] : -1;
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+#pragma unroll
+            for (int q = 0; q < 6; ++q) J[k][q] = t0 + 32 * k < e ? a.b.jrow[(long)(t0 + 32 * k) * 6 + q] : 0.f;
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) rd[k] = c[k] >= 0 ? __ldcg(a.b.rdepth + c[k]) : 0.f;
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+#pragma unroll
+            for (int q = 0; q < 6; ++q) acc[q] = c[k] >= 0 ? acc[q] + J[k][q] * rd[k] : acc[q];
     }
     const unsigned io = a.b.ioff[node], nin = a.b.ioff[node + 1] - io;
     for (unsigned u = lane; u < nin + (unsigned)a.kreg; u += 32) {
@@ -816,9 +848,9 @@ AFX_D float spmv_entry(const GnBuffers& b, int node, int i, const float* z) {
 // and keeps, in its shared memory, the rows of J^T J for its nodes (diagonal block, then the
 // neighbour blocks in ascending neighbour order, lower ones stored transposed so every block
 // is row-major B_ij), their block inverses, its slices of x, r, p, A p, and a full copy of z.
-// After each update a CTA writes its new z slice into every CTA's copy (st.shared::cluster), so
+// After each update a CTA writes its new z slice into every CTA's copy (st.async), so
 // the SpMV reads only local shared memory.  Partial sums are written into every CTA's slot
-// array and summed locally in rank order after the cluster barrier: identical totals in all
+// array the same way and summed locally in one fixed order: identical totals in all
 // CTAs.  J^T J does not change during the Gauss-Newton loop, so the rows are staged once.
 
 constexpr int kDsNodes = 1024;   // node limit of this path (full z copy)
@@ -838,16 +870,20 @@ struct DsLayout {
     int* rowptr;    // [kDsNpc + 1]
     double* slot;   // [2][kDsMaxCta][4]
     int* misc;      // [4]
+    unsigned long long* bar;  // [2] mbarriers: p.Ap exchange, r.z exchange
+    float* scal;    // [2] beta, stop
 };
 
 constexpr size_t kDsSmem = sizeof(float) * ((size_t)kDsNodes * 12 + 3 * kDsNpc * 6 + kDsNpc * 36 + (size_t)kDsBlocks * 36) +
-                           sizeof(int) * (kDsBlocks + kDsNpc + 1 + 4) + sizeof(double) * 2 * kDsMaxCta * 4 + 64;
+                           sizeof(int) * (kDsBlocks + kDsNpc + 1 + 4) + sizeof(double) * (2 * kDsMaxCta * 4 + 4) + 64;
 
 AFX_D DsLayout ds_layout(void* base) {
     DsLayout d;
     double* dp = static_cast<double*>(base);
     d.slot = dp;
-    float* f = reinterpret_cast<float*>(dp + 2 * kDsMaxCta * 4);
+    d.bar = reinterpret_cast<unsigned long long*>(dp + 2 * kDsMaxCta * 4);
+    d.scal = reinterpret_cast<float*>(dp + 2 * kDsMaxCta * 4 + 2);
+    float* f = reinterpret_cast<float*>(dp + 2 * kDsMaxCta * 4 + 4);  // 16-byte aligned
     d.z = f;
     f += kDsNodes * 6;
     d.pf = f;
@@ -872,23 +908,62 @@ AFX_D DsLayout ds_layout(void* base) {
 }
 
 // Store to the same shared-memory offset in CTA `rank` of this cluster.
-AFX_D void dsmem_store_f32(float* local, unsigned rank, float v) {
-    unsigned a = (unsigned)__cvta_generic_to_shared(local), ra;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(ra), "f"(v) : "memory");
-}
 AFX_D void dsmem_store_f64(double* local, unsigned rank, double v) {
     unsigned a = (unsigned)__cvta_generic_to_shared(local), ra;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
     asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(ra), "d"(v) : "memory");
 }
-// A double-float into an 8-byte slot of CTA `rank` (hi at the lower address).
-AFX_D void dsmem_store_df(double* local, unsigned rank, DF v) {
+// Asynchronous stores to the same shared-memory offset in CTA `rank` of this cluster, counted on that
+// CTA's mbarrier: the receiver waits for the bytes it expects, so an exchange costs one trip
+// through the cluster's network instead of a store, its acknowledgement and a cluster barrier
+// (16 CTAs of 512 threads: 1,165 cycles that way; here the wait after a CTA's own last store is 230 to 310).
+AFX_D unsigned cluster_addr(const void* local, unsigned rank) {
     unsigned a = (unsigned)__cvta_generic_to_shared(local), ra;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
-    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(ra), "f"(v.hi), "f"(v.lo) : "memory");
+    return ra;
+}
+AFX_D void async_store_df(unsigned addr, unsigned bar, DF v) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(addr),
+                 "f"(v.hi), "f"(v.lo), "r"(bar)
+                 : "memory");
 }
 
+// The two exchanges of a PCG iteration.  Phases alternate: a CTA sends its part of an exchange only
+// after it has received the other one of the step before from every CTA, that is after every CTA has
+// read what this one overwrites.
+struct DsExchange {
+    unsigned parity[2];  // phase of each mbarrier that the next wait is for
+    bool dead;           // a wait ran out (the error is flagged): no further sends or waits
+};
+
+// Before the cluster barrier at the start of the kernel (one thread).
+AFX_D void ds_exchange_init(const DsLayout& d) {
+    for (int i = 0; i < 2; ++i)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(d.bar + i)) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+
+// Expect `bytes` on mbarrier i in its current phase (one thread).
+AFX_D void ds_expect(const DsLayout& d, int i, unsigned bytes) {
+    const unsigned bar = (unsigned)__cvta_generic_to_shared(d.bar + i);
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+
+// Wait (bounded) for the current phase of mbarrier i; every thread, the same number of times.
+AFX_D void ds_wait(const DsLayout& d, int i, DsExchange& x, int* error) {
+    const unsigned bar = (unsigned)__cvta_generic_to_shared(d.bar + i);
+    unsigned ok = 0;
+    for (int it = 0; it < (1 << 20) && !ok; ++it)
+        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                     : "=r"(ok)
+                     : "r"(bar), "r"(x.parity[i])
+                     : "memory");
+    x.parity[i] ^= 1u;
+    if (!ok) {
+        x.dead = true;
+        if (error) atomicOr(error, ERRF_TIMEOUT);
+    }
+}
 
 // Cluster sum through the slot arrays: the CTA's block total is written into slot[ph][rank] of
 // every CTA; after the barrier each CTA adds the slots in rank order.
@@ -981,51 +1056,67 @@ AFX_D bool ds_stage(const GnBuffers& b, int n, const DsLayout& d, ClusterSums& c
     return true;
 }
 
-// Dot products x[i] . y[i] of the CTA's own entries (cnt floats each, in shared memory), summed
-// over the cluster in double-float arithmetic (about 48 bits; each product enters exactly).  Warp 0
-// alone does the work: lane l accumulates entries l, l + 32, ..., a butterfly gives the CTA's sum,
-// and lane q sends it into slot [ph][rank] of CTA q.  After the cluster barrier warp 0 of every CTA
-// adds the slots in one fixed tree, so all CTAs hold bit-identical totals.  Returns true in lane 0
-// of warp 0 only, with the totals in t; the caller turns them into the scalars every thread reads
-// after the next __syncthreads.
+// Dot products x[i] . y[i] of the CTA's own entries (cnt floats each, in shared memory), summed over the
+// cluster (each product enters exactly; a CTA's sum travels as a double-float, 48 bits).  Warp 0 sends:
+// lane l accumulates entries l, l + 32, ..., a butterfly gives the CTA's sum, and lane q puts it
+// into slot [i][rank] of CTA q (i: the exchange, 0 for p.Ap, 1 for r.z).
 template <int NV>
-AFX_D bool ds_dot(const float* const (&x)[NV], const float* const (&y)[NV], int cnt, const DsLayout& d, int& ph,
-                  DF (&t)[NV]) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+AFX_D void ds_dot_send(const float* const (&x)[NV], const float* const (&y)[NV], int cnt, const DsLayout& d, int i) {
+    const int lane = threadIdx.x & 31;
     const unsigned rank = cluster_rank(), ncta = cluster_size();
-    __syncthreads();  // the staged vectors are complete
-    if (w == 0) {
+    const unsigned bar = cluster_addr(d.bar + i, lane < (int)ncta ? lane : 0);
 #pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            DF s = {0.f, 0.f};
-            for (int o = lane; o < cnt; o += 32) s = df_add(s, df_prod(x[i][o], y[i][o]));
+    for (int k = 0; k < NV; ++k) {
+        TF v = {0.f, 0.f, 0.f};
+        constexpr int kAhead = 4;  // terms loaded together
+        for (int o0 = lane; o0 < cnt; o0 += 32 * kAhead) {
+            float xs[kAhead], ys[kAhead];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s = df_add(s, df_shfl_xor(s, o));
-            if (lane < (int)ncta) dsmem_store_df(d.slot + (ph * kDsMaxCta + rank) * 4 + i, lane, s);
+            for (int q = 0; q < kAhead; ++q) {
+                const int o = o0 + 32 * q;
+                xs[q] = o < cnt ? x[k][o] : 0.f;
+                ys[q] = o < cnt ? y[k][o] : 0.f;
+            }
+#pragma unroll
+            for (int q = 0; q < kAhead; ++q)
+                if (q == 0 || o0 - lane + 32 * q < cnt) v = tf_add_prod(v, xs[q], ys[q]);  // a zero product adds nothing
         }
+        const DF s = tf_butterfly<16>(v);
+        if (lane < (int)ncta) async_store_df(cluster_addr(d.slot + (i * kDsMaxCta + rank) * 4 + k, lane), bar, s);
     }
-    cluster_barrier();
-    const int p = ph;
-    ph ^= 1;
-    if (w != 0) return false;
+}
+
+// The totals of exchange i, in every lane of every warp: the slots in one fixed tree, so all CTAs hold the
+// same bits.
+template <int NV>
+AFX_D void ds_dot_total(const DsLayout& d, int i, DF (&t)[NV]) {
+    const int lane = threadIdx.x & 31;
+    const unsigned ncta = cluster_size();
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
+    for (int k = 0; k < NV; ++k) {
+        // lanes 16 .. 31 hold the same slots again, so every lane ends with the total
+        const int q = lane & (kDsMaxCta - 1);
         DF v = {0.f, 0.f};
-        if (lane < (int)ncta) v = lds_df_local(d.slot + (p * kDsMaxCta + lane) * 4 + i);
-#pragma unroll
-        for (int o = kDsMaxCta / 2; o > 0; o >>= 1) v = df_add(v, df_shfl_xor(v, o));
-        t[i] = v;
+        if (q < (int)ncta) v = lds_df_local(d.slot + (i * kDsMaxCta + q) * 4 + k);
+        t[k] = tf_butterfly<kDsMaxCta / 2>({v.hi, v.lo, 0.f});
     }
-    return lane == 0;
 }
 
 // One PCG solve (same recurrences as the global-memory path), then T_pending -= [x] for the own
 // nodes.  J^T r is read from b.jtr.  Per iteration: p = z + beta p over all nodes (each CTA keeps a
 // full copy of p and of z), A p of the own rows with up to 32 lanes per row (each summing a fixed
-// stride of the row's blocks, then a butterfly), p.Ap (cluster dot), the own x / r / z updates with
-// z sent to every CTA's copy, r.z (and r.r when a tolerance is set; cluster dot).  The step sizes
-// are formed once per CTA by lane 0 (df_quotient) and read from shared memory.
-AFX_D void pcg_ds(const LoopArgs& L, int n, const DsLayout& d, ClusterSums& cs, int& ph) {
+// stride of the row's blocks, then a butterfly), p.Ap (exchange 0), the own x / r / z updates, and z to
+// every CTA's copy -- one warp per destination -- while warp 0 sums r.z (and r.r when a tolerance is
+// set; exchange 1).  A thread keeps its share of its row (up to kRegBlocks blocks), and its entry of x,
+// r and the inverse, in registers for the whole solve.
+// Bound: the chain of those steps, CTA barriers and two exchanges, about 6,000 cycles an iteration with 169 nodes
+// on 16 CTAs (A p 750, the two sums with their sending 2,700, updates 700, waits 550).  gn_loop_kernel in
+// the 256^3 sequence (169 nodes): 305 us with cluster barriers, double-float sums and the matrix rows read from
+// shared memory in each iteration, 267 us so.
+constexpr int kRegBlocks = 6;
+
+template <bool kTol>
+AFX_D void pcg_ds(const LoopArgs& L, int n, const DsLayout& d, DsExchange& ex) {
     const GnBuffers& b = L.g.b;
     const unsigned rank = cluster_rank(), ncta = cluster_size();
     const int npc = (n + (int)ncta - 1) / (int)ncta;
@@ -1035,123 +1126,150 @@ AFX_D void pcg_ds(const LoopArgs& L, int n, const DsLayout& d, ClusterSums& cs, 
     const int li = w * 5 + grp;  // kLoopWarps * 5 >= kDsNpc: one own node per lane group
     const bool act = lane < 30 && li < own;
     const int o = li * 6 + ei;
-    const int gnode = start + li;
     const int cnt = own * 6;
-    const bool tol = L.tol > 0;
+    constexpr int NV = kTol ? 2 : 1;
     float* zown = d.z + (long)start * 6;
     float* pown = d.pf + (long)start * 6;
-    // SpMV lanes per row: the largest power of two with every own row covered in one pass
+    // what arrives: every CTA's sums, and for exchange 1 every other CTA's z
+    const unsigned dot_bytes = ncta * 8u, rz_bytes = ncta * 8u * NV + (unsigned)(n - own) * 24u;
+    // SpMV lanes per row: the largest power of two with every own row covered at once
     int R = 1;
     while (R < 32 && 2 * R * cnt <= (int)blockDim.x) R <<= 1;
-    // x = 0, r = b, z = M^-1 r
-    {
-        const float ji = act ? __ldcg(b.jtr + (long)gnode * 6 + ei) : 0.f;
+    static_assert(kDsNpc * 6 <= kLoopThreads, "a thread per row");
+    const int row = (int)threadIdx.x / R, part = (int)threadIdx.x % R;
+    const int re = row % 6;  // row within its block
+    int b0 = 0, b1 = 0;
+    if (row < cnt) {
+        b0 = d.rowptr[row / 6] + part;
+        b1 = d.rowptr[row / 6 + 1];
+    }
+    float A[kRegBlocks][6];
+    int col[kRegBlocks];
+#pragma unroll
+    for (int k = 0; k < kRegBlocks; ++k) {
+        const int bk = b0 + k * R;
+        col[k] = bk < b1 ? d.col[bk] * 3 : 0;  // in float2
+#pragma unroll
+        for (int j = 0; j < 6; ++j) A[k][j] = bk < b1 ? d.blk[bk * 36 + re * 6 + j] : 0.f;
+    }
+    auto row_times = [&](const float (&B)[6], int c) {
+        const float2* xv = reinterpret_cast<const float2*>(d.pf) + c;
+        const float2 x0 = xv[0], x1 = xv[1], x2 = xv[2];
+        float s = 0.f;
+        s = s + B[0] * x0.x;
+        s = s + B[1] * x0.y;
+        s = s + B[2] * x1.x;
+        s = s + B[3] * x1.y;
+        s = s + B[4] * x2.x;
+        s = s + B[5] * x2.y;
+        return s;
+    };
+    float minv[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) minv[q] = act ? d.minv[li * 36 + ei * 6 + q] : 0.f;
+    // z = M^-1 r of the own entry; r and z where warp 0 and the senders read them
+    auto precondition = [&](float rv, bool stop) {
+        float rq[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) rq[q] = __shfl_sync(0xffffffffu, rv, lane < 30 ? grp * 6 + q : q);
         float zi = 0.f;
 #pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            const float rq = __shfl_sync(0xffffffffu, ji, lane < 30 ? grp * 6 + q : q);
-            if (act) zi = zi + d.minv[li * 36 + ei * 6 + q] * rq;
-        }
+        for (int q = 0; q < 6; ++q) zi = zi + minv[q] * rq[q];
         if (act) {
-            d.x[o] = 0.f;
-            d.r[o] = ji;
+            d.r[o] = rv;
             zown[o] = zi;
-            for (unsigned q = 0; q < ncta; ++q)
-                if (q != rank) dsmem_store_f32(d.z + (long)gnode * 6 + ei, q, zi);
         }
-    }
-    // tol^2 in binary32, for the stopping test of lane 0 of warp 0
-    const float tol2 = (tol && threadIdx.x == 0) ? (float)(L.tol * L.tol) : 0.f;
-    {
-        DF t[2];
-        bool lead;
-        if (tol) lead = ds_dot<2>({d.r, d.r}, {zown, d.r}, cnt, d, ph, t);
-        else {
-            DF t1[1];
-            lead = ds_dot<1>({d.r}, {zown}, cnt, d, ph, t1);
-            t[0] = t1[0];
-            t[1] = {0.f, 0.f};
+        if (__syncthreads_or(stop)) return false;
+        if (ex.dead) return true;
+        if (w == 0) {
+            if constexpr (kTol) ds_dot_send<2>({d.r, d.r}, {zown, d.r}, cnt, d, 1);
+            else ds_dot_send<1>({d.r}, {zown}, cnt, d, 1);
         }
-        if (lead) {
-            cs.rz_df = t[0];
-            cs.bn_df = t[1];
-            cs.stop = 0;
+        for (unsigned k = (unsigned)w; k < ncta; k += kLoopWarps - 1) {  // warp w: the w-th CTA after this one
+            if (k == 0) break;
+            const unsigned q = rank + k < ncta ? rank + k : rank + k - ncta;
+            const unsigned to = cluster_addr(zown, q), bar = cluster_addr(d.bar + 1, q);
+            for (int i = lane; i < cnt / 2; i += 32) {
+                const float2 v = reinterpret_cast<const float2*>(zown)[i];
+                async_store_df(to + 8 * i, bar, {v.x, v.y});
+            }
         }
-    }
-    __syncthreads();
+        return true;
+    };
+    // x = 0, r = b, z = M^-1 r
+    float x = 0.f, rv = act ? __ldcg(b.jtr + (long)(start + li) * 6 + ei) : 0.f;
+    if (threadIdx.x == 0) ds_expect(d, 1, rz_bytes);
+    precondition(rv, false);
+    if (!ex.dead) ds_wait(d, 1, ex, L.g.error);
+    DF t[NV];
+    ds_dot_total<NV>(d, 1, t);
+    DF rz = t[0];
+    const bool mine = w * 5 < own;  // the warp has entries
+    const float tol2 = kTol ? (float)(L.tol * L.tol) : 0.f, bn = t[NV - 1].hi;
     float beta = 0.f;
     for (int it = 0; it < L.pcg_iters; ++it) {
         // p = z (first iteration) or z + beta p, formed for all nodes by every CTA from its copies
-        for (int i = threadIdx.x; i < n * 6; i += blockDim.x) d.pf[i] = it ? d.z[i] + beta * d.pf[i] : d.z[i];
+#pragma unroll 2
+        for (int i = threadIdx.x; i < n * 3; i += kLoopThreads) {
+            const float2 zv = reinterpret_cast<const float2*>(d.z)[i];
+            float2* pv = reinterpret_cast<float2*>(d.pf) + i;
+            if (it) {
+                const float2 pp = *pv;
+                *pv = make_float2(zv.x + beta * pp.x, zv.y + beta * pp.y);
+            } else {
+                *pv = zv;
+            }
+        }
         __syncthreads();
         // A p of the own rows
-        const int rows_per_pass = (int)blockDim.x / R;
-        for (int base = 0; base < cnt; base += rows_per_pass) {
-            const int q = base + (int)threadIdx.x / R, part = (int)threadIdx.x % R;
-            float acc = 0.f;
-            if (q < cnt) {
-                const int l = q / 6, e = q - 6 * l;
-                const int r1 = d.rowptr[l + 1];
-                for (int bk = d.rowptr[l] + part; bk < r1; bk += R) {
-                    const float* B = d.blk + bk * 36 + e * 6;
-                    const float* xv = d.pf + d.col[bk] * 6;
-                    float s = 0.f;
+        float acc = 0.f, prod[kRegBlocks];
 #pragma unroll
-                    for (int j = 0; j < 6; ++j) s = s + B[j] * xv[j];
-                    acc = acc + s;
-                }
-            }
-            for (int m = R / 2; m > 0; m >>= 1) acc = acc + __shfl_xor_sync(0xffffffffu, acc, m);
-            if (q < cnt && part == 0) d.ap[q] = acc;
+        for (int k = 0; k < kRegBlocks; ++k) prod[k] = row_times(A[k], col[k]);
+#pragma unroll
+        for (int k = 0; k < kRegBlocks; ++k) acc = b0 + k * R < b1 ? acc + prod[k] : acc;
+        for (int bk = b0 + kRegBlocks * R; bk < b1; bk += R) {
+            float B[6];
+#pragma unroll
+            for (int j = 0; j < 6; ++j) B[j] = d.blk[bk * 36 + re * 6 + j];
+            acc = acc + row_times(B, d.col[bk] * 3);
         }
-        {
-            DF t[1];
-            if (ds_dot<1>({pown}, {d.ap}, cnt, d, ph, t)) {
-                cs.stop = df_zero_or_nan(t[0]) ? 1 : 0;
-                cs.alpha = cs.stop ? 0.f : df_quotient(cs.rz_df, t[0]);
+        for (int m = R / 2; m > 0; m >>= 1) acc = acc + __shfl_xor_sync(0xffffffffu, acc, m);
+        if (row < cnt && part == 0) d.ap[row] = acc;
+        if (threadIdx.x == 0) ds_expect(d, 0, dot_bytes);
+        __syncthreads();
+        if (w == 0 && !ex.dead) ds_dot_send<1>({pown}, {d.ap}, cnt, d, 0);
+        const float pv = act ? pown[o] : 0.f, apv = act ? d.ap[o] : 0.f;
+        // the totals and step sizes: alpha by the warps that have entries, beta by one warp (all warps
+        // forming them costs more, by their instructions, than handing beta round)
+        bool stop = false;
+        if (mine || w == 0) {
+            if (!ex.dead) ds_wait(d, 0, ex, L.g.error);
+            DF pap[1];
+            ds_dot_total<1>(d, 0, pap);
+            stop = df_zero_or_nan(pap[0]);  // the same in every CTA
+            const float alpha = df_quotient(rz, pap[0]);
+            x = stop ? x : x + alpha * pv;
+            rv = rv - alpha * apv;
+        } else {
+            ex.parity[0] ^= 1u;
+        }
+        if (threadIdx.x == 0 && !stop) ds_expect(d, 1, rz_bytes);
+        // every CTA has read z (forming p) before it sent its part of p.Ap, so it can be overwritten here
+        if (!precondition(rv, stop)) break;
+        if (!ex.dead) ds_wait(d, 1, ex, L.g.error);
+        if (mine || w == 0) {
+            ds_dot_total<NV>(d, 1, t);
+            if (threadIdx.x == 0) {
+                d.scal[0] = df_quotient(t[0], rz);
+                d.scal[1] = kTol && t[NV - 1].hi <= tol2 * bn ? 1.f : 0.f;
             }
+            rz = t[0];
         }
         __syncthreads();
-        if (cs.stop) break;
-        const float alpha = cs.alpha;
-        float rv = 0.f;
-        if (act) {
-            d.x[o] = d.x[o] + alpha * pown[o];
-            rv = d.r[o] - alpha * d.ap[o];
-            d.r[o] = rv;
-        }
-        float zi = 0.f;
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            const float rq = __shfl_sync(0xffffffffu, rv, lane < 30 ? grp * 6 + q : q);
-            if (act) zi = zi + d.minv[li * 36 + ei * 6 + q] * rq;
-        }
-        // z is read (forming p) before the p.Ap barrier in every CTA, so it can be overwritten here
-        if (act) {
-            zown[o] = zi;
-            for (unsigned q = 0; q < ncta; ++q)
-                if (q != rank) dsmem_store_f32(d.z + (long)gnode * 6 + ei, q, zi);
-        }
-        {
-            DF t[2];
-            bool lead;
-            if (tol) lead = ds_dot<2>({d.r, d.r}, {zown, d.r}, cnt, d, ph, t);
-            else {
-                DF t1[1];
-                lead = ds_dot<1>({d.r}, {zown}, cnt, d, ph, t1);
-                t[0] = t1[0];
-                t[1] = {0.f, 0.f};
-            }
-            if (lead) {
-                cs.beta = df_quotient(t[0], cs.rz_df);
-                cs.rz_df = t[0];
-                cs.stop = (tol && t[1].hi <= tol2 * cs.bn_df.hi) ? 1 : 0;
-            }
-        }
-        __syncthreads();
-        beta = cs.beta;
-        if (cs.stop) break;
+        beta = d.scal[0];
+        if (kTol && d.scal[1] != 0.f) break;
     }
+    if (act) d.x[o] = x;
     // T_pending -= [[x_rot]x, x_t; 0] for the own nodes (updateTransformsKernel,
     // src/MotionOptimization.cu:483-498); x also to global memory for inspection
     __syncthreads();
@@ -1179,20 +1297,81 @@ AFX_D void pcg_ds(const LoopArgs& L, int n, const DsLayout& d, ClusterSums& cs, 
 
 // ---- phases of the Gauss-Newton loop (all CTAs of the cluster unless stated) ----
 
+// The node transforms as the phases read them (rows 0 to 2; what the fourth row holds is never used):
+// from global memory through L2 (T is written by other CTAs of the launch), or, when the system lives in
+// shared memory, from a copy in the room of z and p, which are free between solves.  A vertex reads four
+// transforms and an edge two, each transform many times: 3 loads of 16 bytes of shared memory instead of 12
+// loads from L2.  With this, the loads of several items in flight in each phase, half the FP64 additions
+// in the energy sum and the nodes of J^T r dealt over all CTAs, gn_loop_kernel in the 256^3 sequence went
+// from 267 to 232 us.
+template <bool kStaged>
+struct NodeT {
+    const float* T;     // [n][16]
+    const float4* rows;  // kStaged: [n][3] rows (T[r], T[4 + r], T[8 + r], T[12 + r])
+    int n;
+    AFX_D void load(uint32_t i, float (&M)[16]) const {
+        if (kStaged && i < (uint32_t)n) {
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                const float4 v = rows[3 * i + r];
+                M[r] = v.x;
+                M[4 + r] = v.y;
+                M[8 + r] = v.z;
+                M[12 + r] = v.w;
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) M[e] = (e & 3) < 3 ? __ldcg(T + 16 * (long)i + e) : 0.f;
+        }
+    }
+};
+
+// Stage the transforms of all n <= kDsNodes nodes (every thread of the CTA; ends with a CTA barrier).  Other CTAs
+// must be past their last store into this CTA's z, and the next solve must begin after a cluster barrier.
+AFX_D void stage_node_T(const float* T, int n, const DsLayout& d) {
+    float4* rows = reinterpret_cast<float4*>(d.z);
+    static_assert(kDsNodes * 12 * sizeof(float) == 2 * sizeof(float) * kDsNodes * 6, "z and p hold the rows");
+#pragma unroll 2
+    for (int t = threadIdx.x; t < 3 * n; t += kLoopThreads) {
+        const float* p = T + 16 * (long)(t / 3) + t % 3;
+        rows[t] = make_float4(__ldcg(p), __ldcg(p + 4), __ldcg(p + 8), __ldcg(p + 12));
+    }
+    __syncthreads();
+}
+
 // Residuals (fill_r_DepthKernel / fill_r_MRegKernel, src/MotionOptimization.cu:163-227) with
 // the transforms T; partial FP64 energies of this thread (runSquareKernel + reductions,
 // src/VolumeFusion.cu:575-588).
-AFX_D void gn_residuals(const GnArgs& a, const float* warped, const float* T, int n, long ncorr, long gt, long gstride,
-                        double (&e2)[2]) {
+template <bool kStaged>
+AFX_D void gn_residuals(const GnArgs& a, const float* warped, const NodeT<kStaged>& T, int n, long ncorr, long gt,
+                        long gstride, double (&e2)[2]) {
     const GnBuffers& b = a.b;
     const long nreg = (long)n * a.kreg;
-    for (long c = gt; c < ncorr; c += gstride) {
-        const long v = a.corr[2 * c], px = a.corr[2 * c + 1];
-        const float* f = a.frame + 3 * px;
-        float d[3] = {__ldcg(warped + 3 * v) - f[0], __ldcg(warped + 3 * v + 1) - f[1], __ldcg(warped + 3 * v + 2) - f[2]};
-        const float r = a.lam_d * dot3(a.normals + 3 * px, d);
-        __stcg(b.rdepth + c, r);
-        e2[0] += (double)(r * r);
+    constexpr int kAhead = 4;  // correspondences whose loads are in flight together
+    for (long c0 = gt; c0 < ncorr; c0 += kAhead * gstride) {
+        long v[kAhead], px[kAhead];
+        float d[kAhead][3], nr[kAhead][3];
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+            const long c = c0 + k * gstride < ncorr ? c0 + k * gstride : c0;
+            v[k] = a.corr[2 * c];
+            px[k] = a.corr[2 * c + 1];
+        }
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+#pragma unroll
+            for (int ax = 0; ax < 3; ++ax) {
+                d[k][ax] = __ldcg(warped + 3 * v[k] + ax) - a.frame[3 * px[k] + ax];
+                nr[k][ax] = a.normals[3 * px[k] + ax];
+            }
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+            const long c = c0 + k * gstride;
+            if (c >= ncorr) break;
+            const float r = a.lam_d * dot3(nr[k], d[k]);
+            __stcg(b.rdepth + c, r);
+            e2[0] += (double)(r * r);
+        }
     }
     for (long t = gt; t < nreg; t += gstride) {
         const int i = (int)(t / a.kreg);
@@ -1205,11 +1384,8 @@ AFX_D void gn_residuals(const GnArgs& a, const float* warped, const float* T, in
             continue;
         }
         float Ti[16], Tn[16], tc[3], tn[3];
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-            Ti[e] = __ldcg(T + 16 * (long)i + e);
-            Tn[e] = __ldcg(T + 16 * (long)nb + e);
-        }
+        T.load((uint32_t)i, Ti);
+        T.load(nb, Tn);
         mat4_point(Ti, a.nodes + 3 * (long)i, tc);
         mat4_point(Tn, a.nodes + 3 * (long)i, tn);
         for (int ax = 0; ax < 3; ++ax) {
@@ -1354,22 +1530,66 @@ AFX_D void update_transforms_range(float* T, const float* x, int lo, int hi, lon
 }
 
 // Canonical vertices warped by T (warpKernel, src/ComputeCorrespondence.cu:13-30, or the dual-quaternion
-// blend of afx_dqb.cuh).  T is written by other CTAs of this launch: read through L2.
-AFX_D void gn_rewarp(const GnArgs& a, const float* points, float* warped, const float* T, long m, long gt,
+// blend of afx_dqb.cuh).
+template <bool kStaged>
+AFX_D void gn_rewarp(const GnArgs& a, const float* points, float* warped, const NodeT<kStaged>& T, long m, long gt,
                      long gstride) {
     if (a.blend == AFX_BLEND_DQB) {
         for (long i = gt; i < m; i += gstride) {
             const float p[3] = {points[3 * i], points[3 * i + 1], points[3 * i + 2]};
             float o[3];
-            dq_blend_point(
-                [T](uint32_t nb, float* Tn) {
-#pragma unroll
-                    for (int e = 0; e < 16; ++e) Tn[e] = __ldcg(T + 16 * (long)nb + e);
-                },
-                a.midx + i * a.k, a.mw + i * a.k, a.k, AFX_INVALID_INDEX, p, o);
+            dq_blend_point([&](uint32_t nb, float(&Tn)[16]) { T.load(nb, Tn); }, a.midx + i * a.k, a.mw + i * a.k, a.k,
+                           AFX_INVALID_INDEX, p, o);
             __stcg(warped + 3 * i, o[0]);
             __stcg(warped + 3 * i + 1, o[1]);
             __stcg(warped + 3 * i + 2, o[2]);
+        }
+        return;
+    }
+    // one neighbour's part of a point's sum
+    auto blend = [&](const float (&p)[3], uint32_t nb, float wj, float (&acc)[3]) {
+        if (nb == AFX_INVALID_INDEX) return;
+        float Tn[16], o[3];
+        T.load(nb, Tn);
+        mat4_point(Tn, p, o);
+        acc[0] = acc[0] + wj * o[0];
+        acc[1] = acc[1] + wj * o[1];
+        acc[2] = acc[2] + wj * o[2];
+    };
+    auto finish = [&](long i, const float (&p)[3], bool zero, const float (&acc)[3]) {
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) __stcg(warped + 3 * i + ax, zero ? p[ax] : acc[ax]);
+    };
+    if (kStaged && a.k == 4 && !(((size_t)a.midx | (size_t)a.mw) & 15)) {
+        // four neighbours, rows on 16 bytes: whole rows, and the loads of several points in flight together
+        constexpr int kAhead = 4;
+        for (long i0 = gt; i0 < m; i0 += kAhead * gstride) {
+            float p[kAhead][3];
+            uint4 nb[kAhead];
+            float4 w[kAhead];
+#pragma unroll
+            for (int q = 0; q < kAhead; ++q) {
+                const long i = i0 + q * gstride < m ? i0 + q * gstride : i0;
+                nb[q] = reinterpret_cast<const uint4*>(a.midx)[i];
+                w[q] = reinterpret_cast<const float4*>(a.mw)[i];
+#pragma unroll
+                for (int ax = 0; ax < 3; ++ax) p[q][ax] = points[3 * i + ax];
+            }
+#pragma unroll
+            for (int q = 0; q < kAhead; ++q) {
+                const long i = i0 + q * gstride;
+                if (i >= m) break;
+                const bool zero = fabsf(w[q].x) <= 1e-5f && fabsf(w[q].y) <= 1e-5f && fabsf(w[q].z) <= 1e-5f &&
+                                  fabsf(w[q].w) <= 1e-5f;
+                float acc[3] = {0.f, 0.f, 0.f};
+                if (!zero) {
+                    blend(p[q], nb[q].x, w[q].x, acc);
+                    blend(p[q], nb[q].y, w[q].y, acc);
+                    blend(p[q], nb[q].z, w[q].z, acc);
+                    blend(p[q], nb[q].w, w[q].w, acc);
+                }
+                finish(i, p[q], zero, acc);
+            }
         }
         return;
     }
@@ -1378,34 +1598,20 @@ AFX_D void gn_rewarp(const GnArgs& a, const float* points, float* warped, const 
         bool zero = true;
         for (int j = 0; j < a.k; ++j)
             if (!(fabsf(a.mw[i * a.k + j]) <= 1e-5f)) zero = false;
-        float acc[3] = {p[0], p[1], p[2]};
-        if (!zero) {
-            acc[0] = acc[1] = acc[2] = 0.f;
-            for (int j = 0; j < a.k; ++j) {
-                const uint32_t nb = a.midx[i * a.k + j];
-                if (nb == AFX_INVALID_INDEX) continue;
-                float Tn[16], o[3];
-#pragma unroll
-                for (int e = 0; e < 16; ++e) Tn[e] = __ldcg(T + 16 * (long)nb + e);
-                mat4_point(Tn, p, o);
-                const float wj = a.mw[i * a.k + j];
-                acc[0] = acc[0] + wj * o[0];
-                acc[1] = acc[1] + wj * o[1];
-                acc[2] = acc[2] + wj * o[2];
-            }
-        }
-        __stcg(warped + 3 * i, acc[0]);
-        __stcg(warped + 3 * i + 1, acc[1]);
-        __stcg(warped + 3 * i + 2, acc[2]);
+        float acc[3] = {0.f, 0.f, 0.f};
+        if (!zero)
+            for (int j = 0; j < a.k; ++j) blend(p, a.midx[i * a.k + j], a.mw[i * a.k + j], acc);
+        finish(i, p, zero, acc);
     }
 }
 
 // One solve from b.jtr: x in b.x (and in the own slices of the shared-memory layout); with
 // L.T_pending set, T_pending -= [x] as well.  Ends with a cluster barrier.
-AFX_D void gn_solve(const LoopArgs& L, int n, bool ds, const DsLayout& dsl, ClusterSums& cs, int& ds_ph, long gt,
+AFX_D void gn_solve(const LoopArgs& L, int n, bool ds, const DsLayout& dsl, ClusterSums& cs, DsExchange& ex, long gt,
                     long gstride) {
     if (ds) {
-        pcg_ds(L, n, dsl, cs, ds_ph);
+        if (L.tol > 0) pcg_ds<true>(L, n, dsl, ex);
+        else pcg_ds<false>(L, n, dsl, ex);
     } else {
         pcg_global(L, n, cs);
         cluster_barrier();  // x complete
@@ -1419,7 +1625,11 @@ __global__ void __launch_bounds__(kLoopThreads, 1) gn_loop_kernel(LoopArgs L) {
     const GnBuffers& b = a.b;
     __shared__ ClusterSums cs;
     extern __shared__ double ds_smem[];
-    if (threadIdx.x == 0) cs.phase = 0;
+    const DsLayout dsl = ds_layout(ds_smem);
+    if (threadIdx.x == 0) {
+        cs.phase = 0;
+        ds_exchange_init(dsl);
+    }
     // Every CTA of the cluster must be running before any thread touches another CTA's shared
     // memory (the first such store is in ds_stage).  Under load the CTAs of a cluster need not
     // start together; a store into a CTA that has not started is an SM fault.
@@ -1427,7 +1637,8 @@ __global__ void __launch_bounds__(kLoopThreads, 1) gn_loop_kernel(LoopArgs L) {
     const unsigned rank = cluster_rank(), ncta = cluster_size();
     const int w = threadIdx.x >> 5;
     const long gt = (long)rank * kLoopThreads + threadIdx.x, gstride = (long)ncta * kLoopThreads;
-    const int gw = (int)rank * kLoopWarps + w, nw = (int)ncta * kLoopWarps;
+    // nodes dealt to the CTAs in turn: a small graph's fill every CTA alike
+    const int gw = w * (int)ncta + (int)rank, nw = (int)ncta * kLoopWarps;
     const bool leader = rank == 0 && threadIdx.x == 0;
     const int n = min(*a.n_nodes, a.n_max);
     const long ncorr = min((long)*a.corr_count, a.c_max);
@@ -1436,13 +1647,17 @@ __global__ void __launch_bounds__(kLoopThreads, 1) gn_loop_kernel(LoopArgs L) {
     double e_prev = s->e_prev;
     bool done = s->done != 0;
     // small graphs: the system lives in distributed shared memory for the whole loop
-    const DsLayout dsl = ds_layout(ds_smem);
     int ds_ph = 0;
+    DsExchange ex{{0u, 0u}, false};
     const bool ds = !done && n > 0 && (n + (int)ncta - 1) / (int)ncta <= kDsNpc && ds_stage(b, n, dsl, cs, ds_ph);
+    const NodeT<true> Ts{L.T_pending, reinterpret_cast<const float4*>(dsl.z), n};
+    const NodeT<false> Tg{L.T_pending, nullptr, n};
+    if (ds) stage_node_T(L.T_pending, n, dsl);
     for (int iter = 0; iter < L.gn_iters && !done; ++iter) {
         double e2[2] = {0.0, 0.0};
-        gn_residuals(a, L.warped, L.T_pending, n, ncorr, gt, gstride, e2);
-        cluster_sum<2>(e2, cs);
+        if (ds) gn_residuals(a, L.warped, Ts, n, ncorr, gt, gstride, e2);
+        else gn_residuals(a, L.warped, Tg, n, ncorr, gt, gstride, e2);
+        cluster_sum_pair(e2, cs);
         // ---- energy test and commit decision (src/VolumeFusion.cu:589-598)
         const double e = e2[0] + e2[1];
         if (leader) {
@@ -1463,11 +1678,16 @@ __global__ void __launch_bounds__(kLoopThreads, 1) gn_loop_kernel(LoopArgs L) {
             s->iters = iter + 1;
         }
         if (commit)
-            for (long t = gt; t < (long)n * 16; t += gstride) L.T_committed[t] = __ldcg(L.T_pending + t);
+            for (long t = gstride - 1 - gt; t < (long)n * 16; t += gstride) L.T_committed[t] = __ldcg(L.T_pending + t);
         gn_jtr(a, n, gw, nw);
         cluster_barrier();
-        gn_solve(L, n, ds, dsl, cs, ds_ph, gt, gstride);
-        gn_rewarp(a, L.points, L.warped, L.T_pending, m, gt, gstride);
+        gn_solve(L, n, ds, dsl, cs, ex, gt, gstride);
+        if (ds) {
+            stage_node_T(L.T_pending, n, dsl);
+            gn_rewarp(a, L.points, L.warped, Ts, m, gt, gstride);
+        } else {
+            gn_rewarp(a, L.points, L.warped, Tg, m, gt, gstride);
+        }
         cluster_barrier();
     }
     // no CTA leaves while another may still read its shared memory
@@ -1480,15 +1700,19 @@ __global__ void __launch_bounds__(kLoopThreads, 1) gn_solve_kernel(LoopArgs L) {
     const GnArgs& a = L.g;
     __shared__ ClusterSums cs;
     extern __shared__ double ds_smem[];
-    if (threadIdx.x == 0) cs.phase = 0;
+    const DsLayout dsl = ds_layout(ds_smem);
+    if (threadIdx.x == 0) {
+        cs.phase = 0;
+        ds_exchange_init(dsl);
+    }
     cluster_barrier();  // every CTA running before any access to another CTA's shared memory
     const unsigned rank = cluster_rank(), ncta = cluster_size();
     const long gt = (long)rank * kLoopThreads + threadIdx.x, gstride = (long)ncta * kLoopThreads;
     const int n = min(*a.n_nodes, a.n_max);
-    const DsLayout dsl = ds_layout(ds_smem);
     int ds_ph = 0;
+    DsExchange ex{{0u, 0u}, false};
     const bool ds = n > 0 && (n + (int)ncta - 1) / (int)ncta <= kDsNpc && ds_stage(a.b, n, dsl, cs, ds_ph);
-    gn_solve(L, n, ds, dsl, cs, ds_ph, gt, gstride);
+    gn_solve(L, n, ds, dsl, cs, ex, gt, gstride);
     // no CTA leaves while another may still read its shared memory
     cluster_barrier();
 }
@@ -1724,7 +1948,8 @@ __global__ void __launch_bounds__(256) gn_residual_kernel(GnArgs a, const float*
     const int n = min(*a.n_nodes, a.n_max);
     const long ncorr = min((long)*a.corr_count, a.c_max);
     double e2[2] = {0.0, 0.0};
-    gn_residuals(a, warped, T, n, ncorr, blockIdx.x * (long)blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x, e2);
+    gn_residuals(a, warped, NodeT<false>{T, nullptr, n}, n, ncorr, blockIdx.x * (long)blockDim.x + threadIdx.x,
+                 (long)gridDim.x * blockDim.x, e2);
 }
 
 __global__ void __launch_bounds__(256) gn_jtr_kernel(GnArgs a) {
