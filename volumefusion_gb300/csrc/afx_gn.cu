@@ -13,6 +13,7 @@
 // assembled once per ICP iteration; J^T r is rebuilt every Gauss-Newton iteration.
 // The solve is a block-Jacobi PCG in one kernel on one cluster: FP32 block SpMV, dot products in
 // triple- (shared-memory path) or double-binary32 (global-memory path), FP64 6x6 block inverses.
+#include <algorithm>
 #include <cfloat>
 #include <cstring>
 #include <new>
@@ -42,39 +43,68 @@ AFX_D void jdepth(const float* n, float w, const float G[3][6], float lam, float
 }
 
 // ---- per-frame node lists ----
+//
+// Two sets of lists, both ascending: the (vertex, slot) entries of every node and its incoming
+// regularisation edges.  Count, offsets, fill and sort take one launch each for the two sets
+// together: the launches are what these steps cost (a few us each for tens of kB).
 
-__global__ void lst_count_kernel(GnArgs a) {
+__global__ void list_count_kernel(GnArgs a) {
     const long m = min((long)*a.mesh_count, a.m_max);
-    const uint32_t n = (uint32_t)*a.n_nodes;
-    AFX_GRID_STRIDE(t, m * a.k) {
-        if (a.mw[t] == 0.f) continue;
-        const uint32_t node = a.midx[t];
-        if (node < n) atomicAdd(a.b.lcnt + node, 1u);
-    }
-}
-
-__global__ void lst_fill_kernel(GnArgs a) {
-    const long m = min((long)*a.mesh_count, a.m_max);
-    const uint32_t n = (uint32_t)*a.n_nodes;
-    AFX_GRID_STRIDE(t, m * a.k) {
-        if (a.mw[t] == 0.f) continue;
-        const uint32_t node = a.midx[t];
-        if (node >= n) continue;
-        const unsigned p = a.b.loff[node] + atomicAdd(a.b.lcur + node, 1u);
-        a.b.lst[p] = (unsigned)t;
-    }
-}
-
-__global__ void in_count_kernel(GnArgs a) {
     const int n = min(*a.n_nodes, a.n_max);
+    AFX_GRID_STRIDE(t, m * a.k) {
+        if (a.mw[t] == 0.f) continue;
+        const uint32_t node = a.midx[t];
+        if (node < (uint32_t)n) atomicAdd(a.b.lcnt + node, 1u);
+    }
     AFX_GRID_STRIDE(t, (long)n * a.kreg) {
         const uint32_t nb = a.gidx[t];
         if (nb < (uint32_t)n) atomicAdd(a.b.icnt + nb, 1u);
     }
 }
 
-__global__ void in_fill_kernel(GnArgs a) {
+// Exclusive prefix sums over the live nodes, one CTA per set: off[0..n].
+__global__ void __launch_bounds__(1024) list_scan_kernel(GnArgs a) {
+    __shared__ unsigned ws[32];
     const int n = min(*a.n_nodes, a.n_max);
+    const unsigned* cnt = blockIdx.x ? a.b.icnt : a.b.lcnt;
+    unsigned* off = blockIdx.x ? a.b.ioff : a.b.loff;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    unsigned carry = 0;
+    for (int base = 0; base < n; base += 1024) {
+        const int i = base + (int)threadIdx.x;
+        const unsigned v = i < n ? cnt[i] : 0u;
+        unsigned x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) ws[wid] = x;
+        __syncthreads();
+        unsigned t = ws[lane];  // every warp scans the 32 warp sums for itself
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned y = __shfl_up_sync(0xffffffffu, t, o);
+            if (lane >= o) t += y;
+        }
+        const unsigned before = __shfl_sync(0xffffffffu, t, wid > 0 ? wid - 1 : 0);
+        if (i < n) off[i] = carry + (wid > 0 ? before : 0u) + x - v;
+        carry += __shfl_sync(0xffffffffu, t, 31);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) off[n] = carry;
+}
+
+__global__ void list_fill_kernel(GnArgs a) {
+    const long m = min((long)*a.mesh_count, a.m_max);
+    const int n = min(*a.n_nodes, a.n_max);
+    AFX_GRID_STRIDE(t, m * a.k) {
+        if (a.mw[t] == 0.f) continue;
+        const uint32_t node = a.midx[t];
+        if (node >= (uint32_t)n) continue;
+        const unsigned p = a.b.loff[node] + atomicAdd(a.b.lcur + node, 1u);
+        a.b.lst[p] = (unsigned)t;
+    }
     AFX_GRID_STRIDE(t, (long)n * a.kreg) {
         const uint32_t nb = a.gidx[t];
         if (nb >= (uint32_t)n) continue;
@@ -83,159 +113,115 @@ __global__ void in_fill_kernel(GnArgs a) {
     }
 }
 
-// Bitonic sort of one list (len <= kSegMax) through shared memory, by the whole CTA.
+// Ascending bitonic steps of one value per lane: partners `from`, from / 2, .. 1 lanes apart.
+AFX_D unsigned lane_merge(unsigned x, int from, bool asc) {
+    const int lane = threadIdx.x & 31;
+    for (int o = from; o > 0; o >>= 1) {
+        const unsigned y = __shfl_xor_sync(0xffffffffu, x, o);
+        x = (((lane & o) == 0) == asc) ? min(x, y) : max(x, y);
+    }
+    return x;
+}
+
+// Bitonic sort of one list (len <= kSegMax) through shared memory, by the whole CTA.  Partners
+// less than 32 apart are lanes of a warp: only the wider steps need a barrier (15 instead of 55
+// for 1024 entries).
 AFX_D void seg_sort_one(unsigned* lst, int len, unsigned* s) {
-    int P = 1;
+    int P = 32;
     while (P < len) P <<= 1;
     __syncthreads();  // the previous list's write-back is done with s
-    for (int i = threadIdx.x; i < P; i += blockDim.x) s[i] = i < len ? lst[i] : 0xffffffffu;
-    __syncthreads();
-    for (int size = 2; size <= P; size <<= 1)
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+    for (int i = threadIdx.x; i < P; i += blockDim.x) {
+        unsigned x = i < len ? lst[i] : 0xffffffffu;
+        for (int size = 2; size <= 32; size <<= 1) x = lane_merge(x, size >> 1, (i & size) == 0);
+        s[i] = x;
+    }
+    for (int size = 64; size <= P; size <<= 1) {
+        for (int stride = size >> 1; stride >= 32; stride >>= 1) {
+            __syncthreads();
             for (int pidx = threadIdx.x; pidx < P / 2; pidx += blockDim.x) {
-                int i = 2 * stride * (pidx / stride) + (pidx % stride), j = i + stride;
-                bool asc = (i & size) == 0;
-                unsigned x = s[i], y = s[j];
+                const int i = 2 * stride * (pidx / stride) + (pidx % stride), j = i + stride;
+                const bool asc = (i & size) == 0;
+                const unsigned x = s[i], y = s[j];
                 if ((y < x) == asc) {
                     s[i] = y;
                     s[j] = x;
                 }
             }
-            __syncthreads();
         }
+        __syncthreads();
+        for (int i = threadIdx.x; i < P; i += blockDim.x) s[i] = lane_merge(s[i], 16, (i & size) == 0);
+    }
+    __syncthreads();
     for (int i = threadIdx.x; i < len; i += blockDim.x) lst[i] = s[i];
 }
 
-// Sort each node's list ascending (bitonic in shared memory); one CTA per node at a time.
-__global__ void __launch_bounds__(256) seg_sort_kernel(unsigned* lst, const unsigned* off, const int* n_nodes, int n_max,
-                                                       int* error) {
+// Sort both sets: one CTA per node's entries at a time; the edge lists (about kreg entries) one per
+// warp in registers, and by the whole CTA where one is longer than a warp.
+__global__ void __launch_bounds__(256) list_sort_kernel(GnArgs a) {
     __shared__ unsigned s[kSegMax];
-    const int n = min(*n_nodes, n_max);
-    for (int a = blockIdx.x; a < n; a += gridDim.x) {
-        const unsigned o = off[a];
-        const int len = (int)(off[a + 1] - o);
+    const int n = min(*a.n_nodes, a.n_max);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int node = blockIdx.x; node < n; node += gridDim.x) {
+        const unsigned o = a.b.loff[node];
+        const int len = (int)(a.b.loff[node + 1] - o);
         if (len > kSegMax) {
-            if (threadIdx.x == 0) atomicOr(error, ERRF_CAPACITY);
+            if (threadIdx.x == 0) atomicOr(a.error, ERRF_CAPACITY);
             continue;
         }
-        if (len > 1) seg_sort_one(lst + o, len, s);
+        if (len > 1) seg_sort_one(a.b.lst + o, len, s);
+    }
+    for (int base = blockIdx.x * 8; base < n; base += gridDim.x * 8) {
+        const int node = base + w;
+        if (node < n) {
+            const unsigned o = a.b.ioff[node];
+            const int len = (int)(a.b.ioff[node + 1] - o);
+            if (len > 1 && len <= 32) {
+                unsigned x = lane < len ? a.b.ilst[o + lane] : 0xffffffffu;
+                for (int size = 2; size <= 32; size <<= 1) x = lane_merge(x, size >> 1, (lane & size) == 0);
+                if (lane < len) a.b.ilst[o + lane] = x;
+            }
+        }
+        for (int q = 0; q < 8 && base + q < n; ++q) {
+            const unsigned o = a.b.ioff[base + q];
+            const int len = (int)(a.b.ioff[base + q + 1] - o);
+            if (len > kSegMax) {
+                if (threadIdx.x == 0) atomicOr(a.error, ERRF_CAPACITY);
+            } else if (len > 32) {
+                seg_sort_one(a.b.ilst + o, len, s);
+            }
+        }
     }
 }
-
 
 // ---- per-ICP assembly ----
 
-// Neighbour discovery: distinct nodes b != a sharing a corresponding vertex with a (both
-// weights non-zero) or joined to a by a regularisation edge.  One warp per node, bitmap in
-// shared memory, so the list comes out sorted.
-__global__ void __launch_bounds__(32 * kGnWarps) nbr_discover_kernel(GnArgs a, int words) {
-    extern __shared__ unsigned bm[];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n = min(*a.n_nodes, a.n_max);
-    unsigned* my = bm + (long)w * words;
-    for (int node = blockIdx.x * kGnWarps + w; node < n; node += gridDim.x * kGnWarps) {
-        for (int i = lane; i < words; i += 32) my[i] = 0u;
-        __syncwarp();
-        const unsigned o = a.b.loff[node], e = a.b.loff[node + 1];
-        for (unsigned t = o + lane; t < e; t += 32) {
-            unsigned ent = a.b.lst[t];
-            long v = ent / a.k;
-            if (a.corr_of_vertex[v] < 0) continue;
-            for (int s = 0; s < a.k; ++s) {
-                if (a.mw[v * a.k + s] == 0.f) continue;
-                uint32_t bnode = a.midx[v * a.k + s];
-                if (bnode != (uint32_t)node && bnode < (uint32_t)n) atomicOr(my + (bnode >> 5), 1u << (bnode & 31));
-            }
-        }
-        for (int kk = lane; kk < a.kreg; kk += 32) {
-            uint32_t nb = a.gidx[(long)node * a.kreg + kk];
-            if (nb < (uint32_t)n && nb != (uint32_t)node) atomicOr(my + (nb >> 5), 1u << (nb & 31));
-        }
-        for (unsigned t = a.b.ioff[node] + lane; t < a.b.ioff[node + 1]; t += 32) {
-            unsigned x = a.b.ilst[t] / a.kreg;
-            if (x != (unsigned)node) atomicOr(my + (x >> 5), 1u << (x & 31));
-        }
-        __syncwarp();
-        // ordered extraction
-        int base = 0;
-        for (int w0 = 0; w0 < words; w0 += 32) {
-            int wi = w0 + lane;
-            unsigned bits = wi < words ? my[wi] : 0u;
-            int c = __popc(bits);
-            int incl = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += y;
-            }
-            int pos = base + incl - c;
-            while (bits) {
-                int bit = __ffs(bits) - 1;
-                bits &= bits - 1;
-                if (pos < kMaxNbr) a.b.nbr[(long)node * kMaxNbr + pos] = wi * 32 + bit;
-                ++pos;
-            }
-            base += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        if (lane == 0) {
-            a.b.nbr_cnt[node] = min(base, kMaxNbr);
-            if (base > kMaxNbr) atomicOr(a.error, ERRF_CAPACITY);
-        }
-        __syncwarp();  // the bitmap is cleared for the warp's next node
-    }
-}
-
 // For neighbour slots below the diagonal, find the owner's slot (binary search).
-__global__ void nbr_ref_kernel(GnArgs a) {
-    const int n = min(*a.n_nodes, a.n_max);
-    AFX_GRID_STRIDE(t, (long)n * kMaxNbr) {
-        const int node = (int)(t / kMaxNbr), u = (int)(t % kMaxNbr);
-        if (u >= a.b.nbr_cnt[node]) continue;
-        const int bnode = a.b.nbr[t];
-        if (bnode > node) {
-            a.b.nbr_ref[t] = (int)t;
-            continue;
-        }
-        const int* L = a.b.nbr + (long)bnode * kMaxNbr;
-        int lo = 0, hi = a.b.nbr_cnt[bnode] - 1, f = -1;
-        while (lo <= hi) {
-            const int mid = (lo + hi) >> 1;
-            if (L[mid] == node) {
-                f = mid;
-                break;
-            }
-            if (L[mid] < node) lo = mid + 1;
-            else hi = mid - 1;
-        }
-        if (f < 0) {
-            atomicOr(a.error, ERRF_CAPACITY);
-            a.b.nbr_ref[t] = 0;
-            continue;
-        }
-        a.b.nbr_ref[t] = -((int)((long)bnode * kMaxNbr + f) + 1);
+AFX_D void nbr_ref_one(const GnArgs& a, long t) {
+    const int node = (int)(t / kMaxNbr), u = (int)(t % kMaxNbr);
+    if (u >= a.b.nbr_cnt[node]) return;
+    const int bnode = a.b.nbr[t];
+    if (bnode > node) {
+        a.b.nbr_ref[t] = (int)t;
+        return;
     }
+    const int* L = a.b.nbr + (long)bnode * kMaxNbr;
+    int lo = 0, hi = a.b.nbr_cnt[bnode] - 1, f = -1;
+    while (lo <= hi) {
+        const int mid = (lo + hi) >> 1;
+        if (L[mid] == node) {
+            f = mid;
+            break;
+        }
+        if (L[mid] < node) lo = mid + 1;
+        else hi = mid - 1;
+    }
+    if (f < 0) {
+        atomicOr(a.error, ERRF_CAPACITY);
+        a.b.nbr_ref[t] = 0;
+        return;
+    }
+    a.b.nbr_ref[t] = -((int)((long)bnode * kMaxNbr + f) + 1);
 }
-
-// J^T J: node a's warp accumulates D_a and its upper blocks (a, b > a).  Lane l owns block
-// entries l and l + 32 of every block; each entry is summed in a fixed sequential order:
-// depth rows by ascending node-list entry, then regularisation rows by ascending row.  The
-// rows are staged 32 at a time, one per lane, with their Jacobian blocks already formed
-// (jdepth for every contributing slot, or lam_r * G for a regularisation row), so the ordered
-// loop is shared-memory loads and adds only; the upper blocks accumulate in shared memory.
-constexpr int kJtjWarps = 2;
-constexpr int kJtjMaxK = 8;
-
-struct JtjStage {
-    float blk[kMaxNbr * 36];           // upper blocks of this node
-    int L[kMaxNbr];                    // sorted neighbour ids
-    float J[32][kJtjMaxK][6];          // depth rows: jdepth of each slot; reg rows: lam_r * G (3 x 6)
-    signed char slot[32][kJtjMaxK];    // -1: diagonal, >= 0: upper block, -2: no contribution
-    int own[32];                       // depth rows: the row's own slot, -1 without correspondence;
-                                       // reg rows: 1 own edge, 0 incoming edge, -1 skipped
-    unsigned qt[32];                   // depth rows with a correspondence, queued in entry order:
-    unsigned qe[32];                   // node-list position, entry (vertex * k + slot)
-    int qc[32];                        // and correspondence
-};
 
 AFX_D int find_slot(const int* L, int cnt, int b) {
     int lo = 0, hi = cnt - 1;
@@ -248,135 +234,283 @@ AFX_D int find_slot(const int* L, int cnt, int b) {
     return -1;
 }
 
-__global__ void __launch_bounds__(32 * kJtjWarps) jtj_assemble_kernel(GnArgs a) {
-    __shared__ JtjStage stage[kJtjWarps];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    JtjStage& S = stage[w];
-    const int n = min(*a.n_nodes, a.n_max);
-    const int k = a.k;
-    const int e0 = lane, e1 = lane + 32;  // entries this lane owns (e1 valid for lanes 0..3)
-    const int i0 = e0 / 6, j0 = e0 % 6, i1 = e1 / 6, j1 = e1 % 6;
-    const bool has1 = e1 < 36;
-    for (int node = blockIdx.x * kJtjWarps + w; node < n; node += gridDim.x * kJtjWarps) {
-        const int cnt = a.b.nbr_cnt[node];
-        for (int u = lane; u < cnt; u += 32) S.L[u] = a.b.nbr[(long)node * kMaxNbr + u];
-        for (int x = lane; x < cnt * 36; x += 32) S.blk[x] = 0.f;
-        __syncwarp();
-        float d0 = 0.f, d1 = 0.f;
-        bool touched = false;
-        // Depth rows: the node list is read 128 entries at a time (4 per lane, their loads in
-        // flight together); entries whose vertex has a correspondence are queued in entry order
-        // and, 32 at a time, staged (one row per lane: the Jacobian block of every slot) and then
-        // accumulated in order.  Entries without a correspondence contribute nothing.
-        auto run_queue = [&](int nq) {
-            if (lane < nq) {
-                const unsigned t = S.qt[lane], ent = S.qe[lane];
-                const long v = ent / k;
-                const int s = (int)(ent % k);
-                const int c = S.qc[lane];
-                S.own[lane] = s;
-                const int px = a.corr[2 * (long)c + 1];
-                const float nrm[3] = {a.normals[3 * (long)px], a.normals[3 * (long)px + 1], a.normals[3 * (long)px + 2]};
-                const float p[3] = {a.mesh[3 * v], a.mesh[3 * v + 1], a.mesh[3 * v + 2]};
-                float G[3][6];
-                grad_rows(p, G);
-                for (int tt = 0; tt < k; ++tt) {
-                    const float wt = a.mw[v * k + tt];
-                    const uint32_t bnode = a.midx[v * k + tt];
-                    int sl = -2;
-                    if (wt != 0.f && bnode >= (uint32_t)node) {
-                        if (bnode == (uint32_t)node) sl = -1;
-                        else {
-                            const int f = find_slot(S.L, cnt, (int)bnode);
-                            if (f >= 0) sl = f;
-                        }
-                    }
-                    S.slot[lane][tt] = (signed char)sl;
-                    if (sl != -2 || tt == s) {
-                        float Jt[6];
-                        jdepth(nrm, wt, G, a.lam_d, Jt);
-#pragma unroll
-                        for (int q = 0; q < 6; ++q) S.J[lane][tt][q] = Jt[q];
-                        if (tt == s)  // this row's J block, for J^T r
-#pragma unroll
-                            for (int q = 0; q < 6; ++q) a.b.jrow[(long)t * 6 + q] = Jt[q];
-                    }
-                }
-            }
-            __syncwarp();
-            for (int r = 0; r < nq; ++r) {
-                const int s = S.own[r];
-                touched = true;
-                const float ja0 = S.J[r][s][i0];
-                const float ja1 = has1 ? S.J[r][s][i1] : 0.f;
-                for (int tt = 0; tt < k; ++tt) {
-                    const int sl = S.slot[r][tt];
-                    if (sl == -2) continue;
-                    const float jb0 = S.J[r][tt][j0];
-                    const float jb1 = S.J[r][tt][j1];
-                    if (sl == -1) {
-                        d0 = d0 + ja0 * jb0;
-                        if (has1) d1 = d1 + ja1 * jb1;
-                    } else {
-                        float* blk = S.blk + sl * 36;
-                        blk[e0] = blk[e0] + ja0 * jb0;
-                        if (has1) blk[e1] = blk[e1] + ja1 * jb1;
-                    }
-                }
-            }
-            __syncwarp();
-        };
+// J^T J of one node per CTA: its neighbour list, its diagonal block D_a and its upper blocks
+// (a, b > a).
+//
+// Neighbours: distinct nodes b != a sharing a corresponding vertex with a (both weights non-zero)
+// or joined to a by a regularisation edge, as a bitmap in shared memory, so the list is sorted.
+//
+// Every block entry is a sum in a fixed order: depth rows by ascending node-list entry, then
+// regularisation rows by ascending row.  Entries of different blocks are independent, so the rows
+// are staged 256 at a time (one per thread, the Jacobian block of every slot formed: jdepth, or
+// lam_r * G for a regularisation row) and the blocks are dealt over the CTA: warp 0 sums the
+// diagonal, each of the other warps up to five upper blocks at a time, six lanes to a block, one
+// row of it per lane in registers.  A group visits only the rows of its block (a ballot over the slot
+// bytes of 32 rows gives each group its rows).  The bound is the serial sum of the longest lists:
+// with one warp per node walking all rows and the upper blocks in shared memory, the graph of the
+// 256^3 sequence (169 nodes, 900 entries each) took 70 us + 16 us for the neighbours.
+constexpr int kAsmThreads = 256;
+constexpr int kAsmUpWarps = kAsmThreads / 32 - 1;
+constexpr int kAsmGroups = 5;
+constexpr int kAsmPass = kAsmUpWarps * kAsmGroups;            // upper blocks in registers at a time
+constexpr int kAsmPasses = (kMaxNbr + kAsmPass - 1) / kAsmPass;
+constexpr unsigned kSlotDiag = 0xfeu, kSlotNone = 0xffu;       // else the number of the upper block
+
+// Floats per staged row: even, so that pairs stay aligned, and not a multiple of four, so that
+// rows 32 lanes write spread over the banks (two lanes to a bank).
+AFX_HD int asm_stride(int k) {
+    const int s = 6 * (k > 3 ? k : 3) + 2;
+    return s % 4 == 0 ? s + 2 : s;
+}
+
+__global__ void __launch_bounds__(kAsmThreads) jtj_assemble_kernel(GnArgs a) {
+    extern __shared__ float2 asm_dyn[];
+    float* const J = reinterpret_cast<float*>(asm_dyn);             // [256][stride]
+    unsigned* const bm = reinterpret_cast<unsigned*>(asm_dyn);      // neighbour bitmap, before the rows
+    __shared__ int s_L[kMaxNbr];
+    __shared__ uint2 s_slot[kAsmThreads];
+    __shared__ unsigned char s_own[kAsmThreads];
+    __shared__ int s_rows[kAsmThreads / 32];
+    __shared__ int s_dup[kAsmThreads / 32];
+    __shared__ int s_cnt, s_first, s_touched;
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const int n = min(*a.n_nodes, a.n_max), k = a.k, stride = asm_stride(k);
+    const int g = lane / 6, gi = lane % 6;                  // upper blocks: group and block row
+    const int di = lane / 3, dj = (lane % 3) * 2;           // diagonal: lanes 0..17, two entries each
+    for (int node = blockIdx.x; node < n; node += gridDim.x) {
+        const int words = (n + 31) / 32;
+        for (int i = tid; i < words; i += kAsmThreads) bm[i] = 0u;
+        if (tid == 0) s_touched = 0;
+        __syncthreads();
         const unsigned o = a.b.loff[node], e = a.b.loff[node + 1];
-        int qn = 0;  // queued rows (warp-uniform)
-        for (unsigned base = o; base < e; base += 128) {
-            unsigned ent[4];
-            int cj[4];
+        const unsigned io = a.b.ioff[node], nin = a.b.ioff[node + 1] - io;
+        for (unsigned base = o + tid; base < e; base += 2 * kAsmThreads) {
+            const unsigned t1 = base + kAsmThreads;
+            const bool two = t1 < e;
+            const unsigned ent[2] = {a.b.lst[base], two ? a.b.lst[t1] : 0u};
+            long v[2] = {(long)(ent[0] / k), (long)(ent[1] / k)};
+            bool on[2] = {a.corr_of_vertex[v[0]] >= 0, two && a.corr_of_vertex[v[1]] >= 0};
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const unsigned t = base + (unsigned)(j * 32 + lane);
-                ent[j] = t < e ? a.b.lst[t] : 0u;
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const unsigned t = base + (unsigned)(j * 32 + lane);
-                cj[j] = -1;
-                if (t < e) {
-                    cj[j] = a.corr_of_vertex[ent[j] / k];
-                    a.b.jc[t] = cj[j];
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                unsigned bal = __ballot_sync(0xffffffffu, cj[j] >= 0);
-                while (bal) {
-                    unsigned take = bal;
-                    for (int drop = __popc(bal) - (32 - qn); drop > 0; --drop) take &= ~(0x80000000u >> __clz(take));
-                    if (take & (1u << lane)) {
-                        const int pos = qn + __popc(take & ((1u << lane) - 1u));
-                        S.qt[pos] = base + (unsigned)(j * 32 + lane);
-                        S.qe[pos] = ent[j];
-                        S.qc[pos] = cj[j];
-                    }
-                    qn += __popc(take);
-                    bal &= ~take;
-                    __syncwarp();
-                    if (qn == 32) {
-                        run_queue(32);
-                        qn = 0;
-                    }
+            for (int j = 0; j < 2; ++j) {
+                if (!on[j]) continue;
+#pragma unroll 4
+                for (int s = 0; s < k; ++s) {
+                    const uint32_t b = a.midx[v[j] * k + s];
+                    if (a.mw[v[j] * k + s] != 0.f && b != (uint32_t)node && b < (uint32_t)n)
+                        atomicOr(bm + (b >> 5), 1u << (b & 31));
                 }
             }
         }
-        if (qn) run_queue(qn);
+        if (tid < a.kreg) {
+            const uint32_t nb = a.gidx[(long)node * a.kreg + tid];
+            if (nb < (uint32_t)n && nb != (uint32_t)node) atomicOr(bm + (nb >> 5), 1u << (nb & 31));
+        }
+        for (unsigned t = tid; t < nin; t += kAsmThreads) {
+            const unsigned x = a.b.ilst[io + t] / a.kreg;
+            if (x != (unsigned)node) atomicOr(bm + (x >> 5), 1u << (x & 31));
+        }
+        __syncthreads();
+        if (w == 0) {  // ordered extraction
+            int base = 0, first = 0;
+            for (int w0 = 0; w0 < words; w0 += 32) {
+                const int wi = w0 + lane;
+                unsigned bits = wi < words ? bm[wi] : 0u;
+                const int c = __popc(bits);
+                int incl = c;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, incl, d);
+                    if (lane >= d) incl += y;
+                }
+                int pos = base + incl - c;
+                while (bits) {
+                    const int b = wi * 32 + __ffs(bits) - 1;
+                    bits &= bits - 1;
+                    if (pos < kMaxNbr) {
+                        s_L[pos] = b;
+                        a.b.nbr[(long)node * kMaxNbr + pos] = b;
+                        first += b < node;
+                    }
+                    ++pos;
+                }
+                base += __shfl_sync(0xffffffffu, incl, 31);
+            }
+            first = warp_sum(first);
+            if (lane == 0) {
+                s_cnt = min(base, kMaxNbr);
+                s_first = first;
+                a.b.nbr_cnt[node] = min(base, kMaxNbr);
+                if (base > kMaxNbr) atomicOr(a.error, ERRF_CAPACITY);
+            }
+        }
+        __syncthreads();  // the list is complete, the bitmap's room is free
+        const int first = s_first, nup = s_cnt - first;
+        const int* up = s_L + first;
+        float d0 = 0.f, d1 = 0.f;
+        float acc[kAsmPasses][6];
+#pragma unroll
+        for (int p = 0; p < kAsmPasses; ++p)
+#pragma unroll
+            for (int q = 0; q < 6; ++q) acc[p][q] = 0.f;
+
+        // The staged rows (s_rows of every 32) that each group's block takes part in, in order:
+        // calls use(row, slots equal to the block as a byte mask of two words).
+        auto each_row = [&](int pass, auto&& use) {
+            const int u = pass * kAsmPass + g * kAsmUpWarps + w - 1;
+            const unsigned rep = (unsigned)u * 0x01010101u;
+            for (int sub = 0; sub < kAsmThreads / 32; ++sub) {
+                const int nr = s_rows[sub];
+                if (nr == 0) continue;
+                const uint2 x = lane < nr ? s_slot[sub * 32 + lane] : make_uint2(~0u, ~0u);
+                unsigned mask = 0;
+#pragma unroll
+                for (int gg = 0; gg < kAsmGroups; ++gg) {
+                    const int uu = pass * kAsmPass + gg * kAsmUpWarps + w - 1;
+                    if (uu >= nup) break;
+                    const unsigned r4 = (unsigned)uu * 0x01010101u;
+                    const unsigned bal = __ballot_sync(0xffffffffu, (__vcmpeq4(x.x, r4) | __vcmpeq4(x.y, r4)) != 0u);
+                    if (g == gg) mask = bal;
+                }
+                while (mask) {
+                    const int r = sub * 32 + __ffs(mask) - 1;
+                    mask &= mask - 1;
+                    const uint2 y = s_slot[r];
+                    use(r, __vcmpeq4(y.x, rep), __vcmpeq4(y.y, rep));
+                }
+                __syncwarp();
+            }
+        };
+
+        for (unsigned base = o; base < e; base += kAsmThreads) {
+            const unsigned t = base + tid;
+            const unsigned ent = t < e ? a.b.lst[t] : 0u;
+            const long v = ent / k;
+            const int s = (int)(ent % k);
+            const int c = t < e ? a.corr_of_vertex[v] : -1;
+            if (t < e) a.b.jc[t] = c;
+            const unsigned bal = __ballot_sync(0xffffffffu, c >= 0);
+            bool dup = false;
+            if (c >= 0) {
+                const int row = (tid & ~31) + __popc(bal & ((1u << lane) - 1u));
+                const int px = a.corr[2 * (long)c + 1];
+                const float p[3] = {a.mesh[3 * v], a.mesh[3 * v + 1], a.mesh[3 * v + 2]};
+                float wt[8];
+                uint32_t bn[8];
+#pragma unroll
+                for (int tt = 0; tt < 8; ++tt) {
+                    wt[tt] = tt < k ? a.mw[v * k + tt] : 0.f;
+                    bn[tt] = tt < k ? a.midx[v * k + tt] : 0u;
+                }
+                const float nrm[3] = {a.normals[3 * (long)px], a.normals[3 * (long)px + 1], a.normals[3 * (long)px + 2]};
+                float G[3][6];
+                grad_rows(p, G);
+                unsigned lo = ~0u, hi = ~0u;
+                int ndiag = 0;
+                float2* out = reinterpret_cast<float2*>(J + row * stride);
+#pragma unroll
+                for (int tt = 0; tt < 8; ++tt) {
+                    if (tt >= k) break;
+                    unsigned sl = kSlotNone;
+                    if (wt[tt] != 0.f && bn[tt] >= (uint32_t)node) {
+                        if (bn[tt] == (uint32_t)node) {
+                            sl = kSlotDiag;
+                            ++ndiag;
+                        } else {
+                            const int f = find_slot(up, nup, (int)bn[tt]);
+                            if (f >= 0) sl = (unsigned)f;
+                        }
+                    }
+                    if (tt < 4) lo = (lo & ~(0xffu << (8 * tt))) | (sl << (8 * tt));
+                    else hi = (hi & ~(0xffu << (8 * (tt - 4)))) | (sl << (8 * (tt - 4)));
+                    if (sl != kSlotNone || tt == s) {
+                        float Jt[6];
+                        jdepth(nrm, wt[tt], G, a.lam_d, Jt);
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) out[tt * 3 + q] = make_float2(Jt[2 * q], Jt[2 * q + 1]);
+                        if (tt == s) {  // this row's J block, for J^T r
+                            float2* jr = reinterpret_cast<float2*>(a.b.jrow + (long)t * 6);
+#pragma unroll
+                            for (int q = 0; q < 3; ++q) jr[q] = make_float2(Jt[2 * q], Jt[2 * q + 1]);
+                        }
+                    }
+                }
+                s_slot[row] = make_uint2(lo, hi);
+                s_own[row] = (unsigned char)s;
+                dup = ndiag > 1;
+                s_touched = 1;
+            }
+            const bool any_dup = __any_sync(0xffffffffu, dup);
+            if (lane == 0) {
+                s_rows[w] = __popc(bal);
+                s_dup[w] = any_dup;
+            }
+            __syncthreads();
+            if (w == 0) {
+                if (lane < 18)
+                    for (int sub = 0; sub < kAsmThreads / 32; ++sub) {
+                        const int nr = s_rows[sub];
+                        if (!s_dup[sub]) {  // the row's own slot is the only one of this node
+#pragma unroll 4
+                            for (int r = sub * 32; r < sub * 32 + nr; ++r) {
+                                const float* row = J + r * stride + s_own[r] * 6;
+                                const float ja = row[di];
+                                const float2 jb = *reinterpret_cast<const float2*>(row + dj);
+                                d0 = d0 + ja * jb.x;
+                                d1 = d1 + ja * jb.y;
+                            }
+                        } else {
+                            for (int r = sub * 32; r < sub * 32 + nr; ++r) {
+                                const float* row = J + r * stride;
+                                const float ja = row[s_own[r] * 6 + di];
+                                const uint2 y = s_slot[r];
+                                for (int tt = 0; tt < k; ++tt) {
+                                    const unsigned sl = ((tt < 4 ? y.x >> (8 * tt) : y.y >> (8 * (tt - 4))) & 0xffu);
+                                    if (sl != kSlotDiag) continue;
+                                    const float2 jb = *reinterpret_cast<const float2*>(row + tt * 6 + dj);
+                                    d0 = d0 + ja * jb.x;
+                                    d1 = d1 + ja * jb.y;
+                                }
+                            }
+                        }
+                    }
+            } else {
+#pragma unroll
+                for (int pass = 0; pass < kAsmPasses; ++pass) {
+                    if (pass * kAsmPass + w - 1 >= nup) break;
+                    each_row(pass, [&](int r, unsigned lo, unsigned hi) {
+                        const float* row = J + r * stride;
+                        const float ja = row[s_own[r] * 6 + gi];
+                        do {  // slots in order; more than one only where a vertex lists a node twice
+                            int tt;
+                            if (lo) {
+                                tt = (__ffs(lo) - 1) >> 3;
+                                lo &= ~(0xffu << (8 * tt));
+                            } else {
+                                tt = (__ffs(hi) - 1) >> 3;
+                                hi &= ~(0xffu << (8 * tt));
+                                tt += 4;
+                            }
+                            const float2* jb = reinterpret_cast<const float2*>(row + tt * 6);
+#pragma unroll
+                            for (int q = 0; q < 3; ++q) {
+                                const float2 b2 = jb[q];
+                                acc[pass][2 * q] = acc[pass][2 * q] + ja * b2.x;
+                                acc[pass][2 * q + 1] = acc[pass][2 * q + 1] + ja * b2.y;
+                            }
+                        } while (lo | hi);
+                    });
+                }
+            }
+            __syncthreads();
+        }
         // regularisation rows in ascending row order: incoming edges x -> node with x < node,
         // then node's own edges, then incoming edges with x > node (src/MotionOptimization.cu:298-340)
-        const unsigned io = a.b.ioff[node], nin = a.b.ioff[node + 1] - io;
         unsigned nlo = 0;  // incoming rows with source below node (ilst is ascending)
         for (unsigned x = lane; x < nin; x += 32) nlo += (a.b.ilst[io + x] / a.kreg < (unsigned)node) ? 1u : 0u;
         nlo = warp_sum(nlo);
         const unsigned nrows = nin + (unsigned)a.kreg;
-        for (unsigned base = 0; base < nrows; base += 32) {
-            const unsigned r = base + lane;
+        for (unsigned base = 0; base < nrows; base += kAsmThreads) {
+            const unsigned r = base + tid;
             if (r < nrows) {
                 int src, kk;
                 if (r < nlo) {
@@ -393,61 +527,81 @@ __global__ void __launch_bounds__(32 * kJtjWarps) jtj_assemble_kernel(GnArgs a) 
                 }
                 const uint32_t nbk = a.gidx[(long)src * a.kreg + kk];
                 const bool live = !(src == node && nbk >= (uint32_t)n);  // own edge filtered out
-                S.own[lane] = live ? (src == node ? 1 : 0) : -1;
                 float G[3][6];
                 grad_rows(a.nodes + 3 * (long)src, G);
+                float2* out = reinterpret_cast<float2*>(J + tid * stride);
 #pragma unroll
                 for (int ax = 0; ax < 3; ++ax)
 #pragma unroll
-                    for (int q = 0; q < 6; ++q) S.J[lane][ax][q] = G[ax][q] * a.lam_r;
+                    for (int q = 0; q < 3; ++q)
+                        out[ax * 3 + q] = make_float2(G[ax][2 * q] * a.lam_r, G[ax][2 * q + 1] * a.lam_r);
                 const int other = (src == node) ? (int)nbk : src;
-                int sl = -2;
-                if (other > node) {
-                    const int f = find_slot(S.L, cnt, other);
-                    if (f >= 0) sl = f;
+                unsigned sl = kSlotNone;
+                if (live && other > node) {
+                    const int f = find_slot(up, nup, other);
+                    if (f >= 0) sl = (unsigned)f;
                 }
-                S.slot[lane][0] = (signed char)sl;
+                s_slot[tid] = make_uint2(0xffffff00u | sl, ~0u);
+                s_own[tid] = live ? 1 : 0;
+                if (live) s_touched = 1;
             }
-            __syncwarp();
-            const int nb = (int)min(32u, nrows - base);
-            for (int rr = 0; rr < nb; ++rr) {
-                const int self = S.own[rr];
-                if (self < 0) continue;
-                touched = true;
-                const int sl = S.slot[rr][0];
+            if (lane == 0) s_rows[w] = max(0, min(32, (int)(nrows - base) - w * 32));
+            __syncthreads();
+            // the node is an edge's source (coefficient +g) or its target (-g): g_i g_j on the
+            // diagonal and -(g_i g_j) between the two either way
+            if (w == 0) {
+                if (lane < 18) {
+                    const int nb = (int)min((unsigned)kAsmThreads, nrows - base);
+                    for (int r2 = 0; r2 < nb; ++r2) {
+                        if (!s_own[r2]) continue;
 #pragma unroll
-                for (int ax = 0; ax < 3; ++ax) {
-                    const float g_i0 = S.J[rr][ax][i0], g_j0 = S.J[rr][ax][j0];
-                    const float g_i1 = has1 ? S.J[rr][ax][i1] : 0.f, g_j1 = S.J[rr][ax][j1];
-                    // this node is `src` (coefficient +g) or the edge's target (coefficient -g)
-                    const float n_i0 = self ? g_i0 : -g_i0, n_j0 = self ? g_j0 : -g_j0;
-                    const float n_i1 = self ? g_i1 : -g_i1, n_j1 = self ? g_j1 : -g_j1;
-                    d0 = d0 + n_i0 * n_j0;
-                    if (has1) d1 = d1 + n_i1 * n_j1;
-                    if (sl >= 0) {
-                        const float o_j0 = self ? -g_j0 : g_j0, o_j1 = self ? -g_j1 : g_j1;
-                        float* blk = S.blk + sl * 36;
-                        blk[e0] = blk[e0] + n_i0 * o_j0;
-                        if (has1) blk[e1] = blk[e1] + n_i1 * o_j1;
+                        for (int ax = 0; ax < 3; ++ax) {
+                            const float* row = J + r2 * stride + ax * 6;
+                            const float ga = row[di];
+                            const float2 gb = *reinterpret_cast<const float2*>(row + dj);
+                            d0 = d0 + ga * gb.x;
+                            d1 = d1 + ga * gb.y;
+                        }
                     }
                 }
+            } else {
+#pragma unroll
+                for (int pass = 0; pass < kAsmPasses; ++pass) {
+                    if (pass * kAsmPass + w - 1 >= nup) break;
+                    each_row(pass, [&](int r2, unsigned, unsigned) {
+#pragma unroll
+                        for (int ax = 0; ax < 3; ++ax) {
+                            const float* row = J + r2 * stride + ax * 6;
+                            const float ga = row[gi];
+#pragma unroll
+                            for (int q = 0; q < 3; ++q) {
+                                const float2 gb = reinterpret_cast<const float2*>(row)[q];
+                                acc[pass][2 * q] = acc[pass][2 * q] - ga * gb.x;
+                                acc[pass][2 * q + 1] = acc[pass][2 * q + 1] - ga * gb.y;
+                            }
+                        }
+                    });
+                }
             }
-            __syncwarp();
+            __syncthreads();
         }
-        if (!touched) {  // identity diagonal block (src/VolumeFusion.cu:637-640)
-            d0 = (i0 == j0) ? 1.f : 0.f;
-            d1 = (i1 == j1) ? 1.f : 0.f;
+        if (w == 0) {
+            if (!s_touched) {  // identity diagonal block (src/VolumeFusion.cu:637-640)
+                d0 = di == dj ? 1.f : 0.f;
+                d1 = di == dj + 1 ? 1.f : 0.f;
+            }
+            if (lane < 18) reinterpret_cast<float2*>(a.b.diag + (long)node * 36)[lane] = make_float2(d0, d1);
+        } else if (g < kAsmGroups) {
+#pragma unroll
+            for (int pass = 0; pass < kAsmPasses; ++pass) {
+                const int u = pass * kAsmPass + g * kAsmUpWarps + w - 1;
+                if (u >= nup) continue;
+                float2* B = reinterpret_cast<float2*>(a.b.blocks + ((long)node * kMaxNbr + first + u) * 36 + gi * 6);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) B[q] = make_float2(acc[pass][2 * q], acc[pass][2 * q + 1]);
+            }
         }
-        float* D = a.b.diag + (long)node * 36;
-        D[e0] = d0;
-        if (has1) D[e1] = d1;
-        float* B = a.b.blocks + (long)node * kMaxNbr * 36;
-        for (int u = 0; u < cnt; ++u) {
-            if (S.L[u] <= node) continue;
-            B[u * 36 + e0] = S.blk[u * 36 + e0];
-            if (has1) B[u * 36 + e1] = S.blk[u * 36 + e1];
-        }
-        __syncwarp();
+        __syncthreads();  // the shared state is the next node's
     }
 }
 
@@ -509,10 +663,30 @@ AFX_D void diag_inverse_node(const GnArgs& a, int node) {
         for (int i = 0; i < 6; ++i) out[i * 6 + lane - 6] = (float)col[i];
 }
 
-__global__ void __launch_bounds__(128) diag_inverse_kernel(GnArgs a) {
+// What the Gauss-Newton loop needs besides the blocks, in one launch: the inverses (the first `half`
+// CTAs, one node per warp: a serial chain in binary64), and meanwhile the references of the
+// lower blocks, the pending transforms as a copy of the committed ones and the loop's state.
+__global__ void __launch_bounds__(128) gn_icp_finish_kernel(GnArgs a, float4* T_pending, const float4* T_committed,
+                                                           int half) {
     const int n = min(*a.n_nodes, a.n_max);
-    for (int node = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); node < n; node += gridDim.x * (blockDim.x >> 5))
-        diag_inverse_node(a, node);
+    if ((int)blockIdx.x < half) {
+        for (int node = blockIdx.x * 4 + (threadIdx.x >> 5); node < n; node += half * 4) diag_inverse_node(a, node);
+        return;
+    }
+    const long first = (long)(blockIdx.x - half) * blockDim.x + threadIdx.x;
+    const long step = (long)(gridDim.x - half) * blockDim.x;
+    for (long t = first; t < (long)n * kMaxNbr; t += step) nbr_ref_one(a, t);
+    if (T_pending)
+        for (long t = first; t < (long)a.n_max * 4; t += step) T_pending[t] = T_committed[t];
+    if (first == 0) {
+        GnState* s = a.b.state;
+        s->e_prev = 3.4028234663852886e+38;  // std::numeric_limits<float>::max() (src/VolumeFusion.cu:570)
+        s->e_last = 0;
+        s->e_depth = s->e_reg = 0;
+        s->done = 0;
+        s->commit = 0;
+        s->iters = 0;
+    }
 }
 
 // ---- Gauss-Newton loop: one thread-block cluster per ICP iteration ----
@@ -1781,7 +1955,6 @@ size_t gn_workspace_size(long m_max, int n_max, int k, int kreg) {
     s += al((size_t)n_max * 6 * 4) * 5 + al((size_t)n_max * 6 * 4 * 2);  // jtr x r z p, ap + p2
     s += al(m_max * 4) + al((size_t)n_max * kreg * 3 * 4);        // rdepth rreg
     s += al(sizeof(GnState));
-    s += al(scan_workspace_size(m_max > n_max ? m_max : n_max));
     return s + 1024;
 }
 
@@ -1793,13 +1966,13 @@ bool gn_carve(void* ws, size_t bytes, long m_max, int n_max, int k, int kreg, Gn
         p += al(n);
         return q;
     };
-    b->lcnt = (unsigned*)take((n_max + 1) * 4);
-    b->loff = (unsigned*)take((n_max + 1) * 4);
+    b->lcnt = (unsigned*)take((n_max + 1) * 4);  // the four counters together: cleared as one
     b->lcur = (unsigned*)take((n_max + 1) * 4);
-    b->lst = (unsigned*)take(m_max * k * 4);
     b->icnt = (unsigned*)take((n_max + 1) * 4);
-    b->ioff = (unsigned*)take((n_max + 1) * 4);
     b->icur = (unsigned*)take((n_max + 1) * 4);
+    b->loff = (unsigned*)take((n_max + 1) * 4);
+    b->lst = (unsigned*)take(m_max * k * 4);
+    b->ioff = (unsigned*)take((n_max + 1) * 4);
     b->ilst = (unsigned*)take((size_t)n_max * kreg * 4);
     b->nbr_cnt = (int*)take(n_max * 4);
     b->nbr = (int*)take((size_t)n_max * kMaxNbr * 4);
@@ -1818,77 +1991,45 @@ bool gn_carve(void* ws, size_t bytes, long m_max, int n_max, int k, int kreg, Gn
     b->rdepth = (float*)take(m_max * 4);
     b->rreg = (float*)take((size_t)n_max * kreg * 3 * 4);
     b->state = (GnState*)take(sizeof(GnState));
-    b->scan_ws = take(scan_workspace_size(m_max > n_max ? m_max : n_max));
     return true;
 }
+
+constexpr int kNodeCtas = 608;  // CTAs that take one node at a time: four of 256 threads per SM
 
 // Per frame: node -> vertex lists and incoming regularisation edges.
 int gn_frame_setup(const GnArgs& a, cudaStream_t st) {
     const GnBuffers& b = a.b;
-    AFX_CUDA(cudaMemsetAsync(b.lcnt, 0, (a.n_max + 1) * 4, st));
-    AFX_CUDA(cudaMemsetAsync(b.lcur, 0, (a.n_max + 1) * 4, st));
-    AFX_CUDA(cudaMemsetAsync(b.icnt, 0, (a.n_max + 1) * 4, st));
-    AFX_CUDA(cudaMemsetAsync(b.icur, 0, (a.n_max + 1) * 4, st));
-    const long mk = a.m_max * a.k;
-    if (mk > 0) {
-        lst_count_kernel<<<grid_for(mk, 256), 256, 0, st>>>(a);
-        AFX_LAUNCH_CHECK();
-    }
-    int rc = scan_exclusive(b.lcnt, b.loff, a.n_max + 1, nullptr, b.scan_ws, st);
-    if (rc) return rc;
-    if (mk > 0) {
-        lst_fill_kernel<<<grid_for(mk, 256), 256, 0, st>>>(a);
-        AFX_LAUNCH_CHECK();
-    }
-    seg_sort_kernel<<<grid_for_nodes(a.n_max, 1), 256, 0, st>>>(b.lst, b.loff, a.n_nodes, a.n_max, a.error);
+    AFX_CUDA(cudaMemsetAsync(b.lcnt, 0, 4 * al((a.n_max + 1) * 4), st));  // lcnt lcur icnt icur
+    const long items = std::max(a.m_max * a.k, (long)a.n_max * a.kreg);
+    list_count_kernel<<<grid_for(items, 256), 256, 0, st>>>(a);
     AFX_LAUNCH_CHECK();
-    const long nk = (long)a.n_max * a.kreg;
-    in_count_kernel<<<grid_for(nk, 256), 256, 0, st>>>(a);
+    list_scan_kernel<<<2, 1024, 0, st>>>(a);
     AFX_LAUNCH_CHECK();
-    rc = scan_exclusive(b.icnt, b.ioff, a.n_max + 1, nullptr, b.scan_ws, st);
-    if (rc) return rc;
-    in_fill_kernel<<<grid_for(nk, 256), 256, 0, st>>>(a);
+    list_fill_kernel<<<grid_for(items, 256), 256, 0, st>>>(a);
     AFX_LAUNCH_CHECK();
-    seg_sort_kernel<<<grid_for_nodes(a.n_max, 1), 256, 0, st>>>(b.ilst, b.ioff, a.n_nodes, a.n_max, a.error);
+    list_sort_kernel<<<std::min(a.n_max, kNodeCtas), 256, 0, st>>>(a);
     AFX_LAUNCH_CHECK();
     return AFX_OK;
 }
 
-__global__ void gn_state_reset_kernel(GnState* s) {
-    s->e_prev = 3.4028234663852886e+38;  // std::numeric_limits<float>::max() (src/VolumeFusion.cu:570)
-    s->e_last = 0;
-    s->e_depth = s->e_reg = 0;
-    s->done = 0;
-    s->commit = 0;
-    s->iters = 0;
-}
-
 // Per ICP iteration (after correspondences): J^T J structure, blocks and block inverses.
 int gn_icp_setup(const GnArgs& a, float* T_pending, const float* T_committed, cudaStream_t st) {
-    const GnBuffers& b = a.b;
-    gn_state_reset_kernel<<<1, 1, 0, st>>>(b.state);
-    AFX_LAUNCH_CHECK();
-    if (T_pending)
-        AFX_CUDA(cudaMemcpyAsync(T_pending, T_committed, (size_t)a.n_max * 64, cudaMemcpyDeviceToDevice, st));
-    const unsigned nb = grid_for_nodes(a.n_max, kGnWarps);  // grid-stride over the live nodes
     const int words = (a.n_max + 31) / 32;
-    const size_t smem = (size_t)kGnWarps * words * 4;
-    if (smem > 200 * 1024) return AFX_ERR_UNSUPPORTED;
+    if (words > kGnMaxWords) return AFX_ERR_UNSUPPORTED;
+    const size_t smem = std::max((size_t)kAsmThreads * asm_stride(a.k) * 4, (size_t)words * 4);
     static ContextOnce once;  // the opt-in covers every size accepted above
-    if (smem > 48 * 1024) {
+    if (smem > 40 * 1024) {
         const int rc = once_per_context(once, [](int) {
             return note_cuda_error(
-                cudaFuncSetAttribute(nbr_discover_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+                cudaFuncSetAttribute(jtj_assemble_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
         });
         if (rc) return rc;
     }
-    nbr_discover_kernel<<<nb, 32 * kGnWarps, smem, st>>>(a, words);
+    jtj_assemble_kernel<<<std::min(a.n_max, kNodeCtas), kAsmThreads, smem, st>>>(a);
     AFX_LAUNCH_CHECK();
-    nbr_ref_kernel<<<grid_for((long)a.n_max * kMaxNbr, 256), 256, 0, st>>>(a);
-    AFX_LAUNCH_CHECK();
-    jtj_assemble_kernel<<<grid_for_nodes(a.n_max, kJtjWarps), 32 * kJtjWarps, 0, st>>>(a);
-    AFX_LAUNCH_CHECK();
-    diag_inverse_kernel<<<grid_for_nodes(a.n_max, 4), 128, 0, st>>>(a);
+    const int half = std::min((a.n_max + 3) / 4, kNodeCtas);
+    gn_icp_finish_kernel<<<half + grid_for((long)a.n_max * kMaxNbr, 128), 128, 0, st>>>(
+        a, reinterpret_cast<float4*>(T_pending), reinterpret_cast<const float4*>(T_committed), half);
     AFX_LAUNCH_CHECK();
     return AFX_OK;
 }

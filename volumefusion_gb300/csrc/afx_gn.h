@@ -7,7 +7,7 @@ namespace afx {
 
 constexpr int kMaxNbr = 64;      // neighbours per node in J^T J (both sides of the diagonal)
 constexpr int kSegMax = 8192;    // vertices per node list sortable in shared memory
-constexpr int kGnWarps = 4;
+constexpr int kGnMaxWords = 12800;  // bitmap words of the neighbour search: up to 409,600 nodes
 
 struct GnState {
     double e_prev;
@@ -43,7 +43,6 @@ struct GnBuffers {
     float* rdepth;         // [C_max]
     float* rreg;           // [N*kreg*3]
     float* x, *r, *z, *p, *ap;  // PCG vectors [N*6]
-    void* scan_ws;
     GnState* state;
 };
 
