@@ -245,10 +245,12 @@ AFX_D int find_slot(const int* L, int cnt, int b) {
 // are staged 256 at a time (one per thread, the Jacobian block of every slot formed: jdepth, or
 // lam_r * G for a regularisation row) and the blocks are dealt over the CTA: warp 0 sums the
 // diagonal, each of the other warps up to five upper blocks at a time, six lanes to a block, one
-// row of it per lane in registers.  A group visits only the rows of its block (a ballot over the slot
-// bytes of 32 rows gives each group its rows).  The bound is the serial sum of the longest lists:
+// row of it per lane in registers.  A group lists the rows of its block first (ballots over the slot
+// bytes of 32 rows at a time), so that the loads of four rows are in flight while it sums in order; the
+// diagonal takes eight rows at a time.  The bound is the serial sum of the longest lists:
 // with one warp per node walking all rows and the upper blocks in shared memory, the graph of the
-// 256^3 sequence (169 nodes, 900 entries each) took 70 us + 16 us for the neighbours.
+// 256^3 sequence took 70 us and 16 us for the neighbours, against 15 us for both so (and 20 us, or
+// 115 instead of 57 us for 1,500 nodes over 60,000 points, with one row in flight per group).
 constexpr int kAsmThreads = 256;
 constexpr int kAsmUpWarps = kAsmThreads / 32 - 1;
 constexpr int kAsmGroups = 5;
@@ -263,20 +265,30 @@ AFX_HD int asm_stride(int k) {
     return s % 4 == 0 ? s + 2 : s;
 }
 
-__global__ void __launch_bounds__(kAsmThreads) jtj_assemble_kernel(GnArgs a) {
+// Dynamic shared memory: the staged rows (or the neighbour bitmap before them), then a list of
+// rows for every group (row << 6 | own slot << 3 | slot).
+AFX_HD size_t asm_rows_bytes(int k, int words) {
+    const size_t rows = (size_t)kAsmThreads * asm_stride(k) * 4, bits = ((size_t)words * 4 + 7) / 8 * 8;
+    return rows > bits ? rows : bits;
+}
+constexpr size_t kAsmListBytes = (size_t)kAsmPass * kAsmThreads * sizeof(unsigned short);
+
+template <int KM>  // at least k slots per vertex
+__global__ void __launch_bounds__(kAsmThreads, KM <= 4 ? 4 : 3) jtj_assemble_kernel(GnArgs a) {
     extern __shared__ float2 asm_dyn[];
     float* const J = reinterpret_cast<float*>(asm_dyn);             // [256][stride]
     unsigned* const bm = reinterpret_cast<unsigned*>(asm_dyn);      // neighbour bitmap, before the rows
     __shared__ int s_L[kMaxNbr];
     __shared__ uint2 s_slot[kAsmThreads];
-    __shared__ unsigned char s_own[kAsmThreads];
+    __shared__ __align__(8) unsigned char s_own[kAsmThreads];
     __shared__ int s_rows[kAsmThreads / 32];
-    __shared__ int s_dup[kAsmThreads / 32];
     __shared__ int s_cnt, s_first, s_touched;
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const int n = min(*a.n_nodes, a.n_max), k = a.k, stride = asm_stride(k);
     const int g = lane / 6, gi = lane % 6;                  // upper blocks: group and block row
     const int di = lane / 3, dj = (lane % 3) * 2;           // diagonal: lanes 0..17, two entries each
+    unsigned short* const lists = reinterpret_cast<unsigned short*>(
+        reinterpret_cast<char*>(asm_dyn) + asm_rows_bytes(k, (a.n_max + 31) / 32)) + (w - 1) * kAsmGroups * kAsmThreads;
     for (int node = blockIdx.x; node < n; node += gridDim.x) {
         const int words = (n + 31) / 32;
         for (int i = tid; i < words; i += kAsmThreads) bm[i] = 0u;
@@ -353,32 +365,80 @@ __global__ void __launch_bounds__(kAsmThreads) jtj_assemble_kernel(GnArgs a) {
 #pragma unroll
             for (int q = 0; q < 6; ++q) acc[p][q] = 0.f;
 
-        // The staged rows (s_rows of every 32) that each group's block takes part in, in order:
-        // calls use(row, slots equal to the block as a byte mask of two words).
-        auto each_row = [&](int pass, auto&& use) {
-            const int u = pass * kAsmPass + g * kAsmUpWarps + w - 1;
-            const unsigned rep = (unsigned)u * 0x01010101u;
+        // The staged rows (s_rows of every 32) that the block of a group takes part in: a list per group of
+        // this warp, in row order, for rows that name a block once; returns this lane's group's length.
+        auto list_rows = [&](int pass) {
+            int len[kAsmGroups] = {};
             for (int sub = 0; sub < kAsmThreads / 32; ++sub) {
-                const int nr = s_rows[sub];
+                const int nr = s_rows[sub], row = sub * 32 + lane;
                 if (nr == 0) continue;
-                const uint2 x = lane < nr ? s_slot[sub * 32 + lane] : make_uint2(~0u, ~0u);
-                unsigned mask = 0;
+                const uint2 x = lane < nr ? s_slot[row] : make_uint2(~0u, ~0u);
+                const unsigned tag = lane < nr ? (unsigned)row << 6 | (unsigned)s_own[row] << 3 : 0u;
 #pragma unroll
                 for (int gg = 0; gg < kAsmGroups; ++gg) {
                     const int uu = pass * kAsmPass + gg * kAsmUpWarps + w - 1;
                     if (uu >= nup) break;
                     const unsigned r4 = (unsigned)uu * 0x01010101u;
-                    const unsigned bal = __ballot_sync(0xffffffffu, (__vcmpeq4(x.x, r4) | __vcmpeq4(x.y, r4)) != 0u);
-                    if (g == gg) mask = bal;
+                    const unsigned lo = __vcmpeq4(x.x, r4), hi = KM > 4 ? __vcmpeq4(x.y, r4) : 0u;
+                    const unsigned bal = __ballot_sync(0xffffffffu, (lo | hi) != 0u);
+                    if (lo | hi)
+                        lists[gg * kAsmThreads + len[gg] + __popc(bal & ((1u << lane) - 1u))] =
+                            (unsigned short)(tag | (lo ? (__ffs(lo) - 1) >> 3 : 4 + ((__ffs(hi) - 1) >> 3)));
+                    len[gg] += __popc(bal);
                 }
-                while (mask) {
-                    const int r = sub * 32 + __ffs(mask) - 1;
-                    mask &= mask - 1;
-                    const uint2 y = s_slot[r];
-                    use(r, __vcmpeq4(y.x, rep), __vcmpeq4(y.y, rep));
-                }
-                __syncwarp();
             }
+            __syncwarp();
+            int mine = 0;
+#pragma unroll
+            for (int gg = 0; gg < kAsmGroups; ++gg)
+                if (g == gg) mine = len[gg];
+            return mine;
+        };
+        // Upper blocks over the staged depth rows: listed rows, four in flight; or every row looked at
+        // where a vertex of the chunk names a node twice.
+        auto sum_listed = [&](int pass, float (&c)[6]) {
+            const int len = list_rows(pass);
+            const unsigned short* l = lists + min(g, kAsmGroups - 1) * kAsmThreads;
+            for (int i0 = 0; i0 < len; i0 += 4) {
+                float ja[4];
+                float2 jb[4][3];
+                const ushort4 q4 = *reinterpret_cast<const ushort4*>(l + i0);
+                const unsigned q[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const unsigned v = i0 + r < len ? q[r] : q[0];
+                    const float* row = J + (v >> 6) * stride;
+                    ja[r] = row[((v >> 3) & 7u) * 6 + gi];
+#pragma unroll
+                    for (int x = 0; x < 3; ++x) jb[r][x] = reinterpret_cast<const float2*>(row + (v & 7u) * 6)[x];
+                }
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    if (i0 + r >= len) break;
+#pragma unroll
+                    for (int x = 0; x < 3; ++x) {
+                        c[2 * x] = c[2 * x] + ja[r] * jb[r][x].x;
+                        c[2 * x + 1] = c[2 * x + 1] + ja[r] * jb[r][x].y;
+                    }
+                }
+            }
+            __syncwarp();
+        };
+        auto sum_all = [&](int pass, float (&c)[6]) {
+            const int u = pass * kAsmPass + g * kAsmUpWarps + w - 1;
+            if (g < kAsmGroups && u < nup)
+                for (int sub = 0; sub < kAsmThreads / 32; ++sub)
+                    for (int r = sub * 32; r < sub * 32 + s_rows[sub]; ++r) {
+                        const float* row = J + r * stride;
+                        const uint2 y = s_slot[r];
+                        for (int tt = 0; tt < k; ++tt) {
+                            if (((tt < 4 ? y.x >> (8 * tt) : y.y >> (8 * (tt - 4))) & 0xffu) != (unsigned)u) continue;
+                            const float ja = row[s_own[r] * 6 + gi];
+#pragma unroll
+                            for (int q = 0; q < 6; ++q) c[q] = c[q] + ja * row[tt * 6 + q];
+                        }
+                    }
+            __syncwarp();
         };
 
         for (unsigned base = o; base < e; base += kAsmThreads) {
@@ -394,34 +454,33 @@ __global__ void __launch_bounds__(kAsmThreads) jtj_assemble_kernel(GnArgs a) {
                 const int row = (tid & ~31) + __popc(bal & ((1u << lane) - 1u));
                 const int px = a.corr[2 * (long)c + 1];
                 const float p[3] = {a.mesh[3 * v], a.mesh[3 * v + 1], a.mesh[3 * v + 2]};
-                float wt[8];
-                uint32_t bn[8];
+                float wt[KM];
+                uint32_t bn[KM];
 #pragma unroll
-                for (int tt = 0; tt < 8; ++tt) {
+                for (int tt = 0; tt < KM; ++tt) {
                     wt[tt] = tt < k ? a.mw[v * k + tt] : 0.f;
                     bn[tt] = tt < k ? a.midx[v * k + tt] : 0u;
                 }
                 const float nrm[3] = {a.normals[3 * (long)px], a.normals[3 * (long)px + 1], a.normals[3 * (long)px + 2]};
                 float G[3][6];
                 grad_rows(p, G);
-                unsigned lo = ~0u, hi = ~0u;
-                int ndiag = 0;
+                unsigned slots[2] = {~0u, ~0u};
                 float2* out = reinterpret_cast<float2*>(J + row * stride);
 #pragma unroll
-                for (int tt = 0; tt < 8; ++tt) {
+                for (int tt = 0; tt < KM; ++tt) {
                     if (tt >= k) break;
                     unsigned sl = kSlotNone;
                     if (wt[tt] != 0.f && bn[tt] >= (uint32_t)node) {
                         if (bn[tt] == (uint32_t)node) {
                             sl = kSlotDiag;
-                            ++ndiag;
                         } else {
                             const int f = find_slot(up, nup, (int)bn[tt]);
                             if (f >= 0) sl = (unsigned)f;
                         }
                     }
-                    if (tt < 4) lo = (lo & ~(0xffu << (8 * tt))) | (sl << (8 * tt));
-                    else hi = (hi & ~(0xffu << (8 * (tt - 4)))) | (sl << (8 * (tt - 4)));
+                    if (sl != kSlotNone)
+                        dup = dup || ((__vcmpeq4(slots[0], sl * 0x01010101u) | __vcmpeq4(slots[1], sl * 0x01010101u)) != 0u);
+                    slots[tt / 4] ^= (sl ^ 0xffu) << (8 * (tt % 4));
                     if (sl != kSlotNone || tt == s) {
                         float Jt[6];
                         jdepth(nrm, wt[tt], G, a.lam_d, Jt);
@@ -434,29 +493,35 @@ __global__ void __launch_bounds__(kAsmThreads) jtj_assemble_kernel(GnArgs a) {
                         }
                     }
                 }
-                s_slot[row] = make_uint2(lo, hi);
+                s_slot[row] = make_uint2(slots[0], slots[1]);
                 s_own[row] = (unsigned char)s;
-                dup = ndiag > 1;
                 s_touched = 1;
             }
-            const bool any_dup = __any_sync(0xffffffffu, dup);
-            if (lane == 0) {
-                s_rows[w] = __popc(bal);
-                s_dup[w] = any_dup;
-            }
-            __syncthreads();
+            if (lane == 0) s_rows[w] = __popc(bal);
+            const bool twice = __syncthreads_or(dup);
             if (w == 0) {
                 if (lane < 18)
                     for (int sub = 0; sub < kAsmThreads / 32; ++sub) {
                         const int nr = s_rows[sub];
-                        if (!s_dup[sub]) {  // the row's own slot is the only one of this node
-#pragma unroll 4
-                            for (int r = sub * 32; r < sub * 32 + nr; ++r) {
-                                const float* row = J + r * stride + s_own[r] * 6;
-                                const float ja = row[di];
-                                const float2 jb = *reinterpret_cast<const float2*>(row + dj);
-                                d0 = d0 + ja * jb.x;
-                                d1 = d1 + ja * jb.y;
+                        if (!twice) {  // the row's own slot is the only one of this node
+                            for (int r0 = 0; r0 < nr; r0 += 8) {
+                                const uint2 own = *reinterpret_cast<const uint2*>(s_own + sub * 32 + r0);
+                                float ja[8];
+                                float2 jb[8];
+#pragma unroll
+                                for (int r = 0; r < 8; ++r) {
+                                    const unsigned t8 = (r < 4 ? own.x >> (8 * r) : own.y >> (8 * (r - 4))) & 0xffu;
+                                    const bool in = r0 + r < nr;
+                                    const float* row = J + (in ? (sub * 32 + r0 + r) * stride + (int)t8 * 6 : 0);
+                                    ja[r] = row[di];
+                                    jb[r] = *reinterpret_cast<const float2*>(row + dj);
+                                }
+#pragma unroll
+                                for (int r = 0; r < 8; ++r) {
+                                    if (r0 + r >= nr) break;
+                                    d0 = d0 + ja[r] * jb[r].x;
+                                    d1 = d1 + ja[r] * jb[r].y;
+                                }
                             }
                         } else {
                             for (int r = sub * 32; r < sub * 32 + nr; ++r) {
@@ -477,28 +542,8 @@ __global__ void __launch_bounds__(kAsmThreads) jtj_assemble_kernel(GnArgs a) {
 #pragma unroll
                 for (int pass = 0; pass < kAsmPasses; ++pass) {
                     if (pass * kAsmPass + w - 1 >= nup) break;
-                    each_row(pass, [&](int r, unsigned lo, unsigned hi) {
-                        const float* row = J + r * stride;
-                        const float ja = row[s_own[r] * 6 + gi];
-                        do {  // slots in order; more than one only where a vertex lists a node twice
-                            int tt;
-                            if (lo) {
-                                tt = (__ffs(lo) - 1) >> 3;
-                                lo &= ~(0xffu << (8 * tt));
-                            } else {
-                                tt = (__ffs(hi) - 1) >> 3;
-                                hi &= ~(0xffu << (8 * tt));
-                                tt += 4;
-                            }
-                            const float2* jb = reinterpret_cast<const float2*>(row + tt * 6);
-#pragma unroll
-                            for (int q = 0; q < 3; ++q) {
-                                const float2 b2 = jb[q];
-                                acc[pass][2 * q] = acc[pass][2 * q] + ja * b2.x;
-                                acc[pass][2 * q + 1] = acc[pass][2 * q + 1] + ja * b2.y;
-                            }
-                        } while (lo | hi);
-                    });
+                    if (!twice) sum_listed(pass, acc[pass]);
+                    else sum_all(pass, acc[pass]);
                 }
             }
             __syncthreads();
@@ -542,7 +587,7 @@ __global__ void __launch_bounds__(kAsmThreads) jtj_assemble_kernel(GnArgs a) {
                     if (f >= 0) sl = (unsigned)f;
                 }
                 s_slot[tid] = make_uint2(0xffffff00u | sl, ~0u);
-                s_own[tid] = live ? 1 : 0;
+                s_own[tid] = live ? 1 : 0;  // skipped rows name no block and no diagonal
                 if (live) s_touched = 1;
             }
             if (lane == 0) s_rows[w] = max(0, min(32, (int)(nrows - base) - w * 32));
@@ -568,10 +613,12 @@ __global__ void __launch_bounds__(kAsmThreads) jtj_assemble_kernel(GnArgs a) {
 #pragma unroll
                 for (int pass = 0; pass < kAsmPasses; ++pass) {
                     if (pass * kAsmPass + w - 1 >= nup) break;
-                    each_row(pass, [&](int r2, unsigned, unsigned) {
+                    const int len = list_rows(pass);
+                    const unsigned short* l = lists + min(g, kAsmGroups - 1) * kAsmThreads;
+                    for (int x = 0; x < len; ++x) {
 #pragma unroll
                         for (int ax = 0; ax < 3; ++ax) {
-                            const float* row = J + r2 * stride + ax * 6;
+                            const float* row = J + (l[x] >> 6) * stride + ax * 6;
                             const float ga = row[gi];
 #pragma unroll
                             for (int q = 0; q < 3; ++q) {
@@ -580,7 +627,8 @@ __global__ void __launch_bounds__(kAsmThreads) jtj_assemble_kernel(GnArgs a) {
                                 acc[pass][2 * q + 1] = acc[pass][2 * q + 1] - ga * gb.y;
                             }
                         }
-                    });
+                    }
+                    __syncwarp();
                 }
             }
             __syncthreads();
@@ -2016,16 +2064,17 @@ int gn_frame_setup(const GnArgs& a, cudaStream_t st) {
 int gn_icp_setup(const GnArgs& a, float* T_pending, const float* T_committed, cudaStream_t st) {
     const int words = (a.n_max + 31) / 32;
     if (words > kGnMaxWords) return AFX_ERR_UNSUPPORTED;
-    const size_t smem = std::max((size_t)kAsmThreads * asm_stride(a.k) * 4, (size_t)words * 4);
+    const size_t smem = asm_rows_bytes(a.k, words) + kAsmListBytes;
     static ContextOnce once;  // the opt-in covers every size accepted above
-    if (smem > 40 * 1024) {
-        const int rc = once_per_context(once, [](int) {
-            return note_cuda_error(
-                cudaFuncSetAttribute(jtj_assemble_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-        });
-        if (rc) return rc;
-    }
-    jtj_assemble_kernel<<<std::min(a.n_max, kNodeCtas), kAsmThreads, smem, st>>>(a);
+    int rc = once_per_context(once, [](int) {
+        const int most = (int)(std::max(asm_rows_bytes(8, 0), (size_t)kGnMaxWords * 4) + kAsmListBytes);
+        const cudaError_t e = cudaFuncSetAttribute(jtj_assemble_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e != cudaSuccess) return note_cuda_error(e);
+        return note_cuda_error(cudaFuncSetAttribute(jtj_assemble_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    });
+    if (rc) return rc;
+    if (a.k <= 4) jtj_assemble_kernel<4><<<std::min(a.n_max, kNodeCtas), kAsmThreads, smem, st>>>(a);
+    else jtj_assemble_kernel<8><<<std::min(a.n_max, kNodeCtas), kAsmThreads, smem, st>>>(a);
     AFX_LAUNCH_CHECK();
     const int half = std::min((a.n_max + 3) / 4, kNodeCtas);
     gn_icp_finish_kernel<<<half + grid_for((long)a.n_max * kMaxNbr, 128), 128, 0, st>>>(
