@@ -12,7 +12,7 @@
 // J^T J depends only on the canonical geometry, weights and correspondences, so it is
 // assembled once per ICP iteration; J^T r is rebuilt every Gauss-Newton iteration.
 // The solve is a block-Jacobi PCG in one kernel on one cluster: FP32 block SpMV, dot products in
-// triple- (shared-memory path) or double-binary32 (global-memory path), FP64 6x6 block inverses.
+// triple-binary32, FP64 6x6 block inverses.
 #include <algorithm>
 #include <cfloat>
 #include <cstring>
@@ -194,34 +194,6 @@ __global__ void __launch_bounds__(256) list_sort_kernel(GnArgs a) {
 }
 
 // ---- per-ICP assembly ----
-
-// For neighbour slots below the diagonal, find the owner's slot (binary search).
-AFX_D void nbr_ref_one(const GnArgs& a, long t) {
-    const int node = (int)(t / kMaxNbr), u = (int)(t % kMaxNbr);
-    if (u >= a.b.nbr_cnt[node]) return;
-    const int bnode = a.b.nbr[t];
-    if (bnode > node) {
-        a.b.nbr_ref[t] = (int)t;
-        return;
-    }
-    const int* L = a.b.nbr + (long)bnode * kMaxNbr;
-    int lo = 0, hi = a.b.nbr_cnt[bnode] - 1, f = -1;
-    while (lo <= hi) {
-        const int mid = (lo + hi) >> 1;
-        if (L[mid] == node) {
-            f = mid;
-            break;
-        }
-        if (L[mid] < node) lo = mid + 1;
-        else hi = mid - 1;
-    }
-    if (f < 0) {
-        atomicOr(a.error, ERRF_CAPACITY);
-        a.b.nbr_ref[t] = 0;
-        return;
-    }
-    a.b.nbr_ref[t] = -((int)((long)bnode * kMaxNbr + f) + 1);
-}
 
 AFX_D int find_slot(const int* L, int cnt, int b) {
     int lo = 0, hi = cnt - 1;
@@ -711,9 +683,36 @@ AFX_D void diag_inverse_node(const GnArgs& a, int node) {
         for (int i = 0; i < 6; ++i) out[i * 6 + lane - 6] = (float)col[i];
 }
 
+// The blocks of one node below the diagonal, as transposes of the owners' (one warp): with them a
+// node's row of J^T J is its diagonal block and one contiguous run of blocks, in neighbour order.
+AFX_D void lower_blocks_node(const GnArgs& a, int node) {
+    const int lane = threadIdx.x & 31;
+    const int* L = a.b.nbr + (long)node * kMaxNbr;
+    const int cnt = a.b.nbr_cnt[node];
+    for (int u0 = 0; u0 < cnt; u0 += 32) {
+        const int u = u0 + lane;
+        const int owner = u < cnt ? L[u] : node;
+        int f = -1;
+        if (owner < node) {
+            f = find_slot(a.b.nbr + (long)owner * kMaxNbr, a.b.nbr_cnt[owner], node);
+            if (f < 0) atomicOr(a.error, ERRF_CAPACITY);
+        }
+        const int lower = __popc(__ballot_sync(0xffffffffu, owner < node));  // lists ascend: the first ones
+        float* dst = a.b.blocks + ((long)node * kMaxNbr + u0) * 36;
+        const long from = f >= 0 ? ((long)owner * kMaxNbr + f) * 36 : -1;
+#pragma unroll 4
+        for (int e0 = 0; e0 < lower * 36; e0 += 32) {
+            const int e = e0 + lane, q = e / 36, x = e - 36 * q;
+            const long src = __shfl_sync(0xffffffffu, from, q & 31);
+            if (e < lower * 36) dst[e] = src >= 0 ? a.b.blocks[src + (x % 6) * 6 + x / 6] : 0.f;
+        }
+        if (lower < 32) break;
+    }
+}
+
 // What the Gauss-Newton loop needs besides the blocks, in one launch: the inverses (the first `half`
-// CTAs, one node per warp: a serial chain in binary64), and meanwhile the references of the
-// lower blocks, the pending transforms as a copy of the committed ones and the loop's state.
+// CTAs, one node per warp: a serial chain in binary64), and meanwhile the lower blocks, the
+// pending transforms as a copy of the committed ones and the loop's state.
 __global__ void __launch_bounds__(128) gn_icp_finish_kernel(GnArgs a, float4* T_pending, const float4* T_committed,
                                                            int half) {
     const int n = min(*a.n_nodes, a.n_max);
@@ -723,7 +722,7 @@ __global__ void __launch_bounds__(128) gn_icp_finish_kernel(GnArgs a, float4* T_
     }
     const long first = (long)(blockIdx.x - half) * blockDim.x + threadIdx.x;
     const long step = (long)(gridDim.x - half) * blockDim.x;
-    for (long t = first; t < (long)n * kMaxNbr; t += step) nbr_ref_one(a, t);
+    for (int node = (int)(first >> 5); node < n; node += (int)(step >> 5)) lower_blocks_node(a, node);
     if (T_pending)
         for (long t = first; t < (long)a.n_max * 4; t += step) T_pending[t] = T_committed[t];
     if (first == 0) {
@@ -865,10 +864,13 @@ AFX_D float df_quotient(DF a, DF b) {
 
 AFX_D bool df_zero_or_nan(DF v) { return v.hi == 0.f || v.hi != v.hi; }
 
+constexpr int kClusterMax = 16;
+
 struct ClusterSums {
     double slot[2][4];            // this CTA's block sums, double-buffered across calls
     double warp[kLoopWarps * 4];  // per-warp sums
     double total[4];
+    double in[2][kClusterMax][2];  // every CTA's sums (cluster_sum_tf)
     int phase;
 };
 
@@ -883,25 +885,22 @@ AFX_D DF lds_df_local(const double* local) {
     asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.hi), "=f"(v.lo) : "r"(a) : "memory");
     return v;
 }
-AFX_D DF dsmem_load_df(const double* p, unsigned rank) {
-    unsigned local = (unsigned)__cvta_generic_to_shared(p), remote;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
-    DF v;
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.hi), "=f"(v.lo) : "r"(remote) : "memory");
-    return v;
+AFX_D void dsmem_store_df(double* local, unsigned rank, DF v) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(local), ra;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(ra), "f"(v.hi), "f"(v.lo) : "memory");
 }
 
-// The like in double-float arithmetic: the same fixed-shape trees (warp butterfly, the CTA's
-// warps, the CTAs by rank) with df_add, so every thread of every CTA gets identical totals.
-// Contains one cluster barrier.
+// Sums over every thread of the cluster as double-floats, in fixed-shape trees (butterfly within each
+// warp, the CTA's warps, the CTAs by rank): warp 0 puts the CTA's sums into slot [rank] of every
+// CTA, and after the barrier every warp adds its CTA's slots, so all threads of all CTAs hold the same
+// totals.  Contains one cluster barrier.
 template <int NV>
-AFX_D void cluster_sum_df(DF (&v)[NV], ClusterSums& cs) {
+AFX_D void cluster_sum_tf(const TF (&v)[NV], DF (&t)[NV], ClusterSums& cs) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-        DF s = v[i];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s = df_add(s, df_shfl_xor(s, o));
+        const DF s = tf_butterfly<16>(v[i]);
         if (lane == 0) sts_df(&cs.warp[w * 4 + i], s);
     }
     __syncthreads();
@@ -909,28 +908,19 @@ AFX_D void cluster_sum_df(DF (&v)[NV], ClusterSums& cs) {
     if (w == 0) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
-            DF s = {0.f, 0.f};
-            if (lane < kLoopWarps) s = lds_df_local(&cs.warp[lane * 4 + i]);
-#pragma unroll
-            for (int o = kLoopWarps / 2; o > 0; o >>= 1) s = df_add(s, df_shfl_xor(s, o));
-            if (lane == 0) sts_df(&cs.slot[ph][i], s);
+            DF s = lds_df_local(&cs.warp[(lane & (kLoopWarps - 1)) * 4 + i]);
+            s = tf_butterfly<kLoopWarps / 2>({s.hi, s.lo, 0.f});
+            if (lane < (int)cluster_size()) dsmem_store_df(&cs.in[ph][cluster_rank()][i], lane, s);
         }
     }
     cluster_barrier();
-    if (w == 0) {
-        const unsigned ncta = cluster_size();
 #pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            DF t = {0.f, 0.f};
-            if (lane < (int)ncta) t = dsmem_load_df(&cs.slot[ph][i], lane);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) t = df_add(t, df_shfl_xor(t, o));
-            if (lane == 0) sts_df(&cs.total[i], t);
-        }
+    for (int i = 0; i < NV; ++i) {
+        const int q = lane & (kClusterMax - 1);
+        DF s = {0.f, 0.f};
+        if (q < (int)cluster_size()) s = lds_df_local(&cs.in[ph][q][i]);
+        t[i] = tf_butterfly<kClusterMax / 2>({s.hi, s.lo, 0.f});
     }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < NV; ++i) v[i] = lds_df_local(&cs.total[i]);
     if (threadIdx.x == 0) cs.phase = ph ^ 1;
 }
 
@@ -1045,20 +1035,13 @@ AFX_D float spmv_entry(const GnBuffers& b, int node, int i, const float* z) {
         for (int j = 0; j < 6; ++j) s = s + B[j] * __ldcg(x + j);
         acc = acc + s;
     }
-#pragma unroll 2
+#pragma unroll 4
     for (int u = 0; u < cnt; ++u) {
-        const int ref = b.nbr_ref[(long)node * kMaxNbr + u];
         const float* x = z + (long)b.nbr[(long)node * kMaxNbr + u] * 6;
+        const float* B = b.blocks + ((long)node * kMaxNbr + u) * 36 + i * 6;
         float s = 0.f;
-        if (ref >= 0) {
-            const float* B = b.blocks + (long)ref * 36 + i * 6;
 #pragma unroll
-            for (int j = 0; j < 6; ++j) s = s + B[j] * __ldcg(x + j);
-        } else {
-            const float* B = b.blocks + (long)(-ref - 1) * 36 + i;
-#pragma unroll
-            for (int j = 0; j < 6; ++j) s = s + B[j * 6] * __ldcg(x + j);
-        }
+        for (int j = 0; j < 6; ++j) s = s + B[j] * __ldcg(x + j);
         acc = acc + s;
     }
     return acc;
@@ -1080,6 +1063,39 @@ constexpr int kDsNpc = 64;       // nodes per CTA
 constexpr int kDsBlocks = 1024;  // blocks per CTA (diagonal included)
 constexpr int kDsMaxCta = 16;
 
+// Copies of 4 or 16 bytes from global to shared memory that no register waits for; stage_wait before the
+// barrier after which they are read.
+AFX_D void stage_word(int* dst, const int* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+AFX_D void stage_quad(float* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+AFX_D void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// rowptr[0..own] of the nodes from `start` on: a diagonal block and the neighbours' each (whole CTA).
+AFX_D void stage_rowptr(const GnBuffers& b, int* rowptr, int start, int own) {
+    for (int li = threadIdx.x; li < own; li += kLoopThreads) rowptr[li] = 1 + b.nbr_cnt[start + li];
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        int carry = 0;
+        for (int base = 0; base < own; base += 32) {
+            const int li = base + (int)threadIdx.x;
+            const int c = li < own ? rowptr[li] : 0;
+            int incl = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                if ((int)threadIdx.x >= o) incl += y;
+            }
+            if (li < own) rowptr[li] = carry + incl - c;
+            carry += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (threadIdx.x == 0) rowptr[own] = carry;
+    }
+    __syncthreads();
+}
+
 struct DsLayout {
     float* z;       // [kDsNodes * 6] full copy
     float* pf;      // [kDsNodes * 6] full copy of the search direction (each CTA forms it)
@@ -1091,7 +1107,6 @@ struct DsLayout {
     int* col;       // [kDsBlocks] neighbour node of each block
     int* rowptr;    // [kDsNpc + 1]
     double* slot;   // [2][kDsMaxCta][4]
-    int* misc;      // [4]
     unsigned long long* bar;  // [2] mbarriers: p.Ap exchange, r.z exchange
     float* scal;    // [2] beta, stop
 };
@@ -1124,8 +1139,6 @@ AFX_D DsLayout ds_layout(void* base) {
     d.col = ip;
     ip += kDsBlocks;
     d.rowptr = ip;
-    ip += kDsNpc + 1;
-    d.misc = ip;
     return d;
 }
 
@@ -1232,48 +1245,25 @@ AFX_D bool ds_stage(const GnBuffers& b, int n, const DsLayout& d, ClusterSums& c
     const unsigned rank = cluster_rank(), ncta = cluster_size();
     const int npc = (n + (int)ncta - 1) / (int)ncta;
     const int start = min(n, (int)rank * npc), own = min(n, start + npc) - start;
-    if (threadIdx.x < 32) {
-        // row pointers: diagonal + neighbour blocks per own node (one warp, inclusive scan)
-        int carry = 0;
-        for (int base = 0; base < own; base += 32) {
-            const int li = base + (int)threadIdx.x;
-            const int c = li < own ? 1 + b.nbr_cnt[start + li] : 0;
-            int incl = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if ((int)threadIdx.x >= o) incl += y;
-            }
-            if (li < own) d.rowptr[li] = carry + incl - c;
-            carry += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        if (threadIdx.x == 0) {
-            d.rowptr[own] = carry;
-            d.misc[0] = carry;
-        }
-    }
-    __syncthreads();
-    double need[1] = {d.misc[0] > kDsBlocks ? 1.0 : 0.0};
+    stage_rowptr(b, d.rowptr, start, own);
+    double need[1] = {d.rowptr[own] > kDsBlocks ? 1.0 : 0.0};
     ds_sum<1>(need, d, cs, ph);
     if (need[0] != 0.0) return false;
-    // copy the rows (block-major, 36 floats each) and the inverses
+    // the rows (block-major, 36 floats each) and the inverses
     for (int li = threadIdx.x >> 5; li < own; li += kLoopWarps) {
-        const int node = start + li;
+        const long node = start + li;
         const int lane = threadIdx.x & 31;
         const int r0 = d.rowptr[li], cnt = d.rowptr[li + 1] - r0 - 1;
-        for (int e = lane; e < 36; e += 32) {
-            d.blk[r0 * 36 + e] = b.diag[(long)node * 36 + e];
-            d.minv[li * 36 + e] = b.minv[(long)node * 36 + e];
+        if (lane < 9) {
+            stage_quad(d.blk + r0 * 36 + lane * 4, b.diag + node * 36 + lane * 4);
+            stage_quad(d.minv + li * 36 + lane * 4, b.minv + node * 36 + lane * 4);
         }
-        if (lane == 0) d.col[r0] = node;
-        for (int u = 0; u < cnt; ++u) {
-            const int ref = b.nbr_ref[(long)node * kMaxNbr + u];
-            const float* src = b.blocks + (long)(ref >= 0 ? ref : -ref - 1) * 36;
-            float* dst = d.blk + (r0 + 1 + u) * 36;
-            for (int e = lane; e < 36; e += 32) dst[e] = ref >= 0 ? src[e] : src[(e % 6) * 6 + e / 6];
-            if (lane == 0) d.col[r0 + 1 + u] = b.nbr[(long)node * kMaxNbr + u];
-        }
+        if (lane == 0) d.col[r0] = (int)node;
+        for (int u = lane; u < cnt; u += 32) stage_word(d.col + r0 + 1 + u, b.nbr + node * kMaxNbr + u);
+        for (int e = lane; e < cnt * 9; e += 32)
+            stage_quad(d.blk + (r0 + 1) * 36 + e * 4, b.blocks + node * kMaxNbr * 36 + e * 4);
     }
+    stage_wait();
     __syncthreads();
     return true;
 }
@@ -1634,9 +1624,312 @@ AFX_D void gn_jtr(const GnArgs& a, int n, int gw, int nw) {
     }
 }
 
-// PCG with the vectors in global memory (graphs above the shared-memory limit); J^T r from
-// b.jtr, solution in b.x.  Same recurrences and arithmetic as pcg_ds.
-AFX_D void pcg_global(const LoopArgs& L, int n, ClusterSums& cs) {
+// ---- PCG with the vectors in shared memory and the matrix where it fits ----
+//
+// For graphs past the path above: each CTA owns a contiguous node range and keeps in shared memory
+// a full copy of the search direction, its own x, r and A p, its rows' neighbours, and as many of
+// its blocks as there is room for (staged once per Gauss-Newton loop); the rest are read from L2.
+// z travels through global memory: the CTA writes its slice before the barrier of the r.z sum,
+// and after it every CTA forms p = z + beta p over all nodes, so an iteration has two cluster
+// barriers.
+// Bound: for 1,500 nodes the chain of barriers and sums, for 5,000 the blocks from L2 (16 SMs).
+// 1,500 nodes, ten iterations: 103 us; 119 us with all blocks read from shared memory in each, and
+// 298 us with all vectors in global memory (three barriers, one dependent load after the other).
+constexpr int kWideFloats = kDsNodes * 12 + 3 * kDsNpc * 6 + kDsNpc * 36 + kDsBlocks * 36;  // the room from d.z on
+
+struct WideLayout {
+    float *pf, *x, *r, *ap;
+    int *rowptr, *col;  // col: null where the neighbours did not fit
+    float* blk;
+    int cap;            // blocks [0, cap) of the CTA are in shared memory
+};
+
+AFX_D bool wide_fits(int n, int ncta) {
+    const int npc = (n + ncta - 1) / ncta;
+    return ((long)n * 6 + 3) / 4 * 4 + (long)npc * 19 + 1 <= kWideFloats;
+}
+
+AFX_D WideLayout wide_layout(float* room, int n, int npc) {
+    WideLayout d;
+    d.pf = room;
+    d.x = room + (n * 6 + 3) / 4 * 4;
+    d.r = d.x + npc * 6;
+    d.ap = d.r + npc * 6;
+    d.rowptr = reinterpret_cast<int*>(d.ap + npc * 6);
+    return d;
+}
+
+// Row pointers, neighbours and blocks of the own rows; the layout is the same on later calls (`stage` false).
+AFX_D void wide_stage(const GnBuffers& b, WideLayout& d, float* room, int start, int own, bool stage) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (stage) stage_rowptr(b, d.rowptr, start, own);
+    const int nblk = d.rowptr[own];
+    float* p = reinterpret_cast<float*>(d.rowptr + own + 1);
+    float* const end = room + kWideFloats;
+    d.col = nblk <= end - p ? reinterpret_cast<int*>(p) : nullptr;
+    if (d.col) p += nblk;
+    p = room + ((p - room) + 3) / 4 * 4;
+    d.blk = p;
+    d.cap = p < end ? min(nblk, (int)((end - p) / 36)) : 0;
+    if (!stage) return;
+    for (int li = w; li < own; li += kLoopWarps) {
+        const long node = start + li;
+        const int r0 = d.rowptr[li], cnt = d.rowptr[li + 1] - r0 - 1;
+        if (d.col) {
+            if (lane == 0) d.col[r0] = (int)node;
+            for (int u = lane; u < cnt; u += 32) stage_word(d.col + r0 + 1 + u, b.nbr + node * kMaxNbr + u);
+        }
+        const int in = min(cnt + 1, max(0, d.cap - r0)) * 9;
+        for (int e = lane; e < in; e += 32)
+            stage_quad(d.blk + (long)r0 * 36 + e * 4, e < 9 ? b.diag + node * 36 + e * 4 : b.blocks + node * kMaxNbr * 36 + (e - 9) * 4);
+    }
+    stage_wait();
+    __syncthreads();
+}
+
+// A p of the own rows from `first` on, into d.ap, and this thread's part of p.Ap.  kR lanes per row: each
+// multiplies one of kR blocks and the products are added in block order in every lane, as one lane alone would.
+template <int kR>
+AFX_D void wide_spmv(const GnBuffers& b, const WideLayout& d, int start, int own, int first, TF& pap) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, part = lane % kR, cnt = own * 6;
+    constexpr int kRows = 32 / kR;      // per warp
+    constexpr int kH = kR == 1 ? 4 : 2;  // blocks of a lane in flight
+    for (int base = first + w * kRows; base < cnt; base += kLoopWarps * kRows) {
+        const int row = base + lane / kR;
+        const bool on = row < cnt;
+        const int li = on ? row / 6 : 0, i = on ? row - 6 * li : 0;
+        const int r0 = d.rowptr[li], nb = on ? d.rowptr[li + 1] - r0 : 0;
+        const int most = __reduce_max_sync(0xffffffffu, nb);
+        float acc = 0.f;
+        auto add = [&](const float2 (&B)[kH][3], const int (&c)[kH], int k0) {
+            float s[kH];
+#pragma unroll
+            for (int h = 0; h < kH; ++h) {
+                const float2* xv = reinterpret_cast<const float2*>(d.pf) + c[h] * 3;
+                s[h] = 0.f;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    const float2 x = xv[q];
+                    s[h] = s[h] + B[h][q].x * x.x;
+                    s[h] = s[h] + B[h][q].y * x.y;
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < kH; ++h)
+#pragma unroll
+                for (int q = 0; q < kR; ++q) {
+                    const float sq = kR == 1 ? s[h] : __shfl_sync(0xffffffffu, s[h], (lane & ~(kR - 1)) + q);
+                    if (k0 + kR * h + q < nb) acc = acc + sq;
+                }
+        };
+        if (__all_sync(0xffffffffu, r0 + nb <= d.cap) && d.col) {
+            const float2* Bp = reinterpret_cast<const float2*>(d.blk) + r0 * 18 + i * 3;
+            const int* cp = d.col + r0;
+            for (int k0 = 0; k0 < most; k0 += kR * kH) {
+                float2 B[kH][3];
+                int c[kH];
+#pragma unroll
+                for (int h = 0; h < kH; ++h) {
+                    const int u = k0 + kR * h + part < nb ? k0 + kR * h + part : 0;
+                    c[h] = cp[u];
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) B[h][q] = Bp[u * 18 + q];
+                }
+                add(B, c, k0);
+            }
+        } else {
+            const long node = start + li;
+            for (int k0 = 0; k0 < most; k0 += kR * kH) {
+                float2 B[kH][3];
+                int c[kH];
+#pragma unroll
+                for (int h = 0; h < kH; ++h) {
+                    const int u = k0 + kR * h + part < nb ? k0 + kR * h + part : 0;
+                    c[h] = d.col ? d.col[r0 + u] : (u ? b.nbr[node * kMaxNbr + u - 1] : (int)node);
+                    const float2* src =
+                        reinterpret_cast<const float2*>((u ? b.blocks + (node * kMaxNbr + u - 1) * 36 : b.diag + node * 36) + i * 6);
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) B[h][q] = __ldg(src + q);
+                }
+                add(B, c, k0);
+            }
+        }
+        if (on && part == 0) {
+            d.ap[row] = acc;
+            pap = tf_add_prod(pap, d.pf[start * 6 + row], acc);
+        }
+    }
+}
+
+template <bool kTol>
+AFX_D void pcg_wide(const LoopArgs& L, int n, float* room, ClusterSums& cs, bool stage) {
+    const GnBuffers& b = L.g.b;
+    const unsigned rank = cluster_rank(), ncta = cluster_size();
+    const int npc = (n + (int)ncta - 1) / (int)ncta;
+    const int start = min(n, (int)rank * npc), own = min(n, start + npc) - start, cnt = own * 6;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int grp = lane / 6, ei = lane - 6 * grp;
+    WideLayout d = wide_layout(room, n, npc);
+    wide_stage(b, d, room, start, own, stage);
+    constexpr int NV = kTol ? 2 : 1;
+    TF sum[NV];
+    DF tot[NV];
+    // r -= alpha A p, x += alpha p (first: x = 0, r = b), z = M^-1 r to global memory, r.z (and r.r);
+    // kAhead nodes of a lane group at a time, so that their loads are in flight together
+    auto update = [&](bool first, float alpha) {
+        constexpr int kAhead = 3;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) sum[i] = {0.f, 0.f, 0.f};
+        for (int base = w * 5; base < own; base += kAhead * kLoopWarps * 5) {
+            float rv[kAhead];
+            float2 M[kAhead][3];
+            bool act[kAhead];
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) {
+                const int li = base + k * kLoopWarps * 5 + grp;
+                act[k] = lane < 30 && li < own;
+                const float2* Mi = reinterpret_cast<const float2*>(b.minv + (long)(act[k] ? start + li : 0) * 36 + ei * 6);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) M[k][q] = lane < 30 ? Mi[q] : make_float2(0.f, 0.f);
+                const int o = li * 6 + ei;
+                rv[k] = 0.f;
+                if (!act[k]) continue;
+                if (first) {
+                    d.x[o] = 0.f;
+                    rv[k] = __ldcg(b.jtr + (long)start * 6 + o);
+                } else {
+                    d.x[o] = d.x[o] + alpha * d.pf[start * 6 + o];
+                    rv[k] = d.r[o] - alpha * d.ap[o];
+                }
+                d.r[o] = rv[k];
+            }
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) {
+                const int li = base + k * kLoopWarps * 5 + grp;
+                float rq[6], zi = 0.f;
+#pragma unroll
+                for (int q = 0; q < 6; ++q) rq[q] = __shfl_sync(0xffffffffu, rv[k], lane < 30 ? grp * 6 + q : q);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    zi = zi + M[k][q].x * rq[2 * q];
+                    zi = zi + M[k][q].y * rq[2 * q + 1];
+                }
+                if (!act[k]) continue;
+                __stcg(b.z + (long)(start + li) * 6 + ei, zi);
+                sum[0] = tf_add_prod(sum[0], rv[k], zi);
+                if constexpr (kTol) sum[NV - 1] = tf_add_prod(sum[NV - 1], rv[k], rv[k]);
+            }
+        }
+        cluster_sum_tf<NV>(sum, tot, cs);
+    };
+    update(true, 0.f);
+    // a thread keeps the first blocks of one of the first rows in registers for the whole solve
+    constexpr int kRowBlocks = 6;
+    const int row = threadIdx.x, re = row % 6;
+    const int r0 = row < cnt ? d.rowptr[row / 6] : 0, nb = row < cnt ? d.rowptr[row / 6 + 1] - r0 : 0;
+    auto block_row = [&](int u, int& c) {
+        const long node = start + row / 6;
+        c = d.col ? d.col[r0 + u] : (u ? b.nbr[node * kMaxNbr + u - 1] : (int)node);
+        const float* B = r0 + u < d.cap ? d.blk + (r0 + u) * 36
+                                        : (u ? b.blocks + (node * kMaxNbr + u - 1) * 36 : b.diag + node * 36);
+        return reinterpret_cast<const float2*>(B + re * 6);
+    };
+    float2 A[kRowBlocks][3];
+    int off[kRowBlocks];  // in float2
+#pragma unroll
+    for (int k = 0; k < kRowBlocks; ++k) {
+        off[k] = 0;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) A[k][q] = make_float2(0.f, 0.f);
+        if (k >= nb) continue;
+        int c;
+        const float2* src = block_row(k, c);
+        off[k] = c * 3;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) A[k][q] = src[q];
+    }
+    DF rz = tot[0];
+    const float tol2 = kTol ? (float)(L.tol * L.tol) : 0.f, bn = tot[NV - 1].hi;
+    float beta = 0.f;
+    for (int it = 0; it < L.pcg_iters; ++it) {
+        // p = z (first iteration) or z + beta p for all nodes
+        const float4* z4 = reinterpret_cast<const float4*>(b.z);
+        float4* p4 = reinterpret_cast<float4*>(d.pf);
+        constexpr int kBatch = 6;
+        for (int i0 = threadIdx.x; i0 < n * 6 / 4; i0 += kBatch * kLoopThreads) {
+            float4 v[kBatch];
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q) {
+                const int i = i0 + q * kLoopThreads;
+                v[q] = __ldcg(z4 + (i < n * 6 / 4 ? i : i0));
+            }
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q) {
+                const int i = i0 + q * kLoopThreads;
+                if (i >= n * 6 / 4) break;
+                if (it) {
+                    const float4 o = p4[i];
+                    v[q] = make_float4(v[q].x + beta * o.x, v[q].y + beta * o.y, v[q].z + beta * o.z, v[q].w + beta * o.w);
+                }
+                p4[i] = v[q];
+            }
+        }
+        for (int i = n * 6 / 4 * 4 + threadIdx.x; i < n * 6; i += kLoopThreads) {
+            const float zi = __ldcg(b.z + i);
+            d.pf[i] = it ? zi + beta * d.pf[i] : zi;
+        }
+        __syncthreads();
+        TF pap[1] = {{0.f, 0.f, 0.f}};
+        DF tp[1];
+        if (row < cnt) {
+            float acc = 0.f;
+#pragma unroll
+            for (int k = 0; k < kRowBlocks; ++k) {
+                const float2* xv = reinterpret_cast<const float2*>(d.pf) + off[k];
+                float s = 0.f;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    const float2 x = xv[q];
+                    s = s + A[k][q].x * x.x;
+                    s = s + A[k][q].y * x.y;
+                }
+                if (k < nb) acc = acc + s;
+            }
+#pragma unroll 2
+            for (int u = kRowBlocks; u < nb; ++u) {
+                int c;
+                const float2* src = block_row(u, c);
+                const float2* xv = reinterpret_cast<const float2*>(d.pf) + c * 3;
+                float s = 0.f;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    const float2 B = src[q], x = xv[q];
+                    s = s + B.x * x.x;
+                    s = s + B.y * x.y;
+                }
+                acc = acc + s;
+            }
+            d.ap[row] = acc;
+            pap[0] = tf_add_prod(pap[0], d.pf[start * 6 + row], acc);
+        }
+        // further rows: one lane each where they fill the CTA about three times more, else four
+        if (cnt >= 4 * kLoopThreads - 32) wide_spmv<1>(b, d, start, own, kLoopThreads, pap[0]);
+        else wide_spmv<4>(b, d, start, own, kLoopThreads, pap[0]);
+        cluster_sum_tf<1>(pap, tp, cs);
+        if (df_zero_or_nan(tp[0])) break;
+        update(false, df_quotient(rz, tp[0]));
+        beta = df_quotient(tot[0], rz);
+        rz = tot[0];
+        if (kTol && tot[NV - 1].hi <= tol2 * bn) break;
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < cnt; t += kLoopThreads) __stcg(b.x + (long)start * 6 + t, d.x[t]);
+}
+
+// PCG with the vectors in global memory, for graphs whose search direction does not fit in shared memory
+// either (past kWideFloats, about 7,300 nodes); J^T r from b.jtr, solution in b.x.  Same
+// recurrences and arithmetic as pcg_wide.
+__device__ __noinline__ void pcg_global(const LoopArgs& L, int n, ClusterSums& cs) {
     const GnBuffers& b = L.g.b;
     const unsigned rank = cluster_rank(), ncta = cluster_size();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1645,7 +1938,8 @@ AFX_D void pcg_global(const LoopArgs& L, int n, ClusterSums& cs) {
     const bool glane = lane < 30;
     const int gstep = nw * 5;
     // x = 0, r = b, z = M^-1 r; rz = r.z, bb = b.b
-    DF d2[2] = {{0.f, 0.f}, {0.f, 0.f}};
+    TF d2[2] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+    DF tot[2], tp[1];
     for (int base = gw * 5; base < n; base += gstep) {  // warp-uniform trip count
         const int node = base + grp;
         const bool act = glane && node < n;
@@ -1662,14 +1956,14 @@ AFX_D void pcg_global(const LoopArgs& L, int n, ClusterSums& cs) {
             __stcg(b.x + o, 0.f);
             __stcg(b.r + o, ji);
             __stcg(b.z + o, zi);
-            d2[0] = df_add(d2[0], df_prod(ji, zi));
-            d2[1] = df_add(d2[1], df_prod(ji, ji));
+            d2[0] = tf_add_prod(d2[0], ji, zi);
+            d2[1] = tf_add_prod(d2[1], ji, ji);
         }
     }
-    cluster_sum_df<2>(d2, cs);
+    cluster_sum_tf<2>(d2, tot, cs);
     // six lanes per node (entry i = lane % 6 of node group lane / 6, five groups per warp)
-    DF rz = d2[0];
-    const DF bnorm2 = d2[1];
+    DF rz = tot[0];
+    const DF bnorm2 = tot[1];
     const float tol2 = L.tol > 0 ? (float)(L.tol * L.tol) : 0.f;
     float beta = 0.f;
     for (int it = 0; it < L.pcg_iters; ++it) {
@@ -1683,19 +1977,19 @@ AFX_D void pcg_global(const LoopArgs& L, int n, ClusterSums& cs) {
             }
         }
         cluster_barrier();
-        DF pap[1] = {{0.f, 0.f}};
+        TF pap[1] = {{0.f, 0.f, 0.f}};
         if (glane)
             for (int node = gw * 5 + grp; node < n; node += gstep) {
                 const long o = (long)node * 6 + ei;
                 const float api = spmv_entry(b, node, ei, b.p);
                 __stcg(b.ap + o, api);
-                pap[0] = df_add(pap[0], df_prod(__ldcg(b.p + o), api));
+                pap[0] = tf_add_prod(pap[0], __ldcg(b.p + o), api);
             }
-        cluster_sum_df<1>(pap, cs);
-        if (df_zero_or_nan(pap[0])) break;
-        const float alpha = df_quotient(rz, pap[0]);
+        cluster_sum_tf<1>(pap, tp, cs);
+        if (df_zero_or_nan(tp[0])) break;
+        const float alpha = df_quotient(rz, tp[0]);
         // x += alpha p; r -= alpha A p; z = M^-1 r; r.z, r.r
-        DF q2[2] = {{0.f, 0.f}, {0.f, 0.f}};
+        TF q2[2] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
         for (int base = gw * 5; base < n; base += gstep) {
             const int node = base + grp;
             const bool act = glane && node < n;
@@ -1715,14 +2009,14 @@ AFX_D void pcg_global(const LoopArgs& L, int n, ClusterSums& cs) {
             }
             if (act) {
                 __stcg(b.z + o, zi);
-                q2[0] = df_add(q2[0], df_prod(rv, zi));
-                q2[1] = df_add(q2[1], df_prod(rv, rv));
+                q2[0] = tf_add_prod(q2[0], rv, zi);
+                q2[1] = tf_add_prod(q2[1], rv, rv);
             }
         }
-        cluster_sum_df<2>(q2, cs);
-        beta = df_quotient(q2[0], rz);
-        rz = q2[0];
-        if (L.tol > 0 && q2[1].hi <= tol2 * bnorm2.hi) break;
+        cluster_sum_tf<2>(q2, tot, cs);
+        beta = df_quotient(tot[0], rz);
+        rz = tot[0];
+        if (L.tol > 0 && tot[1].hi <= tol2 * bnorm2.hi) break;
     }
 }
 
@@ -1829,13 +2123,16 @@ AFX_D void gn_rewarp(const GnArgs& a, const float* points, float* warped, const 
 
 // One solve from b.jtr: x in b.x (and in the own slices of the shared-memory layout); with
 // L.T_pending set, T_pending -= [x] as well.  Ends with a cluster barrier.
+// `first`: the first solve of the launch.
 AFX_D void gn_solve(const LoopArgs& L, int n, bool ds, const DsLayout& dsl, ClusterSums& cs, DsExchange& ex, long gt,
-                    long gstride) {
+                    long gstride, bool first) {
     if (ds) {
         if (L.tol > 0) pcg_ds<true>(L, n, dsl, ex);
         else pcg_ds<false>(L, n, dsl, ex);
     } else {
-        pcg_global(L, n, cs);
+        if (!wide_fits(n, (int)cluster_size())) pcg_global(L, n, cs);
+        else if (L.tol > 0) pcg_wide<true>(L, n, dsl.z, cs, first);
+        else pcg_wide<false>(L, n, dsl.z, cs, first);
         cluster_barrier();  // x complete
         if (L.T_pending) update_transforms_range(L.T_pending, L.g.b.x, 0, n, gt, gstride);
     }
@@ -1903,7 +2200,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) gn_loop_kernel(LoopArgs L) {
             for (long t = gstride - 1 - gt; t < (long)n * 16; t += gstride) L.T_committed[t] = __ldcg(L.T_pending + t);
         gn_jtr(a, n, gw, nw);
         cluster_barrier();
-        gn_solve(L, n, ds, dsl, cs, ex, gt, gstride);
+        gn_solve(L, n, ds, dsl, cs, ex, gt, gstride, iter == 0);
         if (ds) {
             stage_node_T(L.T_pending, n, dsl);
             gn_rewarp(a, L.points, L.warped, Ts, m, gt, gstride);
@@ -1934,7 +2231,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) gn_solve_kernel(LoopArgs L) {
     int ds_ph = 0;
     DsExchange ex{{0u, 0u}, false};
     const bool ds = n > 0 && (n + (int)ncta - 1) / (int)ncta <= kDsNpc && ds_stage(a.b, n, dsl, cs, ds_ph);
-    gn_solve(L, n, ds, dsl, cs, ex, gt, gstride);
+    gn_solve(L, n, ds, dsl, cs, ex, gt, gstride, true);
     // no CTA leaves while another may still read its shared memory
     cluster_barrier();
 }
@@ -1997,7 +2294,7 @@ size_t gn_workspace_size(long m_max, int n_max, int k, int kreg) {
     size_t s = 0;
     s += 3 * al((n_max + 1) * 4) + al(m_max * k * 4);           // lcnt loff lcur lst
     s += 3 * al((n_max + 1) * 4) + al((size_t)n_max * kreg * 4);  // icnt ioff icur ilst
-    s += al(n_max * 4) + 2 * al((size_t)n_max * kMaxNbr * 4);     // nbr_cnt nbr nbr_ref
+    s += al(n_max * 4) + al((size_t)n_max * kMaxNbr * 4);         // nbr_cnt nbr
     s += al((size_t)n_max * kMaxNbr * 36 * 4) + al((size_t)n_max * 36 * 4) + al((size_t)n_max * 36 * 4);
     s += al((size_t)m_max * k * 6 * 4) + al((size_t)m_max * k * 4);  // jrow jc
     s += al((size_t)n_max * 6 * 4) * 5 + al((size_t)n_max * 6 * 4 * 2);  // jtr x r z p, ap + p2
@@ -2024,7 +2321,6 @@ bool gn_carve(void* ws, size_t bytes, long m_max, int n_max, int k, int kreg, Gn
     b->ilst = (unsigned*)take((size_t)n_max * kreg * 4);
     b->nbr_cnt = (int*)take(n_max * 4);
     b->nbr = (int*)take((size_t)n_max * kMaxNbr * 4);
-    b->nbr_ref = (int*)take((size_t)n_max * kMaxNbr * 4);
     b->blocks = (float*)take((size_t)n_max * kMaxNbr * 36 * 4);
     b->diag = (float*)take((size_t)n_max * 36 * 4);
     b->minv = (float*)take((size_t)n_max * 36 * 4);
@@ -2077,7 +2373,7 @@ int gn_icp_setup(const GnArgs& a, float* T_pending, const float* T_committed, cu
     else jtj_assemble_kernel<8><<<std::min(a.n_max, kNodeCtas), kAsmThreads, smem, st>>>(a);
     AFX_LAUNCH_CHECK();
     const int half = std::min((a.n_max + 3) / 4, kNodeCtas);
-    gn_icp_finish_kernel<<<half + grid_for((long)a.n_max * kMaxNbr, 128), 128, 0, st>>>(
+    gn_icp_finish_kernel<<<half + grid_for((long)a.n_max * 32, 128), 128, 0, st>>>(
         a, reinterpret_cast<float4*>(T_pending), reinterpret_cast<const float4*>(T_committed), half);
     AFX_LAUNCH_CHECK();
     return AFX_OK;

@@ -32,8 +32,7 @@ struct GnBuffers {
     // per ICP iteration
     int* nbr_cnt;          // [N]
     int* nbr;              // [N*kMaxNbr] sorted neighbour ids
-    int* nbr_ref;          // [N*kMaxNbr] block index (owner*kMaxNbr + slot), negative = transpose of -(ref+1)
-    float* blocks;         // [N*kMaxNbr*36] upper blocks (a,b), b > a, row-major
+    float* blocks;         // [N*kMaxNbr*36] blocks (a, b) of the neighbours b, row-major; b < a: the transpose of (b, a)
     float* diag;           // [N*36]
     float* minv;           // [N*36] inverse diagonal blocks (FP64 Gauss-Jordan, stored FP32)
     float* jrow;           // [M*K*6] depth-row Jacobian block of each node-list entry (per ICP iteration)
