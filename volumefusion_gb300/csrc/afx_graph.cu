@@ -717,78 +717,409 @@ int build_graph_impl(float* nodes, float* radii, float* T, int* n_nodes, int cap
 }
 
 // ------------------------------------------------------------------------------------
-// KNN (getKnnData<K>): brute force over node tiles in shared memory, per-thread sorted
-// top-(K[+1]) list by (nanoflann squared distance, node index).
+// KNN (getKnnData<K>): the K[+1] nodes first by (nanoflann squared distance, node index).
 // ------------------------------------------------------------------------------------
+//
+// Searches, by what the call brings:
+//   few queries (kKnnFewQueries, as when the nodes are the queries): a warp per query.  Each lane finds its
+//   smallest distance; the KK-th smallest of those bounds the KK-th of all, so a second pass
+//   collects few candidates, which are then ranked;
+//   many queries: a thread per query with its best KK in registers.  Every CTA sorts the nodes by x into shared
+//   memory (bins: about 3 us), and a warp goes outwards from the x range of its 32 queries until the
+//   gap exceeds every lane's KK-th distance.  Point clouds come sorted by x, so that range is narrow;
+//   few nodes, a shape whose windows would be wide, or warps whose queries are in no order: all nodes in
+//   index order, from shared memory;
+//   more nodes than fit there, or coordinates that are not finite: tile by tile.
+// Bound: instructions, about 15 per distance and 25 per insertion, and below some thousand queries the latency of
+// building and of one query.  In the 512^3 sequence (1,300 nodes): 330,000 points, K = 4, 83 -> 16 us; the nodes
+// among themselves, K = 8, 99 -> 8 us; in the 256^3 sequence (170 nodes) 10.2 -> 8.3 and 15.4 -> 4.2 us (before:
+// every thread walked all nodes).
+// kKnnFewQueries: a warp per query takes 8.4, 12.7 and 31 us for 2,000 queries and 170, 1,300 and 5,000 nodes of
+// a sphere, all nodes by a thread 12.7, 56 and 189; 10, 25 and 75 us for 8,000 (12.6, 56, 188, and a window 15, 35, 60),
+// 31, 101 and 328 us for 40,000 (14.6, 66, 216, and a window 17, 36, 62).
+// kKnnWindowShare: 300 nodes, K = 4: on a sphere (0.39 by the estimate) a window takes 21 us for 16,000 queries and all
+// nodes 17; on a tube along x (0.15) 13 and 17.
 
 constexpr int kKnnTile = 1024;
-constexpr int kKnnThreads = 128;
+constexpr int kKnnThreads = 1024;
+constexpr int kKnnWarps = kKnnThreads / 32;
+constexpr long kKnnFewQueries = 8192;
+constexpr int kKnnCandidates = 96;     // per query of the first search
+constexpr int kKnnBins = 1024;
+constexpr int kKnnScanNodes = 128;       // fewer are not worth sorting
+constexpr float kKnnWindowShare = 0.35f;  // of the nodes: windows not narrower are not worth their bookkeeping
+static_assert(kKnnBins == kKnnThreads, "a thread scans a bin");
+constexpr size_t kKnnRoom = 220 * 1024;
+constexpr size_t kKnnSide = (size_t)kKnnWarps * kKnnCandidates * 8;  // candidates, or the bins
+constexpr int kKnnMaxNodes = (int)((kKnnRoom - kKnnSide) / sizeof(float4));
 
-// One thread per query point (grid-stride over blocks of points, so a block that has no points
-// left loads no nodes).  The running list holds the best KK (distance, index) pairs in
-// registers: a candidate that beats the last entry (or fills an empty slot) replaces it and
-// bubbles up past strictly larger distances, so equal distances keep the earlier index, as the
-// ordered insertion did.  Empty slots carry index -1 and sort last.
 template <int KK>
-__global__ void __launch_bounds__(kKnnThreads) knn_kernel(uint32_t* idx, float* dist, const float* __restrict__ nodes,
-                                                          const int* n_nodes, int n_max, const float* __restrict__ pts,
-                                                          const unsigned* count, long m_max, int k, int excl) {
-    __shared__ float s_n[kKnnTile * 3];
+struct KnnList {
+    float d[KK];
+    int i[KK];
+    AFX_D void clear() {
+#pragma unroll
+        for (int s = 0; s < KK; ++s) {
+            d[s] = INFINITY;
+            i[s] = 0x7fffffff;  // empty: after every node at any distance
+        }
+    }
+    // In any order of calls, for distances that are not NaN.
+    AFX_D void offer(float nd, int ni) {
+        if (!(nd <= d[KK - 1])) return;
+        if (nd == d[KK - 1] && ni > i[KK - 1]) return;
+        d[KK - 1] = nd;
+        i[KK - 1] = ni;
+#pragma unroll
+        for (int p = KK - 1; p > 0; --p) {
+            const bool up = d[p] < d[p - 1] || (d[p] == d[p - 1] && i[p] < i[p - 1]);
+            const float dp = d[p], dq = d[p - 1];
+            const int ip = i[p], iq = i[p - 1];
+            d[p] = up ? dq : dp;
+            d[p - 1] = up ? dp : dq;
+            i[p] = up ? iq : ip;
+            i[p - 1] = up ? ip : iq;
+        }
+    }
+    // In ascending index order (any distances): a candidate that beats the last entry, or fills an empty
+    // slot, replaces it and passes strictly larger distances, so equal ones keep the earlier index.
+    AFX_D void offer_next(float nd, int ni) {
+        if (i[KK - 1] != 0x7fffffff && !(nd < d[KK - 1])) return;
+        d[KK - 1] = nd;
+        i[KK - 1] = ni;
+#pragma unroll
+        for (int p = KK - 1; p > 0; --p) {
+            if (i[p - 1] == 0x7fffffff || d[p] < d[p - 1]) {
+                const float td = d[p];
+                d[p] = d[p - 1];
+                d[p - 1] = td;
+                const int ti = i[p];
+                i[p] = i[p - 1];
+                i[p - 1] = ti;
+            }
+        }
+    }
+    AFX_D void store(uint32_t* idx, float* dist, long q, int k, int excl) const {
+#pragma unroll
+        for (int s = 0; s < KK; ++s) {
+            const int o = s - excl;
+            if (o < 0 || o >= k) continue;
+            const bool have = i[s] != 0x7fffffff;
+            idx[q * k + o] = have ? (uint32_t)i[s] : AFX_INVALID_INDEX;
+            dist[q * k + o] = have ? sqrtf(d[s]) : FLT_MAX;
+        }
+    }
+};
+
+// One query by a warp over nodes in index order (`p`, in shared or global memory).
+template <int KK>
+AFX_D void knn_by_warp(const float (&q)[3], const float* p, int n, unsigned long long* cand, uint32_t* idx, float* dist, long i,
+                       int k, int excl) {
+    const int lane = threadIdx.x & 31;
+    float least = INFINITY;
+    bool nan = false;
+#pragma unroll 4
+    for (int j = lane; j < n; j += 32) {
+        const float d = l2sq_nanoflann(q, p + 3 * j);
+        nan |= d != d;
+        least = fminf(least, d);
+    }
+    int rank = 0;
+#pragma unroll 8
+    for (int o = 0; o < 32; ++o) {
+        const float v = __shfl_sync(0xffffffffu, least, o);
+        rank += v < least || (v == least && o < lane);
+    }
+    const float bound = __shfl_sync(0xffffffffu, least, __ffs(__ballot_sync(0xffffffffu, rank == KK - 1)) - 1);
+    int have = 0;
+    if (!__any_sync(0xffffffffu, nan))
+        for (int j0 = 0; j0 < n && have <= kKnnCandidates; j0 += 32) {
+            const int j = j0 + lane;
+            const float d = j < n ? l2sq_nanoflann(q, p + 3 * j) : INFINITY;
+            const bool in = j < n && d <= bound;
+            const unsigned bal = __ballot_sync(0xffffffffu, in);
+            const int at = have + __popc(bal & ((1u << lane) - 1u));
+            if (in && at < kKnnCandidates) cand[at] = (unsigned long long)__float_as_uint(d) << 32 | (unsigned)j;
+            have += __popc(bal);
+        }
+    else
+        have = kKnnCandidates + 1;
+    if (have > kKnnCandidates) {  // distances that are not numbers, or a crowd of equal ones: in index order
+        if (lane == 0) {
+            KnnList<KK> best;
+            best.clear();
+            for (int j = 0; j < n; ++j) best.offer_next(l2sq_nanoflann(q, p + 3 * j), j);
+            best.store(idx, dist, i, k, excl);
+        }
+        __syncwarp();
+        return;
+    }
+    __syncwarp();
+    for (int c = lane; c < have; c += 32) {
+        const unsigned long long key = cand[c];
+        int r = 0;
+#pragma unroll 4
+        for (int o = 0; o < have; ++o) r += cand[o] < key;
+        r -= excl;
+        if (r >= 0 && r < k) {
+            idx[i * k + r] = (uint32_t)key;
+            dist[i * k + r] = sqrtf(__uint_as_float((unsigned)(key >> 32)));
+        }
+    }
+    for (int r = max(have - excl, 0) + lane; r < k; r += 32) {
+        idx[i * k + r] = AFX_INVALID_INDEX;
+        dist[i * k + r] = FLT_MAX;
+    }
+    __syncwarp();
+}
+
+AFX_D unsigned knn_key(float v) {  // ascending
+    const unsigned b = __float_as_uint(v);
+    return b & 0x80000000u ? ~b : b | 0x80000000u;
+}
+AFX_D float knn_unkey(unsigned k) { return __uint_as_float(k & 0x80000000u ? k & 0x7fffffffu : ~k); }
+
+// The nodes by ascending bin of x, with their indices (the whole CTA; n <= kKnnMaxNodes).  Returns the x that a node
+// may lie before another one further on by, or a negative value where nothing was sorted: a coordinate is not finite,
+// or a window would not be much narrower than all nodes.
+template <int KK>
+AFX_D float knn_sort_x(const float* __restrict__ nodes, int n, float4* list, unsigned* bins, float& x0, float& scale,
+                       bool& finite) {
+    __shared__ unsigned s_min[3], s_max[3], s_bad, s_sum[kKnnWarps];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    if (tid < 3) {
+        s_min[tid] = 0xffffffffu;
+        s_max[tid] = 0u;
+    }
+    if (tid == 3) s_bad = 0u;
+    bins[tid] = 0u;
+    __syncthreads();
+    unsigned lo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, hi[3] = {0u, 0u, 0u};
+    bool bad = false;
+    for (int j = tid; j < n; j += kKnnThreads)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float v = nodes[3 * j + c];
+            bad |= !isfinite(v);
+            lo[c] = min(lo[c], knn_key(v));
+            hi[c] = max(hi[c], knn_key(v));
+        }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        lo[c] = __reduce_min_sync(0xffffffffu, lo[c]);
+        hi[c] = __reduce_max_sync(0xffffffffu, hi[c]);
+        if (lane == 0 && lo[c] <= hi[c]) {
+            atomicMin(s_min + c, lo[c]);
+            atomicMax(s_max + c, hi[c]);
+        }
+    }
+    if (bad) s_bad = 1u;
+    __syncthreads();
+    x0 = knn_unkey(s_min[0]);
+    const float ext = knn_unkey(s_max[0]) - x0, ey = knn_unkey(s_max[1]) - knn_unkey(s_min[1]),
+                ez = knn_unkey(s_max[2]) - knn_unkey(s_min[2]);
+    scale = ext > 0.f ? (kKnnBins - 0.5f) / ext : 0.f;
+    finite = !s_bad && isfinite(ext) && isfinite(scale);  // the same in every thread, as what follows
+    if (!finite) return -1.f;
+    // The distance of the KK-th node, if they lie evenly on a surface of half the bounding box's: a window is about
+    // three of it wide (the farthest of 32 queries sets it).
+    const float reach = sqrtf(0.41f * KK * (ext * ey + ey * ez + ext * ez) / (float)n);
+    if (!(3.f * reach < kKnnWindowShare * ext)) return -1.f;
+    auto bin = [&](float x) { return min(kKnnBins - 1, (int)((x - x0) * scale)); };
+    for (int j = tid; j < n; j += kKnnThreads) atomicAdd(bins + bin(nodes[3 * j]), 1u);
+    __syncthreads();
+    const unsigned v = bins[tid];
+    unsigned x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) s_sum[w] = x;
+    __syncthreads();
+    unsigned t = s_sum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, t, o);
+        if (lane >= o) t += y;
+    }
+    t = __shfl_sync(0xffffffffu, t, w > 0 ? w - 1 : 0);
+    bins[tid] = x - v + (w > 0 ? t : 0u);
+    __syncthreads();
+    for (int j = tid; j < n; j += kKnnThreads) {
+        const float p[3] = {nodes[3 * j], nodes[3 * j + 1], nodes[3 * j + 2]};
+        list[atomicAdd(bins + bin(p[0]), 1u)] = make_float4(p[0], p[1], p[2], __int_as_float(j));
+    }
+    __syncthreads();
+    return ext * (1.02f / kKnnBins);
+}
+
+// The nodes of a warp's 32 queries (those with `on`).  Bin b's nodes end at bins[b]; `copy`: the nodes in
+// index order in shared memory, if they fit.
+template <int KK>
+AFX_D void knn_window(const float (&q)[3], bool on, const float4* list, const float* copy, const float* nodes, int n,
+                      const unsigned* bins, float x0, float scale, float slack, KnnList<KK>& best) {
+    const unsigned key = knn_key(q[0]);
+    const float qlo = knn_unkey(__reduce_min_sync(0xffffffffu, on ? key : 0xffffffffu));
+    const float qhi = knn_unkey(__reduce_max_sync(0xffffffffu, on ? key : 0u));
+    auto look = [&](int a, int b) {
+#pragma unroll 4
+        for (int j = a; j < b; ++j) {
+            const float4 v = list[j];
+            const float p[3] = {v.x, v.y, v.z};
+            best.offer(l2sq_nanoflann(q, p), __float_as_int(v.w));
+        }
+    };
+    auto bin = [&](float x) { return (int)fminf(fmaxf((x - x0) * scale, 0.f), (float)(kKnnBins - 1)); };
+    const int b0 = bin(qlo), b1 = bin(qhi);
+    int left = b0 > 0 ? (int)bins[b0 - 1] : 0, right = (int)bins[b1];
+    if (right - left > kKnnWindowShare * n) {  // queries in no order: all nodes, in theirs
+        if (copy) {
+#pragma unroll 4
+            for (int j = 0; j < n; ++j) best.offer_next(l2sq_nanoflann(q, copy + 3 * j), j);
+        } else {
+#pragma unroll 4
+            for (int j = 0; j < n; ++j) best.offer_next(l2sq_nanoflann(q, nodes + 3 * j), j);
+        }
+        return;
+    }
+    look(left, right);
+    constexpr int kStep = 8;
+    bool more_left = left > 0, more_right = right < n;
+    while (more_left || more_right) {
+        const float worst = __uint_as_float(__reduce_max_sync(0xffffffffu, on ? __float_as_uint(best.d[KK - 1]) : 0u));
+        if (more_right) {
+            const float gap = list[right].x - slack - qhi;
+            if (gap > 0.f && gap * gap * 0.9999f > worst) {
+                more_right = false;
+            } else {
+                const int to = min(right + kStep, n);
+                look(right, to);
+                right = to;
+                more_right = right < n;
+            }
+        }
+        if (more_left) {
+            const float gap = qlo - slack - list[left - 1].x;
+            if (gap > 0.f && gap * gap * 0.9999f > worst) {
+                more_left = false;
+            } else {
+                const int to = max(left - kStep, 0);
+                look(to, left);
+                left = to;
+                more_left = left > 0;
+            }
+        }
+    }
+}
+
+template <int KK>
+__global__ void __launch_bounds__(kKnnThreads, 1) knn_kernel(uint32_t* idx, float* dist, const float* __restrict__ nodes,
+                                                             const int* n_nodes, int n_max, const float* __restrict__ pts,
+                                                             const unsigned* count, long m_max, int k, int excl, size_t room) {
+    extern __shared__ float4 knn_smem[];
     const int n = min(*n_nodes, n_max);
     const long m = count ? min((long)*count, m_max) : m_max;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long first = (long)w * gridDim.x + blockIdx.x, step = (long)gridDim.x * kKnnWarps;  // of warps, over all SMs first
+    if ((long)blockIdx.x >= m) return;
+    float4* const list = knn_smem + kKnnSide / sizeof(float4);
+    if (m <= kKnnFewQueries) {
+        unsigned long long* cand = reinterpret_cast<unsigned long long*>(knn_smem) + w * kKnnCandidates;
+        const float* p = nodes;
+        if (n <= kKnnMaxNodes) {
+            float* s = reinterpret_cast<float*>(list);
+            for (int t = threadIdx.x; t < 3 * n; t += kKnnThreads) s[t] = nodes[t];
+            __syncthreads();
+            p = s;
+        }
+        for (long i = first; i < m; i += step) {
+            const float q[3] = {pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]};
+            knn_by_warp<KK>(q, p, n, cand, idx, dist, i, k, excl);
+        }
+        return;
+    }
+    unsigned* const bins = reinterpret_cast<unsigned*>(knn_smem);
+    float x0 = 0.f, scale = 0.f;
+    bool scan = n <= kKnnScanNodes, finite = true;
+    const float slack = !scan && n <= kKnnMaxNodes ? knn_sort_x<KK>(nodes, n, list, bins, x0, scale, finite) : -1.f;
+    scan = scan || (n <= kKnnMaxNodes && finite && slack < 0.f);
+    if (scan || slack >= 0.f) {
+        // in index order: the scan's nodes, or those of warps that leave the window (beside the sorted ones if there is room)
+        float* const copy = reinterpret_cast<float*>(list + n);
+        const bool copied = !scan && 28 * (size_t)n <= room;
+        if (scan) {
+            for (int j = threadIdx.x; j < n; j += kKnnThreads)
+                list[j] = make_float4(nodes[3 * j], nodes[3 * j + 1], nodes[3 * j + 2], 0.f);
+        } else if (copied) {
+            for (int t = threadIdx.x; t < 3 * n; t += kKnnThreads) copy[t] = nodes[t];
+        }
+        __syncthreads();
+        for (long t = first; t * 32 < m; t += step) {
+            const long i = t * 32 + lane;
+            float q[3] = {0.f, 0.f, 0.f};
+            if (i < m)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) q[c] = pts[3 * i + c];
+            const bool on = i < m && isfinite(q[0]) && isfinite(q[1]) && isfinite(q[2]);
+            KnnList<KK> best;
+            best.clear();
+            if (scan) {
+#pragma unroll 4
+                for (int j = 0; j < n; ++j) {
+                    const float4 v = list[j];
+                    const float p[3] = {v.x, v.y, v.z};
+                    best.offer_next(l2sq_nanoflann(q, p), j);
+                }
+            } else if (__any_sync(0xffffffffu, on)) {
+                knn_window<KK>(q, on, list, copied ? copy : nullptr, nodes, n, bins, x0, scale, slack, best);
+            }
+            if (!scan && i < m && !on) {
+                best.clear();
+                for (int j = 0; j < n; ++j) best.offer_next(l2sq_nanoflann(q, nodes + 3 * j), j);
+            }
+            if (i < m) best.store(idx, dist, i, k, excl);
+            __syncwarp();
+        }
+        return;
+    }
+    __syncthreads();
+    float* s_n = reinterpret_cast<float*>(knn_smem);
     for (long blk = blockIdx.x; blk * kKnnThreads < m; blk += gridDim.x) {
         const long i = blk * kKnnThreads + threadIdx.x;
         float q[3] = {0.f, 0.f, 0.f};
-        if (i < m) {
-            q[0] = pts[3 * i];
-            q[1] = pts[3 * i + 1];
-            q[2] = pts[3 * i + 2];
-        }
-        float bd[KK];
-        int bi[KK];
+        if (i < m)
 #pragma unroll
-        for (int s = 0; s < KK; ++s) {
-            bd[s] = 0.f;
-            bi[s] = -1;
-        }
+            for (int c = 0; c < 3; ++c) q[c] = pts[3 * i + c];
+        KnnList<KK> best;
+        best.clear();
         for (int base = 0; base < n; base += kKnnTile) {
             const int nt = min(kKnnTile, n - base);
             __syncthreads();
-            for (int t = threadIdx.x; t < nt * 3; t += blockDim.x) s_n[t] = nodes[3 * (long)base + t];
+            for (int t = threadIdx.x; t < nt * 3; t += kKnnThreads) s_n[t] = nodes[3 * (long)base + t];
             __syncthreads();
             if (i < m)
-                for (int j = 0; j < nt; ++j) {
-                    const float d = l2sq_nanoflann(q, s_n + 3 * j);
-                    if (bi[KK - 1] >= 0 && !(d < bd[KK - 1])) continue;
-                    bd[KK - 1] = d;
-                    bi[KK - 1] = base + j;
-#pragma unroll
-                    for (int p = KK - 1; p > 0; --p) {
-                        if (bi[p - 1] < 0 || bd[p] < bd[p - 1]) {
-                            const float td = bd[p];
-                            bd[p] = bd[p - 1];
-                            bd[p - 1] = td;
-                            const int ti = bi[p];
-                            bi[p] = bi[p - 1];
-                            bi[p - 1] = ti;
-                        }
-                    }
-                }
+                for (int j = 0; j < nt; ++j) best.offer_next(l2sq_nanoflann(q, s_n + 3 * j), base + j);
         }
-        if (i < m)
-#pragma unroll
-            for (int s = 0; s < KK; ++s) {
-                const int o = s - excl;
-                if (o < 0 || o >= k) continue;
-                if (bi[s] >= 0) {
-                    idx[i * k + o] = (uint32_t)bi[s];
-                    dist[i * k + o] = sqrtf(bd[s]);
-                } else {
-                    idx[i * k + o] = AFX_INVALID_INDEX;
-                    dist[i * k + o] = FLT_MAX;
-                }
-            }
+        if (i < m) best.store(idx, dist, i, k, excl);
     }
+}
+
+template <int KK>
+static int launch_knn(uint32_t* idx, float* dist, const float* nodes, const int* n_nodes, int n_max, const float* pts,
+                      const unsigned* count, long m_max, int k, int excl, cudaStream_t st) {
+    static ContextOnce once;
+    const int rc = once_per_context(once, [](int) {
+        return note_cuda_error(
+            cudaFuncSetAttribute(knn_kernel<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kKnnRoom));
+    });
+    if (rc) return rc;
+    // for the nodes: sorted, and in index order while both fit
+    const size_t most = kKnnRoom - kKnnSide, room = 28 * (size_t)n_max < most ? 28 * (size_t)n_max : most;
+    knn_kernel<KK><<<(unsigned)(m_max < 152 ? m_max : 152), kKnnThreads, kKnnSide + room, st>>>(
+        idx, dist, nodes, n_nodes, n_max, pts, count, m_max, k, excl, room);
+    AFX_LAUNCH_CHECK();
+    return AFX_OK;
 }
 
 int knn_impl(uint32_t* idx, float* dist, const float* nodes, const int* n_nodes, int n_max, const float* pts,
@@ -796,12 +1127,7 @@ int knn_impl(uint32_t* idx, float* dist, const float* nodes, const int* n_nodes,
     if (m_max <= 0) return AFX_OK;
     const int e = excl ? 1 : 0;
     const int kk = k + e;
-    // grid-stride over the live points; the search loop is long, so up to 8 blocks per SM
-    const long want = (m_max + kKnnThreads - 1) / kKnnThreads;
-    const unsigned blocks = (unsigned)(want < 1216 ? want : 1216);
-#define AFX_KNN(KK)                                                                                              \
-    knn_kernel<KK><<<blocks, kKnnThreads, 0, st>>>(idx, dist, nodes, n_nodes, n_max, pts, count, m_max, k, e); \
-    break
+#define AFX_KNN(KK) return launch_knn<KK>(idx, dist, nodes, n_nodes, n_max, pts, count, m_max, k, e, st)
     switch (kk) {
         case 1: AFX_KNN(1);
         case 2: AFX_KNN(2);
@@ -822,8 +1148,6 @@ int knn_impl(uint32_t* idx, float* dist, const float* nodes, const int* n_nodes,
             }
     }
 #undef AFX_KNN
-    AFX_LAUNCH_CHECK();
-    return AFX_OK;
 }
 
 __global__ void filter_disconnected_kernel(uint32_t* idx, float* dist, const int* n_nodes, int n_max, int k,
