@@ -49,6 +49,9 @@ const char* afx_status_string(int status);
 int afx_version(void);
 /* Last CUDA error seen by the library on this thread (cudaError_t value), 0 if none. */
 int afx_last_cuda_error(void);
+/* Wait until the work enqueued on `stream` is done: what the reference's CUDA_CHECK(cudaDeviceSynchronize())
+ * after every operator is for its callers (src/Helper.cu:7-20). */
+int afx_stream_synchronize(void* stream);
 
 /* af::CameraDistortion (include/af/CameraModel.h:21-33), filled from depthDistortion.txt
  * (af::loadCameraDistortion, src/dataset.cpp:44-79: file order k1 k2 p1 p2 k3 k4 k5 k6). */

@@ -58,6 +58,7 @@ SIGNATURES = {
     "afx_status_string": (C.c_char_p, [i32]),
     "afx_version": (i32, []),
     "afx_last_cuda_error": (i32, []),
+    "afx_stream_synchronize": (i32, [vp]),
     "afx_depth_from_mm": (i32, [vp, vp, i64, vp]),
     "afx_filter_depth": (i32, [vp, i64, f32, vp]),
     "afx_filter_depth_fill": (i32, [vp, i64, f32, f32, vp]),

@@ -303,6 +303,8 @@ int afx_version(void) { return 100; }
 
 int afx_last_cuda_error(void) { return g_last_cuda_error; }
 
+int afx_stream_synchronize(void* stream) { return note_cuda_error(cudaStreamSynchronize(as_stream(stream))); }
+
 void afx_fusion_default_params(afx_fusion_params* p) {
     std::memset(p, 0, sizeof(*p));
     p->width = 640;
