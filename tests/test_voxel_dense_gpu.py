@@ -1,0 +1,89 @@
+"""The dense per-voxel kernels at the sizes of their splits: rows of a multiple of four voxels and others, volumes
+around the 128 voxels a warp takes, and arrays that start on 16 bytes or do not.  Voxel centres against their
+formula in binary32; the warp, weights, collisions and integration of sparse counts against numpy or the other path,
+bit for bit."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+F = np.float32
+
+
+def cu(a, offset=0):
+    """On the GPU, `offset` elements after a 16-byte boundary."""
+    a = np.ascontiguousarray(a)
+    buf = torch.empty(a.size + offset, dtype=torch.from_numpy(a).dtype, device="cuda")
+    out = buf[offset:].view(a.shape)
+    out.copy_(torch.from_numpy(a))
+    return out
+
+
+@pytest.mark.parametrize("dims", [(4, 1, 1), (1, 1, 1), (3, 5, 2), (8, 7, 9), (64, 5, 3), (66, 5, 3), (132, 17, 2)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_vertices(dims, offset):
+    from volumefusion_gb300 import af
+    size = tuple(F(0.013) * d for d in dims)
+    vs = tuple(F(s) / F(d) for s, d in zip(size, dims))
+    S = int(np.prod(dims))
+    v = cu(np.full((S, 3), 7, F), offset)
+    af.runGenerateTsdfVerticesKernel(v, vs, size, dims)
+    ax = [np.arange(d, dtype=F) * x - F(s) * F(0.5) for d, x, s in zip(dims, vs, size)]
+    z, y, x = np.meshgrid(ax[2], ax[1], ax[0], indexing="ij")
+    assert np.array_equal(v.cpu().numpy(), np.stack([x, y, z], -1).reshape(-1, 3))
+
+
+@pytest.mark.parametrize("S", [1, 127, 128, 129, 1024, 1025, 70001])
+@pytest.mark.parametrize("k", [4, 6])
+def test_weights_and_warp(S, k):
+    from volumefusion_gb300 import af
+    rng = np.random.default_rng(S + k)
+    n = 40
+    cnt = np.where(rng.random(S) < 0.3, rng.integers(1, k + 1, S), 0).astype(np.int32)
+    idx = rng.integers(0, n, (S, k)).astype(np.int32)
+    idx[np.arange(k)[None] >= cnt[:, None]] = -1
+    dist = rng.uniform(0, 0.04, (S, k)).astype(F)
+    radii = rng.uniform(0.01, 0.03, n).astype(F)
+    T = np.tile(np.eye(4, dtype=F).reshape(-1), (n, 1)) + rng.normal(0, 0.01, (n, 16)).astype(F)
+    verts = rng.normal(size=(S, 3)).astype(F)
+    out = []
+    for offset in (0, 1):
+        w = cu(np.full((S, k), 3, F), offset)
+        v = cu(verts, offset)
+        c, i = cu(cnt, offset), cu(idx, offset)
+        af.runComputeTsdfWarpWeightsKernel(w, cu(radii), i, cu(dist, offset), c, S)
+        w[torch.from_numpy(rng.random(S) < 0.05).cuda()] = 0.0
+        if out:
+            w.copy_(torch.from_numpy(out[0][0]))
+        af.runWarpTsdfKernel(v, cu(T, offset), i, w, c, None, None, (S, 1, 1))
+        out.append((w.cpu().numpy(), v.cpu().numpy()))
+    assert np.array_equal(out[0][1], out[1][1])
+    w, v = out[0]
+    assert (w[(cnt == 0) & (w != 0).all(1)] == 3).all()
+    zero = (np.abs(w) <= F(1e-5)).all(1) | (cnt == 0)
+    q = np.zeros((S, 3), F)
+    for s in range(k):
+        M = T[np.maximum(idx[:, s], 0)].reshape(-1, 4, 4)
+        o = ((M[:, 0, :3] * verts[:, :1] + M[:, 1, :3] * verts[:, 1:2]) + M[:, 2, :3] * verts[:, 2:]) + M[:, 3, :3]
+        q = np.where((s < cnt)[:, None], q + w[:, s:s + 1] * o, q)
+    assert np.array_equal(v, np.where(zero[:, None], verts, q))
+
+
+@pytest.mark.parametrize("dims", [(1, 1, 1), (127, 1, 1), (128, 1, 1), (43, 3, 1), (64, 16, 1), (41, 25, 1), (50, 40, 30)])
+def test_collisions(dims):
+    from volumefusion_gb300 import af
+    rng = np.random.default_rng(dims[0])
+    S = int(np.prod(dims))
+    size = tuple(F(0.01) * F(d) for d in dims)
+    vs = tuple(F(s) / F(d) for s, d in zip(size, dims))
+    cnt = (rng.random(S) < 0.3).astype(np.int32)
+    target = rng.integers(-1, max(S // 3, 1), S)  # several voxels to a target; -1: outside
+    t = np.maximum(target, 0)
+    cell = np.stack([t % dims[0], (t // dims[0]) % dims[1], t // (dims[0] * dims[1])], -1)
+    verts = ((cell + 0.5) * np.array(vs, np.float64) - 0.5 * np.array(size, np.float64)).astype(F)
+    verts[target < 0] = 9.0
+    counts = torch.zeros(S, dtype=torch.int32, device="cuda")
+    af.runCountCollisionsPerVoxelKernel(counts, cu(verts), cu(cnt), vs, size, dims, np.eye(3), (0.0, 0.0, 0.0))
+    want = np.bincount(target[(target >= 0) & (cnt > 0)], minlength=S)
+    assert np.array_equal(counts.cpu().numpy(), want)
