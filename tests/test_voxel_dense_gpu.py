@@ -87,3 +87,47 @@ def test_collisions(dims):
     af.runCountCollisionsPerVoxelKernel(counts, cu(verts), cu(cnt), vs, size, dims, np.eye(3), (0.0, 0.0, 0.0))
     want = np.bincount(target[(target >= 0) & (cnt > 0)], minlength=S)
     assert np.array_equal(counts.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("dims,n,k,lattice", [((8, 8, 8), 1, 4, False), ((9, 7, 17), 30, 3, False), ((24, 16, 8), 190, 8, False),
+                                              ((16, 16, 16), 125, 4, True), ((20, 9, 12), 60, 1, True), ((16, 8, 8), 40, 6, False)])
+def test_supporters(dims, n, k, lattice):
+    """More supporters than k, equal distances (by node), up to the number of nodes a brick holds."""
+    from volumefusion_gb300 import af
+    rng = np.random.default_rng(n + k)
+    size = tuple(F(0.01) * F(d) for d in dims)
+    vs = tuple(F(s) / F(d) for s, d in zip(size, dims))
+    half = np.array([F(s) * F(0.5) for s in size], F)
+    if lattice:
+        m = int(round(n ** (1 / 3)) + 1)
+        grid = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+        nodes = (grid * F(0.02) + np.array(vs, F) - half).astype(F)
+    else:
+        nodes = (rng.uniform(-0.6, 0.6, (n, 3)) * np.array(size)).astype(F)
+    radii = rng.uniform(0.012, 0.03, n).astype(F) if not lattice else np.full(n, 0.02, F)
+    per = np.array([2 * (int(F(0.02) / v) + 1) + 1 for v in vs], np.int32)
+    S = int(np.prod(dims))
+    idx = torch.empty((S, k), dtype=torch.int32, device="cuda")
+    dist = torch.empty((S, k), device="cuda")
+    cnt = torch.empty(S, dtype=torch.int32, device="cuda")
+    af.runTsdfKNNGraph(idx, dist, cnt, cu(nodes), cu(radii), n, vs, size, dims, per)
+    ax = [np.arange(d, dtype=F) * v - h for d, v, h in zip(dims, vs, half)]
+    z, y, x = np.meshgrid(*[np.arange(d) for d in (dims[2], dims[1], dims[0])], indexing="ij")
+    vox = np.stack([x, y, z], -1).reshape(-1, 3)
+    p = np.stack([ax[c][vox[:, c]] for c in range(3)], -1)
+    inv = np.array([F(1.0 / float(v)) for v in vs], F)
+    base = np.trunc((nodes + half) * inv).astype(np.int64)
+    lo = base - (per - 1) // 2
+    D = np.full((S, n), np.inf, F)
+    for j in range(n):
+        d = p - nodes[j]
+        r = np.sqrt(d[:, 0] * d[:, 0] + (d[:, 1] * d[:, 1] + d[:, 2] * d[:, 2]))
+        ok = ((vox >= lo[j]) & (vox <= lo[j] + per - 1)).all(1) & ~(r > radii[j] * F(2))
+        D[ok, j] = r[ok]
+    order = np.argsort(D, axis=1, kind="stable")[:, :k]
+    want_d = np.take_along_axis(D, order, 1)
+    have = np.isfinite(want_d)
+    c = np.minimum(np.isfinite(D).sum(1), k)
+    assert np.array_equal(cnt.cpu().numpy(), c)
+    gi, gd = idx.cpu().numpy(), dist.cpu().numpy()
+    assert np.array_equal(gi[:, :order.shape[1]][have], order[have]) and np.array_equal(gd[:, :order.shape[1]][have], want_d[have])

@@ -393,63 +393,115 @@ AFX_D int coll_get(const unsigned* w, unsigned epoch) {
     return ((v >> 8) == epoch) ? (int)(v & 255u) : 0;
 }
 
+// The K nearest supporters of every voxel of the active bricks, their weights, and the voxel's centre moved by
+// them.  The brick's candidate nodes are staged in shared memory with their transforms, so that what a voxel does
+// after its search waits for no further gather, and a voxel is inside a node's cube where three bits of the
+// candidate's word say so.  The list is kept sorted in registers (indexed ones went to local memory).
+// Bound: the chain active brick -> candidates -> nodes in front of each brick.  200^3 voxels, 600 nodes, dense lists: 24.4 ->
+// 14.6 us; a frame of the 256^3 sequence 23 -> 17 us, of the 512^3 sequence 57 -> 40 us.
 template <int K>
 __global__ void __launch_bounds__(kBrickVox) brick_warp_kernel(WarpArgs a) {
-    __shared__ float s_pos[kMaxBrickNodes * 3];
-    __shared__ float s_rad[kMaxBrickNodes];
-    __shared__ int s_lo[kMaxBrickNodes * 3], s_hi[kMaxBrickNodes * 3];
-    __shared__ int s_id[kMaxBrickNodes];
+    __shared__ float4 s_node[kMaxBrickNodes];      // position, radius
+    __shared__ float4 s_T[kMaxBrickNodes * 4];     // columns of the transform
+    __shared__ unsigned s_cube[kMaxBrickNodes];    // x, y, z of the brick inside the node's cube, eight bits each
+    __shared__ unsigned s_id[kMaxBrickNodes];      // node << 8 | place here
+    static_assert(kMaxBrickNodes <= 256, "a place fits in eight bits");
     const unsigned n_active = *a.n_active;
+    const int lx = threadIdx.x % kBrick, ly = (threadIdx.x / kBrick) % kBrick, lz = threadIdx.x / (kBrick * kBrick);
+    const unsigned here = 1u << lx | 1u << (8 + ly) | 1u << (16 + lz);
     for (unsigned slot = blockIdx.x; slot < n_active; slot += gridDim.x) {
-    __syncthreads();  // the previous brick's staged nodes are no longer read
-    [&] {
     const unsigned b = a.active[slot];
     const unsigned off = a.brick_offset[b];
     const int nc = min((int)a.brick_count[b], kMaxBrickNodes);
+    const int bx = b % a.bg.nb[0], by = (b / a.bg.nb[0]) % a.bg.nb[1], bz = b / ((unsigned)a.bg.nb[0] * a.bg.nb[1]);
+    __syncthreads();  // the previous brick's staged nodes are no longer read
     if (threadIdx.x == 0 && a.brick_count[b] > kMaxBrickNodes) atomicOr(a.error, ERRF_CAPACITY);
+    bool odd = false;  // a position that is not a number
     for (int i = threadIdx.x; i < nc; i += blockDim.x) {
-        int j = (int)a.brick_nodes[off + i];
-        s_id[i] = j;
-        const float* p = a.nodes_t + 3 * j;
-        s_pos[3 * i] = p[0];
-        s_pos[3 * i + 1] = p[1];
-        s_pos[3 * i + 2] = p[2];
-        s_rad[i] = a.radii[j];
+        const unsigned j = a.brick_nodes[off + i];
+        const float p[3] = {a.nodes_t[3 * (long)j], a.nodes_t[3 * (long)j + 1], a.nodes_t[3 * (long)j + 2]};
+        s_id[i] = j << 8 | (unsigned)i;
+        s_node[i] = make_float4(p[0], p[1], p[2], a.radii[j]);
+        odd |= p[0] != p[0] || p[1] != p[1] || p[2] != p[2];
         NodeCube c;
         node_cube(p, a.vol, a.per, &c);
+        const int base[3] = {bx * kBrick, by * kBrick, bz * kBrick};
+        unsigned cube = 0;
+#pragma unroll
         for (int q = 0; q < 3; ++q) {
-            s_lo[3 * i + q] = c.lo[q];
-            s_hi[3 * i + q] = c.hi[q];
+            const int lo = max(c.lo[q] - base[q], 0), hi = min(c.hi[q] - base[q], kBrick - 1);
+            if (lo <= hi) cube |= ((2u << hi) - (1u << lo)) << (8 * q);
         }
+        s_cube[i] = cube;
     }
-    __syncthreads();
-    const int bx = b % a.bg.nb[0], by = (b / a.bg.nb[0]) % a.bg.nb[1], bz = b / ((unsigned)a.bg.nb[0] * a.bg.nb[1]);
-    const int lx = threadIdx.x % kBrick, ly = (threadIdx.x / kBrick) % kBrick, lz = threadIdx.x / (kBrick * kBrick);
+    if (a.out)
+        for (int t = threadIdx.x; t < nc * 4; t += blockDim.x)
+            s_T[t] = reinterpret_cast<const float4*>(a.transforms)[4 * (long)a.brick_nodes[off + (t >> 2)] + (t & 3)];
+    odd = __syncthreads_or(odd);
+    [&] {
     const int x = bx * kBrick + lx, y = by * kBrick + ly, z = bz * kBrick + lz;
     const long local = (long)slot * kBrickVox + threadIdx.x;
     const int X = a.vol.dims[0], Y = a.vol.dims[1], Z = a.vol.dims[2];
     const bool inside = x < X && y < Y && z < Z;
+    constexpr unsigned kEmpty = 0xffffffffu;
     float kd[K];
-    int ki[K];
-    int cnt = 0;
+    unsigned ki[K];  // as s_id: in node order
+#pragma unroll
+    for (int s = 0; s < K; ++s) {
+        kd[s] = INFINITY;
+        ki[s] = kEmpty;
+    }
     float p[3];
     voxel_to_world(x, y, z, a.vol.vs, a.vol.half, p);
-    if (inside) {
+    if (inside && !odd) {
         for (int i = 0; i < nc; ++i) {
-            if (x < s_lo[3 * i] || x > s_hi[3 * i] || y < s_lo[3 * i + 1] || y > s_hi[3 * i + 1] ||
-                z < s_lo[3 * i + 2] || z > s_hi[3 * i + 2])
-                continue;
-            float d3[3] = {p[0] - s_pos[3 * i], p[1] - s_pos[3 * i + 1], p[2] - s_pos[3 * i + 2]};
-            float d = norm3(d3);
-            if (d > s_rad[i] * 2.0f) continue;
-            topk_insert(kd, ki, cnt, K < a.k ? K : a.k, d, s_id[i]);
+            if ((s_cube[i] & here) != here) continue;
+            const float4 v = s_node[i];
+            const float d3[3] = {p[0] - v.x, p[1] - v.y, p[2] - v.z};
+            const float d = norm3(d3);
+            if (d > v.w * 2.0f) continue;
+            const unsigned id = s_id[i];
+            if (!(d < kd[K - 1] || (d == kd[K - 1] && id < ki[K - 1]))) continue;
+            kd[K - 1] = d;
+            ki[K - 1] = id;
+#pragma unroll
+            for (int s = K - 1; s > 0; --s) {
+                const bool up = kd[s] < kd[s - 1] || (kd[s] == kd[s - 1] && ki[s] < ki[s - 1]);
+                const float ds = kd[s], dt = kd[s - 1];
+                const unsigned is = ki[s], it = ki[s - 1];
+                kd[s] = up ? dt : ds;
+                kd[s - 1] = up ? ds : dt;
+                ki[s] = up ? it : is;
+                ki[s - 1] = up ? is : it;
+            }
+        }
+    } else if (inside) {  // distances that are not numbers keep the place they were put at
+        float ld[K];
+        int li[K];
+        int n = 0;
+        for (int i = 0; i < nc; ++i) {
+            if ((s_cube[i] & here) != here) continue;
+            const float4 v = s_node[i];
+            const float d3[3] = {p[0] - v.x, p[1] - v.y, p[2] - v.z};
+            const float d = norm3(d3);
+            if (d > v.w * 2.0f) continue;
+            topk_insert(ld, li, n, K < a.k ? K : a.k, d, (int)s_id[i]);
+        }
+        for (int s = 0; s < n; ++s) {
+            kd[s] = ld[s];
+            ki[s] = (unsigned)li[s];
         }
     }
+    int cnt = 0;
+#pragma unroll
+    for (int s = 0; s < K; ++s) cnt += s < a.k && ki[s] != kEmpty;
     if (a.dense_count && inside) {
         const long v = ((long)z * Y + y) * X + x;
         a.dense_count[v] = cnt;
-        for (int s = 0; s < a.k; ++s) {
-            a.dense_idx[v * a.k + s] = s < cnt ? (uint32_t)ki[s] : AFX_INVALID_INDEX;
+#pragma unroll
+        for (int s = 0; s < K; ++s) {
+            if (s >= a.k) break;
+            a.dense_idx[v * a.k + s] = s < cnt ? ki[s] >> 8 : AFX_INVALID_INDEX;
             a.dense_dist[v * a.k + s] = s < cnt ? kd[s] : 3.402823466e+38f;
         }
     }
@@ -459,29 +511,39 @@ __global__ void __launch_bounds__(kBrickVox) brick_warp_kernel(WarpArgs a) {
     // weights (computeTsdfWarpWeightsKernel, src/TSDFWarp.cu:88-116: no cut-off)
     float w[K];
     float sum = 0.f;
-    for (int s = 0; s < cnt; ++s) {
-        float r = a.radii[ki[s]], d = kd[s];
+#pragma unroll
+    for (int s = 0; s < K; ++s) {
+        w[s] = 0.f;
+        if (s >= cnt) continue;
+        const float r = s_node[ki[s] & 0xffu].w, d = kd[s];
         w[s] = afx_expf(-(d * d) / (2.0f * (r * r)));
         sum = sum + w[s];
     }
-    if (sum != 0.f)
-        for (int s = 0; s < cnt; ++s) w[s] = w[s] / sum;
     bool zero = true;
-    for (int s = 0; s < cnt; ++s)
+#pragma unroll
+    for (int s = 0; s < K; ++s) {
+        if (s >= cnt) continue;
+        if (sum != 0.f) w[s] = w[s] / sum;
         if (!(fabsf(w[s]) <= 1e-5f)) zero = false;
+    }
     // voxel centre in camera space (generateTsdfVertices + translate, src/VolumeFusion.cu:718-723)
     const float cen[3] = {a.centroid_dev[0], a.centroid_dev[1], a.centroid_dev[2]};
     float c[3] = {p[0] + cen[0], p[1] + cen[1], p[2] + cen[2]};
     float q[3] = {c[0], c[1], c[2]};
     if (!zero && a.blend == AFX_BLEND_DQB) {  // dual-quaternion blend (afx_dqb.cuh)
         uint32_t kidx[K];
-        for (int s = 0; s < cnt; ++s) kidx[s] = (uint32_t)ki[s];
+        for (int s = 0; s < cnt; ++s) kidx[s] = ki[s] >> 8;
         dq_blend_point(a.transforms, kidx, w, cnt, AFX_INVALID_INDEX, c, q);
     } else if (!zero) {  // warpTsdfKernel (src/TSDFWarp.cu:158-190)
         q[0] = q[1] = q[2] = 0.f;
-        for (int s = 0; s < cnt; ++s) {
+#pragma unroll
+        for (int s = 0; s < K; ++s) {
+            if (s >= cnt) continue;
+            const float4* T = s_T + 4 * (ki[s] & 0xffu);
+            const float4 t0 = T[0], t1 = T[1], t2 = T[2], t3 = T[3];
+            const float M[16] = {t0.x, t0.y, t0.z, 0.f, t1.x, t1.y, t1.z, 0.f, t2.x, t2.y, t2.z, 0.f, t3.x, t3.y, t3.z, 0.f};
             float o[3];
-            mat4_point(a.transforms + 16 * (long)ki[s], c, o);
+            mat4_point(M, c, o);
             q[0] = q[0] + w[s] * o[0];
             q[1] = q[1] + w[s] * o[1];
             q[2] = q[2] + w[s] * o[2];
