@@ -625,52 +625,54 @@ __global__ void __launch_bounds__(kAsmThreads, KM <= 4 ? 4 : 3) jtj_assemble_ker
     }
 }
 
-// Inverse of each diagonal block: Gauss-Jordan with partial pivoting in FP64, one warp per
-// node with lane j < 12 owning column j of [D | I]; stored rounded to FP32 (the preconditioner
-// is applied in FP32).
-AFX_D void diag_inverse_node(const GnArgs& a, int node) {
-    const int lane = threadIdx.x & 31;
-    const float* D = a.b.diag + (long)node * 36;
-    const bool own = lane < 12;
+// Inverses of the diagonal blocks of nodes `node` and `node` + 1: Gauss-Jordan with partial pivoting in FP64, half
+// a warp per node with lane j < 12 of it owning column j of [D | I]; stored rounded to FP32 (the
+// preconditioner is applied in FP32).  Bound: FP64 issue (16 cycles a warp) with many nodes, the chain of six
+// pivots with few; so two nodes share a warp, and a pivot is searched by the lane that owns its column,
+// on the bits of the magnitudes.  1,300 nodes: the launch took 23 us with a node per warp, 17 so.
+AFX_D void diag_inverse_pair(const GnArgs& a, int node0, int n) {
+    const int lane = threadIdx.x & 15, node = node0 + ((threadIdx.x >> 4) & 1);
+    const bool on = node < n, own = on && lane < 12;
+    const float* D = a.b.diag + (long)(on ? node : node0) * 36;
+    constexpr unsigned long long kInf = 0x7ff0000000000000ull;
     double col[6];
 #pragma unroll
     for (int i = 0; i < 6; ++i) col[i] = !own ? 0.0 : (lane < 6 ? (double)D[i * 6 + lane] : (lane - 6 == i ? 1.0 : 0.0));
     bool ok = true;
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
-        // pivot: the largest |m[r][c]|, r >= c (first on ties), read from lane c
+        // pivot: the largest |m[r][c]|, r >= c (first on ties; one that is not a number is never larger or passed)
         int p = c;
-        double best = fabs(__shfl_sync(0xffffffffu, col[c], c));
+        unsigned long long best = (unsigned long long)__double_as_longlong(fabs(col[c]));
 #pragma unroll
         for (int r = c + 1; r < 6; ++r) {
-            double v = fabs(__shfl_sync(0xffffffffu, col[r], c));
-            if (v > best) {
+            const unsigned long long v = (unsigned long long)__double_as_longlong(fabs(col[r]));
+            if (v > best && v <= kInf) {
                 best = v;
                 p = r;
             }
         }
-        if (best == 0.0) {
-            ok = false;
-            break;
-        }
+        p = __shfl_sync(0xffffffffu, best == 0ull ? -1 : p, c, 16);
+        if (p < 0) ok = false;  // the rest is not used
         if (p != c) {
 #pragma unroll
             for (int r = c + 1; r < 6; ++r)
                 if (r == p) {
-                    double t = col[r];
+                    const double t = col[r];
                     col[r] = col[c];
                     col[c] = t;
                 }
         }
-        const double d = __shfl_sync(0xffffffffu, col[c], c);
+        const double d = __shfl_sync(0xffffffffu, col[c], c, 16);
         col[c] /= d;
 #pragma unroll
         for (int r = 0; r < 6; ++r)
             if (r != c) {
-                double f = __shfl_sync(0xffffffffu, col[r], c);
+                const double f = __shfl_sync(0xffffffffu, col[r], c, 16);
                 col[r] -= f * col[c];
             }
     }
+    if (!on) return;
     float* out = a.b.minv + (long)node * 36;
     if (!ok) {
         if (lane == 0) atomicOr(a.error, ERRF_SINGULAR);
@@ -711,13 +713,13 @@ AFX_D void lower_blocks_node(const GnArgs& a, int node) {
 }
 
 // What the Gauss-Newton loop needs besides the blocks, in one launch: the inverses (the first `half`
-// CTAs, one node per warp: a serial chain in binary64), and meanwhile the lower blocks, the
+// CTAs: a serial chain in binary64), and meanwhile the lower blocks, the
 // pending transforms as a copy of the committed ones and the loop's state.
 __global__ void __launch_bounds__(128) gn_icp_finish_kernel(GnArgs a, float4* T_pending, const float4* T_committed,
                                                            int half) {
     const int n = min(*a.n_nodes, a.n_max);
     if ((int)blockIdx.x < half) {
-        for (int node = blockIdx.x * 4 + (threadIdx.x >> 5); node < n; node += half * 4) diag_inverse_node(a, node);
+        for (int node = (blockIdx.x * 4 + (threadIdx.x >> 5)) * 2; node < n; node += half * 8) diag_inverse_pair(a, node, n);
         return;
     }
     const long first = (long)(blockIdx.x - half) * blockDim.x + threadIdx.x;
@@ -2372,7 +2374,7 @@ int gn_icp_setup(const GnArgs& a, float* T_pending, const float* T_committed, cu
     if (a.k <= 4) jtj_assemble_kernel<4><<<std::min(a.n_max, kNodeCtas), kAsmThreads, smem, st>>>(a);
     else jtj_assemble_kernel<8><<<std::min(a.n_max, kNodeCtas), kAsmThreads, smem, st>>>(a);
     AFX_LAUNCH_CHECK();
-    const int half = std::min((a.n_max + 3) / 4, kNodeCtas);
+    const int half = std::min((a.n_max + 7) / 8, kNodeCtas);
     gn_icp_finish_kernel<<<half + grid_for((long)a.n_max * 32, 128), 128, 0, st>>>(
         a, reinterpret_cast<float4*>(T_pending), reinterpret_cast<const float4*>(T_committed), half);
     AFX_LAUNCH_CHECK();
