@@ -266,7 +266,7 @@ size_t afx_correspondences_workspace_size(long n_points_max);
  * not allocate device memory during the frame (real-time loops on a preallocated memory
  * budget, code running under an allocator lock or inside a host callback).  This entry
  * point has no counterpart in the reference.  Scratch is a fixed device array of the
- * library sized for AFX_CORR_STATIC_MAX_POINTS vertices (about 3 MiB); n_points_max above
+ * library sized for AFX_CORR_STATIC_MAX_POINTS vertices (about 1 MiB); n_points_max above
  * that returns AFX_ERR_CAPACITY before any work.  The first call on each device looks up
  * the array's address, and so does the first call after a device reset (make that first
  * call before any stream capture).  All calls on a

@@ -227,9 +227,13 @@ __global__ void copy_new_nodes_kernel(float* dst, const float* src, const int* n
     }
 }
 
-__global__ void record_n_old_kernel(const int* n_nodes, int* n_old) { *n_old = *n_nodes; }
-
-__global__ void frame_begin_kernel(unsigned* epoch, unsigned* ncorr, int* error, unsigned* nmverts, unsigned* nmfaces) {
+// Counters of the frame: those that start at zero, the nodes there were, and `words` words of list counters.
+__global__ void frame_begin_kernel(unsigned* epoch, unsigned* ncorr, unsigned* nmverts, unsigned* nmfaces, unsigned* next_points,
+                                   const int* n_nodes, int* n_old, unsigned* counters, long words) {
+    AFX_GRID_STRIDE(i, words) counters[i] = 0u;
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    *next_points = 0;
+    *n_old = *n_nodes;
     unsigned e = *epoch + 1;
     if (e >= (1u << 24)) e = 1;  // collision words are cleared by the host when this wraps
     *epoch = e;
@@ -238,9 +242,15 @@ __global__ void frame_begin_kernel(unsigned* epoch, unsigned* ncorr, int* error,
     *nmfaces = 0;
 }
 
+// Statistics of the frame, and (nonrigid) the graph's positions moved back in place as the reference leaves its device
+// graph: p = (p - c) + c (src/VolumeFusion.cu:721).
 __global__ void stats_kernel(FrameStats* s, int* frame, const int* n_nodes, const int* n_old, const unsigned* npoints,
                              const unsigned* ncorr, const GnState* gn, const unsigned* nv, const unsigned* nf,
-                             const int* error, int nonrigid) {
+                             const int* error, int nonrigid, float* nodes, const float* nodes_t, int n_max, const float* c) {
+    if (nonrigid)
+        AFX_GRID_STRIDE(i, (long)n_max)
+            for (int q = 0; q < 3; ++q) nodes[3 * i + q] = nodes_t[3 * i + q] + c[q];
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
     s->frame = *frame;
     *frame = *frame + 1;
     s->n_nodes = *n_nodes;
@@ -622,11 +632,11 @@ static int finish_output_mesh(afx_fusion* f, bool nonrigid, cudaStream_t st) {
     return rc;
 }
 
+// (the point counter of the other buffer is zero)
 static int extract_frame_mesh(afx_fusion* f, int cur, cudaStream_t st) {
     // canonical point cloud for the next frame (runMarchingCubesMeshKernel on the volume the next
     // frame starts from) and, if asked, the output mesh (runMarchingCubesFullKernel), in one pass
     const int next = cur ^ 1;
-    AFX_CUDA(cudaMemsetAsync(f->npoints_buf[next], 0, 4, st));
     const bool mesh = f->p.extract_mesh != 0;
     return mc_fused_impl(f->tsdf, f->weights, f->fmt, f->vol, 0.f, f->points_buf[next], f->npoints_buf[next], f->p.mesh_capacity,
                          mesh ? f->mverts : nullptr, mesh ? f->nmverts : nullptr, f->p.triangle_capacity * 3,
@@ -641,7 +651,9 @@ static int enqueue_frame(afx_fusion* f, const uint16_t* depth_mm, cudaStream_t s
     const afx_fusion_params& p = f->p;
     int rc;
     static const float I3[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
-    frame_begin_kernel<<<1, 1, 0, st>>>(f->epoch, f->ncorr, f->error, f->nmverts, f->nmfaces);
+    const long words = f->frame == 0 ? 0 : (long)gn_counter_words(p.node_capacity);
+    frame_begin_kernel<<<grid_for(words, 256), 256, 0, st>>>(f->epoch, f->ncorr, f->nmverts, f->nmfaces, f->npoints_buf[cur ^ 1],
+                                                             f->n_nodes, f->n_old, f->gn.lcnt, words);
     AFX_LAUNCH_CHECK();
     // af::loadProcessFrame (src/VolumeFusion.cu:151-220)
     afx_prep_params pp;
@@ -670,7 +682,7 @@ static int enqueue_frame(afx_fusion* f, const uint16_t* depth_mm, cudaStream_t s
         if (rc) return rc;
         stage_mark(f, -1, st);
         stats_kernel<<<1, 1, 0, st>>>(f->stats, f->frame_dev, f->n_nodes, f->n_old, f->mesh_used, f->ncorr, f->gn.state,
-                                      f->nmverts, f->nmfaces, f->error, 0);
+                                      f->nmverts, f->nmfaces, f->error, 0, nullptr, nullptr, 0, nullptr);
         AFX_LAUNCH_CHECK();
         return AFX_OK;
     }
@@ -680,16 +692,11 @@ static int enqueue_frame(afx_fusion* f, const uint16_t* depth_mm, cudaStream_t s
     stage_mark(f, ST_SORT, st);
     float* points = f->points_buf[cur];
     unsigned* npoints = f->npoints_buf[cur];
-    rc = sort_unique_volume_impl(points, npoints, M, f->ws_sort, f->ws_sort_bytes, f->vol, st, f->error);
-    if (rc) return rc;
-    AFX_CUDA(cudaMemcpyAsync(f->mesh_used, npoints, 4, cudaMemcpyDeviceToDevice, st));
-    if (rc) return rc;
-    rc = translate_dev_impl(points, points, npoints, M, f->centroid0, 1.f, st);
+    rc = sort_unique_volume_impl(points, npoints, M, f->ws_sort, f->ws_sort_bytes, f->vol, st, f->error, f->centroid0,
+                                 f->mesh_used);
     if (rc) return rc;
     // motion graph (src/VolumeFusion.cu:394-404)
     stage_mark(f, ST_GRAPH, st);
-    record_n_old_kernel<<<1, 1, 0, st>>>(f->n_nodes, f->n_old);
-    AFX_LAUNCH_CHECK();
     if (build) {
         rc = build_graph_impl(f->nodes_host, f->radii, f->T, f->n_nodes, N, points, npoints, M, p.graph_radius,
                               f->ws_graph, f->ws_graph_bytes, f->error, st);
@@ -717,9 +724,9 @@ static int enqueue_frame(afx_fusion* f, const uint16_t* depth_mm, cudaStream_t s
     rc = knn_impl(f->gidx, f->gdist, f->nodes_host, f->n_nodes, N, f->nodes_host,
                   reinterpret_cast<const unsigned*>(f->n_nodes), N, p.kreg, 1, st);
     if (rc) return rc;
-    rc = afx_filter_disconnected(f->gidx, f->gdist, f->n_nodes, N, p.kreg, f->radii, st);
-    if (rc) return rc;
-    rc = warp_weights_impl(f->mw, f->radii, f->midx, f->mdist, npoints, M, p.knn, f->n_nodes, st);
+    GraphWeightArgs gw{f->mw, f->midx, f->mdist, npoints, M, p.knn, f->gidx, f->gdist, p.kreg, f->radii, f->n_nodes, N,
+                       f->gn.lcnt, f->gn.icnt};
+    rc = graph_weights_impl(gw, st);
     if (rc) return rc;
     GnArgs g;
     std::memset(&g, 0, sizeof(g));
@@ -747,7 +754,7 @@ static int enqueue_frame(afx_fusion* f, const uint16_t* depth_mm, cudaStream_t s
     g.b = f->gn;
     g.error = f->error;
     stage_mark(f, ST_GN_SETUP, st);
-    rc = gn_frame_setup(g, st);
+    rc = gn_frame_setup(g, st, true);
     if (rc) return rc;
     const double tol = p.solver == 2 ? p.pcg_tol : 0.0;
     for (int icp = 0; icp < p.icp_iterations; ++icp) {
@@ -773,9 +780,6 @@ static int enqueue_frame(afx_fusion* f, const uint16_t* depth_mm, cudaStream_t s
         rc = build_support(f->sup, f->vol, f->per, f->nodes_t, f->radii, f->n_nodes, N, f->error, st);
         if (rc) return rc;
     }
-    // the reference translates its device graph back in place: p = (p - c) + c (src/VolumeFusion.cu:721)
-    rc = translate_dev_impl(f->nodes_dev, f->nodes_t, nullptr, N, f->centroid0, 1.f, st);
-    if (rc) return rc;
     WarpArgs wa;
     std::memset(&wa, 0, sizeof(wa));
     wa.vol = f->vol;
@@ -829,8 +833,9 @@ static int enqueue_frame(afx_fusion* f, const uint16_t* depth_mm, cudaStream_t s
     if (!rc) rc = finish_output_mesh(f, true, st);
     if (rc) return rc;
     stage_mark(f, -1, st);
-    stats_kernel<<<1, 1, 0, st>>>(f->stats, f->frame_dev, f->n_nodes, f->n_old, f->mesh_used, f->ncorr, f->gn.state,
-                                  f->nmverts, f->nmfaces, f->error, 1);
+    stats_kernel<<<grid_for(N, 256), 256, 0, st>>>(f->stats, f->frame_dev, f->n_nodes, f->n_old, f->mesh_used, f->ncorr,
+                                                   f->gn.state, f->nmverts, f->nmfaces, f->error, 1, f->nodes_dev, f->nodes_t, N,
+                                                   f->centroid0);
     AFX_LAUNCH_CHECK();
     return AFX_OK;
 }
@@ -1114,8 +1119,9 @@ int afx_fusion_autotune(afx_fusion* f, int* tile_out, float* ms_out, void* strea
         f->mc_tile = tile;
         float t_min = 1e30f;
         for (int rep = 0; rep < 4 && rc == AFX_OK; ++rep) {  // the first run of a tile also sets it up
+            if (cudaMemsetAsync(f->npoints_buf[f->cur ^ 1], 0, 4, st) != cudaSuccess) rc = AFX_ERR_CUDA;
             cudaEventRecord(e0, st);
-            rc = extract_frame_mesh(f, f->cur, st);
+            if (!rc) rc = extract_frame_mesh(f, f->cur, st);
             cudaEventRecord(e1, st);
             if (cudaEventSynchronize(e1) != cudaSuccess) rc = AFX_ERR_CUDA;
             float ms = 0.f;

@@ -2343,12 +2343,16 @@ bool gn_carve(void* ws, size_t bytes, long m_max, int n_max, int k, int kreg, Gn
 constexpr int kNodeCtas = 608;  // CTAs that take one node at a time: four of 256 threads per SM
 
 // Per frame: node -> vertex lists and incoming regularisation edges.
-int gn_frame_setup(const GnArgs& a, cudaStream_t st) {
+size_t gn_counter_words(int n_max) { return 4 * al((n_max + 1) * 4) / 4; }
+
+int gn_frame_setup(const GnArgs& a, cudaStream_t st, bool counted) {
     const GnBuffers& b = a.b;
-    AFX_CUDA(cudaMemsetAsync(b.lcnt, 0, 4 * al((a.n_max + 1) * 4), st));  // lcnt lcur icnt icur
     const long items = std::max(a.m_max * a.k, (long)a.n_max * a.kreg);
-    list_count_kernel<<<grid_for(items, 256), 256, 0, st>>>(a);
-    AFX_LAUNCH_CHECK();
+    if (!counted) {
+        AFX_CUDA(cudaMemsetAsync(b.lcnt, 0, gn_counter_words(a.n_max) * 4, st));  // lcnt lcur icnt icur
+        list_count_kernel<<<grid_for(items, 256), 256, 0, st>>>(a);
+        AFX_LAUNCH_CHECK();
+    }
     list_scan_kernel<<<2, 1024, 0, st>>>(a);
     AFX_LAUNCH_CHECK();
     list_fill_kernel<<<grid_for(items, 256), 256, 0, st>>>(a);
@@ -2588,7 +2592,7 @@ int afx_gn_build(afx_gn* g, const float* canonical, const unsigned* n_points, co
     AFX_CUDA(cudaMemsetAsync(g->cov, 0xff, (size_t)g->m_max * 4, st));
     gn_corr_of_vertex_kernel<<<grid_for(g->m_max, 256), 256, 0, st>>>(corr, n_corr, g->m_max, g->cov);
     AFX_LAUNCH_CHECK();
-    int rc = gn_frame_setup(a, st);
+    int rc = gn_frame_setup(a, st, false);
     if (rc) return rc;
     rc = gn_icp_setup(a, nullptr, nullptr, st);
     if (rc) return rc;

@@ -1164,25 +1164,67 @@ __global__ void filter_disconnected_kernel(uint32_t* idx, float* dist, const int
 }
 
 // computeWarpWeightsKernel (src/VertexManipulation.cu:105-132)
+// Weights of point i over its k nearest nodes; ws: its k weights.
+AFX_D void warp_weights_of(const float* radii, const uint32_t* idx, const float* dist, int k, int n, float* ws) {
+    float sum = 0.f;
+    for (int j = 0; j < k; ++j) {
+        const uint32_t nb = idx[j];
+        float wj = 0.f;
+        if (nb < (uint32_t)n) {
+            const float r = radii[nb], d = dist[j];
+            wj = (d >= r) ? 0.f : afx_expf(-(d * d) / (2.0f * (r * r)));
+        }
+        ws[j] = wj;
+        sum = sum + wj;
+    }
+    for (int j = 0; j < k; ++j) ws[j] = (sum != 0.f) ? ws[j] / sum : ws[j];
+}
+
 __global__ void warp_weights_kernel(float* w, const float* radii, const uint32_t* idx, const float* dist,
                                     const unsigned* count, long m_max, int k, const int* n_nodes) {
     const long m = count ? min((long)*count, m_max) : m_max;
     const int n = *n_nodes;
     AFX_GRID_STRIDE(i, m) {
         float ws[17];
-        float sum = 0.f;
-        for (int j = 0; j < k; ++j) {
-            uint32_t nb = idx[i * k + j];
-            float wj = 0.f;
-            if (nb < (uint32_t)n) {
-                float r = radii[nb], d = dist[i * k + j];
-                wj = (d >= r) ? 0.f : afx_expf(-(d * d) / (2.0f * (r * r)));
-            }
-            ws[j] = wj;
-            sum = sum + wj;
-        }
-        for (int j = 0; j < k; ++j) w[i * k + j] = (sum != 0.f) ? ws[j] / sum : ws[j];
+        warp_weights_of(radii, idx + i * k, dist + i * k, k, n, ws);
+        for (int j = 0; j < k; ++j) w[i * k + j] = ws[j];
     }
+}
+
+// What follows the two searches of a frame, in one launch: the points' weights, the graph's edges without those
+// too long (filter_disconnected_kernel), and how many entries and edges each node gets (the Gauss-Newton
+// stage's lists; both counters start at zero).
+__global__ void graph_weights_kernel(GraphWeightArgs a) {
+    const long m = min((long)*a.count, a.m_max);
+    const int n = min(*a.n_nodes, a.n_max);
+    AFX_GRID_STRIDE(i, m) {
+        float ws[17];
+        warp_weights_of(a.radii, a.idx + i * a.k, a.dist + i * a.k, a.k, *a.n_nodes, ws);
+        for (int j = 0; j < a.k; ++j) {
+            a.w[i * a.k + j] = ws[j];
+            const uint32_t node = a.idx[i * a.k + j];
+            if (ws[j] != 0.f && node < (uint32_t)n) atomicAdd(a.entries + node, 1u);
+        }
+    }
+    AFX_GRID_STRIDE(t, (long)n * a.kreg) {
+        const uint32_t nb = a.gidx[t];
+        if (nb >= (uint32_t)n) continue;
+        if (a.gdist[t] <= a.radii[t / a.kreg] * 1.3f) {
+            atomicAdd(a.edges + nb, 1u);
+        } else {
+            a.gidx[t] = AFX_INVALID_INDEX;
+            a.gdist[t] = FLT_MAX;
+        }
+    }
+}
+
+int graph_weights_impl(const GraphWeightArgs& a, cudaStream_t st) {
+    if (a.k > 17) return AFX_ERR_UNSUPPORTED;
+    const long items = a.m_max > (long)a.n_max * a.kreg ? a.m_max : (long)a.n_max * a.kreg;
+    if (items <= 0) return AFX_OK;
+    graph_weights_kernel<<<grid_for(items, 256), 256, 0, st>>>(a);
+    AFX_LAUNCH_CHECK();
+    return AFX_OK;
 }
 
 // warpKernel (src/ComputeCorrespondence.cu:5-30)
@@ -1283,33 +1325,66 @@ AFX_D int corr_pixel(const CorrArgs& a, long i) {
     return (int)px;
 }
 
-__global__ void corr_flags_kernel(CorrArgs a, unsigned* flags, int* pix) {
-    long m = a.count ? min((long)*a.count, a.m_max) : a.m_max;
-    AFX_GRID_STRIDE(i, m) {
-        int px = corr_pixel(a, i);
-        pix[i] = px;
-        flags[i] = px >= 0 ? 1u : 0u;
+// Pixels of the vertices, and how many of each tile of 256 have one.
+constexpr int kCorrTile = 256;
+
+__global__ void __launch_bounds__(kCorrTile) corr_pixel_kernel(CorrArgs a, int* pix, unsigned* sums) {
+    const long m = a.count ? min((long)*a.count, a.m_max) : a.m_max;
+    for (long tile = blockIdx.x; tile * kCorrTile < m; tile += gridDim.x) {
+        const long i = tile * kCorrTile + threadIdx.x;
+        const int px = i < m ? corr_pixel(a, i) : -1;
+        if (i < m) pix[i] = px;
+        const int n = __syncthreads_count(px >= 0);
+        if (threadIdx.x == 0) sums[tile] = (unsigned)n;
     }
 }
 
-__global__ void corr_scatter_kernel(CorrArgs a, const unsigned* flags, const int* pix, const unsigned* pos, int* corr,
-                                    long cap, int* corr_of_vertex) {
-    long m = a.count ? min((long)*a.count, a.m_max) : a.m_max;
-    AFX_GRID_STRIDE(i, m) {
-        if (flags[i]) {
-            unsigned p = pos[i];
+// The pairs in vertex order: a CTA adds up the tiles before its own (a few hundred numbers) instead of
+// waiting for three launches of a prefix sum.
+__global__ void __launch_bounds__(kCorrTile) corr_scatter_kernel(CorrArgs a, const int* pix, const unsigned* sums, int* corr,
+                                                                 unsigned* corr_count, long cap, int* corr_of_vertex) {
+    __shared__ unsigned s_before[2][kCorrTile / 32], s_have[2][kCorrTile / 32];
+    const long m = a.count ? min((long)*a.count, a.m_max) : a.m_max;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (m <= 0 && blockIdx.x == 0 && threadIdx.x == 0) *corr_count = 0u;
+    unsigned base = 0;
+    long done = 0;
+    int par = 0;
+    for (long tile = blockIdx.x; tile * kCorrTile < m; tile += gridDim.x, par ^= 1) {
+        unsigned v = 0;
+        for (long t = done + threadIdx.x; t < tile; t += kCorrTile) v += sums[t];
+        done = tile;
+        v = warp_sum(v);
+        const long i = tile * kCorrTile + threadIdx.x;
+        const int px = i < m ? pix[i] : -1;
+        const unsigned bal = __ballot_sync(0xffffffffu, px >= 0);
+        if (lane == 0) {
+            s_before[par][w] = v;
+            s_have[par][w] = (unsigned)__popc(bal);
+        }
+        __syncthreads();  // the arrays alternate: the next tile's are written while these are read
+        unsigned at = 0, all = 0;
+#pragma unroll
+        for (int q = 0; q < kCorrTile / 32; ++q) {
+            base += s_before[par][q];
+            if (q < w) at += s_have[par][q];
+            all += s_have[par][q];
+        }
+        if (px >= 0) {
+            const unsigned p = base + at + (unsigned)__popc(bal & ((1u << lane) - 1u));
             if (p < cap) {
                 corr[2 * (long)p] = (int)i;
-                corr[2 * (long)p + 1] = pix[i];
+                corr[2 * (long)p + 1] = px;
             }
             if (corr_of_vertex) corr_of_vertex[i] = (int)p;
-        } else if (corr_of_vertex) {
+        } else if (corr_of_vertex && i < m) {
             corr_of_vertex[i] = -1;
         }
+        if (threadIdx.x == 0 && (tile + 1) * kCorrTile >= m) *corr_count = base + all;
     }
 }
 
-size_t corr_ws(long m_max) { return 3 * al(m_max * 4) + al(scan_workspace_size(m_max)) + 256; }
+size_t corr_ws(long m_max) { return al(m_max * 4) + al((m_max / kCorrTile + 1) * 4) + 256; }
 
 int correspondences_impl(int* corr, unsigned* corr_count, long cap, const float* warped, const unsigned* count,
                          long m_max, const float* K, const float* depth, int rows, int cols, const float* frame,
@@ -1320,13 +1395,9 @@ int correspondences_impl(int* corr, unsigned* corr_count, long cap, const float*
         return AFX_OK;
     }
     char* p = static_cast<char*>(ws);
-    unsigned* flags = (unsigned*)p;
-    p += al(m_max * 4);
     int* pix = (int*)p;
     p += al(m_max * 4);
-    unsigned* pos = (unsigned*)p;
-    p += al(m_max * 4);
-    void* scan_ws = p;
+    unsigned* sums = (unsigned*)p;
     CorrArgs a;
     a.warped = warped;
     a.count = count;
@@ -1337,11 +1408,9 @@ int correspondences_impl(int* corr, unsigned* corr_count, long cap, const float*
     a.cols = cols;
     a.frame = frame;
     a.thresh = thresh;
-    corr_flags_kernel<<<grid_for(m_max, 256), 256, 0, st>>>(a, flags, pix);
+    corr_pixel_kernel<<<grid_for(m_max, kCorrTile), kCorrTile, 0, st>>>(a, pix, sums);
     AFX_LAUNCH_CHECK();
-    int rc = scan_exclusive_dev(flags, pos, count, m_max, corr_count, scan_ws, st);
-    if (rc) return rc;
-    corr_scatter_kernel<<<grid_for(m_max, 256), 256, 0, st>>>(a, flags, pix, pos, corr, cap, corr_of_vertex);
+    corr_scatter_kernel<<<grid_for(m_max, kCorrTile), kCorrTile, 0, st>>>(a, pix, sums, corr, corr_count, cap, corr_of_vertex);
     AFX_LAUNCH_CHECK();
     return AFX_OK;
 }
@@ -1466,7 +1535,7 @@ namespace afx {
 
 constexpr long kCorrStaticMaxPoints = AFX_CORR_STATIC_MAX_POINTS;
 // flags, pixels, scan output (4 bytes each per vertex) + scan block sums + alignment slack
-constexpr size_t kCorrStaticBytes = 3 * (size_t)kCorrStaticMaxPoints * 4 + 64 * 1024;
+constexpr size_t kCorrStaticBytes = (size_t)kCorrStaticMaxPoints * 4 + 64 * 1024;
 
 static __device__ __align__(256) unsigned char g_corr_static_scratch[kCorrStaticBytes];
 

@@ -68,8 +68,10 @@ size_t sort_unique_workspace_size(long n_max);
 int sort_unique_impl(float* pts, unsigned* count, long n_max, void* ws, size_t ws_bytes, cudaStream_t st);
 // The same result for a marching-cubes cloud of `vol` (x within the volume), by voxel-column buckets.
 size_t sort_unique_volume_workspace_size(long n_max, int nb);
+// `shift` (may be null): added to the distinct points; `count_copy` (may be null): gets the new count too.
 int sort_unique_volume_impl(float* pts, unsigned* count, long n_max, void* ws, size_t ws_bytes, const Volume& vol,
-                            cudaStream_t st, int* error = nullptr);
+                            cudaStream_t st, int* error = nullptr, const float* shift = nullptr,
+                            unsigned* count_copy = nullptr);
 int mc_fused_impl(const void* tsdf, const void* weights, int fmt, const Volume& vol, float iso, float* points,
                   unsigned* point_count, long point_cap, float* verts, unsigned* vert_count, long vert_cap, int* faces,
                   unsigned* face_count, long face_cap, cudaStream_t st, int* error = nullptr, int tile = 0,
@@ -99,6 +101,24 @@ int build_graph_impl(float* nodes, float* radii, float* T, int* n_nodes, int cap
                      cudaStream_t st);
 int knn_impl(uint32_t* idx, float* dist, const float* nodes, const int* n_nodes, int n_max, const float* pts,
              const unsigned* count, long m_max, int k, int excl, cudaStream_t st);
+struct GraphWeightArgs {
+    // points: w from idx, dist [m * k]
+    float* w;
+    const uint32_t* idx;
+    const float* dist;
+    const unsigned* count;
+    long m_max;
+    int k;
+    // graph edges [n * kreg]
+    uint32_t* gidx;
+    float* gdist;
+    int kreg;
+    const float* radii;
+    const int* n_nodes;
+    int n_max;
+    unsigned *entries, *edges;  // per node
+};
+int graph_weights_impl(const GraphWeightArgs& a, cudaStream_t st);
 int warp_weights_impl(float* w, const float* radii, const uint32_t* idx, const float* dist, const unsigned* count,
                       long m_max, int k, const int* n_nodes, cudaStream_t st);
 // blend: AFX_BLEND_LBS (the reference's linear blend) or AFX_BLEND_DQB (dual quaternions, afx_dqb.cuh)

@@ -1125,11 +1125,10 @@ AFX_D int bucket_of(float x, const BucketArgs& a) {
 }
 
 struct BucketWs {
-    unsigned* cnt;     // [nb]
-    unsigned* off;     // [nb + 1]
+    unsigned* cnt;     // [nb] points; cleared together with the next
     unsigned* cursor;  // [nb]
-    unsigned* ucnt;    // [nb]
-    unsigned* uoff;    // [nb + 1]
+    unsigned* off;     // [nb + 1]
+    unsigned* ucnt;    // [nb] distinct points
 };
 
 __global__ void bucket_count_kernel(const float* __restrict__ pts, const unsigned* count, long n_max, BucketArgs a,
@@ -1138,44 +1137,42 @@ __global__ void bucket_count_kernel(const float* __restrict__ pts, const unsigne
     AFX_GRID_STRIDE(i, n) atomicAdd(cnt + bucket_of(pts[3 * i], a), 1u);
 }
 
-// Exclusive scan of n values by one CTA of 1024 threads (n up to a few thousand); out[n] = total.
-// With `total`, the total is written there too.
-__global__ void __launch_bounds__(1024) small_scan_kernel(const unsigned* in, int n, unsigned* out, unsigned* copy,
-                                                          unsigned* total) {
-    __shared__ unsigned part[1024];
-    const int per = (n + 1023) / 1024;
-    const int lo = threadIdx.x * per, hi = min(n, lo + per);
-    unsigned sum = 0;
-    for (int i = lo; i < hi; ++i) sum += in[i];
-    part[threadIdx.x] = sum;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-        const unsigned v = threadIdx.x >= o ? part[threadIdx.x - o] : 0u;
-        __syncthreads();
-        part[threadIdx.x] += v;
-        __syncthreads();
-    }
-    unsigned run = part[threadIdx.x] - sum;
-    for (int i = lo; i < hi; ++i) {
-        out[i] = run;
-        if (copy) copy[i] = run;
-        run += in[i];
-    }
-    if (threadIdx.x == 1023) {
-        out[n] = part[1023];
-        if (total) *total = part[1023];
-    }
-}
-
-__global__ void bucket_scatter_kernel(const float* __restrict__ pts, const unsigned* count, long n_max, BucketArgs a,
-                                      unsigned* cursor, Key3* keys, int* error) {
+// The points into their buckets.  Every CTA forms the buckets' offsets for itself (a launch of one CTA for a few
+// hundred sums cost more); the first one leaves them for the launches after this.
+__global__ void __launch_bounds__(256) bucket_scatter_kernel(const float* __restrict__ pts, const unsigned* count, long n_max,
+                                                             BucketArgs a, BucketWs ws, Key3* keys, int* error) {
+    extern __shared__ unsigned s_off[];
+    __shared__ unsigned s_sum[8];
     const long n = min((long)*count, n_max);
+    if ((long)blockIdx.x * blockDim.x >= n && blockIdx.x != 0) return;
+    const int per = (a.nb + 255) / 256, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int lo = min(a.nb, (int)threadIdx.x * per), hi = min(a.nb, lo + per);
+    unsigned sum = 0;
+    for (int i = lo; i < hi; ++i) sum += ws.cnt[i];
+    unsigned x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) s_sum[w] = x;
+    __syncthreads();
+    unsigned run = x - sum;
+    for (int q = 0; q < w; ++q) run += s_sum[q];
+    for (int i = lo; i < hi; ++i) {
+        s_off[i] = run;
+        if (blockIdx.x == 0) ws.off[i] = run;
+        run += ws.cnt[i];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 255) ws.off[a.nb] = run;
+    __syncthreads();
     AFX_GRID_STRIDE(i, n) {
         Key3 k;
         k.k[0] = f2key(pts[3 * i]);
         k.k[1] = f2key(pts[3 * i + 1]);
         k.k[2] = f2key(pts[3 * i + 2]);
-        const unsigned pos = atomicAdd(cursor + bucket_of(pts[3 * i], a), 1u);
+        const int b = bucket_of(pts[3 * i], a);
+        const unsigned pos = s_off[b] + atomicAdd(ws.cursor + b, 1u);
         if (pos < (unsigned long)n) keys[pos] = k;
         else if (error) atomicOr(error, ERRF_INDEX);
     }
@@ -1285,18 +1282,35 @@ __global__ void __launch_bounds__(kBucketThreads) bucket_sort_kernel(Key3* keys,
 }
 
 // One CTA per bucket: its unique points, in order, at the bucket's place in the output.
-__global__ void __launch_bounds__(kBucketThreads) bucket_compact_kernel(const Key3* keys, const unsigned* off,
-                                                                      const unsigned* uoff, float* pts, long n_max,
-                                                                      int* error) {
+__global__ void __launch_bounds__(kBucketThreads) bucket_compact_kernel(const Key3* keys, BucketWs ws,
+                                                                      int nb, float* pts, long n_max, int* error,
+                                                                      unsigned* count, const float* shift,
+                                                                      unsigned* count_copy) {
     __shared__ unsigned wsum[kBucketThreads / 32];
+    __shared__ unsigned s_run;
     const int b = blockIdx.x;
-    if (off[b] > off[b + 1] || (long)off[b + 1] > n_max || (long)uoff[b + 1] > n_max) {
+    const unsigned* off = ws.off;
+    // distinct points of the buckets before this one; the last one's total is the new count
+    if (threadIdx.x == 0) s_run = 0u;
+    __syncthreads();
+    unsigned sum = 0;
+    for (int q = threadIdx.x; q < b; q += blockDim.x) sum += ws.ucnt[q];
+    sum = warp_sum(sum);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(&s_run, sum);
+    __syncthreads();
+    const unsigned first = s_run, after = first + ws.ucnt[b];
+    if (b == nb - 1 && threadIdx.x == 0) {
+        *count = after;
+        if (count_copy) *count_copy = after;
+    }
+    if (off[b] > off[b + 1] || (long)off[b + 1] > n_max || (long)after > n_max) {
         if (threadIdx.x == 0 && error) atomicOr(error, ERRF_INDEX);
         return;
     }
     const unsigned lo = off[b], n = off[b + 1] - lo;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    unsigned run = uoff[b];
+    const float t[3] = {shift ? shift[0] : 0.f, shift ? shift[1] : 0.f, shift ? shift[2] : 0.f};
+    unsigned run = first;
     for (unsigned r0 = 0; r0 < n; r0 += blockDim.x) {
         const unsigned i = r0 + threadIdx.x;
         const bool keep = i < n && (i == 0 || !key_same_point(keys[lo + i - 1], keys[lo + i]));
@@ -1313,27 +1327,31 @@ __global__ void __launch_bounds__(kBucketThreads) bucket_compact_kernel(const Ke
         if (keep) {
             const Key3 k = keys[lo + i];
             float* o = pts + 3 * (long)(run + before + __popc(bal & ((1u << lane) - 1)));
-            o[0] = key2f(k.k[0]);
-            o[1] = key2f(k.k[1]);
-            o[2] = key2f(k.k[2]);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) o[c] = shift ? key2f(k.k[c]) + t[c] : key2f(k.k[c]);
         }
         run += all;
     }
 }
 
 size_t sort_unique_volume_workspace_size(long n_max, int nb) {
-    return sort_unique_workspace_size(n_max) + al((size_t)(5 * (nb + 2) + 1) * 4);
+    return sort_unique_workspace_size(n_max) + al((size_t)(4 * nb + 1) * 4);
 }
 
 int sort_unique_volume_impl(float* pts, unsigned* count, long n_max, void* ws, size_t ws_bytes, const Volume& vol,
-                            cudaStream_t st, int* error) {
+                            cudaStream_t st, int* error, const float* shift, unsigned* count_copy) {
     if (n_max <= 0) return AFX_OK;
     const int nb = vol.dims[0] + 1;
-    if (nb > 8 * 1024) return sort_unique_impl(pts, count, n_max, ws, ws_bytes, st);
+    if (nb > 8 * 1024) {
+        int rc = sort_unique_impl(pts, count, n_max, ws, ws_bytes, st);
+        if (!rc && shift) rc = translate_dev_impl(pts, pts, count, n_max, shift, 1.f, st);
+        if (!rc && count_copy) AFX_CUDA(cudaMemcpyAsync(count_copy, count, 4, cudaMemcpyDeviceToDevice, st));
+        return rc;
+    }
     if (!ws || ws_bytes < sort_unique_volume_workspace_size(n_max, nb)) return AFX_ERR_WORKSPACE;
     const size_t base = sort_unique_workspace_size(n_max);
     unsigned* u = reinterpret_cast<unsigned*>(static_cast<char*>(ws) + base);
-    BucketWs w{u, u + nb, u + 2 * nb + 1, u + 3 * nb + 1, u + 4 * nb + 1};
+    BucketWs w{u, u + nb, u + 2 * nb, u + 3 * nb + 1};
     Key3* keys = reinterpret_cast<Key3*>(ws);
     BucketArgs a{vol.half[0], vol.inv[0], nb};
     static ContextOnce once;
@@ -1341,19 +1359,15 @@ int sort_unique_volume_impl(float* pts, unsigned* count, long n_max, void* ws, s
         return note_cuda_error(cudaFuncSetAttribute(bucket_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                     (int)(kBucketCap * sizeof(Key3))));
     });
-    AFX_CUDA(cudaMemsetAsync(w.cnt, 0, nb * 4, st));
+    AFX_CUDA(cudaMemsetAsync(w.cnt, 0, 2 * nb * 4, st));
     bucket_count_kernel<<<grid_for(n_max, 256), 256, 0, st>>>(pts, count, n_max, a, w.cnt);
     AFX_LAUNCH_CHECK();
-    small_scan_kernel<<<1, 1024, 0, st>>>(w.cnt, nb, w.off, w.cursor, nullptr);
-    AFX_LAUNCH_CHECK();
-    bucket_scatter_kernel<<<grid_for(n_max, 256), 256, 0, st>>>(pts, count, n_max, a, w.cursor, keys, error);
+    bucket_scatter_kernel<<<grid_for(n_max, 256), 256, nb * sizeof(unsigned), st>>>(pts, count, n_max, a, w, keys, error);
     AFX_LAUNCH_CHECK();
     Key3* scratch = reinterpret_cast<Key3*>(static_cast<char*>(ws) + al(n_max * sizeof(Key3)));  // the second buffer
     bucket_sort_kernel<<<nb, kBucketThreads, kBucketCap * sizeof(Key3), st>>>(keys, scratch, w.off, w.ucnt, n_max, error);
     AFX_LAUNCH_CHECK();
-    small_scan_kernel<<<1, 1024, 0, st>>>(w.ucnt, nb, w.uoff, nullptr, count);
-    AFX_LAUNCH_CHECK();
-    bucket_compact_kernel<<<nb, kBucketThreads, 0, st>>>(keys, w.off, w.uoff, pts, n_max, error);
+    bucket_compact_kernel<<<nb, kBucketThreads, 0, st>>>(keys, w, nb, pts, n_max, error, count, shift, count_copy);
     AFX_LAUNCH_CHECK();
     return AFX_OK;
 }
