@@ -452,6 +452,9 @@ int afx_fusion_tsdf(afx_fusion* f, float** tsdf, float** weights);  /* FP32 sess
 /* Device view of the volume in either storage format: FP32 values + FP32 weights, or (precision
  * form) IEEE FP16 values + uint16 weights; *precision says which. */
 int afx_fusion_volume(afx_fusion* f, void** tsdf, void** weights, int* precision);
+/* Copies the volume to FP32 arrays of the caller (16-byte aligned, one value per voxel), whatever the storage
+ * format: FP16 values widen exactly, uint16 weights are counts up to 15.  Asynchronous on `stream`. */
+int afx_fusion_export_volume(afx_fusion* f, float* tsdf, float* weights, void* stream);
 /* After writing the session's volume through these views: the session keeps, per brick of 8^3
  * voxels, whether any voxel has a weight (marching cubes skips bricks without, which hold no active
  * cube) and updates it itself when it integrates or loads a volume; this rebuilds it from the

@@ -129,6 +129,7 @@ SIGNATURES = {
     "afx_fusion_process_host": (i32, [vp, vp, vp]),
     "afx_fusion_stats": (i32, [vp, C.POINTER(FrameStats), vp]),
     "afx_fusion_tsdf": (i32, [vp, C.POINTER(vp), C.POINTER(vp)]),
+    "afx_fusion_export_volume": (i32, [vp, vp, vp, vp]),
     "afx_fusion_volume": (i32, [vp, C.POINTER(vp), C.POINTER(vp), C.POINTER(i32)]),
     "afx_fusion_graph": (i32, [vp, C.POINTER(vp), C.POINTER(vp), C.POINTER(vp), C.POINTER(vp)]),
     "afx_fusion_centroid": (i32, [vp, C.POINTER(vp)]),

@@ -7,6 +7,7 @@
 // correspondences and Gauss-Newton control (energy test, commit of pending transforms)
 // all stay on the GPU.  The reference blocks on cudaDeviceSynchronize and copies the
 // point cloud and graph to the host every frame.
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
@@ -20,6 +21,7 @@
 
 #include "afx_gn.h"
 #include "afx_host.h"
+#include "afx_store.cuh"
 #include "afx_voxel.h"
 
 namespace afx {
@@ -115,6 +117,8 @@ struct WorkMarks {
 
 using namespace afx;
 
+constexpr long kEpochsPerClear = 1L << 20;  // of 2^24 epochs
+
 struct afx_fusion {
     afx_fusion_params p;
     Volume vol;
@@ -208,6 +212,7 @@ struct afx_fusion {
     cudaEvent_t ev_in_ready[2] = {nullptr, nullptr}, ev_in_free[2] = {nullptr, nullptr};
     cudaGraphExec_t gexec[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
     cudaGraph_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // kept for batch graphs
+    long epochs_used = 0;      // frames since the collision words were cleared, as of the last reset
     unsigned graph_epoch = 0;  // advanced whenever the captured graphs are dropped
     int mc_tile = kMcTileTma16;  // marching-cubes tile (afx_fusion_autotune)
     long glaunches[2][2] = {{0, 0}, {0, 0}};  // kernels in each captured frame
@@ -262,6 +267,37 @@ __global__ void stats_kernel(FrameStats* s, int* frame, const int* n_nodes, cons
     s->mesh_vertices = *nv;
     s->mesh_faces = *nf;
     s->error = *error;
+}
+
+// `bytes` (even) at p, on 16 bytes, filled with a word: 16 bytes a store, four in flight a thread (an element a thread
+// took 263 us for 512^3 FP16 values, now 43).
+__global__ void __launch_bounds__(256) fill_kernel(uint4* p, long bytes, unsigned word) {
+    const long n = bytes / 16, step = (long)gridDim.x * blockDim.x;
+    const uint4 v = make_uint4(word, word, word, word);
+    const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
+#pragma unroll 4
+    for (long i = t; i < n; i += step) p[i] = v;
+    if (t < bytes % 16 / 2) reinterpret_cast<unsigned short*>(p + n)[t] = (unsigned short)(t & 1 ? word >> 16 : word);
+}
+
+// The volume as FP32: four times four voxels a thread, all read before the first is written.
+constexpr int kExportGroups = 4;
+
+template <class TT, class WT>
+__global__ void __launch_bounds__(256) export_volume_kernel(const TT* __restrict__ t, const WT* __restrict__ w,
+                                                            float* __restrict__ to, float* __restrict__ wo, long n) {
+    const long first = blockIdx.x * (256L * kExportGroups) + threadIdx.x;
+    float tv[kExportGroups][4], wv[kExportGroups][4];
+#pragma unroll
+    for (int g = 0; g < kExportGroups; ++g)
+        if (first + 256 * g < n / 4) vox_get4(t, w, 4 * (first + 256 * g), tv[g], wv[g]);
+#pragma unroll
+    for (int g = 0; g < kExportGroups; ++g)
+        if (first + 256 * g < n / 4) vox_put4(to, wo, 4 * (first + 256 * g), tv[g], wv[g]);
+    if (first < n % 4) {
+        const long i = n / 4 * 4 + first;
+        vox_put(to, wo, i, vox_get_t(t, i), vox_get_w(w, i));
+    }
 }
 
 static size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -570,32 +606,28 @@ int afx_fusion_destroy(afx_fusion* f) {
     return note_cuda_error(e);
 }
 
-__global__ void fill_kernel(float* p, long n, float v) {
-    long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (i < n) p[i] = v;
-}
-
-__global__ void fill_u16_kernel(unsigned short* p, long n, unsigned short v) {
-    long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (i < n) p[i] = v;
-}
-
 int afx_fusion_reset(afx_fusion* f, void* stream) {
     if (!f) return AFX_ERR_INVALID_ARGUMENT;
     cudaStream_t st = as_stream(stream);
     // DeviceTsdf::initDefault: values -1, weights 0 (0xBC00 is -1 in FP16)
-    if (f->fmt == kVoxF16)
-        fill_u16_kernel<<<blocks_for(f->S, 256), 256, 0, st>>>(static_cast<unsigned short*>(f->tsdf), f->S, 0xBC00);
-    else
-        fill_kernel<<<blocks_for(f->S, 256), 256, 0, st>>>(static_cast<float*>(f->tsdf), f->S, -1.f);
+    const long tsdf_bytes = f->S * vox_bytes(f->fmt);
+    const unsigned word = f->fmt == kVoxF16 ? 0xBC00BC00u : 0xBF800000u;
+    fill_kernel<<<(unsigned)std::min<long>(blocks_for(tsdf_bytes / 16, 256), 1216), 256, 0, st>>>(static_cast<uint4*>(f->tsdf),
+                                                                                                tsdf_bytes, word);
     AFX_LAUNCH_CHECK();
     AFX_CUDA(cudaMemsetAsync(f->weights, 0, f->S * vox_bytes(f->fmt), st));
-    AFX_CUDA(cudaMemsetAsync(f->coll, 0, f->S * 4, st));
+    // Collision words are read by their epoch, which goes on over sequences: words of an earlier one count as empty.
+    // They are cleared, and the epoch with them, long before it comes round.
+    f->epochs_used += f->frame;
+    if (f->epochs_used >= kEpochsPerClear) {
+        AFX_CUDA(cudaMemsetAsync(f->coll, 0, f->S * 4, st));
+        AFX_CUDA(cudaMemsetAsync(f->epoch, 0, 64, st));
+        f->epochs_used = 0;
+    }
     AFX_CUDA(cudaMemsetAsync(f->occ, 0, brick_count_total(f->vol), st));
     AFX_CUDA(cudaMemsetAsync(f->centroid0, 0, 64, st));
     AFX_CUDA(cudaMemsetAsync(f->acc, 0, 64, st));
     AFX_CUDA(cudaMemsetAsync(f->error, 0, 64, st));
-    AFX_CUDA(cudaMemsetAsync(f->epoch, 0, 64, st));
     AFX_CUDA(cudaMemsetAsync(f->npoints_buf[0], 0, 64, st));
     AFX_CUDA(cudaMemsetAsync(f->npoints_buf[1], 0, 64, st));
     AFX_CUDA(cudaMemsetAsync(f->mesh_used, 0, 64, st));
@@ -1014,6 +1046,23 @@ int afx_fusion_tsdf(afx_fusion* f, float** tsdf, float** weights) {
     if (f->fmt != kVoxF32) return AFX_ERR_UNSUPPORTED;  // FP16 sessions: afx_fusion_volume
     if (tsdf) *tsdf = static_cast<float*>(f->tsdf);
     if (weights) *weights = static_cast<float*>(f->weights);
+    return AFX_OK;
+}
+
+int afx_fusion_export_volume(afx_fusion* f, float* tsdf, float* weights, void* stream) {
+    if (!f || !tsdf || !weights) return AFX_ERR_INVALID_ARGUMENT;
+    if (((size_t)tsdf | (size_t)weights) & 15) return AFX_ERR_INVALID_ARGUMENT;
+    cudaStream_t st = as_stream(stream);
+    if (f->fmt != kVoxF16) {
+        AFX_CUDA(cudaMemcpyAsync(tsdf, f->tsdf, (size_t)f->S * 4, cudaMemcpyDeviceToDevice, st));
+        AFX_CUDA(cudaMemcpyAsync(weights, f->weights, (size_t)f->S * 4, cudaMemcpyDeviceToDevice, st));
+        f->work.note(st);
+        return AFX_OK;
+    }
+    export_volume_kernel<<<blocks_for(f->S / 4, 256 * kExportGroups), 256, 0, st>>>(
+        static_cast<const __half*>(f->tsdf), static_cast<const unsigned short*>(f->weights), tsdf, weights, f->S);
+    AFX_LAUNCH_CHECK();
+    f->work.note(st);
     return AFX_OK;
 }
 

@@ -109,13 +109,12 @@ class FusionSession:
 
     def tsdf(self):
         """Copies of the volume as FP32 tensors (values, weights), whatever the storage format."""
-        t, w, prec = C.c_void_p(), C.c_void_p(), C.c_int(0)
-        check(lib().afx_fusion_volume(self.h, C.byref(t), C.byref(w), C.byref(prec)), "afx_fusion_volume")
-        if prec.value == 0:
-            return _wrap_device(t.value, self.S, torch.float32), _wrap_device(w.value, self.S, torch.float32)
-        # precision form: FP16 values widen exactly; uint16 weights are counts <= 15
-        return (_wrap_device(t.value, self.S, torch.float16).float(),
-                _wrap_device(w.value, self.S, torch.int16).float())
+        t, w = (torch.empty(self.S, dtype=torch.float32, device="cuda") for _ in range(2))
+        st = torch.cuda.current_stream()
+        check(lib().afx_fusion_export_volume(self.h, C.c_void_p(t.data_ptr()), C.c_void_p(w.data_ptr()),
+                                             C.c_void_p(st.cuda_stream)), "afx_fusion_export_volume")
+        st.synchronize()
+        return t, w
 
     def volume_raw(self):
         """The stored arrays as they are: (values, weights, precision) with FP16 / int16 (bit
