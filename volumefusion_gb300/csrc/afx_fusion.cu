@@ -214,7 +214,7 @@ struct afx_fusion {
     cudaGraph_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // kept for batch graphs
     long epochs_used = 0;      // frames since the collision words were cleared, as of the last reset
     unsigned graph_epoch = 0;  // advanced whenever the captured graphs are dropped
-    int mc_tile = kMcTileTma16;  // marching-cubes tile (afx_fusion_autotune)
+    int mc_tile = kMcTileTma16;  // marching-cubes tile (by size at creation; afx_fusion_autotune)
     long glaunches[2][2] = {{0, 0}, {0, 0}};  // kernels in each captured frame
     long replayed = 0;                        // kernels launched by graph replays
     WorkMarks work;                           // streams holding this session's work (destroy waits on them)
@@ -394,6 +394,11 @@ static void session_layout(const afx_fusion_params& p, afx_fusion* f) {
     for (int c = 0; c < 3; ++c) vs[c] = p.volume_size[c] / (float)p.dims[c];
     f->vol = make_volume(p.dims, vs, p.volume_size);
     f->S = (long)p.dims[0] * p.dims[1] * p.dims[2];
+    // Until the autotuner chooses: a CTA per tile in small volumes, the list of occupied tiles where most tiles are empty.
+    // A capsule pair, a CTA per 16-deep tile against the 4-deep list: 128^3 17.6 and 21.3 us, 192^3 21.8 and 21.1,
+    // 256^3 47 and 38 (but the list's launches wait for each other: the whole sequence took 12.9 and 13.1 ms), 384^3
+    // 50 and 39, 512^3 FP16 108 and 61 (the sequence 7.8 and 7.4 ms).
+    f->mc_tile = f->S >= 20000000 ? kMcTilePipe4 : kMcTileTma16;
     f->P = (long)p.width * p.height;
     // voxels per node cube: 2 * ((r / voxelSize).cast<int>() + 1) + 1 (src/VolumeFusion.cu:702-706)
     for (int c = 0; c < 3; ++c) f->per[c] = 2 * ((int)(p.graph_radius / vs[c]) + 1) + 1;
