@@ -791,7 +791,7 @@ static int enqueue_frame(afx_fusion* f, const uint16_t* depth_mm, cudaStream_t s
     g.b = f->gn;
     g.error = f->error;
     stage_mark(f, ST_GN_SETUP, st);
-    rc = gn_frame_setup(g, st, true);
+    rc = gn_frame_setup(g, st);
     if (rc) return rc;
     const double tol = p.solver == 2 ? p.pcg_tol : 0.0;
     for (int icp = 0; icp < p.icp_iterations; ++icp) {

@@ -45,10 +45,11 @@ AFX_D void jdepth(const float* n, float w, const float G[3][6], float lam, float
 // ---- per-frame node lists ----
 //
 // Two sets of lists, both ascending: the (vertex, slot) entries of every node and its incoming
-// regularisation edges.  Count, offsets, fill and sort take one launch each for the two sets
-// together: the launches are what these steps cost (a few us each for tens of kB).
+// regularisation edges.  The launches are what these steps cost (a few us each for tens of kB), so offsets,
+// fill and sort take one each for the two sets together, and the counts are part of a launch before them
+// (graph_weights_kernel in a session, gn_corr_of_vertex_kernel here).
 
-__global__ void list_count_kernel(GnArgs a) {
+AFX_D void list_counts(const GnArgs& a) {
     const long m = min((long)*a.mesh_count, a.m_max);
     const int n = min(*a.n_nodes, a.n_max);
     AFX_GRID_STRIDE(t, m * a.k) {
@@ -2345,14 +2346,9 @@ constexpr int kNodeCtas = 608;  // CTAs that take one node at a time: four of 25
 // Per frame: node -> vertex lists and incoming regularisation edges.
 size_t gn_counter_words(int n_max) { return 4 * al((n_max + 1) * 4) / 4; }
 
-int gn_frame_setup(const GnArgs& a, cudaStream_t st, bool counted) {
+int gn_frame_setup(const GnArgs& a, cudaStream_t st) {
     const GnBuffers& b = a.b;
     const long items = std::max(a.m_max * a.k, (long)a.n_max * a.kreg);
-    if (!counted) {
-        AFX_CUDA(cudaMemsetAsync(b.lcnt, 0, gn_counter_words(a.n_max) * 4, st));  // lcnt lcur icnt icur
-        list_count_kernel<<<grid_for(items, 256), 256, 0, st>>>(a);
-        AFX_LAUNCH_CHECK();
-    }
     list_scan_kernel<<<2, 1024, 0, st>>>(a);
     AFX_LAUNCH_CHECK();
     list_fill_kernel<<<grid_for(items, 256), 256, 0, st>>>(a);
@@ -2431,9 +2427,24 @@ int gn_loop(const GnArgs& a, const float* points, float* warped, float* T_commit
 
 namespace afx {
 
-__global__ void gn_corr_of_vertex_kernel(const int* corr, const unsigned* n_corr, long c_max, int* cov) {
-    const long nc = min((long)*n_corr, c_max);
-    AFX_GRID_STRIDE(c, nc) cov[corr[2 * c]] = (int)c;
+// The start of a build in one launch (six copies and clears otherwise): the counts that later calls use, no error, no
+// correspondence of any vertex, and the lists' counters at zero.
+__global__ void gn_begin_kernel(unsigned* counts, const unsigned* n_points, const unsigned* n_corr, const int* n_nodes, int* error,
+                                int* cov, long m_max, unsigned* counters, long words) {
+    AFX_GRID_STRIDE(i, m_max) cov[i] = -1;
+    AFX_GRID_STRIDE(i, words) counters[i] = 0u;
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    counts[0] = *n_points;
+    counts[1] = *n_corr;
+    counts[2] = (unsigned)*n_nodes;
+    *error = 0;
+}
+
+// The correspondence of each vertex, and the lists' counts.
+__global__ void gn_corr_of_vertex_kernel(const int* corr, const unsigned* n_corr, long c_max, int* cov, GnArgs a) {
+    const long c = min((long)*n_corr, c_max);
+    AFX_GRID_STRIDE(i, c) cov[corr[2 * i]] = (int)i;
+    list_counts(a);
 }
 
 __global__ void __launch_bounds__(256) gn_residual_kernel(GnArgs a, const float* warped, const float* T) {
@@ -2558,10 +2569,11 @@ int afx_gn_build(afx_gn* g, const float* canonical, const unsigned* n_points, co
         !frame_normals || !warped || !nodes || !transforms || !n_nodes || !graph_idx)
         return AFX_ERR_INVALID_ARGUMENT;
     cudaStream_t st = as_stream(stream);
+    const long words = (long)gn_counter_words(g->n_max);
+    gn_begin_kernel<<<grid_for(std::max(g->m_max, words), 256), 256, 0, st>>>(g->counts, n_points, n_corr, n_nodes, g->error,
+                                                                              g->cov, g->m_max, g->b.lcnt, words);
+    AFX_LAUNCH_CHECK();
     // later calls use these copies, not the caller's counters
-    AFX_CUDA(cudaMemcpyAsync(g->counts, n_points, 4, cudaMemcpyDeviceToDevice, st));
-    AFX_CUDA(cudaMemcpyAsync(g->counts + 1, n_corr, 4, cudaMemcpyDeviceToDevice, st));
-    AFX_CUDA(cudaMemcpyAsync(g->counts + 2, n_nodes, 4, cudaMemcpyDeviceToDevice, st));
     n_points = g->counts;
     n_corr = g->counts + 1;
     n_nodes = reinterpret_cast<const int*>(g->counts + 2);
@@ -2588,11 +2600,10 @@ int afx_gn_build(afx_gn* g, const float* canonical, const unsigned* n_points, co
     a.lam_r = lambda_reg;
     a.b = g->b;
     a.error = g->error;
-    AFX_CUDA(cudaMemsetAsync(g->error, 0, 4, st));
-    AFX_CUDA(cudaMemsetAsync(g->cov, 0xff, (size_t)g->m_max * 4, st));
-    gn_corr_of_vertex_kernel<<<grid_for(g->m_max, 256), 256, 0, st>>>(corr, n_corr, g->m_max, g->cov);
+    gn_corr_of_vertex_kernel<<<grid_for(std::max(g->m_max * g->k, (long)g->n_max * g->kreg), 256), 256, 0, st>>>(
+        corr, n_corr, g->m_max, g->cov, a);
     AFX_LAUNCH_CHECK();
-    int rc = gn_frame_setup(a, st, false);
+    int rc = gn_frame_setup(a, st);
     if (rc) return rc;
     rc = gn_icp_setup(a, nullptr, nullptr, st);
     if (rc) return rc;

@@ -73,10 +73,9 @@ struct GnArgs {
 
 size_t gn_workspace_size(long m_max, int n_max, int k, int kreg);
 bool gn_carve(void* ws, size_t bytes, long m_max, int n_max, int k, int kreg, GnBuffers* b);
-// The counters of the lists (words from b.lcnt on), and the lists; `counted`: the caller has cleared them and counted
-// entries and edges (graph_weights_impl).
+// The lists' counters: words from b.lcnt on, cleared and counted by the caller before gn_frame_setup.
 size_t gn_counter_words(int n_max);
-int gn_frame_setup(const GnArgs& a, cudaStream_t st, bool counted);
+int gn_frame_setup(const GnArgs& a, cudaStream_t st);
 int gn_icp_setup(const GnArgs& a, float* T_pending, const float* T_committed, cudaStream_t st);
 int gn_loop(const GnArgs& a, const float* points, float* warped, float* T_committed, float* T_pending, int gn_iters,
             int pcg_iters, double tol, cudaStream_t st);
