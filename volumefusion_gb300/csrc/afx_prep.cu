@@ -161,6 +161,43 @@ AFX_D float bilateral_at(int x, int y, int w, int h, const BilateralTables& T, A
     return iF / wP;
 }
 
+// The same for a pixel whose window lies inside the image, from a tile in shared memory (c: the pixel; clr: the colour
+// weights, also there: lanes look up different ones, which constant memory serves one by one).  Unrolled, with no
+// clamps, a tap is about a dozen instructions, a third of what the loop above takes; instructions bound these kernels.
+// prep_kernel at 640 x 576: 14.3 -> 11.5 us; the rigid stream, three such cameras: 15.5 -> 14.7 us.
+template <int R>
+AFX_D float bilateral_inside(const float* c, int pitch, const BilateralTables& T, const float* clr) {
+    const float centre = c[0];
+    if (isinf(centre)) return centre;
+    float iF = 0.f, wP = 0.f;
+#pragma unroll
+    for (int a = -R; a <= R; ++a)
+#pragma unroll
+        for (int b = -R; b <= R; ++b) {
+            const float cur = c[b * pitch + a];
+            const float diff = fabsf(centre - cur);
+            if (isinf(cur) || diff > T.thr) continue;
+            const unsigned bucket = min((unsigned)f2i(fabsf(diff * T.norm_factor)), 30u);  // negative: past the end too
+            const float wt = T.g2d[(a + R) * (2 * R + 1) + b + R] * clr[bucket];
+            iF = iF + cur * wt;
+            wP = wP + wt;
+        }
+    return iF / wP;
+}
+
+// Pixel (x, y) of the tile; `at` gives the pixels of windows that the image's border clamps.
+template <class At>
+AFX_D float bilateral_tile(const float* c, int pitch, int x, int y, int w, int h, const BilateralTables& T, const float* clr,
+                           At at) {
+    const int r = T.r;
+    if (x >= r && x + r < w && y >= r && y + r < h) {
+        if (r == 2) return bilateral_inside<2>(c, pitch, T, clr);
+        if (r == 1) return bilateral_inside<1>(c, pitch, T, clr);
+        if (r == 3) return bilateral_inside<3>(c, pitch, T, clr);
+    }
+    return bilateral_at(x, y, w, h, T, at);
+}
+
 // ------------------------------------------------------------------------------------
 // Fused frame preparation
 // ------------------------------------------------------------------------------------
@@ -204,7 +241,9 @@ __global__ void __launch_bounds__(kTW * kTH) prep_kernel(const __grid_constant__
     __shared__ alignas(8) unsigned long long mbar;
     __shared__ long long red[4][kTW * kTH / 32];
 
+    __shared__ float clr[31];
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kTW + tx;
+    if (tid < 31) clr[tid] = (float)A.tab.clr[tid];
     const int x0 = blockIdx.x * kTW, y0 = blockIdx.y * kTH;
     const int W = A.width, H = A.height;
     const int inW = kTW + 2 * A.xhalo, inH = kTH + 2 * A.halo;
@@ -282,7 +321,8 @@ __global__ void __launch_bounds__(kTW * kTH) prep_kernel(const __grid_constant__
         int gx = x0 - 1 + i % bw, gy = y0 - 1 + i / bw;
         float v = __int_as_float(0x7f800000);
         if (gx >= 0 && gx < W && gy >= 0 && gy < H)
-            v = A.bilateral ? bilateral_at(gx, gy, W, H, A.tab, at_dep) : at_dep(gx, gy);
+            v = A.bilateral ? bilateral_tile(dep + (gy - gy0) * inW + (gx - gx0), inW, gx, gy, W, H, A.tab, clr, at_dep)
+                            : at_dep(gx, gy);
         bil[i] = v;
         // back-projection (src/VertexManipulation.cu:43-63)
         float* o = ver + 3 * i;
@@ -356,6 +396,8 @@ __global__ void __launch_bounds__(kTW * kTH) stream_prep_kernel(const __grid_con
     const StreamCamera& cam = A.cam[blockIdx.z];
     const int W = A.width, H = A.height, r = tab.r;
     const int tid = threadIdx.y * kTW + threadIdx.x;
+    __shared__ float clr[31];
+    if (tid < 31) clr[tid] = (float)tab.clr[tid];
     const int inW = kTW + 2 * r, inH = kTH + 2 * r;
     const int gx0 = blockIdx.x * kTW - r, gy0 = blockIdx.y * kTH - r;
     const uint16_t* __restrict__ mm = cam.mm;
@@ -370,7 +412,7 @@ __global__ void __launch_bounds__(kTW * kTH) stream_prep_kernel(const __grid_con
     const int x = blockIdx.x * kTW + threadIdx.x, y = blockIdx.y * kTH + threadIdx.y;
     if (x >= W || y >= H) return;
     auto at = [&](int xx, int yy) -> float { return dep[(yy - gy0) * inW + (xx - gx0)]; };
-    const float d = A.bilateral ? bilateral_at(x, y, W, H, tab, at) : at(x, y);
+    const float d = A.bilateral ? bilateral_tile(dep + (y - gy0) * inW + (x - gx0), inW, x, y, W, H, tab, clr, at) : at(x, y);
     const long p = (long)y * W + x;
     cam.depth[p] = d;
     float v[3] = {0.f, 0.f, 0.f}, o[3];
