@@ -822,6 +822,7 @@ static int enqueue_frame(afx_fusion* f, const uint16_t* depth_mm, cudaStream_t s
     wa.vol = f->vol;
     wa.bg = make_bricks(f->vol);
     wa.k = p.knn;
+    wa.n_max = N;
     wa.nodes_t = f->nodes_t;
     wa.radii = f->radii;
     wa.transforms = f->T;

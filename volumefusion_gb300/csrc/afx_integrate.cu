@@ -367,7 +367,8 @@ __global__ void brick_active_kernel(const unsigned* brick_count, long nb, unsign
     if (on) active[base + __popc(m & ((1u << lane) - 1))] = (unsigned)b;
 }
 
-AFX_D void topk_insert(float* kd, int* ki, int& cnt, int cap, float d, int idx) {
+template <class Id>
+AFX_D void topk_insert(float* kd, Id* ki, int& cnt, int cap, float d, Id idx) {
     if (cnt == cap && !(d < kd[cap - 1] || (d == kd[cap - 1] && idx < ki[cap - 1]))) return;
     int i = (cnt < cap) ? cnt++ : cap - 1;
     while (i > 0 && (d < kd[i - 1] || (d == kd[i - 1] && idx < ki[i - 1]))) {
@@ -399,12 +400,13 @@ AFX_D int coll_get(const unsigned* w, unsigned epoch) {
 // candidate's word say so.  The list is kept sorted in registers (indexed ones went to local memory).
 // Bound: the chain active brick -> candidates -> nodes in front of each brick.  200^3 voxels, 600 nodes, dense lists: 24.4 ->
 // 14.6 us; a frame of the 256^3 sequence 23 -> 17 us, of the 512^3 sequence 57 -> 40 us.
-template <int K>
+// Id: a node and its place in the brick's list in one number, 64 bits for graphs whose nodes do not fit in 24.
+template <int K, class Id>
 __global__ void __launch_bounds__(kBrickVox) brick_warp_kernel(WarpArgs a) {
     __shared__ float4 s_node[kMaxBrickNodes];      // position, radius
     __shared__ float4 s_T[kMaxBrickNodes * 4];     // columns of the transform
     __shared__ unsigned s_cube[kMaxBrickNodes];    // x, y, z of the brick inside the node's cube, eight bits each
-    __shared__ unsigned s_id[kMaxBrickNodes];      // node << 8 | place here
+    __shared__ Id s_id[kMaxBrickNodes];            // node << 8 | place here
     static_assert(kMaxBrickNodes <= 256, "a place fits in eight bits");
     const unsigned n_active = *a.n_active;
     const int lx = threadIdx.x % kBrick, ly = (threadIdx.x / kBrick) % kBrick, lz = threadIdx.x / (kBrick * kBrick);
@@ -420,7 +422,7 @@ __global__ void __launch_bounds__(kBrickVox) brick_warp_kernel(WarpArgs a) {
     for (int i = threadIdx.x; i < nc; i += blockDim.x) {
         const unsigned j = a.brick_nodes[off + i];
         const float p[3] = {a.nodes_t[3 * (long)j], a.nodes_t[3 * (long)j + 1], a.nodes_t[3 * (long)j + 2]};
-        s_id[i] = j << 8 | (unsigned)i;
+        s_id[i] = (Id)j << 8 | (unsigned)i;
         s_node[i] = make_float4(p[0], p[1], p[2], a.radii[j]);
         odd |= p[0] != p[0] || p[1] != p[1] || p[2] != p[2];
         NodeCube c;
@@ -443,9 +445,9 @@ __global__ void __launch_bounds__(kBrickVox) brick_warp_kernel(WarpArgs a) {
     const long local = (long)slot * kBrickVox + threadIdx.x;
     const int X = a.vol.dims[0], Y = a.vol.dims[1], Z = a.vol.dims[2];
     const bool inside = x < X && y < Y && z < Z;
-    constexpr unsigned kEmpty = 0xffffffffu;
+    constexpr Id kEmpty = ~(Id)0;
     float kd[K];
-    unsigned ki[K];  // as s_id: in node order
+    Id ki[K];  // as s_id: in node order
 #pragma unroll
     for (int s = 0; s < K; ++s) {
         kd[s] = INFINITY;
@@ -460,7 +462,7 @@ __global__ void __launch_bounds__(kBrickVox) brick_warp_kernel(WarpArgs a) {
             const float d3[3] = {p[0] - v.x, p[1] - v.y, p[2] - v.z};
             const float d = norm3(d3);
             if (d > v.w * 2.0f) continue;
-            const unsigned id = s_id[i];
+            const Id id = s_id[i];
             if (!(d < kd[K - 1] || (d == kd[K - 1] && id < ki[K - 1]))) continue;
             kd[K - 1] = d;
             ki[K - 1] = id;
@@ -468,7 +470,7 @@ __global__ void __launch_bounds__(kBrickVox) brick_warp_kernel(WarpArgs a) {
             for (int s = K - 1; s > 0; --s) {
                 const bool up = kd[s] < kd[s - 1] || (kd[s] == kd[s - 1] && ki[s] < ki[s - 1]);
                 const float ds = kd[s], dt = kd[s - 1];
-                const unsigned is = ki[s], it = ki[s - 1];
+                const Id is = ki[s], it = ki[s - 1];
                 kd[s] = up ? dt : ds;
                 kd[s - 1] = up ? ds : dt;
                 ki[s] = up ? it : is;
@@ -477,7 +479,7 @@ __global__ void __launch_bounds__(kBrickVox) brick_warp_kernel(WarpArgs a) {
         }
     } else if (inside) {  // distances that are not numbers keep the place they were put at
         float ld[K];
-        int li[K];
+        Id li[K];
         int n = 0;
         for (int i = 0; i < nc; ++i) {
             if ((s_cube[i] & here) != here) continue;
@@ -485,11 +487,11 @@ __global__ void __launch_bounds__(kBrickVox) brick_warp_kernel(WarpArgs a) {
             const float d3[3] = {p[0] - v.x, p[1] - v.y, p[2] - v.z};
             const float d = norm3(d3);
             if (d > v.w * 2.0f) continue;
-            topk_insert(ld, li, n, K < a.k ? K : a.k, d, (int)s_id[i]);
+            topk_insert(ld, li, n, K < a.k ? K : a.k, d, s_id[i]);
         }
         for (int s = 0; s < n; ++s) {
             kd[s] = ld[s];
-            ki[s] = (unsigned)li[s];
+            ki[s] = li[s];
         }
     }
     int cnt = 0;
@@ -501,7 +503,7 @@ __global__ void __launch_bounds__(kBrickVox) brick_warp_kernel(WarpArgs a) {
 #pragma unroll
         for (int s = 0; s < K; ++s) {
             if (s >= a.k) break;
-            a.dense_idx[v * a.k + s] = s < cnt ? ki[s] >> 8 : AFX_INVALID_INDEX;
+            a.dense_idx[v * a.k + s] = s < cnt ? (uint32_t)(ki[s] >> 8) : AFX_INVALID_INDEX;
             a.dense_dist[v * a.k + s] = s < cnt ? kd[s] : 3.402823466e+38f;
         }
     }
@@ -515,7 +517,7 @@ __global__ void __launch_bounds__(kBrickVox) brick_warp_kernel(WarpArgs a) {
     for (int s = 0; s < K; ++s) {
         w[s] = 0.f;
         if (s >= cnt) continue;
-        const float r = s_node[ki[s] & 0xffu].w, d = kd[s];
+        const float r = s_node[(unsigned)ki[s] & 0xffu].w, d = kd[s];
         w[s] = afx_expf(-(d * d) / (2.0f * (r * r)));
         sum = sum + w[s];
     }
@@ -532,14 +534,14 @@ __global__ void __launch_bounds__(kBrickVox) brick_warp_kernel(WarpArgs a) {
     float q[3] = {c[0], c[1], c[2]};
     if (!zero && a.blend == AFX_BLEND_DQB) {  // dual-quaternion blend (afx_dqb.cuh)
         uint32_t kidx[K];
-        for (int s = 0; s < cnt; ++s) kidx[s] = ki[s] >> 8;
+        for (int s = 0; s < cnt; ++s) kidx[s] = (uint32_t)(ki[s] >> 8);
         dq_blend_point(a.transforms, kidx, w, cnt, AFX_INVALID_INDEX, c, q);
     } else if (!zero) {  // warpTsdfKernel (src/TSDFWarp.cu:158-190)
         q[0] = q[1] = q[2] = 0.f;
 #pragma unroll
         for (int s = 0; s < K; ++s) {
             if (s >= cnt) continue;
-            const float4* T = s_T + 4 * (ki[s] & 0xffu);
+            const float4* T = s_T + 4 * ((unsigned)ki[s] & 0xffu);
             const float4 t0 = T[0], t1 = T[1], t2 = T[2], t3 = T[3];
             const float M[16] = {t0.x, t0.y, t0.z, 0.f, t1.x, t1.y, t1.z, 0.f, t2.x, t2.y, t2.z, 0.f, t3.x, t3.y, t3.z, 0.f};
             float o[3];
@@ -676,9 +678,13 @@ static unsigned brick_grid(long max_active) { return (unsigned)(max_active < 608
 
 int launch_brick_warp(const WarpArgs& a, long max_active, cudaStream_t st) {
     if (max_active <= 0) return AFX_OK;
-    switch (a.k <= 4 ? 4 : 8) {
-        case 4: brick_warp_kernel<4><<<brick_grid(max_active), kBrickVox, 0, st>>>(a); break;
-        default: brick_warp_kernel<8><<<brick_grid(max_active), kBrickVox, 0, st>>>(a); break;
+    const unsigned grid = brick_grid(max_active);
+    if (a.n_max > 1 << 24) {  // node numbers past 24 bits
+        if (a.k <= 4) brick_warp_kernel<4, unsigned long long><<<grid, kBrickVox, 0, st>>>(a);
+        else brick_warp_kernel<8, unsigned long long><<<grid, kBrickVox, 0, st>>>(a);
+    } else {
+        if (a.k <= 4) brick_warp_kernel<4, unsigned><<<grid, kBrickVox, 0, st>>>(a);
+        else brick_warp_kernel<8, unsigned><<<grid, kBrickVox, 0, st>>>(a);
     }
     AFX_LAUNCH_CHECK();
     return AFX_OK;
@@ -904,6 +910,7 @@ int afx_tsdf_knn(uint32_t* knn_idx, float* knn_dist, int* knn_counts, const floa
     a.vol = vol;
     a.bg = make_bricks(vol);
     a.k = k;
+    a.n_max = n_nodes;
     a.nodes_t = nodes;
     a.radii = radii;
     a.brick_offset = s.brick_offset;

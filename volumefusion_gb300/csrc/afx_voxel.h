@@ -52,6 +52,7 @@ struct WarpArgs {
     Volume vol;
     BrickGrid bg;
     int k;
+    int n_max;                // most nodes there can be
     const float* nodes_t;     // translated node positions
     const float* radii;
     const float* transforms;  // committed node transforms (column-major 4x4)
