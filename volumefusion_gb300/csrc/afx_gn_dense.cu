@@ -351,6 +351,11 @@ __global__ void __launch_bounds__(kLuMaxPanelThreads) lu_panel_kernel(float* A, 
             failed = true;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
+                if (live[r] && pos[r] == (unsigned)c) {  // the row stays here: no candidate of a later column
+                    live[r] = false;
+#pragma unroll
+                    for (int j = 0; j < kW; ++j) prow[c][j] = a[r][j];
+                }
                 mult[c * rows + r * blockDim.x + t] = a[r][0];
 #pragma unroll
                 for (int j = 1; j < kW; ++j) a[r][j - 1] = a[r][j];
@@ -492,7 +497,11 @@ __global__ void __launch_bounds__(kLuThreads) lu_update_kernel(float* A, int n, 
     const int nc = min(kLuTC, (right ? n : k0) - c0);
     const int bad = *info;  // columns from bad - 1 on have no updates
     const int nk = bad == 0 ? w : max(0, min(w, bad - 1 - k0));
-    if (t < w) p[t] = ipiv[k0 + t] <= n ? ipiv[k0 + t] - 1 : k0 + t;  // a column without a pivot swaps nothing
+    if (t < w) {  // a column without a pivot (its diagonal element is zero or not a number) swaps nothing
+        const int q = ipiv[k0 + t] - 1;
+        const float d = bad != 0 ? A[k0 + t + (long)(k0 + t) * lda] : 1.f;
+        p[t] = q < n && d == d && d != 0.f ? q : k0 + t;
+    }
     __syncthreads();
     if (t < 2 * w) {
         const int d = t < w ? k0 + t : p[t - w];
