@@ -248,7 +248,7 @@ constexpr size_t kAsmListBytes = (size_t)kAsmPass * kAsmThreads * sizeof(unsigne
 
 template <int KM>  // at least k slots per vertex
 __global__ void __launch_bounds__(kAsmThreads, KM <= 4 ? 4 : 3) jtj_assemble_kernel(GnArgs a) {
-    extern __shared__ float2 asm_dyn[];
+    extern __shared__ __align__(16) float2 asm_dyn[];
     float* const J = reinterpret_cast<float*>(asm_dyn);             // [256][stride]
     unsigned* const bm = reinterpret_cast<unsigned*>(asm_dyn);      // neighbour bitmap, before the rows
     __shared__ int s_L[kMaxNbr];
@@ -1117,13 +1117,17 @@ struct DsLayout {
 constexpr size_t kDsSmem = sizeof(float) * ((size_t)kDsNodes * 12 + 3 * kDsNpc * 6 + kDsNpc * 36 + (size_t)kDsBlocks * 36) +
                            sizeof(int) * (kDsBlocks + kDsNpc + 1 + 4) + sizeof(double) * (2 * kDsMaxCta * 4 + 4) + 64;
 
+// `base` on 16 bytes: blocks, inverses, z and p are also copied and read 16 bytes at a time.
 AFX_D DsLayout ds_layout(void* base) {
+    static_assert(sizeof(double) * (2 * kDsMaxCta * 4 + 4) % 16 == 0 && sizeof(float) * kDsNodes * 6 % 16 == 0 &&
+                      sizeof(float) * kDsNpc * 6 % 16 == 0 && sizeof(float) * kDsNpc * 36 % 16 == 0,
+                  "every array from z on starts on 16 bytes");
     DsLayout d;
     double* dp = static_cast<double*>(base);
     d.slot = dp;
     d.bar = reinterpret_cast<unsigned long long*>(dp + 2 * kDsMaxCta * 4);
     d.scal = reinterpret_cast<float*>(dp + 2 * kDsMaxCta * 4 + 2);
-    float* f = reinterpret_cast<float*>(dp + 2 * kDsMaxCta * 4 + 4);  // 16-byte aligned
+    float* f = reinterpret_cast<float*>(dp + 2 * kDsMaxCta * 4 + 4);
     d.z = f;
     f += kDsNodes * 6;
     d.pf = f;
@@ -2146,7 +2150,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) gn_loop_kernel(LoopArgs L) {
     const GnArgs& a = L.g;
     const GnBuffers& b = a.b;
     __shared__ ClusterSums cs;
-    extern __shared__ double ds_smem[];
+    extern __shared__ __align__(16) double ds_smem[];
     const DsLayout dsl = ds_layout(ds_smem);
     if (threadIdx.x == 0) {
         cs.phase = 0;
@@ -2221,7 +2225,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) gn_loop_kernel(LoopArgs L) {
 __global__ void __launch_bounds__(kLoopThreads, 1) gn_solve_kernel(LoopArgs L) {
     const GnArgs& a = L.g;
     __shared__ ClusterSums cs;
-    extern __shared__ double ds_smem[];
+    extern __shared__ __align__(16) double ds_smem[];
     const DsLayout dsl = ds_layout(ds_smem);
     if (threadIdx.x == 0) {
         cs.phase = 0;

@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(kLuMaxPanelThreads) lu_panel_kernel(float* A, 
     __shared__ alignas(16) float cand[2][kWarps][NB];  // each warp's best row, double-buffered over columns
     __shared__ unsigned ckey[2][kWarps], cpos[2][kWarps];
     __shared__ float prow[NB][NB + 1];                 // the chosen rows from their diagonal element on
-    extern __shared__ float mult[];                    // [NB][R * blockDim.x] multipliers of each row
+    extern __shared__ __align__(16) float mult[];      // [NB][R * blockDim.x] multipliers of each row
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = blockDim.x >> 5;
     const int m = n - k0, w = min(NB, m);
     float a[R][NB];
@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(kLuThreads) lu_solve_kernel(const float* A, in
     __shared__ float D[kSolveNB][kSolveNB];  // [column][row]
     __shared__ float xb[kSolveNB];
     __shared__ int p[2][kSolveNB];
-    extern __shared__ float xs[];
+    extern __shared__ __align__(16) float xs[];
     if (*info) return;
     float* x = in_smem ? xs : xg;
     const int t = threadIdx.x, lane = t & 31, r = t & 31, c = t >> 5;  // 32 x 32 threads over a block

@@ -273,7 +273,7 @@ template <class TT, class WT, bool kPoints, bool kMesh>
 __global__ void __launch_bounds__(32 * kSweepWarps) mc_sweep_kernel(const TT* __restrict__ tsdf,
                                                                     const WT* __restrict__ weights, McArgs a) {
     __shared__ unsigned queue[kSweepWarps][64];
-    extern __shared__ unsigned char sweep_raw[];
+    extern __shared__ __align__(16) unsigned char sweep_raw[];
     McScratch<kMesh>* scratch = reinterpret_cast<McScratch<kMesh>*>(sweep_raw);  // one per warp
     constexpr int R = kSweepY + 1;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1141,7 +1141,7 @@ __global__ void bucket_count_kernel(const float* __restrict__ pts, const unsigne
 // hundred sums cost more); the first one leaves them for the launches after this.
 __global__ void __launch_bounds__(256) bucket_scatter_kernel(const float* __restrict__ pts, const unsigned* count, long n_max,
                                                              BucketArgs a, BucketWs ws, Key3* keys, int* error) {
-    extern __shared__ unsigned s_off[];
+    extern __shared__ __align__(16) unsigned s_off[];
     __shared__ unsigned s_sum[8];
     const long n = min((long)*count, n_max);
     if ((long)blockIdx.x * blockDim.x >= n && blockIdx.x != 0) return;
@@ -1254,7 +1254,7 @@ AFX_D void cta_merge(const Key3* A, unsigned la, const Key3* B, unsigned lb, Key
 __global__ void __launch_bounds__(kBucketThreads) bucket_sort_kernel(Key3* keys, Key3* scratch, const unsigned* off,
                                                                    unsigned* ucnt, long n_max,
                                                                    int* error) {
-    extern __shared__ Key3 sk[];
+    extern __shared__ __align__(16) Key3 sk[];
     __shared__ unsigned wsum[kBucketThreads / 32];
     const int b = blockIdx.x;
     const unsigned lo = off[b], n = off[b + 1] - lo;
