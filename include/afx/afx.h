@@ -310,8 +310,15 @@ int afx_gn_export(afx_gn* g, int n_nodes_host, float* jtj, float* jtr, float* r_
 
 /* x = (J^T J)^-1 J^T r by block-Jacobi preconditioned conjugate gradients: `iterations` steps, or
  * until |r| <= tol |b| when tol > 0 (replaces linearSolverLUStable, src/LinearSolver.cu:179-224).
- * x: 6 * n_nodes_max floats, device. */
+ * x: 6 * n_nodes_max floats, device.  Asynchronous: the solver's thread blocks exchange sums and wait for them a
+ * bounded time; where such a wait ran out, parts of x are not a number and afx_gn_status says so. */
 int afx_gn_solve(afx_gn* g, float* x, int iterations, double tol, void* stream);
+
+/* Waits for `stream`; AFX_ERR_TIMEOUT when a wait of a solve since the last call ran out (x holds no solution). */
+int afx_gn_status(afx_gn* g, void* stream);
+
+/* Polls of one wait of a solve before it gives up (2^20 by default).  No counterpart in the reference. */
+int afx_gn_set_wait_limit(afx_gn* g, int polls);
 
 /* runUpdateTransformsKernel (src/MotionOptimization.cu:483-506): T -= [[x_rot]x, x_t; 0]. */
 int afx_update_transforms(float* transforms, const float* x, const int* n_nodes, int n_nodes_max, void* stream);

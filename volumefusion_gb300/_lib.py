@@ -99,6 +99,8 @@ SIGNATURES = {
     "afx_gn_build": (i32, [vp] + [vp] * 13 + [f32, f32, vp]),
     "afx_gn_export": (i32, [vp, i32, vp, vp, vp, vp, vp]),
     "afx_gn_solve": (i32, [vp, vp, i32, C.c_double, vp]),
+    "afx_gn_status": (i32, [vp, vp]),
+    "afx_gn_set_wait_limit": (i32, [vp, i32]),
     "afx_update_transforms": (i32, [vp, vp, vp, i32, vp]),
     "afx_fusion_set_graphs": (i32, [vp, i32]),
     "afx_fusion_graph_count": (i32, [vp]),

@@ -295,7 +295,8 @@ class GaussNewtonSystem:
 
     def solve(self, iterations=10, tol=0.0):
         x = torch.zeros(6 * self.n_nodes_max, dtype=torch.float32, device="cuda")
-        _sync(lib().afx_gn_solve(self.h, _p(x), int(iterations), float(tol), _stream()), "afx_gn_solve")
+        check(lib().afx_gn_solve(self.h, _p(x), int(iterations), float(tol), _stream()), "afx_gn_solve")
+        check(lib().afx_gn_status(self.h, _stream()), "afx_gn_solve")
         return x
 
 

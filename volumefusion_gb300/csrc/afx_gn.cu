@@ -875,6 +875,7 @@ struct ClusterSums {
     double total[4];
     double in[2][kClusterMax][2];  // every CTA's sums (cluster_sum_tf)
     int phase;
+    int dead;  // a wait of some CTA ran out (gn_solve)
 };
 
 // Double-floats in this CTA's shared memory and in CTA `rank`'s (8-byte slots, hi first).
@@ -967,7 +968,9 @@ struct LoopArgs {
     float* T_committed;
     float* T_pending;
     int gn_iters, pcg_iters;
-    double tol;  // <= 0: run exactly pcg_iters PCG iterations
+    double tol;      // <= 0: run exactly pcg_iters PCG iterations
+    int wait_polls;  // polls of an exchange between CTAs before it gives up
+    int* gave_up;    // set when one does (memory the host reads), or null
 };
 
 // J^T r of one node, one warp: lane l sums the node-list entries l, l+32, ... (depth rows, J
@@ -1155,6 +1158,11 @@ AFX_D void dsmem_store_f64(double* local, unsigned rank, double v) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
     asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(ra), "d"(v) : "memory");
 }
+AFX_D void dsmem_store_int(int* local, unsigned rank, int v) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(local), ra;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
+    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(ra), "r"(v) : "memory");
+}
 // Asynchronous stores to the same shared-memory offset in CTA `rank` of this cluster, counted on that
 // CTA's mbarrier: the receiver waits for the bytes it expects, so an exchange costs one trip
 // through the cluster's network instead of a store, its acknowledgement and a cluster barrier
@@ -1173,10 +1181,18 @@ AFX_D void async_store_df(unsigned addr, unsigned bar, DF v) {
 // The two exchanges of a PCG iteration.  Phases alternate: a CTA sends its part of an exchange only
 // after it has received the other one of the step before from every CTA, that is after every CTA has
 // read what this one overwrites.
+//
+// Waits are bounded.  A CTA one of whose waits runs out flags the error and leaves the solve at its next barrier,
+// with no further sends; it then waits, again bounded, for what the others may have sent it until they
+// run out too (ds_drain), so that no store is under way to a CTA that has left.  The others learn of it at the end of
+// the solve (gn_solve), and nobody sends any more in that launch.
 struct DsExchange {
     unsigned parity[2];  // phase of each mbarrier that the next wait is for
-    bool dead;           // a wait ran out (the error is flagged): no further sends or waits
+    bool dead;           // a wait ran out (this thread's within a solve, any CTA's after it)
 };
+
+constexpr int kDsWaitPolls = 1 << 20;
+constexpr int kDsDrainPolls = 1 << 12;
 
 // Before the cluster barrier at the start of the kernel (one thread).
 AFX_D void ds_exchange_init(const DsLayout& d) {
@@ -1191,20 +1207,35 @@ AFX_D void ds_expect(const DsLayout& d, int i, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 
-// Wait (bounded) for the current phase of mbarrier i; every thread, the same number of times.
-AFX_D void ds_wait(const DsLayout& d, int i, DsExchange& x, int* error) {
+// Whether the phase `parity` of mbarrier i ends within `polls` polls.
+AFX_D bool ds_poll(const DsLayout& d, int i, unsigned parity, int polls) {
     const unsigned bar = (unsigned)__cvta_generic_to_shared(d.bar + i);
     unsigned ok = 0;
-    for (int it = 0; it < (1 << 20) && !ok; ++it)
+    for (int it = 0; it < polls && !ok; ++it)
         asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
                      : "=r"(ok)
-                     : "r"(bar), "r"(x.parity[i])
+                     : "r"(bar), "r"(parity)
                      : "memory");
-    x.parity[i] ^= 1u;
-    if (!ok) {
+    return ok != 0;
+}
+
+// Wait (bounded) for the current phase of mbarrier i.
+AFX_D void ds_wait(const DsLayout& d, int i, DsExchange& x, const LoopArgs& L) {
+    if (ds_poll(d, i, x.parity[i], L.wait_polls)) {
+        x.parity[i] ^= 1u;
+    } else {
         x.dead = true;
-        if (error) atomicOr(error, ERRF_TIMEOUT);
+        if (L.g.error) atomicOr(L.g.error, ERRF_TIMEOUT);
     }
+}
+
+// After a wait ran out (one thread, which has made every wait): what the other CTAs have sent or may still send before
+// their own waits run out, that is at most the exchange that was waited for and the one after it.  `armed`: the
+// mbarriers whose bytes are expected already.
+AFX_D void ds_drain(const DsLayout& d, const DsExchange& x, unsigned armed, const unsigned (&bytes)[2]) {
+    for (int i = 0; i < 2; ++i)
+        if (!((armed >> i) & 1u)) ds_expect(d, i, bytes[i]);
+    for (int i = 0; i < 2; ++i) ds_poll(d, i, x.parity[i], kDsDrainPolls);
 }
 
 // Cluster sum through the slot arrays: the CTA's block total is written into slot[ph][rank] of
@@ -1398,8 +1429,7 @@ AFX_D void pcg_ds(const LoopArgs& L, int n, const DsLayout& d, DsExchange& ex) {
             d.r[o] = rv;
             zown[o] = zi;
         }
-        if (__syncthreads_or(stop)) return false;
-        if (ex.dead) return true;
+        if (__syncthreads_or(stop || ex.dead)) return false;
         if (w == 0) {
             if constexpr (kTol) ds_dot_send<2>({d.r, d.r}, {zown, d.r}, cnt, d, 1);
             else ds_dot_send<1>({d.r}, {zown}, cnt, d, 1);
@@ -1419,13 +1449,14 @@ AFX_D void pcg_ds(const LoopArgs& L, int n, const DsLayout& d, DsExchange& ex) {
     float x = 0.f, rv = act ? __ldcg(b.jtr + (long)(start + li) * 6 + ei) : 0.f;
     if (threadIdx.x == 0) ds_expect(d, 1, rz_bytes);
     precondition(rv, false);
-    if (!ex.dead) ds_wait(d, 1, ex, L.g.error);
+    ds_wait(d, 1, ex, L);
     DF t[NV];
     ds_dot_total<NV>(d, 1, t);
     DF rz = t[0];
     const bool mine = w * 5 < own;  // the warp has entries
     const float tol2 = kTol ? (float)(L.tol * L.tol) : 0.f, bn = t[NV - 1].hi;
     float beta = 0.f;
+    int armed = -1;
     for (int it = 0; it < L.pcg_iters; ++it) {
         // p = z (first iteration) or z + beta p, formed for all nodes by every CTA from its copies
 #pragma unroll 2
@@ -1439,7 +1470,7 @@ AFX_D void pcg_ds(const LoopArgs& L, int n, const DsLayout& d, DsExchange& ex) {
                 *pv = zv;
             }
         }
-        __syncthreads();
+        if (__syncthreads_or(ex.dead)) break;  // the wait for r.z ran out
         // A p of the own rows
         float acc = 0.f, prod[kRegBlocks];
 #pragma unroll
@@ -1456,13 +1487,13 @@ AFX_D void pcg_ds(const LoopArgs& L, int n, const DsLayout& d, DsExchange& ex) {
         if (row < cnt && part == 0) d.ap[row] = acc;
         if (threadIdx.x == 0) ds_expect(d, 0, dot_bytes);
         __syncthreads();
-        if (w == 0 && !ex.dead) ds_dot_send<1>({pown}, {d.ap}, cnt, d, 0);
+        if (w == 0) ds_dot_send<1>({pown}, {d.ap}, cnt, d, 0);
         const float pv = act ? pown[o] : 0.f, apv = act ? d.ap[o] : 0.f;
         // the totals and step sizes: alpha by the warps that have entries, beta by one warp (all warps
         // forming them costs more, by their instructions, than handing beta round)
         bool stop = false;
         if (mine || w == 0) {
-            if (!ex.dead) ds_wait(d, 0, ex, L.g.error);
+            ds_wait(d, 0, ex, L);
             DF pap[1];
             ds_dot_total<1>(d, 0, pap);
             stop = df_zero_or_nan(pap[0]);  // the same in every CTA
@@ -1472,10 +1503,13 @@ AFX_D void pcg_ds(const LoopArgs& L, int n, const DsLayout& d, DsExchange& ex) {
         } else {
             ex.parity[0] ^= 1u;
         }
-        if (threadIdx.x == 0 && !stop) ds_expect(d, 1, rz_bytes);
+        if (threadIdx.x == 0 && !stop && !ex.dead) ds_expect(d, 1, rz_bytes);
         // every CTA has read z (forming p) before it sent its part of p.Ap, so it can be overwritten here
-        if (!precondition(rv, stop)) break;
-        if (!ex.dead) ds_wait(d, 1, ex, L.g.error);
+        if (!precondition(rv, stop)) {  // no direction left, or the wait for p.Ap ran out
+            armed = ex.dead ? 1 : (stop ? 0 : 2);
+            break;
+        }
+        ds_wait(d, 1, ex, L);
         if (mine || w == 0) {
             ds_dot_total<NV>(d, 1, t);
             if (threadIdx.x == 0) {
@@ -1490,8 +1524,23 @@ AFX_D void pcg_ds(const LoopArgs& L, int n, const DsLayout& d, DsExchange& ex) {
     }
     if (act) d.x[o] = x;
     // T_pending -= [[x_rot]x, x_t; 0] for the own nodes (updateTransformsKernel,
-    // src/MotionOptimization.cu:483-498); x also to global memory for inspection
-    __syncthreads();
+    // src/MotionOptimization.cu:483-498); x also to global memory for inspection.  After a wait that ran out there is
+    // no x: the transforms stay.
+    const bool mine_dead = ex.dead;
+    ex.dead = __syncthreads_or(mine_dead);
+    if (ex.dead) {
+        if (threadIdx.x == 0) {
+            if (armed < 0) armed = mine_dead ? 2 : 0;  // left at the wait for r.z
+            const unsigned bytes[2] = {dot_bytes, rz_bytes};
+            ds_drain(d, ex, (unsigned)armed, bytes);
+            if (L.gave_up) {
+                *(volatile int*)L.gave_up = 1;
+                __threadfence_system();
+            }
+        }
+        for (int t = threadIdx.x; t < own * 6; t += blockDim.x) __stcg(b.x + (long)start * 6 + t, NAN);
+        return;
+    }
     for (int t = threadIdx.x; L.T_pending && t < own * 16; t += blockDim.x) {
         const int l = t >> 4, e = t & 15;
         const float* u = d.x + l * 6;
@@ -2129,13 +2178,17 @@ AFX_D void gn_rewarp(const GnArgs& a, const float* points, float* warped, const 
 }
 
 // One solve from b.jtr: x in b.x (and in the own slices of the shared-memory layout); with
-// L.T_pending set, T_pending -= [x] as well.  Ends with a cluster barrier.
+// L.T_pending set, T_pending -= [x] as well.  Ends with a cluster barrier, after which every CTA knows whether a
+// wait ran out.
 // `first`: the first solve of the launch.
 AFX_D void gn_solve(const LoopArgs& L, int n, bool ds, const DsLayout& dsl, ClusterSums& cs, DsExchange& ex, long gt,
                     long gstride, bool first) {
     if (ds) {
-        if (L.tol > 0) pcg_ds<true>(L, n, dsl, ex);
-        else pcg_ds<false>(L, n, dsl, ex);
+        if (!ex.dead) {
+            if (L.tol > 0) pcg_ds<true>(L, n, dsl, ex);
+            else pcg_ds<false>(L, n, dsl, ex);
+        }
+        if (ex.dead && threadIdx.x < cluster_size()) dsmem_store_int(&cs.dead, threadIdx.x, 1);
     } else {
         if (!wide_fits(n, (int)cluster_size())) pcg_global(L, n, cs);
         else if (L.tol > 0) pcg_wide<true>(L, n, dsl.z, cs, first);
@@ -2144,6 +2197,7 @@ AFX_D void gn_solve(const LoopArgs& L, int n, bool ds, const DsLayout& dsl, Clus
         if (L.T_pending) update_transforms_range(L.T_pending, L.g.b.x, 0, n, gt, gstride);
     }
     cluster_barrier();
+    if (ds) ex.dead = cs.dead != 0;
 }
 
 __global__ void __launch_bounds__(kLoopThreads, 1) gn_loop_kernel(LoopArgs L) {
@@ -2154,6 +2208,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) gn_loop_kernel(LoopArgs L) {
     const DsLayout dsl = ds_layout(ds_smem);
     if (threadIdx.x == 0) {
         cs.phase = 0;
+        cs.dead = 0;
         ds_exchange_init(dsl);
     }
     // Every CTA of the cluster must be running before any thread touches another CTA's shared
@@ -2229,6 +2284,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) gn_solve_kernel(LoopArgs L) {
     const DsLayout dsl = ds_layout(ds_smem);
     if (threadIdx.x == 0) {
         cs.phase = 0;
+        cs.dead = 0;
         ds_exchange_init(dsl);
     }
     cluster_barrier();  // every CTA running before any access to another CTA's shared memory
@@ -2419,6 +2475,8 @@ int gn_loop(const GnArgs& a, const float* points, float* warped, float* T_commit
     L.gn_iters = gn_iters;
     L.pcg_iters = pcg_iters;
     L.tol = tol;
+    L.wait_polls = kDsWaitPolls;
+    L.gave_up = nullptr;
     return launch_cluster(gn_loop_kernel, L, st);
 }
 
@@ -2519,6 +2577,8 @@ struct afx_gn {
     int* cov;
     int* error;
     unsigned* counts;  // copies of the caller's counters at build time: points, correspondences, nodes
+    int* gave_up;      // pinned: set by a solve one of whose waits ran out, until afx_gn_status reports it
+    int wait_polls;
     afx::GnArgs last;
     bool built;
 };
@@ -2543,11 +2603,20 @@ int afx_gn_create(long n_points_max, int n_nodes_max, int k, int kreg, afx_gn** 
         delete g;
         return AFX_ERR_NO_MEMORY;
     }
+    if (cudaHostAlloc(reinterpret_cast<void**>(&g->gave_up), sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(g->arena);
+        delete g;
+        return AFX_ERR_NO_MEMORY;
+    }
+    *g->gave_up = 0;
+    g->wait_polls = kDsWaitPolls;
     gn_carve(g->arena, ws, n_points_max, n_nodes_max, k, kreg, &g->b);
     g->cov = reinterpret_cast<int*>(static_cast<char*>(g->arena) + ws);
     g->error = reinterpret_cast<int*>(static_cast<char*>(g->arena) + ws + al((size_t)n_points_max * 4));
     g->counts = reinterpret_cast<unsigned*>(static_cast<char*>(g->arena) + ws + al((size_t)n_points_max * 4) + 256);
     if (cudaMemset(g->error, 0, 4) != cudaSuccess) {
+        cudaFreeHost(g->gave_up);
         cudaFree(g->arena);
         delete g;
         return note_cuda_error(cudaGetLastError());
@@ -2560,9 +2629,25 @@ int afx_gn_create(long n_points_max, int n_nodes_max, int k, int kreg, afx_gn** 
 int afx_gn_destroy(afx_gn* g) {
     if (!g) return AFX_ERR_INVALID_ARGUMENT;
     cudaDeviceSynchronize();
+    cudaFreeHost(g->gave_up);
     cudaError_t e = cudaFree(g->arena);
     delete g;
     return note_cuda_error(e);
+}
+
+int afx_gn_set_wait_limit(afx_gn* g, int polls) {
+    if (!g || polls < 0) return AFX_ERR_INVALID_ARGUMENT;
+    g->wait_polls = polls;
+    return AFX_OK;
+}
+
+int afx_gn_status(afx_gn* g, void* stream) {
+    if (!g) return AFX_ERR_INVALID_ARGUMENT;
+    AFX_CUDA(cudaStreamSynchronize(as_stream(stream)));
+    volatile int* w = g->gave_up;
+    if (!*w) return AFX_OK;
+    *w = 0;
+    return AFX_ERR_TIMEOUT;
 }
 
 int afx_gn_build(afx_gn* g, const float* canonical, const unsigned* n_points, const uint32_t* knn_idx,
@@ -2651,6 +2736,8 @@ int afx_gn_solve(afx_gn* g, float* x, int iterations, double tol, void* stream) 
     L.g = g->last;
     L.pcg_iters = iterations;
     L.tol = tol;
+    L.wait_polls = g->wait_polls;
+    L.gave_up = g->gave_up;
     int rc = launch_cluster(gn_solve_kernel, L, st);
     if (rc) return rc;
     AFX_CUDA(cudaMemcpyAsync(x, g->b.x, (size_t)g->n_max * 6 * 4, cudaMemcpyDeviceToDevice, st));
