@@ -497,6 +497,10 @@ int afx_fusion_set_graphs(afx_fusion* f, int on);
 /* Number of frame graphs captured so far (0 while graphs are off or capture fell back). */
 int afx_fusion_graph_count(const afx_fusion* f);
 
+/* A session numbers its frames to tell a frame's collision counts from earlier ones, and clears the counts before a
+ * frame whose number would pass this limit (2^20 by default, below 2^24).  No counterpart in the reference. */
+int afx_fusion_set_epoch_limit(afx_fusion* f, long frames);
+
 /* Marching-cubes tile of the session (no counterpart in the reference): AFX_MC_TILE_TMA16 (default:
  * a CTA's brick of 32x8x16 cubes brought into shared memory by TMA), AFX_MC_TILE_TMA8,
  * AFX_MC_TILE_TMA32 (8 or 32 cubes along z), AFX_MC_TILE_COLUMN (sweep from global memory),

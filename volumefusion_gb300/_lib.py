@@ -104,6 +104,7 @@ SIGNATURES = {
     "afx_update_transforms": (i32, [vp, vp, vp, i32, vp]),
     "afx_fusion_set_graphs": (i32, [vp, i32]),
     "afx_fusion_graph_count": (i32, [vp]),
+    "afx_fusion_set_epoch_limit": (i32, [vp, i64]),
     "afx_fusion_set_tile": (i32, [vp, i32]),
     "afx_fusion_get_tile": (i32, [vp]),
     "afx_fusion_autotune": (i32, [vp, C.POINTER(i32), C.POINTER(C.c_float), vp]),

@@ -117,7 +117,8 @@ struct WorkMarks {
 
 using namespace afx;
 
-constexpr long kEpochsPerClear = 1L << 20;  // of 2^24 epochs
+constexpr long kEpochs = 1L << 24;             // that a collision word can name
+constexpr long kEpochsPerClear = 1L << 20;
 
 struct afx_fusion {
     afx_fusion_params p;
@@ -212,7 +213,8 @@ struct afx_fusion {
     cudaEvent_t ev_in_ready[2] = {nullptr, nullptr}, ev_in_free[2] = {nullptr, nullptr};
     cudaGraphExec_t gexec[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
     cudaGraph_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // kept for batch graphs
-    long epochs_used = 0;      // frames since the collision words were cleared, as of the last reset
+    long epochs = 0;           // frames begun since the collision words were cleared
+    long epoch_limit = kEpochsPerClear;
     unsigned graph_epoch = 0;  // advanced whenever the captured graphs are dropped
     int mc_tile = kMcTileTma16;  // marching-cubes tile (by size at creation; afx_fusion_autotune)
     long glaunches[2][2] = {{0, 0}, {0, 0}};  // kernels in each captured frame
@@ -239,9 +241,7 @@ __global__ void frame_begin_kernel(unsigned* epoch, unsigned* ncorr, unsigned* n
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     *next_points = 0;
     *n_old = *n_nodes;
-    unsigned e = *epoch + 1;
-    if (e >= (1u << 24)) e = 1;  // collision words are cleared by the host when this wraps
-    *epoch = e;
+    *epoch = *epoch + 1;  // (next_epoch sees to it that this stays below kEpochs)
     *ncorr = 0;
     *nmverts = 0;
     *nmfaces = 0;
@@ -621,14 +621,7 @@ int afx_fusion_reset(afx_fusion* f, void* stream) {
                                                                                                 tsdf_bytes, word);
     AFX_LAUNCH_CHECK();
     AFX_CUDA(cudaMemsetAsync(f->weights, 0, f->S * vox_bytes(f->fmt), st));
-    // Collision words are read by their epoch, which goes on over sequences: words of an earlier one count as empty.
-    // They are cleared, and the epoch with them, long before it comes round.
-    f->epochs_used += f->frame;
-    if (f->epochs_used >= kEpochsPerClear) {
-        AFX_CUDA(cudaMemsetAsync(f->coll, 0, f->S * 4, st));
-        AFX_CUDA(cudaMemsetAsync(f->epoch, 0, 64, st));
-        f->epochs_used = 0;
-    }
+    // (the collision words stay: those of earlier frames count as empty, next_epoch)
     AFX_CUDA(cudaMemsetAsync(f->occ, 0, brick_count_total(f->vol), st));
     AFX_CUDA(cudaMemsetAsync(f->centroid0, 0, 64, st));
     AFX_CUDA(cudaMemsetAsync(f->acc, 0, 64, st));
@@ -903,9 +896,30 @@ static int capture_frame(afx_fusion* f, int cur, bool build) {
     return AFX_OK;
 }
 
+// Collision words are read by their epoch, a number per frame that goes on over sequences: words of earlier frames count
+// as empty.  Before a frame whose number would not fit, wherever in a sequence it is, the words are cleared and
+// the numbers start again.
+static int next_epoch(afx_fusion* f, cudaStream_t st) {
+    if (f->epochs >= f->epoch_limit) {
+        AFX_CUDA(cudaMemsetAsync(f->coll, 0, f->S * 4, st));
+        AFX_CUDA(cudaMemsetAsync(f->epoch, 0, 64, st));
+        f->epochs = 0;
+    }
+    ++f->epochs;
+    return AFX_OK;
+}
+
+int afx_fusion_set_epoch_limit(afx_fusion* f, long frames) {
+    if (!f || frames < 1 || frames >= kEpochs) return AFX_ERR_INVALID_ARGUMENT;
+    f->epoch_limit = frames;
+    return AFX_OK;
+}
+
 int afx_fusion_process(afx_fusion* f, const uint16_t* depth_mm, void* stream) {
     if (!f || !depth_mm) return AFX_ERR_INVALID_ARGUMENT;
     cudaStream_t st = as_stream(stream);
+    const int erc = next_epoch(f, st);
+    if (erc) return erc;
     if (f->frame == 0) {
         const int rc = enqueue_frame(f, depth_mm, st, f->cur, false);
         if (rc) return rc;
@@ -1390,6 +1404,10 @@ int afx_batch_process(afx_batch* b, const uint16_t* const* depth_mm, void* strea
                 cudaMemcpyDefault);
             if (e != cudaSuccess) return batch_fail("frame copy update", e);
         }
+    }
+    for (int i : members) {
+        const int rc = next_epoch(b->s[i], st);
+        if (rc) return rc;
     }
     const cudaError_t le = cudaGraphLaunch(it->second.exec, st);
     if (le != cudaSuccess) return batch_fail("launch", le);
