@@ -727,9 +727,9 @@ int build_graph_impl(float* nodes, float* radii, float* T, int* n_nodes, int cap
 //   many queries: a thread per query with its best KK in registers.  Every CTA sorts the nodes by x into shared
 //   memory (bins: about 3 us), and a warp goes outwards from the x range of its 32 queries until the
 //   gap exceeds every lane's KK-th distance.  Point clouds come sorted by x, so that range is narrow;
-//   few nodes, a shape whose windows would be wide, or warps whose queries are in no order: all nodes in
-//   index order, from shared memory;
-//   more nodes than fit there, or coordinates that are not finite: tile by tile.
+//   few nodes, a shape whose windows would be wide, coordinates that are not finite, or warps whose queries are in no
+//   order: all nodes in index order, from shared memory;
+//   more nodes than fit there: the same, as many at a time as fit.
 // Bound: instructions, about 15 per distance and 25 per insertion, and below some thousand queries the latency of
 // building and of one query.  In the 512^3 sequence (1,300 nodes): 330,000 points, K = 4, 83 -> 16 us; the nodes
 // among themselves, K = 8, 99 -> 8 us; in the 256^3 sequence (170 nodes) 10.2 -> 8.3 and 15.4 -> 4.2 us (before:
@@ -737,10 +737,11 @@ int build_graph_impl(float* nodes, float* radii, float* T, int* n_nodes, int cap
 // kKnnFewQueries: a warp per query takes 8.4, 12.7 and 31 us for 2,000 queries and 170, 1,300 and 5,000 nodes of
 // a sphere, all nodes by a thread 12.7, 56 and 189; 10, 25 and 75 us for 8,000 (12.6, 56, 188, and a window 15, 35, 60),
 // 31, 101 and 328 us for 40,000 (14.6, 66, 216, and a window 17, 36, 62).
+// More nodes than fit, 20,000 and K = 4: 570 us for 20,000 queries, 780 for 60,000 and 2.57 ms for 300,000 (the queries in
+// CTAs of 128, or of 1024 one after the other, and 1,024 nodes at a time: 770, 910 and 2.97 ms, and 1.28, 1.28 and 2.54 ms).
 // kKnnWindowShare: 300 nodes, K = 4: on a sphere (0.39 by the estimate) a window takes 21 us for 16,000 queries and all
 // nodes 17; on a tube along x (0.15) 13 and 17.
 
-constexpr int kKnnTile = 1024;
 constexpr int kKnnThreads = 1024;
 constexpr int kKnnWarps = kKnnThreads / 32;
 constexpr long kKnnFewQueries = 8192;
@@ -883,8 +884,7 @@ AFX_D float knn_unkey(unsigned k) { return __uint_as_float(k & 0x80000000u ? k &
 // may lie before another one further on by, or a negative value where nothing was sorted: a coordinate is not finite,
 // or a window would not be much narrower than all nodes.
 template <int KK>
-AFX_D float knn_sort_x(const float* __restrict__ nodes, int n, float4* list, unsigned* bins, float& x0, float& scale,
-                       bool& finite) {
+AFX_D float knn_sort_x(const float* __restrict__ nodes, int n, float4* list, unsigned* bins, float& x0, float& scale) {
     __shared__ unsigned s_min[3], s_max[3], s_bad, s_sum[kKnnWarps];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     if (tid < 3) {
@@ -919,8 +919,7 @@ AFX_D float knn_sort_x(const float* __restrict__ nodes, int n, float4* list, uns
     const float ext = knn_unkey(s_max[0]) - x0, ey = knn_unkey(s_max[1]) - knn_unkey(s_min[1]),
                 ez = knn_unkey(s_max[2]) - knn_unkey(s_min[2]);
     scale = ext > 0.f ? (kKnnBins - 0.5f) / ext : 0.f;
-    finite = !s_bad && isfinite(ext) && isfinite(scale);  // the same in every thread, as what follows
-    if (!finite) return -1.f;
+    if (s_bad || !isfinite(ext) || !isfinite(scale)) return -1.f;  // the same in every thread, as what follows
     // The distance of the KK-th node, if they lie evenly on a surface of half the bounding box's: a window is about
     // three of it wide (the farthest of 32 queries sets it).
     const float reach = sqrtf(0.41f * KK * (ext * ey + ey * ez + ext * ez) / (float)n);
@@ -1041,9 +1040,9 @@ __global__ void __launch_bounds__(kKnnThreads, 1) knn_kernel(uint32_t* idx, floa
     }
     unsigned* const bins = reinterpret_cast<unsigned*>(knn_smem);
     float x0 = 0.f, scale = 0.f;
-    bool scan = n <= kKnnScanNodes, finite = true;
-    const float slack = !scan && n <= kKnnMaxNodes ? knn_sort_x<KK>(nodes, n, list, bins, x0, scale, finite) : -1.f;
-    scan = scan || (n <= kKnnMaxNodes && finite && slack < 0.f);
+    bool scan = n <= kKnnScanNodes;
+    const float slack = !scan && n <= kKnnMaxNodes ? knn_sort_x<KK>(nodes, n, list, bins, x0, scale) : -1.f;
+    scan = scan || (n <= kKnnMaxNodes && slack < 0.f);
     if (scan || slack >= 0.f) {
         // in index order: the scan's nodes, or those of warps that leave the window (beside the sorted ones if there is room)
         float* const copy = reinterpret_cast<float*>(list + n);
@@ -1083,23 +1082,32 @@ __global__ void __launch_bounds__(kKnnThreads, 1) knn_kernel(uint32_t* idx, floa
         }
         return;
     }
-    __syncthreads();
-    float* s_n = reinterpret_cast<float*>(knn_smem);
-    for (long blk = blockIdx.x; blk * kKnnThreads < m; blk += gridDim.x) {
-        const long i = blk * kKnnThreads + threadIdx.x;
+    // (the queries dealt to warps as above; every warp of a CTA loads nodes for those that have some)
+    for (long t0 = blockIdx.x; t0 * 32 < m; t0 += step) {
+        const long i = (t0 + (long)w * gridDim.x) * 32 + lane;
+        const bool any = i - lane < m;
         float q[3] = {0.f, 0.f, 0.f};
         if (i < m)
 #pragma unroll
             for (int c = 0; c < 3; ++c) q[c] = pts[3 * i + c];
         KnnList<KK> best;
         best.clear();
-        for (int base = 0; base < n; base += kKnnTile) {
-            const int nt = min(kKnnTile, n - base);
+        for (int base = 0; base < n; base += kKnnMaxNodes) {
+            const int nt = min(kKnnMaxNodes, n - base);
             __syncthreads();
-            for (int t = threadIdx.x; t < nt * 3; t += kKnnThreads) s_n[t] = nodes[3 * (long)base + t];
+            for (int j = threadIdx.x; j < nt; j += kKnnThreads) {
+                const float* p = nodes + 3 * ((long)base + j);
+                list[j] = make_float4(p[0], p[1], p[2], 0.f);
+            }
             __syncthreads();
-            if (i < m)
-                for (int j = 0; j < nt; ++j) best.offer_next(l2sq_nanoflann(q, s_n + 3 * j), base + j);
+            if (any) {
+#pragma unroll 8
+                for (int j = 0; j < nt; ++j) {
+                    const float4 v = list[j];
+                    const float p[3] = {v.x, v.y, v.z};
+                    best.offer_next(l2sq_nanoflann(q, p), base + j);
+                }
+            }
         }
         if (i < m) best.store(idx, dist, i, k, excl);
     }
