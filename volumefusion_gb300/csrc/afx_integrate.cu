@@ -33,7 +33,7 @@ Volume make_volume(const int dims[3], const float voxel_size[3], const float vol
 // ------------------------------------------------------------------------------------
 // Rigid integration (integrateTSDFFromFrameKernel, src/TSDFIntegration.cu:69-96)
 //
-// The volume is taken in blocks of 32 x 16 x 16 voxels.  The pixels that a block projects to are bounded
+// The volume is taken in blocks of 32 x 16 x 16 voxels (thinner ones in smaller volumes).  The pixels that a block projects to are bounded
 // by its eight corner voxels (the projection of a box in front of the camera lies within theirs) and
 // compared by the largest depth among them: a block that lies outside the image, sees no valid depth,
 // or lies more than the truncation distance behind every one of them has no voxel to update, and most
@@ -68,8 +68,16 @@ AFX_D void mark_brick(unsigned char* occ, int nbx, int nby, int x, int y, int z)
     if (occ) occ[((long)(z >> 3) * nby + (y >> 3)) * nbx + (x >> 3)] = 1;
 }
 
-constexpr int kBlkX = 32, kBlkY = 16, kBlkZ = 16;  // whole 8^3 bricks
+// Blocks of kBlkZ slices.  Below kMidVoxels half as deep, since there are few for the SMs (256^3: an object 29 -> 27.5 us,
+// every voxel updated 70 -> 68; rows of 255 voxels 84 -> 75; at 320^3 the looking costs more than that saves, an
+// object 37 -> 41.5).  Below kThinVoxels a quarter as deep and without looking, for which there is little to leave
+// out (an object and every voxel updated, from kBlkZ slices to these: 64^3 21 -> 11 us both, 128^3 21 -> 11 and 23 -> 13,
+// 192^3 23 -> 21 and 31 -> 29; at 256^3 29 -> 42 and 70 -> 62).
+constexpr int kBlkX = 32, kBlkY = 16, kBlkZ = 16, kMidZ = 8, kThinZ = 4;  // whole 8^3 bricks, but for kThinZ
+constexpr long kThinVoxels = 10000000, kMidVoxels = 20000000;
 constexpr int kBlkThreads = 256;
+// CTAs per SM that the registers of each form are held to.
+__host__ __device__ constexpr int blk_ctas(bool vec, int depth) { return depth == kBlkZ ? 5 : depth == kThinZ && !vec ? 8 : 6; }
 constexpr int kBlkPixels = 4096;        // a block that spans more pixels is evaluated without looking at them
 
 AFX_D void rigid_point(const RigidArgs& a, float t0, float t1, float t2, int x, int y, int z, float* q) {
@@ -95,12 +103,13 @@ struct BoxView {
     float behind;  // a box whose pixels' largest valid depth is below this has nothing to update
 };
 
+template <int kZ>
 AFX_D BoxView box_view(const RigidArgs& a, float t0, float t1, float t2, int x0, int y0, int z0) {
     const int lane = threadIdx.x & 31;
     const int* D = a.vol.dims;
     float q[3];
     rigid_point(a, t0, t1, t2, (lane & 1) ? min(x0 + kBlkX, D[0]) - 1 : x0, (lane & 2) ? min(y0 + kBlkY, D[1]) - 1 : y0,
-                (lane & 4) ? min(z0 + kBlkZ, D[2]) - 1 : z0, q);
+                (lane & 4) ? min(z0 + kZ, D[2]) - 1 : z0, q);
     const float zmin = warp_min8(q[2]), zmax = -warp_min8(-q[2]);
     const float u = a.K.fx * q[0] / q[2] + a.K.cx, v = a.K.fy * q[1] / q[2] + a.K.cy;
     const float umin = warp_min8(u), umax = -warp_min8(-u), vmin = warp_min8(v), vmax = -warp_min8(-v);
@@ -152,8 +161,8 @@ AFX_D bool box_empty(const BoxView& b, unsigned best) { return best == 0u || __u
 
 // The voxels of the block at (x0, y0, z0), by the whole CTA.  kVec: rows of a multiple of four voxels,
 // 16-byte (FP16: 8-byte) aligned.  kFresh: every voxel is written; `seen`: whether any can be updated.
-// Returns the bricks of the block in which this thread left a positive value (kFresh), a bit each.
-template <class TT, class WT, bool kVec, bool kFresh>
+// Returns the bricks of the block in which this thread left a positive value (kFresh), a bit each.  kZ: depth of the block.
+template <class TT, class WT, bool kVec, bool kFresh, int kZ>
 AFX_D unsigned integrate_block(TT* __restrict__ tsdf, WT* __restrict__ weights, const float* __restrict__ depth,
                                const RigidArgs& a, float t0, float t1, float t2, int x0, int y0, int z0, bool seen) {
     constexpr int N = kVec ? 4 : 1;                           // voxels per access
@@ -165,7 +174,7 @@ AFX_D unsigned integrate_block(TT* __restrict__ tsdf, WT* __restrict__ weights, 
     unsigned mine = 0u;
     if (x >= X) return mine;
     for (int y = y0 + ty; y < min(y0 + kBlkY, Y); y += kTy)
-        for (int z = z0 + tz; z < min(z0 + kBlkZ, Z); z += kTz) {
+        for (int z = z0 + tz; z < min(z0 + kZ, Z); z += kTz) {
             float tn[N];
             unsigned upd = 0;
             if (!kFresh || seen) {
@@ -209,11 +218,12 @@ AFX_D unsigned integrate_block(TT* __restrict__ tsdf, WT* __restrict__ weights, 
 }
 
 // Whether any voxel of the CTA's block can be updated (the same answer in every thread).
+template <int kZ>
 AFX_D bool block_seen(const RigidArgs& a, const float* __restrict__ depth, float t0, float t1, float t2, int x0, int y0,
                       int z0) {
     __shared__ unsigned wmax[kBlkThreads / 32];
     const int lane = threadIdx.x & 31;
-    const BoxView b = box_view(a, t0, t1, t2, x0, y0, z0);
+    const BoxView b = box_view<kZ>(a, t0, t1, t2, x0, y0, z0);
     if (b.state != 2) return b.state != 0;
     const unsigned m = box_depth(b, depth, a.W, threadIdx.x, kBlkThreads);
     if (lane == 0) wmax[threadIdx.x >> 5] = m;
@@ -221,34 +231,39 @@ AFX_D bool block_seen(const RigidArgs& a, const float* __restrict__ depth, float
     return !box_empty(b, __reduce_max_sync(0xffffffffu, lane < kBlkThreads / 32 ? wmax[lane] : 0u));
 }
 
-template <class TT, class WT, bool kVec>
-__global__ void __launch_bounds__(kBlkThreads, 5) integrate_rigid_kernel(TT* __restrict__ tsdf, WT* __restrict__ weights,
-                                                                         const float* __restrict__ depth, RigidArgs a) {
-    const int x0 = blockIdx.x * kBlkX, y0 = blockIdx.y * kBlkY, z0 = blockIdx.z * kBlkZ;
+// kZ: depth of the blocks; kLook: leave out those without a voxel to update.
+template <class TT, class WT, bool kVec, int kZ, bool kLook>
+__global__ void __launch_bounds__(kBlkThreads, blk_ctas(kVec, kZ)) integrate_rigid_kernel(TT* __restrict__ tsdf,
+                                                                                         WT* __restrict__ weights,
+                                                                                         const float* __restrict__ depth,
+                                                                                         RigidArgs a) {
+    const int x0 = blockIdx.x * kBlkX, y0 = blockIdx.y * kBlkY, z0 = blockIdx.z * kZ;
     const float t0 = a.t_dev ? a.t_dev[0] : a.t[0], t1 = a.t_dev ? a.t_dev[1] : a.t[1],
                 t2 = a.t_dev ? a.t_dev[2] : a.t[2];
-    if (!block_seen(a, depth, t0, t1, t2, x0, y0, z0)) return;
-    integrate_block<TT, WT, kVec, false>(tsdf, weights, depth, a, t0, t1, t2, x0, y0, z0, true);
+    if (kLook && !block_seen<kZ>(a, depth, t0, t1, t2, x0, y0, z0)) return;
+    integrate_block<TT, WT, kVec, false, kZ>(tsdf, weights, depth, a, t0, t1, t2, x0, y0, z0, true);
 }
 
-// a.occ (optional): every byte of it is written, whether the brick has a weighted voxel with a positive value.
-template <bool kVec>
-__global__ void __launch_bounds__(kBlkThreads, 5) integrate_fresh_kernel(float* __restrict__ tsdf,
-                                                                         float* __restrict__ weights,
-                                                                         const float* __restrict__ depth, RigidArgs a) {
+// a.occ (optional; blocks of whole bricks): every byte of it is written, whether the brick has a weighted voxel with a
+// positive value.
+template <bool kVec, int kZ, bool kLook>
+__global__ void __launch_bounds__(kBlkThreads, blk_ctas(kVec, kZ)) integrate_fresh_kernel(float* __restrict__ tsdf,
+                                                                                         float* __restrict__ weights,
+                                                                                         const float* __restrict__ depth,
+                                                                                         RigidArgs a) {
     __shared__ unsigned bricks;  // bit per 8^3 brick of the block with a positive value
     const int X = a.vol.dims[0], Y = a.vol.dims[1], Z = a.vol.dims[2];
-    const int x0 = blockIdx.x * kBlkX, y0 = blockIdx.y * kBlkY, z0 = blockIdx.z * kBlkZ;
-    const bool seen = block_seen(a, depth, a.t[0], a.t[1], a.t[2], x0, y0, z0);
-    const unsigned mine = __reduce_or_sync(0xffffffffu, integrate_block<float, float, kVec, true>(
+    const int x0 = blockIdx.x * kBlkX, y0 = blockIdx.y * kBlkY, z0 = blockIdx.z * kZ;
+    const bool seen = !kLook || block_seen<kZ>(a, depth, a.t[0], a.t[1], a.t[2], x0, y0, z0);
+    const unsigned mine = __reduce_or_sync(0xffffffffu, integrate_block<float, float, kVec, true, kZ>(
                                                             tsdf, weights, depth, a, a.t[0], a.t[1], a.t[2], x0, y0, z0, seen));
-    if (!a.occ) return;
+    if (kZ % 8 != 0 || !a.occ) return;
     if (threadIdx.x == 0) bricks = 0u;
     __syncthreads();
     if ((threadIdx.x & 31) == 0 && mine) atomicOr(&bricks, mine);
     __syncthreads();
     const int k = threadIdx.x, bx = (x0 >> 3) + (k & 3), by = (y0 >> 3) + ((k >> 2) & 1), bz = (z0 >> 3) + (k >> 3);
-    if (k < 16 && bx * 8 < X && by * 8 < Y && bz * 8 < Z)
+    if (k < kZ && bx * 8 < X && by * 8 < Y && bz * 8 < Z)  // 4 x 2 x kZ / 8 of them
         a.occ[((long)bz * a.nby + by) * a.nbx + bx] = (unsigned char)((bricks >> k) & 1u);
 }
 
@@ -270,10 +285,12 @@ static RigidArgs rigid_args(const Volume& vol, const float* R, const float* t, c
     return a;
 }
 
-static dim3 rigid_grid(const Volume& vol) {
+static dim3 rigid_grid(const Volume& vol, int depth) {
     return dim3((unsigned)((vol.dims[0] + kBlkX - 1) / kBlkX), (unsigned)((vol.dims[1] + kBlkY - 1) / kBlkY),
-                (unsigned)((vol.dims[2] + kBlkZ - 1) / kBlkZ));
+                (unsigned)((vol.dims[2] + depth - 1) / depth));
 }
+
+static long voxels_of(const Volume& vol) { return (long)vol.dims[0] * vol.dims[1] * vol.dims[2]; }
 
 // Whether rows of four voxels are aligned vectors (`elem` bytes per voxel and array).
 static bool rows_vectorize(const void* tsdf, const void* weights, const Volume& vol, size_t elem) {
@@ -284,10 +301,17 @@ static bool rows_vectorize(const void* tsdf, const void* weights, const Volume& 
 int integrate_fresh_impl(float* tsdf, float* weights, const float* depth, int W, int H, float delta, const Volume& vol,
                          const float* R, const float* t, const float* K, cudaStream_t st, unsigned char* occ) {
     const RigidArgs a = rigid_args(vol, R, t, nullptr, K, delta, W, H, occ);
-    if (rows_vectorize(tsdf, weights, vol, sizeof(float)))
-        integrate_fresh_kernel<true><<<rigid_grid(vol), kBlkThreads, 0, st>>>(tsdf, weights, depth, a);
-    else
-        integrate_fresh_kernel<false><<<rigid_grid(vol), kBlkThreads, 0, st>>>(tsdf, weights, depth, a);
+    const bool vec = rows_vectorize(tsdf, weights, vol, sizeof(float));
+    auto launch = [&](auto depth_of, auto look_of) {
+        constexpr int kZ = decltype(depth_of)::value;
+        constexpr bool kLook = decltype(look_of)::value;
+        if (vec) integrate_fresh_kernel<true, kZ, kLook><<<rigid_grid(vol, kZ), kBlkThreads, 0, st>>>(tsdf, weights, depth, a);
+        else integrate_fresh_kernel<false, kZ, kLook><<<rigid_grid(vol, kZ), kBlkThreads, 0, st>>>(tsdf, weights, depth, a);
+    };
+    // (every voxel is written, so only the thin blocks pay here; whole bricks where their marks are asked for)
+    if (voxels_of(vol) >= kThinVoxels) launch(std::integral_constant<int, kBlkZ>(), std::true_type());
+    else if (occ) launch(std::integral_constant<int, kMidZ>(), std::false_type());
+    else launch(std::integral_constant<int, kThinZ>(), std::false_type());
     AFX_LAUNCH_CHECK();
     return AFX_OK;
 }
@@ -300,8 +324,16 @@ int integrate_rigid_impl(void* tsdf, void* weights, int fmt, const float* depth,
     vox_dispatch(fmt, tsdf, weights, [&](auto* tp, auto* wp) {
         using TT = std::remove_pointer_t<decltype(tp)>;
         using WT = std::remove_pointer_t<decltype(wp)>;
-        if (vec) integrate_rigid_kernel<TT, WT, true><<<rigid_grid(vol), kBlkThreads, 0, st>>>(tp, wp, depth, a);
-        else integrate_rigid_kernel<TT, WT, false><<<rigid_grid(vol), kBlkThreads, 0, st>>>(tp, wp, depth, a);
+        auto launch = [&](auto depth_of, auto look_of) {
+            constexpr int kZ = decltype(depth_of)::value;
+            constexpr bool kLook = decltype(look_of)::value;
+            const dim3 grid = rigid_grid(vol, kZ);
+            if (vec) integrate_rigid_kernel<TT, WT, true, kZ, kLook><<<grid, kBlkThreads, 0, st>>>(tp, wp, depth, a);
+            else integrate_rigid_kernel<TT, WT, false, kZ, kLook><<<grid, kBlkThreads, 0, st>>>(tp, wp, depth, a);
+        };
+        if (voxels_of(vol) >= kMidVoxels) launch(std::integral_constant<int, kBlkZ>(), std::true_type());
+        else if (voxels_of(vol) >= kThinVoxels) launch(std::integral_constant<int, kMidZ>(), std::true_type());
+        else launch(std::integral_constant<int, kThinZ>(), std::false_type());
         return 0;
     });
     AFX_LAUNCH_CHECK();
