@@ -1114,7 +1114,7 @@ struct DsLayout {
     int* rowptr;    // [kDsNpc + 1]
     double* slot;   // [2][kDsMaxCta][4]
     unsigned long long* bar;  // [2] mbarriers: p.Ap exchange, r.z exchange
-    float* scal;    // [2] beta, stop
+    float* scal;    // [4] beta, stop, whether a wait of this CTA ran out (on 16 bytes, read together)
 };
 
 constexpr size_t kDsSmem = sizeof(float) * ((size_t)kDsNodes * 12 + 3 * kDsNpc * 6 + kDsNpc * 36 + (size_t)kDsBlocks * 36) +
@@ -1122,9 +1122,9 @@ constexpr size_t kDsSmem = sizeof(float) * ((size_t)kDsNodes * 12 + 3 * kDsNpc *
 
 // `base` on 16 bytes: blocks, inverses, z and p are also copied and read 16 bytes at a time.
 AFX_D DsLayout ds_layout(void* base) {
-    static_assert(sizeof(double) * (2 * kDsMaxCta * 4 + 4) % 16 == 0 && sizeof(float) * kDsNodes * 6 % 16 == 0 &&
+    static_assert(sizeof(double) * (2 * kDsMaxCta * 4 + 2) % 16 == 0 && sizeof(double) * (2 * kDsMaxCta * 4 + 4) % 16 == 0 && sizeof(float) * kDsNodes * 6 % 16 == 0 &&
                       sizeof(float) * kDsNpc * 6 % 16 == 0 && sizeof(float) * kDsNpc * 36 % 16 == 0,
-                  "every array from z on starts on 16 bytes");
+                  "scal and every array from z on start on 16 bytes");
     DsLayout d;
     double* dp = static_cast<double*>(base);
     d.slot = dp;
@@ -1196,6 +1196,7 @@ constexpr int kDsDrainPolls = 1 << 12;
 
 // Before the cluster barrier at the start of the kernel (one thread).
 AFX_D void ds_exchange_init(const DsLayout& d) {
+    d.scal[2] = 0.f;
     for (int i = 0; i < 2; ++i)
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(d.bar + i)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1225,6 +1226,7 @@ AFX_D void ds_wait(const DsLayout& d, int i, DsExchange& x, const LoopArgs& L) {
         x.parity[i] ^= 1u;
     } else {
         x.dead = true;
+        d.scal[2] = 1.f;
         if (L.g.error) atomicOr(L.g.error, ERRF_TIMEOUT);
     }
 }
@@ -1450,6 +1452,8 @@ AFX_D void pcg_ds(const LoopArgs& L, int n, const DsLayout& d, DsExchange& ex) {
     if (threadIdx.x == 0) ds_expect(d, 1, rz_bytes);
     precondition(rv, false);
     ds_wait(d, 1, ex, L);
+    __syncthreads();
+    const int iters = d.scal[2] != 0.f ? 0 : L.pcg_iters;
     DF t[NV];
     ds_dot_total<NV>(d, 1, t);
     DF rz = t[0];
@@ -1457,7 +1461,7 @@ AFX_D void pcg_ds(const LoopArgs& L, int n, const DsLayout& d, DsExchange& ex) {
     const float tol2 = kTol ? (float)(L.tol * L.tol) : 0.f, bn = t[NV - 1].hi;
     float beta = 0.f;
     int armed = -1;
-    for (int it = 0; it < L.pcg_iters; ++it) {
+    for (int it = 0; it < iters; ++it) {
         // p = z (first iteration) or z + beta p, formed for all nodes by every CTA from its copies
 #pragma unroll 2
         for (int i = threadIdx.x; i < n * 3; i += kLoopThreads) {
@@ -1470,7 +1474,7 @@ AFX_D void pcg_ds(const LoopArgs& L, int n, const DsLayout& d, DsExchange& ex) {
                 *pv = zv;
             }
         }
-        if (__syncthreads_or(ex.dead)) break;  // the wait for r.z ran out
+        __syncthreads();
         // A p of the own rows
         float acc = 0.f, prod[kRegBlocks];
 #pragma unroll
@@ -1519,8 +1523,9 @@ AFX_D void pcg_ds(const LoopArgs& L, int n, const DsLayout& d, DsExchange& ex) {
             rz = t[0];
         }
         __syncthreads();
-        beta = d.scal[0];
-        if (kTol && d.scal[1] != 0.f) break;
+        const float4 sc = *reinterpret_cast<const float4*>(d.scal);
+        beta = sc.x;
+        if ((kTol && sc.y != 0.f) || sc.z != 0.f) break;  // close enough, or the wait for r.z ran out
     }
     if (act) d.x[o] = x;
     // T_pending -= [[x_rot]x, x_t; 0] for the own nodes (updateTransformsKernel,
@@ -1530,7 +1535,7 @@ AFX_D void pcg_ds(const LoopArgs& L, int n, const DsLayout& d, DsExchange& ex) {
     ex.dead = __syncthreads_or(mine_dead);
     if (ex.dead) {
         if (threadIdx.x == 0) {
-            if (armed < 0) armed = mine_dead ? 2 : 0;  // left at the wait for r.z
+            if (armed < 0) armed = mine_dead ? 2 : 0;  // left after the wait for r.z
             const unsigned bytes[2] = {dot_bytes, rz_bytes};
             ds_drain(d, ex, (unsigned)armed, bytes);
             if (L.gave_up) {
