@@ -740,25 +740,29 @@ long brick_count_total(const Volume& vol) { return make_bricks(vol).n; }
 // kernels spend their time on is the others' counts: a thread looks at four, 32 apart, whose loads are in
 // flight together, and a warp's idle groups are skipped.  200^3 voxels, a sixth of them supported: collisions 17.7 ->
 // 6.9 us, integration 17.8 -> 11.5 us, weights 18.6 -> 15.2 us (the warp, which is bound by its gathers, gained nothing).
+// In small volumes the weights of the supported voxels bound their kernel, not the counts, and four to a thread leave too few
+// threads to hide them: an eighth of the voxels supported, k = 8, 64^3 8.2 us (14.5 with four), 128^3 17 (21), 160^3 25
+// (26), 200^3 43 (45; a sixth in a block at k = 4, as in a sequence, 35 and 25).
 constexpr int kVoxPerThread = 4;
-constexpr int kVoxBlock = 256 * kVoxPerThread;
+constexpr long kFewVoxels = 3000000;
 
-template <class F>
+template <int kVox, class F>
 AFX_D void each_supported(const int* __restrict__ kcount, long S, F&& f) {
     const int lane = threadIdx.x & 31;
-    const long base = ((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5) * (32 * kVoxPerThread) + lane;
-    int c[kVoxPerThread];
+    const long base = ((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5) * (32 * kVox) + lane;
+    int c[kVox];
 #pragma unroll
-    for (int q = 0; q < kVoxPerThread; ++q) c[q] = base + 32 * q < S ? kcount[base + 32 * q] : 0;
+    for (int q = 0; q < kVox; ++q) c[q] = base + 32 * q < S ? kcount[base + 32 * q] : 0;
 #pragma unroll
-    for (int q = 0; q < kVoxPerThread; ++q)
+    for (int q = 0; q < kVox; ++q)
         if (c[q]) f(base + 32 * q, c[q]);
 }
 
+template <int kVox>
 __global__ void tsdf_weights_kernel(float* kw, const float* radii, const uint32_t* kidx, const float* kdist,
                                     const int* kcount, long S, int k) {
     // as the reference: empty voxels keep whatever the array held
-    each_supported(kcount, S, [&](long i, int cnt) {
+    each_supported<kVox>(kcount, S, [&](long i, int cnt) {
         float w[kMaxK];
         float sum = 0.f;
         for (int s = 0; s < k; ++s) w[s] = 0.f;
@@ -841,7 +845,7 @@ struct DenseWarpArgs {
 };
 
 __global__ void count_collisions_kernel(int* counts, const float* verts, const int* kcount, DenseWarpArgs a) {
-    each_supported(kcount, (long)a.vol.dims[0] * a.vol.dims[1] * a.vol.dims[2], [&](long i, int) {
+    each_supported<kVoxPerThread>(kcount, (long)a.vol.dims[0] * a.vol.dims[1] * a.vol.dims[2], [&](long i, int) {
         const long tg = warped_target(verts + 3 * i, a.vol, a.Rinv, a.t);
         if (tg >= 0) atomicAdd(counts + tg, 1);
     });
@@ -850,7 +854,7 @@ __global__ void count_collisions_kernel(int* counts, const float* verts, const i
 __global__ void integrate_warped_kernel(float* tsdf, float* weights, const float* verts, const int* coll,
                                         const int* kcount, const float* depth, int W, int H, float delta,
                                         Intrinsics K, DenseWarpArgs a) {
-    each_supported(kcount, (long)a.vol.dims[0] * a.vol.dims[1] * a.vol.dims[2], [&](long i, int) {
+    each_supported<kVoxPerThread>(kcount, (long)a.vol.dims[0] * a.vol.dims[1] * a.vol.dims[2], [&](long i, int) {
         const long tg = warped_target(verts + 3 * i, a.vol, a.Rinv, a.t);
         if (tg < 0 || coll[tg] > 1) return;
         float tn;
@@ -968,8 +972,10 @@ int afx_tsdf_warp_weights(float* knn_weights, const float* radii, const uint32_t
     if (!knn_weights || !radii || !knn_idx || !knn_dist || !knn_counts || k < 1 || k > kMaxK)
         return AFX_ERR_INVALID_ARGUMENT;
     if (n_voxels <= 0) return AFX_OK;
-    tsdf_weights_kernel<<<blocks_for(n_voxels, kVoxBlock), 256, 0, as_stream(stream)>>>(knn_weights, radii, knn_idx,
-                                                                                  knn_dist, knn_counts, n_voxels, k);
+    const int per = n_voxels < kFewVoxels ? 1 : kVoxPerThread;
+    const auto kernel = per == 1 ? tsdf_weights_kernel<1> : tsdf_weights_kernel<kVoxPerThread>;
+    kernel<<<blocks_for(n_voxels, 256 * per), 256, 0, as_stream(stream)>>>(knn_weights, radii, knn_idx, knn_dist, knn_counts, n_voxels,
+                                                                          k);
     AFX_LAUNCH_CHECK();
     return AFX_OK;
 }
@@ -1008,7 +1014,7 @@ int afx_count_collisions(int* counts, const float* vertices, const int* knn_coun
     rotation_inverse(rotate, a.Rinv);
     for (int c = 0; c < 3; ++c) a.t[c] = translate[c];
     long S = (long)dims[0] * dims[1] * dims[2];
-    count_collisions_kernel<<<blocks_for(S, kVoxBlock), 256, 0, as_stream(stream)>>>(counts, vertices, knn_counts, a);
+    count_collisions_kernel<<<blocks_for(S, 256 * kVoxPerThread), 256, 0, as_stream(stream)>>>(counts, vertices, knn_counts, a);
     AFX_LAUNCH_CHECK();
     return AFX_OK;
 }
@@ -1024,7 +1030,7 @@ int afx_integrate_warped_tsdf(float* tsdf, float* weights, const float* vertices
     rotation_inverse(rotate, a.Rinv);
     for (int c = 0; c < 3; ++c) a.t[c] = translate[c];
     long S = (long)dims[0] * dims[1] * dims[2];
-    integrate_warped_kernel<<<blocks_for(S, kVoxBlock), 256, 0, as_stream(stream)>>>(
+    integrate_warped_kernel<<<blocks_for(S, 256 * kVoxPerThread), 256, 0, as_stream(stream)>>>(
         tsdf, weights, vertices, collisions, knn_counts, depth, width, height, delta, make_intrinsics(K), a);
     AFX_LAUNCH_CHECK();
     return AFX_OK;
