@@ -43,6 +43,7 @@ constexpr float kCellMargin = 1.02f;  // candidate cells over grid cells: more t
 constexpr int kSmallCells = 2048;     // candidate cells whose state fits in shared memory, with a neighbour table
 constexpr int kGreedyThreads = 1024;
 constexpr int kPickMax = 32;          // candidates inserted per round: a bit each of a cell's word
+constexpr int kNearMax = 8;            // points of a round around a cell: their cells are not adjacent to one another
 constexpr unsigned kNoCell = 0xffffffffu;
 constexpr unsigned kGone = 0xffffffffu;  // point index of a decided candidate
 
@@ -87,8 +88,10 @@ struct GraphState {
     unsigned* ccount;    // number of them,
     unsigned* cmin;      // the earliest undecided one (0xffffffff: none),
     unsigned* cblock;    // the adjacent cell that holds an earlier one,
-    unsigned* cnear;     // and the round's inserted points around it
+    unsigned* cnear;     // and the number of the round's inserted points around it
+    unsigned* cwork;     // cells around the round's points
     float4* cpos;        // its position and index
+    float4* cpick;       // [kNearMax] those of the round's inserted points around it
     unsigned short* nbr; // [kSmallCells * 32] adjacent occupied cells (27 used), 0xffff: none
     float* fac;          // [mesh_max] per new node: d / (0 + d)
     GraphCounters* k;
@@ -354,14 +357,14 @@ __global__ void __launch_bounds__(256) graph_bucket_kernel(GraphState s, const G
 // threads: a warp then examines two cells in turn), where a walk in chunks of 1024 candidates, each
 // tested against every node, took 1.76 ms.  The first frame of the 512^3 sequence, 28,761 candidates
 // and 1,300 nodes: 232 rounds, 0.50 ms from 3.6 ms; a frame with nothing to insert: 2 us from 20 us.
-struct GreedyCells {   // per occupied cell, in shared memory (kSmallCells of them) or in global memory
+struct GreedyCells {   // per occupied cell, in shared memory (up to kSmallCells of them)
     float4* pos;       // the earliest undecided candidate: position, point index
     unsigned* cmin;    // the index again (0xffffffff: none)
     unsigned* block;   // the adjacent cell that held an earlier one (kNoCell: to be examined)
     unsigned* near;    // the round's inserted points around it, a bit each
     unsigned* start;   // its candidates: first place in `sorted`
     unsigned* count;   // and number
-    unsigned short* nbr;  // adjacent occupied cells, kNbr per cell (kSmall only; 0xffff: none)
+    unsigned short* nbr;  // adjacent occupied cells, kNbr per cell (0xffff: none)
 };
 constexpr int kNbr = 28;  // 27 and a pad
 __host__ __device__ constexpr unsigned padded_cells(unsigned n) { return n + n / 32 + 1; }
@@ -375,14 +378,54 @@ struct GreedyLists {
     unsigned wsum[kGreedyThreads / 32];
 };
 
-template <bool kSmall>
-AFX_D void greedy_rounds(const GraphState& s, const Grid& g, unsigned nc, const GreedyCells& C, GreedyLists& L) {
+// What a warp that goes through a cell's candidates keeps: those covered by the round's points around the cell (`near`: the
+// lanes or places that hold one, point(i) gives it) are marked, the earliest of the others is returned in `best` of the
+// lane whose `first` is the result.
+template <class Point>
+AFX_D unsigned mark_covered(float4* list, unsigned n, unsigned near, float r2, Point&& point, unsigned& first, float4& best) {
+    const int lane = threadIdx.x & 31;
+    constexpr int kAhead = 4;  // 32-candidate groups loaded together
+    first = 0xffffffffu;
+    for (unsigned i0 = 0; i0 < n; i0 += 32 * kAhead) {
+        float4 v[kAhead];
+        bool gone[kAhead];
+#pragma unroll
+        for (int a = 0; a < kAhead; ++a) {
+            const unsigned i = i0 + a * 32 + lane;
+            v[a] = i < n ? list[i] : make_float4(0.f, 0.f, 0.f, __uint_as_float(kGone));
+            gone[a] = false;
+        }
+        for (unsigned rest = near; rest; rest &= rest - 1) {
+            const float4 q4 = point(__ffs(rest) - 1);
+            const float q[3] = {q4.x, q4.y, q4.z};
+#pragma unroll
+            for (int a = 0; a < kAhead; ++a) {
+                const float p[3] = {v[a].x, v[a].y, v[a].z};
+                gone[a] |= l2sq_nanoflann(p, q) < r2 || __float_as_uint(v[a].w) == __float_as_uint(q4.w);
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < kAhead; ++a) {
+            const unsigned id = __float_as_uint(v[a].w);
+            if (id == kGone) continue;
+            if (gone[a]) {
+                list[i0 + a * 32 + lane].w = __uint_as_float(kGone);
+            } else if (id < first) {
+                first = id;
+                best = v[a];
+            }
+        }
+    }
+    return __reduce_min_sync(0xffffffffu, first);
+}
+
+AFX_D void greedy_rounds(const GraphState& s, unsigned nc, const GreedyCells& C, GreedyLists& L) {
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const unsigned limit = s.k->ncand + 2;
     constexpr unsigned kWarps = kGreedyThreads / 32;
-    // A warp's share are the cells w, w + kWarps, ...: cells to examine tend to be consecutive ones.  In shared
-    // memory a word of padding per 32 keeps that access free of bank conflicts.
-    auto at = [](unsigned c) { return kSmall ? c + (c >> 5) : c; };
+    // A warp's share are the cells w, w + kWarps, ...: cells to examine tend to be consecutive ones.  A word of
+    // padding per 32 keeps that access free of bank conflicts.
+    auto at = [](unsigned c) { return c + (c >> 5); };
     for (unsigned round = 1; round <= limit; ++round) {
         // (a)
         const int par = round & 1;
@@ -397,11 +440,7 @@ AFX_D void greedy_rounds(const GraphState& s, const Grid& g, unsigned nc, const 
             }
             for (unsigned rest = __ballot_sync(0xffffffffu, check); rest; rest &= rest - 1) {
                 const unsigned c = c0 + kWarps * (__ffs(rest) - 1), m = C.cmin[at(c)];
-                int nb = -1;
-                if (lane < 27) {
-                    if (kSmall) nb = C.nbr[c * kNbr + lane] == 0xffff ? -1 : (int)C.nbr[c * kNbr + lane];
-                    else nb = adjacent_cell(s, g, c, lane);
-                }
+                const int nb = lane < 27 && C.nbr[c * kNbr + lane] != 0xffff ? (int)C.nbr[c * kNbr + lane] : -1;
                 const unsigned mm = nb >= 0 ? C.cmin[at(nb)] : 0xffffffffu;
                 const unsigned wm = __reduce_min_sync(0xffffffffu, mm);
                 if (wm < m) {
@@ -432,46 +471,80 @@ AFX_D void greedy_rounds(const GraphState& s, const Grid& g, unsigned nc, const 
         const unsigned nwork = L.nwork[par];
         if (tid == 0) L.npick[par ^ 1] = L.nwork[par ^ 1] = 0;  // the next round's, unused in this one
         for (unsigned q = w; q < nwork; q += kWarps) {
-            const unsigned c = L.work[q], near = C.near[c], n = C.count[c];
-            float4* list = s.sorted + C.start[c];
-            unsigned first = 0xffffffffu;
+            const unsigned c = L.work[q];
+            unsigned first;
             float4 fp;
-            constexpr int kAhead = 4;  // 32-candidate groups loaded together
-            for (unsigned i0 = 0; i0 < n; i0 += 32 * kAhead) {
-                float4 v[kAhead];
-                bool gone[kAhead];
-#pragma unroll
-                for (int a = 0; a < kAhead; ++a) {
-                    const unsigned i = i0 + a * 32 + lane;
-                    v[a] = i < n ? list[i] : make_float4(0.f, 0.f, 0.f, __uint_as_float(kGone));
-                    gone[a] = false;
-                }
-                for (unsigned rest = near; rest; rest &= rest - 1) {
-                    const float4 q4 = L.pick[__ffs(rest) - 1];
-                    const float q[3] = {q4.x, q4.y, q4.z};
-#pragma unroll
-                    for (int a = 0; a < kAhead; ++a) {
-                        const float p[3] = {v[a].x, v[a].y, v[a].z};
-                        gone[a] |= l2sq_nanoflann(p, q) < s.r2 || __float_as_uint(v[a].w) == __float_as_uint(q4.w);
-                    }
-                }
-#pragma unroll
-                for (int a = 0; a < kAhead; ++a) {
-                    const unsigned id = __float_as_uint(v[a].w);
-                    if (id == kGone) continue;
-                    if (gone[a]) {
-                        list[i0 + a * 32 + lane].w = __uint_as_float(kGone);
-                    } else if (id < first) {
-                        first = id;
-                        fp = v[a];
-                    }
-                }
-            }
-            const unsigned wf = __reduce_min_sync(0xffffffffu, first);
+            const unsigned wf = mark_covered(s.sorted + C.start[c], C.count[c], C.near[c], s.r2,
+                                             [&](int k) { return L.pick[k]; }, first, fp);
             if (wf != 0xffffffffu && first == wf) C.pos[c] = fp;
             if (lane == 0) {
                 C.cmin[at(c)] = wf;
                 C.near[c] = 0u;
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// The same with the cells in global memory and no limit on the points of a round: each is left with the cells around it
+// (at most kNearMax to a cell).  300,000 points in a plane, 29,000 nodes: 28 ms in the cloud's order, and 23,000
+// nodes, 9 ms, in no order; with 32 points a round 42 and 90 ms (the walk in chunks: 45 and 39).
+AFX_D void greedy_rounds_large(const GraphState& s, const Grid& g, unsigned nc, GreedyLists& L) {
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const unsigned limit = s.k->ncand + 2;
+    constexpr unsigned kWarps = kGreedyThreads / 32;
+    for (unsigned round = 1; round <= limit; ++round) {
+        // (a)
+        const int par = round & 1;
+        bool some = false;
+        for (unsigned c0 = w; c0 < nc; c0 += kGreedyThreads) {
+            const unsigned mine = c0 + kWarps * lane;
+            bool check = false;
+            if (mine < nc) {
+                const unsigned m = s.cmin[mine], b = s.cblock[mine];
+                check = m != 0xffffffffu && (b == kNoCell || !(s.cmin[b] < m));
+                some |= m != 0xffffffffu;
+            }
+            for (unsigned rest = __ballot_sync(0xffffffffu, check); rest; rest &= rest - 1) {
+                const unsigned c = c0 + kWarps * (__ffs(rest) - 1), m = s.cmin[c];
+                const int nb = lane < 27 ? adjacent_cell(s, g, c, lane) : -1;
+                const unsigned mm = nb >= 0 ? s.cmin[nb] : 0xffffffffu;
+                const unsigned wm = __reduce_min_sync(0xffffffffu, mm);
+                if (wm < m) {
+                    if (mm == wm) s.cblock[c] = (unsigned)nb;
+                    continue;
+                }
+                if (lane == 0) {
+                    s.cblock[c] = kNoCell;
+                    atomicOr(s.picked + (m >> 5), 1u << (m & 31));
+                }
+                const float4 pick = s.cpos[c];
+                unsigned k = kNearMax;
+                if (nb >= 0 && mm != 0xffffffffu) k = atomicAdd(s.cnear + nb, 1u);
+                if (k < kNearMax) s.cpick[(long)nb * kNearMax + k] = pick;
+                const bool first = k == 0u;
+                const unsigned add = __ballot_sync(0xffffffffu, first);
+                unsigned place = 0;
+                if (lane == 0) place = atomicAdd(&L.nwork[par], (unsigned)__popc(add));
+                place = __shfl_sync(0xffffffffu, place, 0) + __popc(add & ((1u << lane) - 1u));
+                if (first) s.cwork[place] = (unsigned)nb;
+            }
+        }
+        if (!__syncthreads_or(some)) break;
+        // (b)
+        const unsigned nwork = L.nwork[par];
+        if (tid == 0) L.nwork[par ^ 1] = 0;
+        for (unsigned q = w; q < nwork; q += kWarps) {
+            const unsigned c = s.cwork[q], near = min(s.cnear[c], (unsigned)kNearMax);
+            const float4* picks = s.cpick + (long)c * kNearMax;
+            unsigned first;
+            float4 fp;
+            const unsigned wf = mark_covered(s.sorted + s.cstart[c], s.ccount[c], (1u << near) - 1u, s.r2,
+                                             [&](int k) { return picks[k]; }, first, fp);
+            if (wf != 0xffffffffu && first == wf) s.cpos[c] = fp;
+            if (lane == 0) {
+                s.cmin[c] = wf;
+                s.cnear[c] = 0u;
             }
         }
         __syncthreads();
@@ -486,30 +559,29 @@ __global__ void __launch_bounds__(kGreedyThreads) graph_greedy_kernel(GraphState
     const Grid g = *gp;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     if (tid < 2) L.npick[tid] = L.nwork[tid] = 0;
-    const GreedyCells G{s.cpos, s.cmin, s.cblock, s.cnear, s.cstart, s.ccount, nullptr};
     unsigned* u = reinterpret_cast<unsigned*>(cells + nc);
     unsigned* v = u + 2 * padded_cells(nc);
     const GreedyCells S{cells, u, u + padded_cells(nc), v, v + nc, v + 2 * nc, reinterpret_cast<unsigned short*>(v + 3 * nc)};
     const bool small = nc <= kSmallCells;
     for (unsigned c = tid; c < nc; c += kGreedyThreads) {
-        const unsigned m = G.cmin[c];
+        const unsigned m = s.cmin[c];
         const float4 p = make_float4(s.mesh[3 * (long)m], s.mesh[3 * (long)m + 1], s.mesh[3 * (long)m + 2], __uint_as_float(m));
         if (small) {
             S.pos[c] = p;
             S.cmin[c + (c >> 5)] = m;
             S.block[c + (c >> 5)] = kNoCell;
             S.near[c] = 0u;
-            S.start[c] = G.start[c];
-            S.count[c] = G.count[c];
+            S.start[c] = s.cstart[c];
+            S.count[c] = s.ccount[c];
         } else {
-            G.pos[c] = p;
+            s.cpos[c] = p;
         }
     }
     for (unsigned t = tid; small && t < nc * 32; t += kGreedyThreads)
         if ((t & 31) < 27) S.nbr[(t >> 5) * kNbr + (t & 31)] = s.nbr[t];
     __syncthreads();
-    if (small) greedy_rounds<true>(s, g, nc, S, L);
-    else greedy_rounds<false>(s, g, nc, G, L);
+    if (small) greedy_rounds(s, nc, S, L);
+    else greedy_rounds_large(s, g, nc, L);
     __syncthreads();
     // the inserted points in order: nodes n0, n0 + 1, ...
     const long m = min((long)*s.mesh_count, s.mesh_max), words = (m + 31) / 32;
@@ -591,36 +663,35 @@ __global__ void __launch_bounds__(256) graph_transforms_kernel(GraphState s) {
     if (!last_block(&s.k->done[2])) return;
     const int cnt = n - first;
     auto up = [&](int i) { return (int)__ldcg(parent + (i - first)); };
-    constexpr int kJump = 8192;  // new nodes whose ways up are shortened in shared memory
+    constexpr int kJump = 8192;  // new nodes whose ways up are shortened in shared memory, those of more in global memory
     constexpr unsigned kOdd = 0x80000000u;  // a factor other than 1 on the way
     __shared__ unsigned sp[kJump];
-    if (cnt <= kJump) {  // each node's ancestor, doubled until it is one of the old nodes
-        for (int i = threadIdx.x; i < cnt; i += blockDim.x)
-            sp[i] = __ldcg(parent + i) | (__ldcg(s.fac + i) == 1.0f ? 0u : kOdd);
-        bool more = true;
-        while (__syncthreads_or(more)) {  // any ancestor another thread has moved up meanwhile is one too
-            more = false;
-            for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
-                const unsigned a = sp[i], q = a & ~kOdd;
-                if ((int)q < first) continue;
-                sp[i] = sp[q - first] | (a & kOdd);
-                more = true;
-            }
+    unsigned* const gp = reinterpret_cast<unsigned*>(s.sorted);  // (not needed once the rounds are over)
+    const bool small = cnt <= kJump;
+    auto get = [&](int t) { return small ? sp[t] : __ldcg(gp + t); };
+    auto put = [&](int t, unsigned v) {
+        if (small) sp[t] = v;
+        else __stcg(gp + t, v);
+    };
+    // each node's ancestor, doubled until it is one of the old nodes
+    for (int t = threadIdx.x; t < cnt; t += blockDim.x)
+        put(t, __ldcg(parent + t) | (__ldcg(s.fac + t) == 1.0f ? 0u : kOdd));
+    bool more = true;
+    while (__syncthreads_or(more)) {  // any ancestor another thread has moved up meanwhile is one too
+        more = false;
+        for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
+            const unsigned a = get(t), q = a & ~kOdd;
+            if ((int)q < first) continue;
+            put(t, get((int)q - first) | (a & kOdd));
+            more = true;
         }
     }
     for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
         const int i = first + t;
-        bool plain = true;
-        int root = i, hops = 0;
-        if (cnt <= kJump) {
-            plain = !(sp[t] & kOdd);
-            root = (int)(sp[t] & ~kOdd);
-        }
-        if (cnt > kJump || !plain)
-            for (plain = true, root = i; root >= first; ++hops) {
-                plain = plain && __ldcg(s.fac + (root - first)) == 1.0f;
-                root = up(root);
-            }
+        bool plain = !(get(t) & kOdd);
+        int root = (int)(get(t) & ~kOdd), hops = 0;
+        if (!plain)
+            for (root = i; root >= first; ++hops) root = up(root);
         float* out = s.T + 16 * (long)i;
         const float* in = s.T + 16 * (long)root;
         for (int e = 0; e < 16; ++e) {
@@ -689,6 +760,10 @@ int build_graph_impl(float* nodes, float* radii, float* T, int* n_nodes, int cap
     s.cpos = (float4*)take(C * sizeof(float4));
     s.nbr = (unsigned short*)take((size_t)kSmallCells * 32 * 2);
     s.g.slots = (int*)take(C * kGridSlots * 4);
+    // the rounds of large graphs use the room of the node grid, which is not needed any more by then
+    s.cwork = reinterpret_cast<unsigned*>(s.g.cnt);
+    s.cpick = reinterpret_cast<float4*>(s.g.slots);
+    static_assert(kGridSlots * sizeof(int) >= kNearMax * sizeof(float4), "they fit");
     s.pcell = (unsigned*)take(mesh_max * 4);
     s.prank = (unsigned*)take(mesh_max * 4);
     s.sorted = (float4*)take(mesh_max * sizeof(float4));
