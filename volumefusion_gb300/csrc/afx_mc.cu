@@ -845,13 +845,21 @@ AFX_D bool key_le(const Key3& a, const Key3& b) { return !key_less(b, a); }
 // many passes are launched as the capacity can need; those that the live number does not need return
 // at once.  The pass a run length belongs to decides which buffer it reads.
 // Bound: latency of a pass (a search for the split, one load, a merge of kSortPer keys per thread).
-// 450,000 points of a marching-cubes cloud: tiles 20 us, 8 passes of 9 us, unique 15 us; one cluster of
-// 16 CTAs doing all of it took 905 us.
+// 450,000 points in room for a million: 102 us (131 with launches that each wait for the one before to be gone; one cluster of
+// 16 CTAs doing all of it 1,365); 5,000 points in the same room 50 us (78, 70), none 40 (57, 18).
 constexpr int kSortTile = 2048;
 constexpr int kSortPer = 8;  // keys per thread
 constexpr int kSortThreads = kSortTile / kSortPer;
 constexpr int kUniqueThreads = 1024;
 constexpr long kSortBlocks = 608;  // four CTAs per SM
+
+// The launches after the first may start while the one before still runs, and wait here for all of it: an empty pass --
+// most are, where a cloud is small for its capacity -- costs about 1 us instead of 3.5.  The next launch is
+// let in only after that, so a launch waits for all before it.
+AFX_D void sort_pass_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // Passes that merge runs of kSortTile into one of n.
 __host__ __device__ inline int sort_passes(long n) {
@@ -906,6 +914,7 @@ AFX_D void merge_serial(SortTile& s, int at, int la, int lb, int q0, Key3 (&out)
 __global__ void __launch_bounds__(kSortThreads) sort_tiles_kernel(const float* __restrict__ pts, const unsigned* count,
                                                                  long n_max, Key3* out, unsigned* done) {
     __shared__ SortTile s;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const long n = min((long)*count, n_max);
     if (blockIdx.x == 0 && threadIdx.x == 0) *done = 0u;
     for (long base = blockIdx.x * (long)kSortTile; base < n; base += gridDim.x * (long)kSortTile) {
@@ -964,6 +973,7 @@ __global__ void __launch_bounds__(kSortThreads) merge_pass_kernel(const Key3* __
                                                                  const unsigned* count, long n_max, long L) {
     __shared__ SortTile s;
     __shared__ long split[2];
+    sort_pass_begin();
     const long n = min((long)*count, n_max);
     if (L >= n) return;  // one run already
     for (long o0 = blockIdx.x * (long)kSortTile; o0 < n; o0 += gridDim.x * (long)kSortTile) {
@@ -1001,6 +1011,7 @@ AFX_D bool key_same_point(const Key3& a, const Key3& b) {
 // Points of each tile that differ from the one before them.
 __global__ void __launch_bounds__(kUniqueThreads) unique_count_kernel(const Key3* buf0, const Key3* buf1,
                                                                    const unsigned* count, long n_max, unsigned* tile_cnt) {
+    sort_pass_begin();
     const long n = min((long)*count, n_max), tiles = (n + kSortTile - 1) / kSortTile;
     const Key3* src = sort_passes(n) & 1 ? buf1 : buf0;
     for (long t = blockIdx.x; t < tiles; t += gridDim.x) {
@@ -1019,6 +1030,7 @@ __global__ void __launch_bounds__(kUniqueThreads) unique_compact_kernel(float* p
                                                                      unsigned* count, long n_max,
                                                                      const unsigned* __restrict__ tile_cnt, unsigned* done) {
     __shared__ unsigned wsum[kUniqueThreads / 32];
+    sort_pass_begin();
     const long n = min((long)*count, n_max), tiles = (n + kSortTile - 1) / kSortTile;
     const Key3* src = sort_passes(n) & 1 ? buf1 : buf0;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1084,14 +1096,27 @@ int sort_unique_impl(float* pts, unsigned* count, long n_max, void* ws, size_t w
     const unsigned grid = (unsigned)(tiles < kSortBlocks ? tiles : kSortBlocks);
     sort_tiles_kernel<<<grid, kSortThreads, 0, st>>>(pts, count, n_max, buf[0], done);
     AFX_LAUNCH_CHECK();
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kSortThreads);
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
     const int passes = sort_passes(n_max);
     for (int k = 0; k < passes; ++k) {
-        merge_pass_kernel<<<grid, kSortThreads, 0, st>>>(buf[k & 1], buf[(k & 1) ^ 1], count, n_max, (long)kSortTile << k);
+        AFX_CUDA(cudaLaunchKernelEx(&cfg, merge_pass_kernel, (const Key3*)buf[k & 1], buf[(k & 1) ^ 1], (const unsigned*)count, n_max,
+                                    (long)kSortTile << k));
         AFX_LAUNCH_CHECK();
     }
-    unique_count_kernel<<<grid, kUniqueThreads, 0, st>>>(buf[0], buf[1], count, n_max, tile_cnt);
+    cfg.blockDim = dim3(kUniqueThreads);
+    AFX_CUDA(cudaLaunchKernelEx(&cfg, unique_count_kernel, (const Key3*)buf[0], (const Key3*)buf[1], (const unsigned*)count, n_max,
+                                tile_cnt));
     AFX_LAUNCH_CHECK();
-    unique_compact_kernel<<<grid, kUniqueThreads, 0, st>>>(pts, buf[0], buf[1], count, n_max, tile_cnt, done);
+    AFX_CUDA(cudaLaunchKernelEx(&cfg, unique_compact_kernel, pts, (const Key3*)buf[0], (const Key3*)buf[1], count, n_max,
+                                (const unsigned*)tile_cnt, done));
     AFX_LAUNCH_CHECK();
     return AFX_OK;
 }
