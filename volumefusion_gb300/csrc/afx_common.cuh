@@ -61,13 +61,6 @@ inline unsigned grid_for(long n, int threads) {
     long b = (n + threads - 1) / threads;
     return (unsigned)(b < 1 ? 1 : (b > kStrideBlocks ? kStrideBlocks : b));
 }
-// The same for kernels with a long loop per item (one graph node per warp or block): up to 8
-// blocks per SM, so that graphs of thousands of nodes still spread over every SM.
-constexpr long kNodeBlocks = 1216;
-inline unsigned grid_for_nodes(long n, int per_block) {
-    long b = (n + per_block - 1) / per_block;
-    return (unsigned)(b < 1 ? 1 : (b > kNodeBlocks ? kNodeBlocks : b));
-}
 
 // for (i in [start, n)) over the whole grid
 #define AFX_GRID_STRIDE(i, n) \
@@ -188,15 +181,6 @@ AFX_D T warp_sum(T v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
-}
-
-// Bounded spin on a device flag / counter; returns false on timeout.
-AFX_D bool spin_until_geq(volatile unsigned* p, unsigned target, long max_iter) {
-    for (long i = 0; i < max_iter; ++i) {
-        if (*p >= target) return true;
-        __nanosleep(64);
-    }
-    return false;
 }
 
 }  // namespace afx

@@ -785,14 +785,11 @@ AFX_D double dsmem_load(const double* p, unsigned rank) {
     return v;
 }
 
-// Double-binary32 ("double-float") arithmetic: a value is the unevaluated sum hi + lo of two
-// binary32 numbers with |lo| <= ulp(hi) / 2, about 48 significant bits.  A sum is the accurate
-// double-float addition of Hida, Li and Bailey's QD library (2001): Knuth's TwoSum (the exact
-// rounding error of a binary32 sum) on the high and the low parts, then Dekker's Fast2Sum to
-// renormalise; a product of two binary32 values is exact as p + fma(x, y, -p).  TwoSum's error term
-// is exact whatever the operand order, so df_add(a, b) and df_add(b, a) agree bit for bit and
-// every lane of a butterfly ends with the same total.  On this part a dependent binary64 add takes
-// ~150-200 cycles; a double-float add is a chain of ~8 binary32 operations.
+// Double-binary32 ("double-float") numbers: the unevaluated sum hi + lo of two binary32 numbers with
+// |lo| <= ulp(hi) / 2, about 48 significant bits.  Knuth's TwoSum gives a binary32 sum and its exact rounding error,
+// the same whatever the operands' order, so every lane of a butterfly ends with the same total; Dekker's Fast2Sum does
+// so for |a| >= |b|; a product of two binary32 numbers is exact as p + fma(x, y, -p).  On this part a dependent
+// binary64 add takes ~150-200 cycles.
 struct DF {
     float hi, lo;
 };
@@ -807,21 +804,9 @@ AFX_D DF fast_two_sum(float a, float b) {
     return {s, b - (s - a)};
 }
 
-AFX_D DF df_add(DF a, DF b) {
-    DF s = two_sum(a.hi, b.hi);
-    const DF t = two_sum(a.lo, b.lo);
-    s = fast_two_sum(s.hi, s.lo + t.hi);
-    return fast_two_sum(s.hi, s.lo + t.lo);
-}
-
-AFX_D DF df_prod(float x, float y) {
-    const float p = x * y;
-    return {p, fmaf(x, y, -p)};
-}
-
 // A sum under way: hi is the running binary32 sum, lo the running sum of its exact rounding errors and c
 // that of lo's.  Adding two of them waits for one addition on hi and two on lo; the error terms follow
-// behind, so a butterfly step costs a shuffle and two additions instead of a double-float addition's
+// behind, so a butterfly step costs a shuffle and two additions where adding double-floats takes
 // thirteen, and the result carries more bits (errors of the PCG's dot products against exact sums, over
 // 12 to 384 terms per CTA and 16 CTAs, relative to the sum of |x y|: about a third of a double-float's; with
 // 66 terms at most 1.8e-15 and 3.2e-16 on average, against 4.7e-15 and 9.5e-16).
@@ -850,10 +835,6 @@ AFX_D DF tf_butterfly(TF v) {
     }
     const DF s = fast_two_sum(v.hi, v.lo);
     return fast_two_sum(s.hi, s.lo + v.c);
-}
-
-AFX_D DF df_shfl_xor(DF v, int o) {
-    return {__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
 }
 
 // a / b rounded to binary32 (within about half an ulp): the binary32 quotient of the high parts,
@@ -1240,15 +1221,13 @@ AFX_D void ds_drain(const DsLayout& d, const DsExchange& x, unsigned armed, cons
 
 // Cluster sum through the slot arrays: the CTA's block total is written into slot[ph][rank] of
 // every CTA; after the barrier each CTA adds the slots in rank order.
-// `live` (warp-uniform) is false for warps whose lanes hold only zeros: they skip the FP64
-// butterfly (FP64 issue is scarce on this part) and contribute an exact 0.
 template <int NV>
-AFX_D void ds_sum(double (&v)[NV], const DsLayout& d, ClusterSums& cs, int& ph, bool live = true) {
+AFX_D void ds_sum(double (&v)[NV], const DsLayout& d, ClusterSums& cs, int& ph) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned rank = cluster_rank(), ncta = cluster_size();
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-        const double s = live ? warp_sum(v[i]) : 0.0;
+        const double s = warp_sum(v[i]);
         if (lane == 0) cs.warp[w * 4 + i] = s;
     }
     __syncthreads();
@@ -2363,7 +2342,7 @@ size_t gn_workspace_size(long m_max, int n_max, int k, int kreg) {
     s += al(n_max * 4) + al((size_t)n_max * kMaxNbr * 4);         // nbr_cnt nbr
     s += al((size_t)n_max * kMaxNbr * 36 * 4) + al((size_t)n_max * 36 * 4) + al((size_t)n_max * 36 * 4);
     s += al((size_t)m_max * k * 6 * 4) + al((size_t)m_max * k * 4);  // jrow jc
-    s += al((size_t)n_max * 6 * 4) * 5 + al((size_t)n_max * 6 * 4 * 2);  // jtr x r z p, ap + p2
+    s += al((size_t)n_max * 6 * 4) * 6;                           // jtr x r z p ap
     s += al(m_max * 4) + al((size_t)n_max * kreg * 3 * 4);        // rdepth rreg
     s += al(sizeof(GnState));
     return s + 1024;
@@ -2397,7 +2376,7 @@ bool gn_carve(void* ws, size_t bytes, long m_max, int n_max, int k, int kreg, Gn
     b->r = (float*)take((size_t)n_max * 6 * 4);
     b->z = (float*)take((size_t)n_max * 6 * 4);
     b->p = (float*)take((size_t)n_max * 6 * 4);
-    b->ap = (float*)take((size_t)n_max * 6 * 4 * 2);  // A p, then the second search-direction buffer
+    b->ap = (float*)take((size_t)n_max * 6 * 4);
     b->rdepth = (float*)take(m_max * 4);
     b->rreg = (float*)take((size_t)n_max * kreg * 3 * 4);
     b->state = (GnState*)take(sizeof(GnState));

@@ -19,9 +19,6 @@ inline size_t vox_bytes(int fmt) { return fmt == kVoxF16 ? 2 : 4; }  // per arra
 // sum of all n values is written there (device).  Workspace: scan_workspace_size(n).
 size_t scan_workspace_size(long n);
 int scan_exclusive(const unsigned* in, unsigned* out, long n, unsigned* total, void* ws, cudaStream_t st);
-// Same, with the element count read from the device (n = min(*count, n_max)).
-int scan_exclusive_dev(const unsigned* in, unsigned* out, const unsigned* count, long n_max, unsigned* total, void* ws,
-                       cudaStream_t st);
 
 // ---- prep (afx_prep.cu) ----
 // undistort_map: a cv::undistort map of the frame (afx_undistort_map, AFX_UNDISTORT_LINEAR) to sample the

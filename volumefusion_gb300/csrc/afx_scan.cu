@@ -1,8 +1,7 @@
 // afx_scan.cu -- exclusive prefix sums used for stream compaction and CSR offsets.
 // Three phases: per-tile sums, a single-block scan of those sums, then the tile-local scans
 // with their offsets added.  Deterministic (integer arithmetic).  The tile phases are
-// grid-stride loops over the tiles that hold live items (the live count is read on the device),
-// on a grid of at most kScanBlocks, so a large capacity with few items costs one short wave.
+// grid-stride loops over the tiles, on a grid of at most kScanBlocks.
 #include "afx_internal.h"
 
 namespace afx {
@@ -38,16 +37,10 @@ AFX_D unsigned block_exclusive_scan(unsigned v, unsigned* warp_sums, unsigned* b
     return excl;
 }
 
-__device__ __forceinline__ long scan_n(const unsigned* count, long n_max) {
-    return count ? min((long)*count, n_max) : n_max;
-}
-
 constexpr long kScanBlocks = 152;
 
-__global__ void __launch_bounds__(kScanThreads) scan_block_sums(const unsigned* in, const unsigned* count, long n_max,
-                                                                 unsigned* sums) {
+__global__ void __launch_bounds__(kScanThreads) scan_block_sums(const unsigned* in, long n, unsigned* sums) {
     __shared__ unsigned ws[32];
-    const long n = scan_n(count, n_max);
     const long nt = (n + kScanTile - 1) / kScanTile;
     for (long tile = blockIdx.x; tile < nt; tile += gridDim.x) {
         const long base = tile * kScanTile;
@@ -62,10 +55,8 @@ __global__ void __launch_bounds__(kScanThreads) scan_block_sums(const unsigned* 
     }
 }
 
-__global__ void __launch_bounds__(1024) scan_sums_kernel(unsigned* sums, const unsigned* count, long n_max,
-                                                         unsigned* total) {
+__global__ void __launch_bounds__(1024) scan_sums_kernel(unsigned* sums, long nblocks, unsigned* total) {
     __shared__ unsigned ws[32];
-    const long nblocks = (scan_n(count, n_max) + kScanTile - 1) / kScanTile;
     unsigned carry = 0;
     for (long base = 0; base < nblocks; base += blockDim.x) {
         long j = base + threadIdx.x;
@@ -78,10 +69,8 @@ __global__ void __launch_bounds__(1024) scan_sums_kernel(unsigned* sums, const u
     if (threadIdx.x == 0 && total) *total = carry;
 }
 
-__global__ void __launch_bounds__(kScanThreads) scan_apply(const unsigned* in, unsigned* out, const unsigned* count,
-                                                           long n_max, const unsigned* sums) {
+__global__ void __launch_bounds__(kScanThreads) scan_apply(const unsigned* in, unsigned* out, long n, const unsigned* sums) {
     __shared__ unsigned ws[32];
-    const long n = scan_n(count, n_max);
     const long nt = (n + kScanTile - 1) / kScanTile;
     for (long tile = blockIdx.x; tile < nt; tile += gridDim.x) {
         const long base = tile * kScanTile;
@@ -103,26 +92,21 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply(const unsigned* in, u
 
 size_t scan_workspace_size(long n) { return (size_t)((n + kScanTile - 1) / kScanTile + 1) * sizeof(unsigned); }
 
-int scan_exclusive_dev(const unsigned* in, unsigned* out, const unsigned* count, long n_max, unsigned* total, void* ws,
-                       cudaStream_t st) {
-    if (n_max <= 0) {
+int scan_exclusive(const unsigned* in, unsigned* out, long n, unsigned* total, void* ws, cudaStream_t st) {
+    if (n <= 0) {
         if (total) AFX_CUDA(cudaMemsetAsync(total, 0, sizeof(unsigned), st));
         return AFX_OK;
     }
-    const long nb = (n_max + kScanTile - 1) / kScanTile;
+    const long nb = (n + kScanTile - 1) / kScanTile;
     const unsigned grid = (unsigned)(nb < kScanBlocks ? nb : kScanBlocks);
     unsigned* sums = static_cast<unsigned*>(ws);
-    scan_block_sums<<<grid, kScanThreads, 0, st>>>(in, count, n_max, sums);
+    scan_block_sums<<<grid, kScanThreads, 0, st>>>(in, n, sums);
     AFX_LAUNCH_CHECK();
-    scan_sums_kernel<<<1, 1024, 0, st>>>(sums, count, n_max, total);
+    scan_sums_kernel<<<1, 1024, 0, st>>>(sums, nb, total);
     AFX_LAUNCH_CHECK();
-    scan_apply<<<grid, kScanThreads, 0, st>>>(in, out, count, n_max, sums);
+    scan_apply<<<grid, kScanThreads, 0, st>>>(in, out, n, sums);
     AFX_LAUNCH_CHECK();
     return AFX_OK;
-}
-
-int scan_exclusive(const unsigned* in, unsigned* out, long n, unsigned* total, void* ws, cudaStream_t st) {
-    return scan_exclusive_dev(in, out, nullptr, n, total, ws, st);
 }
 
 }  // namespace afx
