@@ -69,7 +69,7 @@ AFX_D void mark_brick(unsigned char* occ, int nbx, int nby, int x, int y, int z)
 }
 
 // Blocks of kBlkZ slices.  Below kMidVoxels half as deep, since there are few for the SMs (256^3: an object 29 -> 27.5 us,
-// every voxel updated 70 -> 68; rows of 255 voxels 84 -> 75; at 320^3 the looking costs more than that saves, an
+// every voxel updated 70 -> 64.5; rows of 255 voxels 84 -> 71; at 320^3 the looking costs more than that saves, an
 // object 37 -> 41.5).  Below kThinVoxels a quarter as deep and without looking, for which there is little to leave
 // out (an object and every voxel updated, from kBlkZ slices to these: 64^3 21 -> 11 us both, 128^3 21 -> 11 and 23 -> 13,
 // 192^3 23 -> 21 and 31 -> 29; at 256^3 29 -> 42 and 70 -> 62).
@@ -139,8 +139,11 @@ AFX_D BoxView box_view(const RigidArgs& a, float t0, float t1, float t2, int x0,
     return b;
 }
 
-// Largest valid depth of the box's pixels, as bits (positive floats compare as integers; 0: none; not a
-// number counts as infinitely far, since it updates), over this thread's share of them.
+// A valid depth as bits: positive floats compare as integers; 0: none; not a number counts as infinitely far, since it
+// updates.
+AFX_D unsigned depth_key(float d) { return d != d ? 0x7f800000u : (isinf(d) || d < 1.e-4f) ? 0u : __float_as_uint(d); }
+
+// Largest of the box's pixels over this thread's share of them.
 AFX_D unsigned box_depth(const BoxView& b, const float* __restrict__ depth, int W, int first, int step) {
     const int n = b.w * b.h;
     const float inv = 1.0f / (float)b.w;  // (i + 1/2) / w is at least 1/2w from an integer: exact for these n
@@ -149,8 +152,7 @@ AFX_D unsigned box_depth(const BoxView& b, const float* __restrict__ depth, int 
     for (int i = first; i < n; i += step) {
         const int row = (int)(((float)i + 0.5f) * inv);
         const float d = __ldg(depth + (long)(b.py0 + row) * W + b.px0 + (i - row * b.w));
-        const unsigned k = d != d ? 0x7f800000u : (isinf(d) || d < 1.e-4f) ? 0u : __float_as_uint(d);
-        best = max(best, k);
+        best = max(best, depth_key(d));
     }
     return __reduce_max_sync(0xffffffffu, best);
 }
@@ -225,6 +227,12 @@ AFX_D bool block_seen(const RigidArgs& a, const float* __restrict__ depth, float
     const int lane = threadIdx.x & 31;
     const BoxView b = box_view<kZ>(a, t0, t1, t2, x0, y0, z0);
     if (b.state != 2) return b.state != 0;
+    const int n = b.w * b.h;
+    if (kZ == kMidZ && n > 4 * kBlkThreads) {  // one pixel a thread first: a block that is seen mostly is by one of these
+        const int i = (int)((unsigned)threadIdx.x * (unsigned)n / kBlkThreads), row = i / b.w;
+        const float d = __ldg(depth + (long)(b.py0 + row) * a.W + b.px0 + (i - row * b.w));
+        if (__syncthreads_or(!box_empty(b, depth_key(d)))) return true;
+    }
     const unsigned m = box_depth(b, depth, a.W, threadIdx.x, kBlkThreads);
     if (lane == 0) wmax[threadIdx.x >> 5] = m;
     __syncthreads();
