@@ -1950,8 +1950,9 @@ AFX_D void pcg_wide(const LoopArgs& L, int n, float* room, ClusterSums& cs, bool
             d.ap[row] = acc;
             pap[0] = tf_add_prod(pap[0], d.pf[start * 6 + row], acc);
         }
-        // further rows: one lane each where they fill the CTA about three times more, else four
-        if (cnt >= 4 * kLoopThreads - 32) wide_spmv<1>(b, d, start, own, kLoopThreads, pap[0]);
+        // further rows: four lanes each while two passes take them all, else one (ten iterations, four lanes and one: 1,500
+        // nodes, 52 rows, 96 and 105 us; 2,000, 238 rows, 110 both; 2,100, 280 rows, 125 and 115; 5,300 248 and 221)
+        if (cnt - kLoopThreads > 2 * kLoopThreads / 4) wide_spmv<1>(b, d, start, own, kLoopThreads, pap[0]);
         else wide_spmv<4>(b, d, start, own, kLoopThreads, pap[0]);
         cluster_sum_tf<1>(pap, tp, cs);
         if (df_zero_or_nan(tp[0])) break;
