@@ -480,7 +480,7 @@ def rigid_integration_arm(stream, barrier, hbm, frame_mm):
     updated = int((weights > 0).sum())
     gbs = 16.0 * S / (ms / 1000.0) / 1e9
     del tsdf, weights
-    return {"kernel": "integrate_rigid_x4_kernel", "volume": "256^3 FP32 @ 4 mm", "ms": ms, "algorithmic_bytes": 16 * S,
+    return {"kernel": "integrate_rigid_kernel", "volume": "256^3 FP32 @ 4 mm", "ms": ms, "algorithmic_bytes": 16 * S,
             "achieved_gbs": gbs, "peak_gbs": hbm, "frac": gbs / hbm, "voxels_updated": updated,
             "note": "16 B per voxel is the reference kernel's traffic; this kernel loads and stores only the 4-voxel "
                     "groups the frame updates (%.1f%% of voxels updated)" % (100.0 * updated / S)}
@@ -1201,11 +1201,11 @@ def main():
     pcg_mean = max(1e-9, 10.0 * gn_step / clip)
     roof["dominant_kernel"] = {
         "kernel": "gn_loop_kernel", "ms_per_frame": per_frame.get("gn_loop", 0.0),
-        "bound": "latency: cluster barriers and the dot products' reduction chains (1.6 MB of DRAM traffic per launch)",
+        "bound": "latency: the exchanges between CTAs and the dot products' reduction chains (1.6 MB of DRAM traffic per launch)",
         "gn_iterations_last_frame": int(st["gn_iterations_done"]), "gn_iterations_per_step": gn_step,
         "pcg_iterations_per_frame_mean": pcg_mean,
         "us_per_pcg_iteration_upper_bound": 1000.0 * per_frame.get("gn_loop", 0.0) / pcg_mean,
-        "cluster_barriers_per_pcg_iteration": 2}
+        "exchanges_per_pcg_iteration": 2}
     # every stage with an exact byte count, against the same peak
     roof["stages"] = {k: {"ms_per_frame": per_frame.get(k, 0.0), "algorithmic_bytes": v,
                           "achieved_gbs": v / (per_frame[k] / 1000.0) / 1e9 if per_frame.get(k) else None}

@@ -501,12 +501,13 @@ int afx_fusion_graph_count(const afx_fusion* f);
  * frame whose number would pass this limit (2^20 by default, below 2^24).  No counterpart in the reference. */
 int afx_fusion_set_epoch_limit(afx_fusion* f, long frames);
 
-/* Marching-cubes tile of the session (no counterpart in the reference): AFX_MC_TILE_TMA16 (default:
- * a CTA's brick of 32x8x16 cubes brought into shared memory by TMA), AFX_MC_TILE_TMA8,
+/* Marching-cubes tile of the session (no counterpart in the reference): AFX_MC_TILE_TMA16
+ * (a CTA's brick of 32x8x16 cubes brought into shared memory by TMA), AFX_MC_TILE_TMA8,
  * AFX_MC_TILE_TMA32 (8 or 32 cubes along z), AFX_MC_TILE_COLUMN (sweep from global memory),
  * AFX_MC_TILE_PIPE8 / AFX_MC_TILE_PIPE16 / AFX_MC_TILE_PIPE4 (a persistent grid whose CTAs keep two
  * bricks of 8, 16 or 4 cubes in flight).  Results are the same with every tile (point and triangle sets; triangle order
- * may differ).  afx_fusion_autotune times each tile on the session's current volume (call it after
+ * may differ).  A session starts with AFX_MC_TILE_TMA16, from 2 10^7 voxels on with AFX_MC_TILE_PIPE4.
+ * afx_fusion_autotune times each tile on the session's current volume (call it after
  * a few frames), keeps the fastest and returns it in *tile (and the best time of each tile in
  * ms[AFX_MC_TILES] if given); it re-extracts the current frame's mesh and blocks on `stream`.
  * Changing the tile drops the captured frame graphs, which are captured again on next use. */

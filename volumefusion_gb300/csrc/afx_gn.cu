@@ -4,15 +4,15 @@
 // The reference fills a dense Jacobian ((C + 3 K_reg N) x N Vec6f), lists contributing
 // node pairs with atomics, sorts and reduces them with thrust, scatters into a dense
 // (6N)^2 matrix and solves it with cuSOLVER LU in FP32 (src/VolumeFusion.cu:454-691,
-// src/MotionOptimization.cu).  Here J is never stored: each node's warp walks the
-// vertices that reference it (ascending vertex order, which is ascending correspondence
-// order) and accumulates its 6x6 blocks J_a^T J_b in binary32 in a fixed order --
-// depth rows by ascending correspondence, then regularisation rows by ascending row.
+// src/MotionOptimization.cu).  Here J is never stored: a node's thread block stages the rows of
+// the vertices that reference it (ascending vertex order, which is ascending correspondence
+// order), and its 6x6 blocks J_a^T J_b, dealt over the warps, are summed in binary32 in a fixed
+// order -- depth rows by ascending correspondence, then regularisation rows by ascending row.
 // Diagonal blocks without any contribution keep the identity (runInitIdentityKernel).
 // J^T J depends only on the canonical geometry, weights and correspondences, so it is
 // assembled once per ICP iteration; J^T r is rebuilt every Gauss-Newton iteration.
 // The solve is a block-Jacobi PCG in one kernel on one cluster: FP32 block SpMV, dot products in
-// triple-binary32, FP64 6x6 block inverses.
+// triple-binary32, FP64 6x6 block inverses.  Its exchanges between CTAs are bounded waits.
 #include <algorithm>
 #include <cfloat>
 #include <cstring>
@@ -1341,7 +1341,8 @@ AFX_D void ds_dot_total(const DsLayout& d, int i, DF (&t)[NV]) {
 // Bound: the chain of those steps, CTA barriers and two exchanges, about 6,000 cycles an iteration with 169 nodes
 // on 16 CTAs (A p 750, the two sums with their sending 2,700, updates 700, waits 550).  gn_loop_kernel in
 // the 256^3 sequence (169 nodes): 305 us with cluster barriers, double-float sums and the matrix rows read from
-// shared memory in each iteration, 267 us so.
+// shared memory in each iteration, 267 us so (with staged transforms, NodeT below, 232, and 203 with the lists and
+// matrix rows of the commits after).
 constexpr int kRegBlocks = 6;
 
 template <bool kTol>

@@ -1606,18 +1606,18 @@ int afx_correspondences(int* corr, unsigned* corr_count, long capacity, const fl
 }  // extern "C"
 
 // ------------------------------------------------------------------------------------
-// Correspondence search without any allocation: the same three steps as
-// afx_correspondences (flag kernel, exclusive scan, scatter kernel), with the scratch in a
+// Correspondence search without any allocation: the same two launches as
+// afx_correspondences (pixels with the tiles' counts, scatter), with the scratch in a
 // fixed file-scope device array instead of a caller-provided workspace.  Every scratch word
-// is written before it is read within one call (flags and pixels for every live vertex,
-// scan block sums, scan output), so nothing has to start at zero and nothing is cleared.
+// is written before it is read within one call (a pixel for every live vertex, a count for
+// every tile of them), so nothing has to start at zero and nothing is cleared.
 // The array is shared by all calls on a device: calls that overlap in time race on it.
 // ------------------------------------------------------------------------------------
 
 namespace afx {
 
 constexpr long kCorrStaticMaxPoints = AFX_CORR_STATIC_MAX_POINTS;
-// flags, pixels, scan output (4 bytes each per vertex) + scan block sums + alignment slack
+// the pixel of each vertex, and the tiles' counts with alignment slack
 constexpr size_t kCorrStaticBytes = (size_t)kCorrStaticMaxPoints * 4 + 64 * 1024;
 
 static __device__ __align__(256) unsigned char g_corr_static_scratch[kCorrStaticBytes];

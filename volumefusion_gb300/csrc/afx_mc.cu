@@ -264,7 +264,7 @@ AFX_D bool tile_occupied(const McArgs& a, int x0, int y0, int z0, int zr) {
 // are read only where the warp's rows hold a weight.  Surface cubes wait in a queue of the warp's own
 // until 32 of them are interpolated together.
 // Bound: the latency of a slice and, where there is surface, the shared-memory traffic of the emission.
-// 257 x 230 x 301 voxels (142 MB) with 0.22 m^2 of surface at 2.5 mm: 65 us, 1.6 TB/s of DRAM reads (a
+// 257 x 230 x 301 voxels (142 MB) with 0.22 m^2 of surface at 2.5 mm: 60 us, 2.4 TB/s of the volume's bytes (a
 // thread per column reading eight corners a cube, and interpolating where it stood, took 400 us; runs of
 // 16 slices 111 us, a warp with much surface holding up the rest).
 constexpr int kSweepY = 4, kSweepZ = 8, kSweepWarps = 8;

@@ -200,8 +200,8 @@ class FusionSession:
         check(lib().afx_fusion_save_mesh_ply(self.h, str(path).encode(), self._st()), "afx_fusion_save_mesh_ply")
 
     def set_tile(self, tile):
-        """Marching-cubes tile: 0 TMA 16 cubes along z (default), 1 TMA 8, 2 TMA 32, 3 sweep from global memory,
-        4 / 5 persistent two-stage TMA 8 / 16."""
+        """Marching-cubes tile: 0 TMA 16 cubes along z (default below 2e7 voxels), 1 TMA 8, 2 TMA 32, 3 sweep from global
+        memory, 4 / 5 / 6 persistent two-stage TMA 8 / 16 / 4 (6: default from 2e7 voxels on)."""
         check(lib().afx_fusion_set_tile(self.h, int(tile)), "afx_fusion_set_tile")
 
     def tile(self):
