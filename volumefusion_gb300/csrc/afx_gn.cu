@@ -1341,8 +1341,7 @@ AFX_D void ds_dot_total(const DsLayout& d, int i, DF (&t)[NV]) {
 // Bound: the chain of those steps, CTA barriers and two exchanges, about 6,000 cycles an iteration with 169 nodes
 // on 16 CTAs (A p 750, the two sums with their sending 2,700, updates 700, waits 550).  gn_loop_kernel in
 // the 256^3 sequence (169 nodes): 305 us with cluster barriers, double-float sums and the matrix rows read from
-// shared memory in each iteration, 267 us so (with staged transforms, NodeT below, 232, and 203 with the lists and
-// matrix rows of the commits after).
+// shared memory in each iteration, 267 us so (232 with the transforms staged, NodeT below; the whole launch takes 203 us).
 constexpr int kRegBlocks = 6;
 
 template <bool kTol>
